@@ -7,6 +7,7 @@ entry point of the package fails with that error.  Build it with
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 from pathlib import Path
 
@@ -73,6 +74,8 @@ SIGNATURES = {
     "fos_linear_workspace_bytes": (_c_i64, [_c_i64, _c_i64]),
     "fos_linear_forward": (_c_int, [_c_ptr, _c_int, _c_i64, _c_i64, _c_i64, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_i64,
                                     _c_ptr, _c_int, _c_i64, _c_ptr, _c_i64, _c_ptr, _c_ptr, _c_ptr]),
+    "fos_linear_forward_bias": (_c_int, [_c_ptr, _c_int, _c_i64, _c_i64, _c_i64, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_i64,
+                                        _c_ptr, _c_ptr, _c_int, _c_i64, _c_ptr, _c_i64, _c_ptr, _c_ptr, _c_ptr]),
     "fos_experts_workspace_bytes": (_c_i64, [_c_i64, _c_int, _c_int, _c_i64, _c_i64]),
     "fos_experts_forward": (_c_int, [_c_ptr, _c_int, _c_i64, _c_i64, _c_i64, _c_ptr, _c_int, _c_ptr, _c_int, _c_int,
                                      _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_i64, _c_int, _c_int,
@@ -96,6 +99,10 @@ SIGNATURES = {
     "fos_reduce_scatter_peer": (_c_int, [_c_ptr, _c_int, _c_i64, _c_i64, _c_i64, _c_i64, _c_ptr, _c_i64, _c_int, _c_int, _c_ptr]),
     "fos_allgather_peer": (_c_int, [_c_ptr, _c_int, _c_i64, _c_i64, _c_ptr, _c_int, _c_ptr]),
     "fos_reduce_gather": (_c_int, [_c_ptr, _c_ptr, _c_int, _c_int, _c_i64, _c_i64, _c_i64, _c_i64, _c_int, _c_ptr]),
+    "fos_gemm_nvfp4_scaled": (_c_int, [_c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_ptr,
+                                       _c_int, _c_i64, _c_i64, _c_i64, _c_i64, _c_i64, _c_i64, _c_ptr, _c_ptr, _c_ptr]),
+    "fos_gemm_mxfp4_unscaled": (_c_int, [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_i64, _c_i64, _c_i64, _c_i64,
+                                         _c_i64, _c_i64, _c_ptr, _c_ptr, _c_ptr]),
     "fos_gemm_if4_workspace_bytes": (_c_i64, [_c_i64, _c_i64, _c_i64]),
     "fos_gemm_if4": (_c_int, [_c_ptr, _c_ptr, _c_int, _c_int, _c_ptr, _c_ptr, _c_int, _c_int, _c_ptr, _c_ptr, _c_int,
                               _c_i64, _c_i64, _c_i64, _c_i64, _c_i64, _c_i64, _c_ptr, _c_i64, _c_ptr, _c_ptr]),
@@ -169,11 +176,23 @@ def raise_on_wait_failure() -> None:
 
 
 def stream_ptr(device: torch.device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    index = device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+
+
+def on_device(device: torch.device):
+    """`torch.cuda.device(device)` where that changes anything (entering it costs microseconds a small call feels)."""
+    if device.index is None or device.index == torch.cuda.current_device():
+        return _SAME_DEVICE
+    return torch.cuda.device(device)
+
+
+_ELEM_CODES = {torch.bfloat16: FOS_BF16, torch.float16: FOS_FP16, torch.float32: FOS_FP32}
+_SAME_DEVICE = contextlib.nullcontext()
 
 
 def elem_code(dtype: torch.dtype) -> int:
     try:
-        return {torch.bfloat16: FOS_BF16, torch.float16: FOS_FP16, torch.float32: FOS_FP32}[dtype]
+        return _ELEM_CODES[dtype]
     except KeyError:
         raise ValueError(f"unsupported element type {dtype}") from None

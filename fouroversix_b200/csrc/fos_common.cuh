@@ -32,11 +32,56 @@ int quantize_mxfp4(const void *x, int x_dtype, int64_t rows, int64_t cols, int64
 int dequantize_mxfp4(const uint8_t *codes, const uint8_t *sf, int sf_layout, int64_t rows_p, int64_t cols_p, int64_t rows,
                      int64_t cols, void *out, int out_dtype, int64_t ld_out, cudaStream_t stream);
 
+// fos_quantize_grouped for callers that read no product of a padding row: what comes out there is not defined.
+int quantize_grouped_rows_in_use(const void *x, int x_dtype, int64_t rows_capacity, int64_t cols, int64_t ld, int format,
+                                 int scale_rule, const int32_t *group_start, const int32_t *group_rows, int num_groups,
+                                 const float *amax_in, uint8_t *codes, uint8_t *sf, float *amax_out, int flags, void *stream);
+
+// How a GEMM's output is scaled without an alpha word: alpha = amax_a * amax_b / denom is formed in the GEMM (the same
+// operations as fos_gemm_alpha; amax_a == nullptr: 1), bias [n] of the output's type (or nullptr) is added to the
+// rounded product. `chained`: the kernel before the GEMM in the stream is this library's, packs A, and lets its
+// dependents start only after its own wait for its predecessors: B may then be fetched before that kernel ends.
+struct GemmScales {
+    const float *amax_a, *amax_b;      // grouped: one per group
+    float denom;
+    const void *bias;
+    bool chained;
+};
+
+int gemm_nvfp4_chained(const uint8_t *a_codes, const uint8_t *a_sf, const uint8_t *b_codes, const uint8_t *b_sf,
+                       const GemmScales &scales, void *d, int out_dtype, int64_t m_p, int64_t n_p, int64_t k_p, int64_t m,
+                       int64_t n, int64_t ldd, const fos_gemm_opts *opts, int32_t *status, void *stream);
+// fos_gemm_nvfp4_grouped with alpha formed in the GEMM;
+int gemm_nvfp4_grouped_scaled(const uint8_t *a_codes, const uint8_t *a_sf, const uint8_t *b_codes, const uint8_t *b_sf,
+                              const GemmScales &scales, void *d, int out_dtype, const int32_t *group_start,
+                              const int32_t *group_rows, int num_groups, int64_t rows_capacity, int64_t n_p, int64_t k_p,
+                              int64_t n, int64_t ldd, int32_t *status, void *stream);
+
 #define FOS_CUDA_TRY(expr)                                         \
     do {                                                           \
         cudaError_t fos_e_ = (expr);                               \
         if (fos_e_ != cudaSuccess) return fos::note_cuda_error(fos_e_); \
     } while (0)
+
+#ifdef __CUDACC__
+// Launch as the programmatic dependent of whatever kernel is before it in the stream: the CTAs may be placed while that
+// one drains. For kernels that execute griddepcontrol.wait before they touch global memory; the earlier kernel is
+// complete then, and so is everything before it if it waited the same way.
+template <typename... Params, typename... Args>
+cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, unsigned threads, int smem_bytes, cudaStream_t stream, Args &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = static_cast<size_t>(smem_bytes);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+#endif
 
 static inline int64_t round_up64(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 
@@ -46,6 +91,15 @@ __host__ __device__ inline float dequant_divisor(int format, int rule) {
     if (rule == FOS_RULE_STATIC_6) return 2688.0f;
     if (rule == FOS_RULE_STATIC_4) return 1792.0f;
     return 1536.0f;
+}
+
+// What alpha divides amax_a * amax_b by: the reference multiplies the constants as Python numbers (exactly, for the
+// integers; 16/17 for each operand rounded by stochastic_unbiased) before the one division.
+inline float alpha_divisor(int format_a, int rule_a, int format_b, int rule_b, int unbiased_a = 0, int unbiased_b = 0) {
+    double product = static_cast<double>(dequant_divisor(format_a, rule_a)) * static_cast<double>(dequant_divisor(format_b, rule_b));
+    if (unbiased_a) product *= 16.0 / 17.0;
+    if (unbiased_b) product *= 16.0 / 17.0;
+    return static_cast<float>(product);
 }
 
 #ifdef __CUDACC__

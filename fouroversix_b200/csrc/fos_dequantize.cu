@@ -290,11 +290,7 @@ extern "C" int fos_gemm_alpha_grouped(const float *amax_a, int format_a, int rul
     if (!amax_a || !amax_b || !alpha || count <= 0) return FOS_ERR_INVALID_ARGUMENT;
     int st = check_device();
     if (st != FOS_OK) return st;
-    // the reference multiplies the constants as Python numbers (exactly, for the integers) before the one division
-    double product = static_cast<double>(dequant_divisor(format_a, rule_a)) * static_cast<double>(dequant_divisor(format_b, rule_b));
-    if (unbiased_a) product *= 16.0 / 17.0;
-    if (unbiased_b) product *= 16.0 / 17.0;
-    const float denom = static_cast<float>(product);
+    const float denom = alpha_divisor(format_a, rule_a, format_b, rule_b, unbiased_a, unbiased_b);
     const int threads = count < 256 ? ((count + 31) / 32) * 32 : 256;
     alpha_kernel<<<(count + threads - 1) / threads, threads, 0, static_cast<cudaStream_t>(stream_)>>>(amax_a, amax_b, denom, alpha, count);
     FOS_CUDA_TRY(cudaGetLastError());

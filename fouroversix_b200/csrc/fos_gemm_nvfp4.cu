@@ -31,7 +31,7 @@
 //               line with the MMAs (372 us at 8192^3); from warps of their own they overlap
 //               them, and two warps issue them faster than one (235 -> 219 us).
 //
-// What bounds the kernel now (8192^3, parts switched off in a -DFOS_GEMM_DEBUG build): MMAs alone
+// What bounds the kernel (8192^3, parts switched off in a -DFOS_GEMM_DEBUG build): MMAs alone
 // 150 us, loads alone 148, loads + MMAs 176, everything 219. The scale copies are the largest
 // single cost: twelve per stage, each about 30 ns of the copying warp and about 14 cycles of the
 // tensor pipe that no MMA gets. Loads and MMAs together lose 26 us to the round trip of a stage
@@ -40,15 +40,12 @@
 // Every mbarrier wait is bounded (in SM cycles). A wait that gives up records where
 // in *status, raises a CTA-wide abort flag, and all roles fall through to the common exit,
 // which lets in-flight copies land, releases tensor memory and returns.
-#include "fos_tcgen05.cuh"
+#include "fos_gemm_skinny.cuh"
+#include "fos_pair.cuh"
 
 namespace fos {
 namespace {
 
-constexpr int BLOCK_M = 128;
-constexpr int BLOCK_K_BYTES = 128;                 // 256 E2M1 values: one 128-byte swizzle row
-constexpr int KB_PER_STAGE = 4;                    // MMA K-blocks (64 values, 32 bytes) per stage
-constexpr int SF_TILE_BYTES = 512;                 // scales of 128 rows x 64 values
 constexpr int A_BYTES = BLOCK_M * BLOCK_K_BYTES;   // 16 KiB
 constexpr int SFA_BYTES = KB_PER_STAGE * SF_TILE_BYTES;
 #ifndef FOS_GEMM_SF_LEAD
@@ -61,6 +58,7 @@ constexpr int SF_LEAD = FOS_GEMM_SF_LEAD;   // 0 or 1: how many stages the scale
 
 constexpr int SF_CP_WARPS = 2;                     // warps 10 and 11 issue the scale copies, taking stages in turn
 constexpr int NUM_THREADS = 384;                   // warps: 0 TMA, 1 MMA, 2-9 epilogue (FUSED_A: also the A operand), 10-11 scale copies
+constexpr int PAIR_MIN_GROUP_ROWS = 640;           // grouped launches: CTA pairs from this many rows of the buffer per group
 constexpr int MAX_GROUPS = 256;                    // of a grouped launch (their row ranges are kept in shared memory)
 constexpr int SF_COL0 = 256;                       // tensor-memory columns: accumulators first, then per
                                                    // stage 16 columns of A scales and N/8 of B scales
@@ -90,7 +88,11 @@ template <int BLOCK_N> struct Cfg {
 struct GemmParams {
     const uint8_t *a_sf;
     const uint8_t *b_sf;
-    const float *alpha;
+    const float *alpha;      // the product's factor, or nullptr:
+    const float *amax_a;     // then it is amax_a * amax_b / alpha_denom (what fos_gemm_alpha computes), 1 without amax_a
+    const float *amax_b;
+    float alpha_denom;
+    const void *bias;        // [n] of the output's type, added to the rounded product, or nullptr
     void *d;
     int32_t *status;         // where a bounded wait that gives up records its site: the caller's word, or the sticky one
     int64_t m_p, n_p, k_p;   // padded problem (k_p in values)
@@ -124,76 +126,39 @@ struct GemmParams {
     int num_groups;
 };
 
-// ---------------------------------------------------------------------------- MMA wrappers
-
-// MXFP4: two E8M0 scales per row and K-block (scale_vec::2X); which two of the four bytes of a
-// scale column an instruction uses is part of its descriptor.
-__device__ __forceinline__ void tc_mma_mxf4(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                            uint32_t sfa_tmem, uint32_t sfb_tmem, uint32_t accumulate) {
-    asm volatile(
-        "{ .reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%5], [%6], p; }\n"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(sfa_tmem), "r"(sfb_tmem)
-        : "memory");
+__device__ __forceinline__ float gemm_alpha(const GemmParams &p, int group = 0) {
+    if (p.alpha) return __ldg(p.alpha + group);
+    if (!p.amax_a) return 1.0f;
+    return __fdiv_rn(__fmul_rn(*static_cast<const volatile float *>(p.amax_a + group), __ldg(p.amax_b + group)), p.alpha_denom);
 }
 
-// Descriptors in two halves. The upper word of a shared-memory matrix descriptor is the same for every
-// tile of a kind (stride byte offset, version, swizzle) and the lower word is the start address >> 4
-// (shared-memory addresses stay below 2^18, so adding a byte offset >> 4 never carries out of the field):
-// the issuing threads keep one lower word per stage and add constants, instead of rebuilding 64-bit
-// descriptors for every instruction - a single thread issues every copy and every MMA of an SM, and
-// what it executes between two of them is what bounds its rate.
-constexpr uint32_t DESC_HI_OPERAND = (1024u >> 4) | (1u << 14) | (2u << 29);   // SBO 1024, version 1, 128-byte swizzle
-constexpr uint32_t DESC_HI_SCALES = (128u >> 4) | (1u << 14);                   // SBO 128, version 1, no swizzle
-__device__ __forceinline__ uint32_t desc_lo(uint32_t addr, uint32_t lbo_bytes = 0) {
-    return ((addr & 0x3ffffu) >> 4) | ((lbo_bytes >> 4) << 16);
-}
-__device__ __forceinline__ void tc_copy_sf_lo(uint32_t taddr, uint32_t lo) {
-    asm volatile("{ .reg .b64 d;\n"
-                 "mov.b64 d, {%1, %2};\n"
-                 "tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], d; }" ::"r"(taddr), "r"(lo), "r"(DESC_HI_SCALES) : "memory");
-}
-__device__ __forceinline__ void tc_copy_sf_pair_lo(uint32_t taddr, uint32_t lo) {
-    asm volatile("{ .reg .b64 d;\n"
-                 "mov.b64 d, {%1, %2};\n"
-                 "tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], d; }" ::"r"(taddr), "r"(lo), "r"(DESC_HI_SCALES) : "memory");
-}
-__device__ __forceinline__ void tc_mma_nvf4_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
-                                               uint32_t sfa_tmem, uint32_t sfb_tmem, uint32_t accumulate) {
-    asm volatile(
-        "{ .reg .pred p;\n"
-        ".reg .b64 da, db;\n"
-        "mov.b64 da, {%1, %7};\n"
-        "mov.b64 db, {%2, %7};\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], da, db, %3, [%5], [%6], p; }\n"
-        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(sfa_tmem), "r"(sfb_tmem), "r"(DESC_HI_OPERAND)
-        : "memory");
-}
-__device__ __forceinline__ void tc_mma_nvf4_pair_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
-                                                    uint32_t sfa_tmem, uint32_t sfb_tmem, uint32_t accumulate) {
-    asm volatile(
-        "{ .reg .pred p;\n"
-        ".reg .b64 da, db;\n"
-        "mov.b64 da, {%1, %7};\n"
-        "mov.b64 db, {%2, %7};\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], da, db, %3, [%5], [%6], p; }\n"
-        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(sfa_tmem), "r"(sfb_tmem), "r"(DESC_HI_OPERAND)
-        : "memory");
-}
+// GROUPED: first row of every group (and one past the last group), and one past each group's last valid row.
+template <bool GROUPED> struct GroupTable {
+    int32_t start[GROUPED ? MAX_GROUPS + 1 : 1], end[GROUPED ? MAX_GROUPS : 1];
+};
 
-// Instruction descriptor of kind::mxf4nvf4 block-scaled MMA: A and B E2M1 (code 1 in bits
-// [7,10) and [10,13)), both K-major, N >> 3 in [17,23), UE4M3 scales (bit 23 = 0), M >> 4 in
-// [24,29), scale-factor byte ids 0, dense K = 64. MXFP4: E8M0 scales (bit 23 = 1) and the byte
-// offset (0 or 2) of the instruction's two scales inside the 32-bit scale column in [4,6) for B
-// and [29,31) for A.
-__device__ __forceinline__ uint32_t mma_idesc(int n, int m = BLOCK_M) {
-    return (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
-}
-__device__ __forceinline__ uint32_t mma_idesc_mx(uint32_t idesc, uint32_t sf_byte) {
-    return idesc | (1u << 23) | (sf_byte << 4) | (sf_byte << 29);
+template <int THREADS> __device__ __forceinline__ void load_groups(const GemmParams &p, GroupTable<true> &groups) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");     // the row ranges come from an earlier kernel
+    const int32_t cap = static_cast<int32_t>(p.m_p);
+    // (the same number of rounds in every thread, and the warps converged again before the warp-wide
+    // instructions that follow - tcgen05.alloc, elect.sync: a loop that only some lanes of a warp enter leaves
+    // the warp split, and those instructions are undefined for a split warp)
+    for (int g0 = 0; g0 <= p.num_groups; g0 += THREADS) {
+        const int g = g0 + static_cast<int>(threadIdx.x);
+        if (g <= p.num_groups) {
+            int32_t s0 = __ldg(p.group_start + g);
+            s0 = (s0 < 0 ? 0 : (s0 > cap ? cap : s0)) & ~127;             // never beyond the buffers
+            groups.start[g] = s0;
+            if (g < p.num_groups) {
+                // valid rows end inside the group's own range, whatever group_rows claims
+                int32_t s1 = __ldg(p.group_start + g + 1);
+                s1 = (s1 < s0 ? s0 : (s1 > cap ? cap : s1)) & ~127;
+                const int32_t r = __ldg(p.group_rows + g), e = s0 + (r < 0 ? 0 : r);
+                groups.end[g] = e > s1 ? s1 : e;
+            }
+        }
+    }
+    __syncwarp();
 }
 
 // ---------------------------------------------------------------------------- kernel
@@ -223,30 +188,8 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    // GROUPED: first row of every group (and one past the last group), and one past each group's last valid row
-    __shared__ int32_t grp_start[GROUPED ? MAX_GROUPS + 1 : 1], grp_end[GROUPED ? MAX_GROUPS : 1];
-    if constexpr (GROUPED) {
-        const int32_t cap = static_cast<int32_t>(p.m_p);
-        // (the same number of rounds in every thread, and the warps converged again before the warp-wide
-        // instructions below - tcgen05.alloc, elect.sync: a loop that only some lanes of a warp enter leaves
-        // the warp split, and those instructions are undefined for a split warp)
-        for (int g0 = 0; g0 <= p.num_groups; g0 += NUM_THREADS) {
-            const int g = g0 + static_cast<int>(threadIdx.x);
-            if (g <= p.num_groups) {
-                int32_t s0 = __ldg(p.group_start + g);
-                s0 = (s0 < 0 ? 0 : (s0 > cap ? cap : s0)) & ~127;             // never beyond the buffers
-                grp_start[g] = s0;
-                if (g < p.num_groups) {
-                    // valid rows end inside the group's own range, whatever group_rows claims
-                    int32_t s1 = __ldg(p.group_start + g + 1);
-                    s1 = (s1 < s0 ? s0 : (s1 > cap ? cap : s1)) & ~127;
-                    const int32_t r = __ldg(p.group_rows + g), e = s0 + (r < 0 ? 0 : r);
-                    grp_end[g] = e > s1 ? s1 : e;
-                }
-            }
-        }
-        __syncwarp();
-    }
+    __shared__ GroupTable<GROUPED> groups;
+    if constexpr (GROUPED) load_groups<NUM_THREADS>(p, groups);
 
     if (threadIdx.x == 0) {
         // FUSED_A: besides the copy engine (B, B's scales), the eight warps that make A and its scales arrive
@@ -278,16 +221,16 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    const int64_t num_m = GROUPED ? grp_start[p.num_groups] / BLOCK_M : p.m_p / BLOCK_M;
+    const int64_t num_m = GROUPED ? groups.start[p.num_groups] / BLOCK_M : p.m_p / BLOCK_M;
     const int64_t num_n = (p.n_p + BLOCK_N - 1) / BLOCK_N;
-    // GROUPED: the group that row block mb lies in (the last g with grp_start[g] <= row; empty groups are skipped)
+    // GROUPED: the group that row block mb lies in (the last g with start[g] <= row; empty groups are skipped)
     auto group_of = [&](int64_t mb) -> int {
         if constexpr (!GROUPED) return 0;
         const int32_t row = static_cast<int32_t>(mb * BLOCK_M);
         int lo = 0, hi = p.num_groups - 1;
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
-            if (grp_start[mid] <= row) lo = mid; else hi = mid - 1;
+            if (groups.start[mid] <= row) lo = mid; else hi = mid - 1;
         }
         return lo;
     };
@@ -342,6 +285,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
         };
         enter_tile();
+        asm volatile("griddepcontrol.wait;" ::: "memory");   // (a dependent launch) the kernel that packs A is done
         for (int i = 0; i < SF_LEAD; ++i) issue_next_scales();
         uint32_t s = 0, ph = 0;
         bool ok = true;
@@ -379,8 +323,11 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         // instructions take directly; a lone thread's values live in ordinary registers and every instruction
         // pays for moving its operands over: 256 -> 235 us at 8192^3, the CTA-pair kernel 343 -> 249 us.)
         const bool issue = elect_one();
+        // (A wait on a barrier that has completed long ago still takes some 190 cycles: the MMAs' operand reads keep shared
+        // memory busy. So the next stage's barriers are probed before this stage's instructions are issued, and the
+        // answer is looked at after them.)
         uint32_t s = 0, ph = 0, j = 0, jph = 0, tile_i = 0;      // operand stage / scale slot and their phases
-        bool ok = true;
+        bool ok = true, ready = false;
         for (int64_t t = blockIdx.x; t < num_tiles && ok; t += gridDim.x, ++tile_i) {
             int64_t mb, nb;
             tile_coords(t, num_m, num_n, mb, nb);
@@ -394,28 +341,30 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + acc * BLOCK_N;
             for (int64_t kt = 0; kt < k_tiles; ++kt) {
-                if (!dbg_no_load) {
+                if (!dbg_no_load && !ready) {
                     ok = mbar_wait(full_bar + 8 * s, ph, abort_flag, p.status, 2);
                     if (ok && !dbg_no_sf) ok = mbar_wait(sf_ready_bar + 8 * j, jph, abort_flag, p.status, 5);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
                 }
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
                 tc_fence_after();
+                const uint32_t s_next = s + 1 == C::STAGES ? 0 : s + 1, ph_next = s + 1 == C::STAGES ? ph ^ 1u : ph;
+                const uint32_t j_next = j + 1 == C::SF_SLOTS ? 0 : j + 1, jph_next = j + 1 == C::SF_SLOTS ? jph ^ 1u : jph;
+                const bool full_next = mbar_test_wait(full_bar + 8 * s_next, ph_next);
+                const bool sf_next = mbar_test_wait(sf_ready_bar + 8 * j_next, jph_next);
                 const int64_t kb0 = kt * KB_PER_STAGE;
                 const int nkb = static_cast<int>((k_blocks - kb0) < KB_PER_STAGE ? (k_blocks - kb0) : KB_PER_STAGE);
                 const uint32_t stage = smem_base + s * C::STAGE_BYTES;
                 // operands: 128-byte swizzled rows, 8-row groups 1024 bytes apart; each K-block
                 // of 64 values is 32 bytes further along the row. Scales: this iteration's ring slot.
-                const uint64_t a_desc = smem_desc(stage, 16, 1024, 2);
-                const uint64_t b_desc = smem_desc(stage + A_BYTES, 16, 1024, 2);
+                const uint32_t a_lo = desc_lo(stage, 16), b_lo = desc_lo(stage + A_BYTES, 16);
                 const uint32_t sfa_tmem = tmem_base + SF_COL0 + j * C::SF_STAGE_COLS, sfb_tmem = sfa_tmem + 16;
                 if (p.mx) {
                     for (int kb = 0; kb < nkb && !dbg_no_mma && issue; ++kb)
-                        tc_mma_mxf4(d_tmem, a_desc + 2 * kb, b_desc + 2 * kb, mma_idesc_mx(idesc, (kb & 1) * 2),
-                                    sfa_tmem + 4 * (kb >> 1), sfb_tmem + (BLOCK_N / 32) * (kb >> 1),
-                                    (kt > 0 || kb > 0) ? 1u : 0u);
+                        tc_mma_mxf4_lo(d_tmem, a_lo + 2 * kb, b_lo + 2 * kb, mma_idesc_mx(idesc, (kb & 1) * 2),
+                                       sfa_tmem + 4 * (kb >> 1), sfb_tmem + (BLOCK_N / 32) * (kb >> 1),
+                                       (kt > 0 || kb > 0) ? 1u : 0u);
                 } else {
-                    const uint32_t a_lo = desc_lo(stage, 16), b_lo = desc_lo(stage + A_BYTES, 16);
 #pragma unroll
                     for (int kb = 0; kb < KB_PER_STAGE; ++kb) {
                         if (kb < nkb && !dbg_no_mma && issue)
@@ -425,8 +374,11 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 }
                 if (issue) tc_commit(empty_bar + 8 * s);          // stage (and scale slot) reusable once these MMAs are done
                 __syncwarp();
-                if (++s == C::STAGES) { s = 0; ph ^= 1u; }
-                if (++j == C::SF_SLOTS) { j = 0; jph ^= 1u; }
+                ready = __all_sync(0xffffffffu, full_next && sf_next);
+                s = s_next;
+                ph = ph_next;
+                j = j_next;
+                jph = jph_next;
             }
             if (ok && issue) tc_commit(acc_full_bar + 8 * acc);  // accumulator complete
         }
@@ -442,7 +394,8 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         const int quad = warp & 3;                       // tensor-memory lanes 32*quad .. +31
         constexpr int COLS = BLOCK_N / 2;                // columns per warp: left or right half
         const int half = (warp - 2) >> 2;
-        float alpha = GROUPED ? 0.0f : __ldg(p.alpha);
+        asm volatile("griddepcontrol.wait;" ::: "memory");   // amax_a, and whoever still reads d
+        float alpha = GROUPED ? 0.0f : gemm_alpha(p);
         int64_t row_end = p.m;
         OUT *out = static_cast<OUT *>(p.d);
         const bool vec_ok = (reinterpret_cast<uintptr_t>(out) % 16 == 0) && ((p.ldd * sizeof(OUT)) % 16 == 0);
@@ -528,8 +481,8 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             const int64_t row = mb * BLOCK_M + quad * 32 + lane, n0 = nb * BLOCK_N + half * COLS;
             if constexpr (GROUPED) {
                 const int grp = group_of(mb);
-                alpha = __ldg(p.alpha + grp);
-                row_end = grp_end[grp];
+                alpha = gemm_alpha(p, grp);
+                row_end = groups.end[grp];
             }
             if (p.scatter_world > 1) {
                 // row block mb belongs to rank mb % world (interleaved, so that the peer traffic is spread
@@ -567,6 +520,11 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 const int64_t left = p.n - n0;
                 if (row_ok && left > 0) {
                     OUT *dst = out + row * p.ldd + n0;
+                    if (p.bias) {
+                        const OUT *bias = static_cast<const OUT *>(p.bias) + n0;
+#pragma unroll
+                        for (int i = 0; i < COLS / 2; ++i) pk[i] = add_bias<OUT>(pk[i], bias + 2 * i, left - 2 * i);
+                    }
                     if (left >= COLS && vec32_ok) {
 #ifdef FOS_GEMM_DEBUG
                         if (p.debug & 8) {
@@ -638,7 +596,6 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 ok = mbar_wait(sf_full_bar + 8 * (me * C::SF_SLOTS + j), jph, abort_flag, p.status, 6);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
-                tc_fence_after();
                 const uint32_t src = sf_base + j * C::SF_SLOT_BYTES, dst = tmem_base + SF_COL0 + j * C::SF_STAGE_COLS;
                 // tiles: 32 rows of 16 bytes, 8-row groups 128 bytes apart, no swizzle
                 // (MXFP4: a tile spans two K-blocks, so a stage has two tiles per group)
@@ -672,104 +629,121 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 //
 // Two CTAs of a cluster (two SMs) compute one 256 x 256 tile with cta_group::2 MMAs: CTA r of
 // the pair holds rows m0 + 128 r .. of A and rows n0 + 128 r .. of B in its shared memory,
-// and the tensor cores of both SMs read both halves of B. Per MMA an SM moves a third less
-// through shared memory than the single-CTA kernel, whose limit that is. Only the even CTA (the
-// leader) issues MMAs; both CTAs run the two TMA producers, scale movers and an epilogue for their
-// own 128 rows of the tile, with the same roles per warp as the single-CTA kernel.
+// and the tensor cores of both SMs read both halves of B. Per MMA an SM fetches a third less
+// than the single-CTA kernel, whose limit that is. Only the even CTA (the leader) issues MMAs;
+// both CTAs run a TMA producer and an epilogue for their own 128 rows of the tile.
 //
-//   full[s]      leader's barrier: one arrive.expect_tx by the leader's producer for the bytes of
-//                BOTH CTAs; the peer's TMA loads complete on it too (cta_group::2 form of the copy)
-//   empty[s]     one per CTA, released in both CTAs by the leader's multicast tcgen05.commit
-//   sf_full[w][j] leader's barriers, one per (copying warp, slot) as in the single-CTA kernel: the scale
-//                tiles of both CTAs have landed (each in its own CTA's shared memory), announced and
-//                completed like full[s]
-//   sf_ready[j]  leader's barrier: one of the leader's two copying warps has moved the slot's scales into
-//                the tensor memory of both CTAs (tcgen05.cp with cta_group::2, one commit)
-//   acc_full     one per CTA, multicast commit
-//   acc_empty    leader's barrier, 16 arrivals: 8 epilogue warps of each CTA
+//   warp 0     (both CTAs) TMA: per stage this CTA's tiles of A and B and its scale tiles (128 rows of A, all 256 of
+//              B: each SM's tensor core needs the scales of every column); everything completes on
+//              the LEADER's barriers (the cta_group::2 form of the copy)
+//   warp 1     (leader) scale copies (tcgen05.cp) and MMAs, all from this one thread: the tensor pipe runs them in issue
+//              order, so neither the copies nor the re-use of their tensor-memory columns need a barrier
+//   warps 2..9 (both CTAs) epilogue
 //
-// Barriers that the other SM arrives on are polled (test_wait) by their single waiting thread: a
-// thread suspended in try_wait did not see such arrivals promptly. Remote arrives use the
-// default (CTA-scope release) form: the cluster-scope release form cost about a microsecond each.
+//   full[s]    leader's barrier: one arrive.expect_tx for the bytes of BOTH CTAs
+//   empty[s]   one per CTA, released in both CTAs by the leader's multicast tcgen05.commit
+//   acc_full   one per CTA, multicast commit
+//   acc_empty  leader's barrier, 16 arrivals: 8 epilogue warps of each CTA
+//
+// The MMA warp issues seventeen instructions per stage of 256 K values, whose MMAs take 512 cycles, so what it does besides
+// counts. Cycles per stage at 8192^3 (NVFP4 / MXFP4), measured with its waits for full[s] as: waits that poll with a
+// suspend limit 716 / 669, a tight test_wait loop 730 / 686, plain try_wait 666 / 623. A wait for a barrier that completed long
+// ago still costs some 190 cycles of those (its access to shared memory queues behind the MMAs' operand reads), so the next
+// stage's barrier is probed before a stage's instructions are issued and the answer is looked at after them (205 -> 197 us,
+// 187 -> 180 us; the single-CTA kernel: 218, 224 us). A second barrier per stage, or per group of stages, for the scales (so that they could be copied for several stages together)
+// costs more than it saves. No tcgen05 fence after a wait for TMA copies: it orders tcgen05 operations of different threads, and
+// only the accumulators pass between threads.
+//
+// Tensor memory: tiles alternate between two accumulators that OVERLAP by the columns that the scales take. The
+// epilogue reads the shared columns first and then releases the barrier, so the next tile's MMAs start while the
+// rest of the accumulator is still being read and stored.
 namespace pair {
 
 constexpr int TILE_N = 256;
 constexpr int B_HALF_BYTES = 128 * BLOCK_K_BYTES;                         // this CTA's 128 rows of B
-constexpr int STAGE_BYTES = A_BYTES + B_HALF_BYTES;                       // 32 KiB
-constexpr int SFB_BYTES = 2 * KB_PER_STAGE * SF_TILE_BYTES;               // scales of all 256 B rows
-constexpr int SF_SLOT_BYTES = SFA_BYTES + SFB_BYTES;                      // 6 KiB
-constexpr int STAGES = 6;
-constexpr int SF_SLOTS = 5;                                               // what tensor memory has room for
-constexpr int BARRIER_BYTES = 512;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + SF_SLOTS * SF_SLOT_BYTES + 1024 + BARRIER_BYTES;
-constexpr int THREADS = 384;                                              // warps: 0 TMA (operands and scales), 1 MMA, 2-9 epilogue, 10-11 scale copies
-constexpr int CP_WARPS = 2;                                               // they take the stages in turn (leader only)
-constexpr int SF_STAGE_COLS = 16 + 32;                                    // A scales, B scales
-static_assert(STAGE_BYTES % 1024 == 0, "stages must keep the 1024-byte swizzle alignment");
-static_assert(SF_COL0 + SF_SLOTS * SF_STAGE_COLS <= TMEM_COLS, "scale ring does not fit tensor memory");
-static_assert(SMEM_BYTES <= 232448, "more shared memory than a CTA can have");
-static_assert((2 * STAGES + (CP_WARPS + 1) * SF_SLOTS + 2) * 8 + 8 <= BARRIER_BYTES, "barrier area too small");
-static_assert(SF_SLOTS < STAGES, "the producer requests a stage's scales one iteration after its operands");
+constexpr int OPERAND_BYTES = A_BYTES + B_HALF_BYTES;                     // 32 KiB
+constexpr int THREADS = 320;
+constexpr int BARRIER_BYTES = 256;
 
-// 3-D form of the same (scale tiles).
-__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap *map, int c0, int c1, int c2, uint32_t cluster_bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3, %4}], [%5];"
-        ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(cluster_bar) : "memory");
-}
+template <bool MX> struct PairCfg {
+    static constexpr int TILES = MX ? KB_PER_STAGE / 2 : KB_PER_STAGE;    // 512-byte scale tiles of a stage per 128 rows
+    static constexpr int SFA_BYTES = TILES * SF_TILE_BYTES;
+    static constexpr int SF_BYTES = 3 * SFA_BYTES;                        // of a stage: this CTA's rows of A, all 256 rows of B
+    static constexpr int STAGE_BYTES = OPERAND_BYTES + SF_BYTES;
+    static constexpr int STAGES = MX ? 6 : 5;
+    static constexpr int SF_COLS = 12 * TILES;                            // tensor-memory columns of a stage's scales: 4 of A, 8 of B per tile
+    static constexpr int SF_COL = TMEM_COLS - 2 * 48;                     // the first of two sets, used in turn
+    static constexpr int ACC1_COL = SF_COL - TILE_N;                      // first column of the odd accumulator
+    static constexpr int OVERLAP = TILE_N - ACC1_COL;                     // columns that both accumulators use
+    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + BARRIER_BYTES;
+    static_assert(SF_COLS <= 48 && OVERLAP == 96, "tensor memory");
+    static_assert(SMEM_BYTES <= 232448, "more shared memory than a CTA can have");
+    static_assert((2 * STAGES + 3) * 8 + 8 <= BARRIER_BYTES, "barrier area too small");
+};
 
-// Arrive (once, on a barrier of this CTA) when the tcgen05 operations this thread issued for the pair are done.
-__device__ __forceinline__ void tc_commit_pair_local(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-// TMA tile load whose completion is signalled on a barrier of either CTA of the pair.
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap *map, int c0, int c1, uint32_t cluster_bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(cluster_bar) : "memory");
-}
-
-template <typename OUT>
+// GROUPED: row tiles run through each group's rows in steps of 256, so a tile never computes two groups' rows (its second
+// half may reach into the next group's, or beyond the last: not stored).
+template <typename OUT, bool MX, bool GROUPED = false>
 __global__ void __launch_bounds__(THREADS, 1)
-gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                       const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_sfb,
-                       const GemmParams p) {
+gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                     const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_sfb,
+                     const GemmParams p) {
+    using C = PairCfg<MX>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t *smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-    const uint32_t sf_base = smem_base + STAGES * STAGE_BYTES;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem_gen + STAGES * STAGE_BYTES + SF_SLOTS * SF_SLOT_BYTES);
+    const uint32_t sf_base = smem_base + C::STAGES * OPERAND_BYTES;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem_gen + C::STAGES * C::STAGE_BYTES);
     const uint32_t full_bar = smem_u32(bars);                 // [STAGES], used in the leader only
-    const uint32_t empty_bar = full_bar + 8 * STAGES;         // [STAGES]
-    const uint32_t sf_full_bar = empty_bar + 8 * STAGES;      // [CP_WARPS][SF_SLOTS], used in the leader only
-    const uint32_t sf_ready_bar = sf_full_bar + 8 * CP_WARPS * SF_SLOTS; // [SF_SLOTS], used in the leader only
-    const uint32_t acc_full_bar = sf_ready_bar + 8 * SF_SLOTS;
+    const uint32_t empty_bar = full_bar + 8 * C::STAGES;      // [STAGES]
+    const uint32_t acc_full_bar = empty_bar + 8 * C::STAGES;
     const uint32_t acc_empty_bar = acc_full_bar + 8;          // used in the leader only
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * STAGES + (CP_WARPS + 1) * SF_SLOTS + 2);
+    const uint32_t drain_bar = acc_empty_bar + 8;             // only used when the leader gives up
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * C::STAGES + 3);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_cta_rank();                 // 0 = leader
     const bool leader = rank == 0;
 
+    __shared__ GroupTable<GROUPED> groups;
+    __shared__ int32_t first_tile[GROUPED ? MAX_GROUPS + 1 : 1];          // of each group, in 256-row tiles
+    if constexpr (GROUPED) {
+        load_groups<THREADS>(p, groups);
+        __syncthreads();
+        if (warp == 2) {
+            int at = 0;                                                     // running sum, 32 groups at a time
+            for (int g0 = 0; g0 < p.num_groups; g0 += 32) {
+                const int g = g0 + lane;
+                int n = g < p.num_groups ? (groups.start[g + 1] - groups.start[g] + 255) / 256 : 0;
+                n = n < 0 ? 0 : n;
+                int sum = n;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int up = __shfl_up_sync(0xffffffffu, sum, o);
+                    if (lane >= o) sum += up;
+                }
+                if (g < p.num_groups) first_tile[g] = at + sum - n;
+                at += __shfl_sync(0xffffffffu, sum, 31);
+            }
+            if (lane == 0) first_tile[p.num_groups] = at;
+        }
+        __syncwarp();
+    }
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) {
+        for (int s = 0; s < C::STAGES; ++s) {
             mbar_init(full_bar + 8 * s, 1);
             mbar_init(empty_bar + 8 * s, 1);
         }
-        for (int j = 0; j < SF_SLOTS; ++j) {
-            for (int w = 0; w < CP_WARPS; ++w)
-                mbar_init(sf_full_bar + 8 * (w * SF_SLOTS + j), 1);   // the scale tiles of BOTH CTAs have landed
-            mbar_init(sf_ready_bar + 8 * j, 1);    // one commit after the copies into tensor memory
-        }
         mbar_init(acc_full_bar, 1);
         mbar_init(acc_empty_bar, 16);
+        mbar_init(drain_bar, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == 1) {
+        __syncwarp();
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
                      ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
@@ -780,238 +754,179 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    const int64_t num_m = p.m_p / 256, num_n = p.n_p / TILE_N;
+    // (the second half of a tile may lie beyond the operands: zero-filled by the copies, not stored)
+    const int64_t num_m = GROUPED ? first_tile[p.num_groups] : (p.m_p + 255) / 256, num_n = (p.n_p + TILE_N - 1) / TILE_N;
     const int64_t num_tiles = num_m * num_n;
+    // the group of row tile mb (the last one whose first tile is not beyond it: empty groups are skipped) and its first row
+    auto locate = [&](int64_t mb, int &group) -> int64_t {
+        group = 0;
+        if constexpr (!GROUPED) return mb * 256;
+        int lo = 0, hi = p.num_groups - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (first_tile[mid] <= mb) lo = mid; else hi = mid - 1;
+        }
+        group = lo;
+        return groups.start[lo] + (mb - first_tile[lo]) * 256;
+    };
     const int64_t k_blocks = p.k_p / 64;
-    const int64_t k_tiles = (k_blocks + KB_PER_STAGE - 1) / KB_PER_STAGE;
+    const int k_tiles = static_cast<int>((k_blocks + KB_PER_STAGE - 1) / KB_PER_STAGE);
     const int64_t pair_id = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-#ifdef FOS_GEMM_DEBUG
-    const bool dbg_no_sf = p.debug & 1, dbg_no_load = p.debug & 2, dbg_no_store = p.debug & 4;
-    const bool dbg_no_mma = p.debug & 16;
-#else
-    constexpr bool dbg_no_sf = false, dbg_no_load = false, dbg_no_store = false, dbg_no_mma = false;
-#endif
 
-    if (warp == 0 && lane == 0 && !dbg_no_load) {
-        // ------------------------------------------------------------------ TMA producer: operands and scales (both CTAs)
-        // Each CTA fetches its 128 rows of A and of B, and the scales of its own rows of A and of all 256 rows of B,
-        // into its own shared memory; everything completes on the LEADER's barriers. The scale ring has one slot
-        // less than the operand ring (tensor memory has room for five), so a stage's scales are requested one
-        // iteration AFTER its operands: the wait that frees operand stage i (the MMAs of iteration i - STAGES are
-        // done) also frees the scale slot of iteration i - 1. The first SF_SLOTS requests need no wait.
-        const uint32_t leader_full = map_to_cta(full_bar, 0), leader_sf_full = map_to_cta(sf_full_bar, 0);
-        int64_t f_t = pair_id, f_kt = 0;             // the stage whose scales are requested next
-        uint32_t slot = 0, f_w = 0;                  // its ring slot, and which copying warp will take it
-        int a_group = 0, b_group = 0;
-        int64_t requested = 0, i = 0;                // scale requests and operand stages issued so far
-        auto enter_tile = [&]() {
-            if (f_t >= num_tiles) return;
-            int64_t mb, nb;
-            tile_coords(f_t, num_m, num_n, mb, nb);
-            a_group = static_cast<int>(mb * 2 + rank);
-            b_group = static_cast<int>(nb * 2);
-        };
-        auto issue_next_scales = [&]() {
-            ++requested;
-            if (f_t >= num_tiles || dbg_no_sf) return;
-            const int kb0 = static_cast<int>(f_kt * KB_PER_STAGE);
-            const uint32_t idx = 8 * (f_w * SF_SLOTS + slot);
-            const uint32_t dst = sf_base + slot * SF_SLOT_BYTES, bar = leader_sf_full + idx;
-            if (leader) mbar_expect_tx(sf_full_bar + idx, 2 * SF_SLOT_BYTES);
-            tma_load_3d_pair(dst, &map_sfa, 0, kb0, a_group, bar);
-            tma_load_3d_pair(dst + SFA_BYTES, &map_sfb, 0, kb0, b_group, bar);
-            if (++slot == SF_SLOTS) slot = 0;
-            if (++f_w == CP_WARPS) f_w = 0;
-            if (++f_kt == k_tiles) {
-                f_kt = 0;
-                f_t += num_pairs;
-                enter_tile();
-            }
-        };
-        enter_tile();
+    if (warp == 0) {
+        // ------------------------------------------------------------------ TMA producer (both CTAs)
+        const bool issue = elect_one();
+        const uint32_t leader_full = map_to_cta(full_bar, 0);
+        asm volatile("griddepcontrol.wait;" ::: "memory");   // (a dependent launch) the kernel that packs A is done
         uint32_t s = 0, ph = 0;
         bool ok = true;
         for (int64_t t = pair_id; t < num_tiles && ok; t += num_pairs) {
             int64_t mb, nb;
             tile_coords(t, num_m, num_n, mb, nb);
-            const int m0 = static_cast<int>(mb * 256 + rank * 128), n0 = static_cast<int>(nb * TILE_N + rank * 128);
-            for (int64_t kt = 0; kt < k_tiles; ++kt, ++i) {
-                if (i < SF_SLOTS) issue_next_scales();
-                ok = mbar_wait_poll(empty_bar + 8 * s, ph ^ 1u, abort_flag, p.status, 1);
+            int group;
+            const int m0 = static_cast<int>(locate(mb, group) + rank * 128);
+            const int n0 = static_cast<int>(nb * TILE_N + rank * 128) + group * static_cast<int>(p.n_p);      // row of B
+            const int a_group = m0 / 128, b_group = static_cast<int>(nb * 2) + group * static_cast<int>(p.n_p / 128);
+            for (int kt = 0; kt < k_tiles; ++kt) {
+                ok = __all_sync(0xffffffffu, mbar_wait(empty_bar + 8 * s, ph ^ 1u, abort_flag, p.status, 1));
                 if (!ok) break;
-                if (i >= STAGES) issue_next_scales();
-                const uint32_t stage = smem_base + s * STAGE_BYTES, bar = leader_full + 8 * s;
+                const uint32_t stage = smem_base + s * OPERAND_BYTES, sf = sf_base + s * C::SF_BYTES, bar = leader_full + 8 * s;
                 // out-of-range parts of a box are zero-filled and still counted: fixed byte counts.
                 // The leader announces the bytes of both CTAs; its barrier may see the peer's bytes
                 // first, which only makes the pending count negative for a moment.
-                if (leader) mbar_expect_tx(full_bar + 8 * s, 2 * STAGE_BYTES);
-                tma_load_2d_pair(stage, &map_a, static_cast<int>(kt * BLOCK_K_BYTES), m0, bar);
-                tma_load_2d_pair(stage + A_BYTES, &map_b, static_cast<int>(kt * BLOCK_K_BYTES), n0, bar);
-                if (++s == STAGES) { s = 0; ph ^= 1u; }
+                if (issue) {
+                    if (leader) mbar_expect_tx(full_bar + 8 * s, 2 * C::STAGE_BYTES);
+                    tma_load_3d_pair(sf, &map_sfa, 0, kt * C::TILES, a_group, bar);
+                    tma_load_3d_pair(sf + C::SFA_BYTES, &map_sfb, 0, kt * C::TILES, b_group, bar);
+                    tma_load_2d_pair(stage, &map_a, kt * BLOCK_K_BYTES, m0, bar);
+                    tma_load_2d_pair(stage + A_BYTES, &map_b, kt * BLOCK_K_BYTES, n0, bar);
+                }
+                __syncwarp();
+                if (++s == C::STAGES) { s = 0; ph ^= 1u; }
             }
         }
-        // the scales of the last iteration (when there were more than SF_SLOTS): their slot is free once the
-        // operand stage that would come next is
-        while (ok && requested < i) {
-            ok = mbar_wait_poll(empty_bar + 8 * s, ph ^ 1u, abort_flag, p.status, 7);
-            if (!ok) break;
-            issue_next_scales();
-            if (++s == STAGES) { s = 0; ph ^= 1u; }
+        // the leader's last releases arrive in both CTAs' shared memory: stay until they have
+        for (int i = 0; i < C::STAGES && ok; ++i) {
+            ok = __all_sync(0xffffffffu, mbar_wait(empty_bar + 8 * s, ph ^ 1u, abort_flag, p.status, 7));
+            if (++s == C::STAGES) { s = 0; ph ^= 1u; }
         }
         if (!ok) {
             const unsigned long long t0 = global_timer_ns();
             while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
         }
     } else if (warp == 1 && leader) {
-        // ------------------------------------------------------------------ MMA issuer (leader only)
+        // ------------------------------------------------------------------ scale copies and MMAs, for both CTAs
         const bool issue = elect_one();
         const uint32_t idesc = mma_idesc(TILE_N, 256);
-        uint32_t s = 0, ph = 0, j = 0, jph = 0, tile_i = 0;
-        bool ok = true;
+        uint32_t s = 0, ph = 0, sf_set = 0, tile_i = 0;
+        bool ok = true, ready = false;
         for (int64_t t = pair_id; t < num_tiles && ok; t += num_pairs, ++tile_i) {
-            ok = mbar_wait_poll(acc_empty_bar, (tile_i & 1u) ^ 1u, abort_flag, p.status, 3);
-            ok = __all_sync(0xffffffffu, ok);
+            // the epilogue of the tile before has read the columns that the two accumulators share
+            ok = __all_sync(0xffffffffu, mbar_wait(acc_empty_bar, (tile_i & 1u) ^ 1u, abort_flag, p.status, 3));
             if (!ok) break;
             tc_fence_after();
-            for (int64_t kt = 0; kt < k_tiles; ++kt) {
-                if (!dbg_no_load) {
-                    ok = mbar_wait_poll(full_bar + 8 * s, ph, abort_flag, p.status, 2);
-                    if (ok && !dbg_no_sf) ok = mbar_wait_poll(sf_ready_bar + 8 * j, jph, abort_flag, p.status, 5);
-                }
-                ok = __all_sync(0xffffffffu, ok);
+            const uint32_t d_tmem = tmem_base + ((tile_i & 1u) ? C::ACC1_COL : 0);
+            for (int kt = 0; kt < k_tiles; ++kt) {
+                if (!ready) ok = __all_sync(0xffffffffu, mbar_wait(full_bar + 8 * s, ph, abort_flag, p.status, 2));
                 if (!ok) break;
-                tc_fence_after();
-                const int64_t kb0 = kt * KB_PER_STAGE;
-                const int nkb = static_cast<int>((k_blocks - kb0) < KB_PER_STAGE ? (k_blocks - kb0) : KB_PER_STAGE);
-                const uint32_t stage = smem_base + s * STAGE_BYTES;
-                const uint32_t sfa_tmem = tmem_base + SF_COL0 + j * SF_STAGE_COLS, sfb_tmem = sfa_tmem + 16;
-                const uint32_t a_lo = desc_lo(stage, 16), b_lo = desc_lo(stage + A_BYTES, 16);
+                // probe the next stage's barrier now (this warp has consumed the slot's phase before): the answer is back by the
+                // time this stage's instructions are issued
+                const uint32_t s_next = s + 1 == C::STAGES ? 0 : s + 1, ph_next = s + 1 == C::STAGES ? ph ^ 1u : ph;
+                const bool next_ready = mbar_test_wait(full_bar + 8 * s_next, ph_next);
+                const int left = static_cast<int>(k_blocks) - kt * KB_PER_STAGE;
+                const int nkb = left < KB_PER_STAGE ? left : KB_PER_STAGE;
+                const uint32_t stage = smem_base + s * OPERAND_BYTES;
+                const uint32_t a_lo = desc_lo(stage, 16), b_lo = desc_lo(stage + A_BYTES, 16), sf_lo = desc_lo(sf_base + s * C::SF_BYTES);
+                const uint32_t sfa = tmem_base + C::SF_COL + sf_set * 48, sfb = sfa + 4 * C::TILES;
+                if (issue) {
+                    // tiles: 32 rows of 16 bytes (one of 512 bytes per 128 rows and K-block; MXFP4: per two K-blocks), copied
+                    // to all four 32-lane quadrants of the tensor memory of each CTA from that CTA's own shared memory
 #pragma unroll
-                for (int kb = 0; kb < KB_PER_STAGE; ++kb) {
-                    if (kb < nkb && !dbg_no_mma && issue)
-                        tc_mma_nvf4_pair_lo(tmem_base, a_lo + 2 * kb, b_lo + 2 * kb, idesc, sfa_tmem + 4 * kb,
-                                            sfb_tmem + 8 * kb, (kt > 0 || kb > 0) ? 1u : 0u);
+                    for (int kb = 0; kb < C::TILES; ++kb) {
+                        tc_copy_sf_pair_lo(sfa + 4 * kb, sf_lo + ((kb * SF_TILE_BYTES) >> 4));
+                        tc_copy_sf_pair_lo(sfb + 8 * kb, sf_lo + ((C::SFA_BYTES + kb * SF_TILE_BYTES) >> 4));
+                        tc_copy_sf_pair_lo(sfb + 8 * kb + 4, sf_lo + ((C::SFA_BYTES + (C::TILES + kb) * SF_TILE_BYTES) >> 4));
+                    }
+#pragma unroll
+                    for (int kb = 0; kb < KB_PER_STAGE; ++kb) {
+                        if (kb >= nkb) break;
+                        const uint32_t accumulate = (kt > 0 || kb > 0) ? 1u : 0u;
+                        if constexpr (MX)
+                            tc_mma_mxf4_pair_lo(d_tmem, a_lo + 2 * kb, b_lo + 2 * kb, mma_idesc_mx(idesc, (kb & 1) * 2),
+                                                sfa + 4 * (kb >> 1), sfb + 8 * (kb >> 1), accumulate);
+                        else
+                            tc_mma_nvf4_pair_lo(d_tmem, a_lo + 2 * kb, b_lo + 2 * kb, idesc, sfa + 4 * kb, sfb + 8 * kb, accumulate);
+                    }
+                    tc_commit_pair(empty_bar + 8 * s);
                 }
-                if (issue) tc_commit_pair(empty_bar + 8 * s);
                 __syncwarp();
-                if (++s == STAGES) { s = 0; ph ^= 1u; }
-                if (++j == SF_SLOTS) { j = 0; jph ^= 1u; }
+                sf_set ^= 1u;
+                ready = __all_sync(0xffffffffu, next_ready);
+                s = s_next;
+                ph = ph_next;
             }
             if (ok && issue) tc_commit_pair(acc_full_bar);
         }
-    } else if (warp >= 2 && warp < 10) {
+        if (!ok) {
+            // giving up: the MMAs already issued must have finished before tensor memory is released
+            if (issue) tc_commit_pair_local(drain_bar);
+            __syncwarp();
+            const long long t0 = clock64();
+            while (!mbar_try_wait(drain_bar, 0) && clock64() - t0 < 20000000ll) {}   // about 10 ms
+        }
+    } else if (warp >= 2) {
         // ------------------------------------------------------------------ epilogue (both CTAs)
         const int quad = warp & 3;                       // tensor-memory lanes 32*quad .. +31
-        const int half = (warp - 2) >> 2;                // which 128 of the 256 columns
-        constexpr int COLS = 128;
-        const float alpha = __ldg(p.alpha);
+        const int half = (warp - 2) >> 2;                // which half of the shared columns, and of the others
+        asm volatile("griddepcontrol.wait;" ::: "memory");   // amax_a, and whoever still reads d
+        float alpha = GROUPED ? 0.0f : gemm_alpha(p);
+        int64_t row_end = p.m;
         OUT *out = static_cast<OUT *>(p.d);
-        const bool vec_ok = (reinterpret_cast<uintptr_t>(out) % 16 == 0) && ((p.ldd * sizeof(OUT)) % 16 == 0);
-        const bool vec32_ok = FOS_GEMM_ST256 && (reinterpret_cast<uintptr_t>(out) % 32 == 0) && ((p.ldd * sizeof(OUT)) % 32 == 0);
+        const bool vec16 = (reinterpret_cast<uintptr_t>(out) % 16 == 0) && ((p.ldd * sizeof(OUT)) % 16 == 0);
+        const bool vec32 = (reinterpret_cast<uintptr_t>(out) % 32 == 0) && ((p.ldd * sizeof(OUT)) % 32 == 0);
         const uint32_t leader_acc_empty = map_to_cta(acc_empty_bar, 0);
         uint32_t tile_i = 0;
         bool ok = true;
         for (int64_t t = pair_id; t < num_tiles && ok; t += num_pairs, ++tile_i) {
             int64_t mb, nb;
             tile_coords(t, num_m, num_n, mb, nb);
-            const int64_t row = mb * 256 + rank * 128 + quad * 32 + lane, n0 = nb * TILE_N + half * COLS;
-            // in the peer this barrier is arrived on from the leader's SM: one lane polls for the warp
+            int group;
+            const int64_t row = locate(mb, group) + rank * 128 + quad * 32 + lane;
+            if constexpr (GROUPED) {
+                alpha = gemm_alpha(p, group);
+                row_end = groups.end[group];
+            }
+            const bool odd = tile_i & 1u;
+            // columns of the tile that this warp takes: half of the shared ones, then half of the others
+            constexpr int FIRST = C::OVERLAP / 2, SECOND = C::ACC1_COL / 2;
+            const int first = (odd ? 0 : C::ACC1_COL) + half * FIRST, second = (odd ? C::OVERLAP : 0) + half * SECOND;
+            // (in the peer this barrier is arrived on from the leader's SM: one lane polls for the warp)
             if (lane == 0) ok = mbar_wait_poll(acc_full_bar, tile_i & 1u, abort_flag, p.status, 4);
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             if (!ok) break;
             tc_fence_after();
-            const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + half * COLS;
-            const bool row_ok = row < p.m && !dbg_no_store;
-            if constexpr (sizeof(OUT) == 2) {
-                uint32_t pk[COLS / 2];
+            const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + (odd ? C::ACC1_COL : 0);
+            OUT *dst = out + row * p.ldd + nb * TILE_N;
+            const OUT *bias = p.bias ? static_cast<const OUT *>(p.bias) + nb * TILE_N : nullptr;
+            const int64_t left = row < row_end ? p.n - nb * TILE_N : 0;
+            auto store = [&](const uint32_t *acc, int col, auto n) {
+                store_columns<OUT, decltype(n)::value>(dst + col, acc, alpha, bias ? bias + col : nullptr, left - col, vec32, vec16);
+            };
+            uint32_t v[FIRST / 48][48];
 #pragma unroll
-                for (int c = 0; c < COLS / 32; ++c) {
-                    uint32_t v[32];
-                    tc_load_32cols_sync(t_acc + 32 * c, v);
-                    if (c + 1 == COLS / 32) {            // everything is in registers: release the accumulator
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive_cluster(leader_acc_empty);
-                    }
+            for (int i = 0; i < FIRST / 48; ++i) tc_load_48cols_sync(t_acc + first + 48 * i, v[i]);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(leader_acc_empty);
 #pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        pk[16 * c + i] = pack_pair<OUT>(alpha * __uint_as_float(v[2 * i]), alpha * __uint_as_float(v[2 * i + 1]));
-                }
-                const int64_t left = p.n - n0;
-                if (row_ok && left > 0) {
-                    OUT *dst = out + row * p.ldd + n0;
-                    if (left >= COLS && vec32_ok) {
-#pragma unroll
-                        for (int i = 0; i < COLS / 16; ++i) stg_32_stream(reinterpret_cast<uint8_t *>(dst) + 32 * i, &pk[8 * i]);
-                    } else if (left >= COLS && vec_ok) {
-#pragma unroll
-                        for (int i = 0; i < COLS / 8; ++i)
-                            reinterpret_cast<uint4 *>(dst)[i] = make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
-                    } else {
-                        uint16_t *d16 = reinterpret_cast<uint16_t *>(dst);
-#pragma unroll
-                        for (int i = 0; i < COLS; ++i)
-                            if (i < left) d16[i] = static_cast<uint16_t>(pk[i >> 1] >> ((i & 1) * 16));
-                    }
-                }
-            } else {
-#pragma unroll 1
-                for (int c = 0; c < 4; c += 2) {
-                    uint32_t v0[32], v1[32];
-                    tc_load_64cols_sync(t_acc + 32 * c, v0, v1);
-                    if (c + 2 >= 4) {
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive_cluster(leader_acc_empty);
-                    }
-                    const int64_t col = n0 + 32 * c;
-                    const int64_t left0 = p.n - col, left1 = left0 - 32;
-                    if (row_ok && left0 > 0)
-                        store_chunk<OUT>(out + row * p.ldd + col, v0, alpha, left0 < 32 ? static_cast<int>(left0) : 32, vec_ok);
-                    if (row_ok && left1 > 0)
-                        store_chunk<OUT>(out + row * p.ldd + col + 32, v1, alpha, left1 < 32 ? static_cast<int>(left1) : 32, vec_ok);
-                }
+            for (int i = 0; i < FIRST / 48; ++i) store(v[i], first + 48 * i, std::integral_constant<int, 48>{});
+            if constexpr (SECOND == 80) {
+                tc_load_48cols_sync(t_acc + second, v[0]);
+                store(v[0], second, std::integral_constant<int, 48>{});
             }
-        }
-    } else if (warp >= 10 && warp < 10 + CP_WARPS && leader && !dbg_no_load && !dbg_no_sf) {
-        // ------------------------------------------------------------------ scale copies (leader, for both CTAs)
-        // tcgen05.cp with cta_group::2 copies, in each CTA, from that CTA's shared memory into its
-        // tensor memory: one thread of the pair moves the scales of both, and no warp of the peer
-        // has to report back. Two warps take the stages in turn (one alone cannot issue twelve copies
-        // per stage as fast as the MMAs consume them), each with a landing barrier of its own per slot.
-        const bool issue = elect_one();
-        const uint32_t me = static_cast<uint32_t>(warp - 10);
-        uint32_t j = 0, turn = 0, seen = 0;          // bit j of `seen`: parity of this warp's next phase of slot j
-        bool ok = true;
-        for (int64_t t = pair_id; t < num_tiles && ok; t += num_pairs) {
-            for (int64_t kt = 0; kt < k_tiles; ++kt) {
-                const bool mine = turn == me;
-                if (++turn == CP_WARPS) turn = 0;
-                if (!mine) {
-                    if (++j == SF_SLOTS) j = 0;
-                    continue;
-                }
-                const uint32_t jph = (seen >> j) & 1u;
-                seen ^= 1u << j;
-                ok = mbar_wait_poll(sf_full_bar + 8 * (me * SF_SLOTS + j), jph, abort_flag, p.status, 6);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t src = sf_base + j * SF_SLOT_BYTES, dst = tmem_base + SF_COL0 + j * SF_STAGE_COLS;
-                const uint32_t src_lo = desc_lo(src);
-#pragma unroll
-                for (int kb = 0; kb < KB_PER_STAGE; ++kb) {
-                    if (!issue) break;
-                    tc_copy_sf_pair_lo(dst + 4 * kb, src_lo + ((kb * SF_TILE_BYTES) >> 4));
-#pragma unroll
-                    for (int g = 0; g < 2; ++g)
-                        tc_copy_sf_pair_lo(dst + 16 + 8 * kb + 4 * g,
-                                           src_lo + ((SFA_BYTES + (g * KB_PER_STAGE + kb) * SF_TILE_BYTES) >> 4));
-                }
-                if (issue) tc_commit_pair_local(sf_ready_bar + 8 * j);
-                __syncwarp();
-                if (++j == SF_SLOTS) j = 0;
-            }
+            uint32_t w[32];
+            tc_load_32cols_sync(t_acc + second + (SECOND - 32), w);
+            store(w, second + (SECOND - 32), std::integral_constant<int, 32>{});
         }
     }
 
@@ -1028,56 +943,21 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 
 // ---------------------------------------------------------------------------- host side
 
-// Scale tiles as a 3-D tensor [row groups][tiles along K][512 bytes]; box = `groups` x the tiles of one stage
-// (four; two for MXFP4, whose tiles span two K-blocks).
-int make_scale_map(CUtensorMap *map, const uint8_t *sf, int64_t row_groups, int64_t k_blocks, int groups,
-                   int tiles_per_stage = KB_PER_STAGE) {
-    EncodeTiledFn fn = encode_tiled_fn();
-    if (!fn) return FOS_ERR_CUDA;
-    cuuint64_t dims[3] = {128, static_cast<cuuint64_t>(k_blocks), static_cast<cuuint64_t>(row_groups)};
-    cuuint64_t strides[2] = {512, static_cast<cuuint64_t>(k_blocks) * 512};
-    cuuint32_t box[3] = {128, static_cast<cuuint32_t>(tiles_per_stage), static_cast<cuuint32_t>(groups)};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<uint8_t *>(sf), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? FOS_OK : FOS_ERR_CUDA;
+template <typename OUT, bool MX, bool GROUPED>
+int launch_pair(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &msa, const CUtensorMap &msb,
+                const GemmParams &p, int max_ctas, cudaStream_t stream) {
+    // (grouped: at most one more row tile per group than the buffer has)
+    const int64_t row_tiles = (p.m_p + 255) / 256 + (GROUPED ? p.num_groups : 0);
+    return pair::launch(pair::gemm_fp4_pair_kernel<OUT, MX, GROUPED>, pair::THREADS, pair::PairCfg<MX>::SMEM_BYTES,
+                        row_tiles * ((p.n_p + 255) / 256), max_ctas, stream, ma, mb, msa, msb, p);
 }
 
-template <typename OUT>
-int launch_pair(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &msa, const CUtensorMap &msb,
-                const GemmParams &p, cudaStream_t stream) {
-    auto kernel = pair::gemm_nvfp4_pair_kernel<OUT>;
-    static int max_clusters[64] = {};   // per device: how many CTA pairs can be resident at once
-    static std::mutex mu;
-    int dev = 0;
-    FOS_CUDA_TRY(cudaGetDevice(&dev));
-    const int slot = (dev >= 0 && dev < 64) ? dev : 0;
-    std::lock_guard<std::mutex> lock(mu);
-    cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(pair::THREADS);
-    cfg.dynamicSmemBytes = pair::SMEM_BYTES;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (max_clusters[slot] == 0) {
-        FOS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, pair::SMEM_BYTES));
-        int sms = 0, n = 0;
-        FOS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        cfg.gridDim = dim3(static_cast<unsigned>(sms & ~1));
-        FOS_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, kernel, &cfg));
-        max_clusters[slot] = n > 0 ? n : 1;
-    }
-    const int64_t tiles = (p.m_p / 256) * (p.n_p / 256);
-    const int64_t pairs = tiles < max_clusters[slot] ? tiles : max_clusters[slot];
-    cfg.gridDim = dim3(static_cast<unsigned>(2 * pairs));
-    FOS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, ma, mb, msa, msb, p));
-    return FOS_OK;
+template <bool MX, bool GROUPED = false>
+int launch_pair_out(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &msa, const CUtensorMap &msb,
+                    const GemmParams &p, int max_ctas, cudaStream_t stream) {
+    if (p.out_dtype == FOS_BF16) return launch_pair<__nv_bfloat16, MX, GROUPED>(ma, mb, msa, msb, p, max_ctas, stream);
+    if (p.out_dtype == FOS_FP16) return launch_pair<__half, MX, GROUPED>(ma, mb, msa, msb, p, max_ctas, stream);
+    return launch_pair<float, MX, GROUPED>(ma, mb, msa, msb, p, max_ctas, stream);
 }
 
 template <int BLOCK_N, typename OUT, bool FUSED_A = false, bool GROUPED = false>
@@ -1093,8 +973,7 @@ int launch(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &msa,
     }));
     const int64_t tiles = (p.m_p / BLOCK_M) * ((p.n_p + BLOCK_N - 1) / BLOCK_N);
     const unsigned grid = static_cast<unsigned>(tiles < sms ? tiles : sms);
-    kernel<<<grid, NUM_THREADS, C::SMEM_BYTES, stream>>>(ma, mb, msa, msb, p);
-    FOS_CUDA_TRY(cudaGetLastError());
+    FOS_CUDA_TRY(launch_dependent(kernel, dim3(grid), NUM_THREADS, C::SMEM_BYTES, stream, ma, mb, msa, msb, p));
     return FOS_OK;
 }
 
@@ -1126,7 +1005,7 @@ static int gemm_fp4_entry(const uint8_t *a_codes, const uint8_t *a_sf, const uin
                           const uint8_t *b_sf, const float *alpha, void *d, int out_dtype, int64_t m_p,
                           int64_t n_p, int64_t k_p, int64_t m, int64_t n, int64_t ldd, const fos_gemm_opts *opts,
                           int32_t *status, void *stream_, int mx, void *const *d_peers = nullptr, int world = 0,
-                          int rank = 0) {
+                          int rank = 0, const fos::GemmScales *scales = nullptr) {
     using namespace fos;
     const int variant = opts ? opts->variant : 0, max_ctas = opts ? opts->max_ctas : 0;
     if ((variant != 0 && variant != 128 && variant != 256 && variant != 2) || max_ctas < 0) return FOS_ERR_INVALID_ARGUMENT;
@@ -1139,7 +1018,7 @@ static int gemm_fp4_entry(const uint8_t *a_codes, const uint8_t *a_sf, const uin
         }
         d = d_peers[rank];
     }
-    if (!a_codes || !a_sf || !b_codes || !b_sf || !alpha || !d) return FOS_ERR_INVALID_ARGUMENT;
+    if (!a_codes || !a_sf || !b_codes || !b_sf || (!alpha && !scales) || !d) return FOS_ERR_INVALID_ARGUMENT;
     if (m_p <= 0 || n_p <= 0 || k_p < 64 || m_p % 128 || n_p % 128 || k_p % (mx ? 128 : 64)) return FOS_ERR_INVALID_ARGUMENT;
     if (m <= 0 || n <= 0 || m > m_p || n > n_p || ldd < n) return FOS_ERR_INVALID_ARGUMENT;
     if (out_dtype != FOS_BF16 && out_dtype != FOS_FP16 && out_dtype != FOS_FP32) return FOS_ERR_INVALID_ARGUMENT;
@@ -1161,8 +1040,18 @@ static int gemm_fp4_entry(const uint8_t *a_codes, const uint8_t *a_sf, const uin
 #else
     const int debug_bits = 0;
 #endif
-    GemmParams p{a_sf, b_sf, alpha, d, status, m_p, n_p, k_p, m, n, ldd, out_dtype, debug_bits, mx, nullptr, 0, nullptr, 0, 0,
-                 0, 0, 0, {}};
+    GemmParams p{};
+    p.a_sf = a_sf; p.b_sf = b_sf;
+    p.alpha = alpha;
+    if (scales) {
+        p.amax_a = scales->amax_a;
+        p.amax_b = scales->amax_b;
+        p.alpha_denom = scales->denom;
+        p.bias = scales->bias;
+    }
+    p.d = d; p.status = status;
+    p.m_p = m_p; p.n_p = n_p; p.k_p = k_p; p.m = m; p.n = n; p.ldd = ldd;
+    p.out_dtype = out_dtype; p.debug = debug_bits; p.mx = mx;
     if (d_peers) {
         p.scatter_world = world;
         p.scatter_rank = rank;
@@ -1178,29 +1067,35 @@ static int gemm_fp4_entry(const uint8_t *a_codes, const uint8_t *a_sf, const uin
     }
     CUtensorMap map_a, map_b;
 
-    // The CTA-pair kernel is correct but still measures slower than the single-CTA kernel on B200
-    // (its hand-overs between the two SMs lengthen the load round trip), so it only runs when
-    // asked for.
-    const bool pair_fits = m_p % 256 == 0 && n_p % 256 == 0;
-    const bool use_pair = pair_fits && variant == 2 && !mx && !d_peers;
-    if (use_pair) {
-        CUtensorMap map_sfa, map_sfb;
-        if ((st = make_operand_map(&map_a, a_codes, m_p, k_p / 2, 128)) != FOS_OK) return st;
-        if ((st = make_operand_map(&map_b, b_codes, n_p, k_p / 2, 128)) != FOS_OK) return st;
-        if ((st = make_scale_map(&map_sfa, a_sf, m_p / 128, k_p / 64, 1)) != FOS_OK) return st;
-        if ((st = make_scale_map(&map_sfb, b_sf, n_p / 128, k_p / 64, 2)) != FOS_OK) return st;
-        if (out_dtype == FOS_BF16) return launch_pair<__nv_bfloat16>(map_a, map_b, map_sfa, map_sfb, p, stream);
-        if (out_dtype == FOS_FP16) return launch_pair<__half>(map_a, map_b, map_sfa, map_sfb, p, stream);
-        return launch_pair<float>(map_a, map_b, map_sfa, map_sfb, p, stream);
+    if (m <= skinny::MAX_TOKENS && variant == 0 && max_ctas == 0 && !d_peers && n_p / 128 <= INT32_MAX / skinny::MAX_SPLIT) {
+        skinny::Params q{};
+        q.alpha = alpha;
+        q.amax_a = p.amax_a; q.amax_b = p.amax_b; q.denom = p.alpha_denom;
+        q.d = d; q.status = p.status;
+        q.bias = p.bias;
+        q.m = static_cast<int>(m); q.n = static_cast<int>(n); q.ldd = ldd;
+        return mx ? skinny::launch_n<true>(a_codes, a_sf, b_codes, b_sf, q, out_dtype, m_p, n_p, k_p, sms, scales && scales->chained, stream)
+                  : skinny::launch_n<false>(a_codes, a_sf, b_codes, b_sf, q, out_dtype, m_p, n_p, k_p, sms, scales && scales->chained, stream);
     }
 
-    // single-CTA kernel: 128 x 256 tiles unless they would fill less than half of the SMs (a 128 x 128
-    // tile takes nine tenths of the time of a 128 x 256 one, so the narrow kernel only pays when it
-    // doubles the number of busy SMs)
-    const int64_t tiles_256 = (m_p / BLOCK_M) * ((n_p + 255) / 256);
+    // 128 x 256 tiles unless they would fill less than half of the SMs (a 128 x 128 tile takes nine tenths of the
+    // time of a 128 x 256 one, so the narrow kernel only pays when it doubles the number of busy SMs); in place of
+    // the wide ones 256 x 256 tiles on CTA pairs wherever those need no more rounds (see pairs_pay)
+    const int64_t tiles_256 = (m_p / BLOCK_M) * ((n_p + 255) / 256), pair_tiles = ((m_p + 255) / 256) * ((n_p + 255) / 256);
     bool wide = n_p >= 256 && tiles_256 * 2 > sms;
+    const bool use_pair = !d_peers && (variant == 2 || (variant == 0 && wide && pairs_pay(tiles_256, pair_tiles, sms)));
     if (variant == 128) wide = false;
     if (variant == 256) wide = true;
+    if (use_pair) {
+        CUtensorMap map_sfa, map_sfb;
+        const int tiles = mx ? KB_PER_STAGE / 2 : KB_PER_STAGE;
+        if ((st = make_operand_map(&map_a, a_codes, m_p, k_p / 2, 128)) != FOS_OK) return st;
+        if ((st = make_operand_map(&map_b, b_codes, n_p, k_p / 2, 128)) != FOS_OK) return st;
+        if ((st = make_scale_map(&map_sfa, a_sf, m_p / 128, sf_k_tiles, 1, tiles)) != FOS_OK) return st;
+        if ((st = make_scale_map(&map_sfb, b_sf, n_p / 128, sf_k_tiles, 2, tiles)) != FOS_OK) return st;
+        return mx ? launch_pair_out<true>(map_a, map_b, map_sfa, map_sfb, p, max_ctas, stream)
+                  : launch_pair_out<false>(map_a, map_b, map_sfa, map_sfb, p, max_ctas, stream);
+    }
     if ((st = make_operand_map(&map_a, a_codes, m_p, k_p / 2, BLOCK_M)) != FOS_OK) return st;
     if ((st = make_operand_map(&map_b, b_codes, n_p, k_p / 2, wide ? 256 : 128)) != FOS_OK) return st;
     CUtensorMap map_sfa, map_sfb;
@@ -1228,6 +1123,33 @@ extern "C" int fos_gemm_nvfp4_ex(const uint8_t *a_codes, const uint8_t *a_sf, co
     return gemm_fp4_entry(a_codes, a_sf, b_codes, b_sf, alpha, d, out_dtype, m_p, n_p, k_p, m, n, ldd, opts, status, stream, 0);
 }
 
+int fos::gemm_nvfp4_chained(const uint8_t *a_codes, const uint8_t *a_sf, const uint8_t *b_codes, const uint8_t *b_sf,
+                            const GemmScales &scales, void *d, int out_dtype, int64_t m_p, int64_t n_p, int64_t k_p,
+                            int64_t m, int64_t n, int64_t ldd, const fos_gemm_opts *opts, int32_t *status, void *stream) {
+    return gemm_fp4_entry(a_codes, a_sf, b_codes, b_sf, nullptr, d, out_dtype, m_p, n_p, k_p, m, n, ldd, opts, status, stream, 0,
+                          nullptr, 0, 0, &scales);
+}
+
+extern "C" int fos_gemm_nvfp4_scaled(const uint8_t *a_codes, const uint8_t *a_sf, const float *amax_a, int rule_a,
+                                     int unbiased_a, const uint8_t *b_codes, const uint8_t *b_sf, const float *amax_b,
+                                     int rule_b, int unbiased_b, void *d, int out_dtype, int64_t m_p, int64_t n_p,
+                                     int64_t k_p, int64_t m, int64_t n, int64_t ldd, const fos_gemm_opts *opts,
+                                     int32_t *status, void *stream) {
+    using namespace fos;
+    if (!amax_a || !amax_b) return FOS_ERR_INVALID_ARGUMENT;
+    const GemmScales scales{amax_a, amax_b, alpha_divisor(FOS_NVFP4, rule_a, FOS_NVFP4, rule_b, unbiased_a, unbiased_b), nullptr, false};
+    return gemm_fp4_entry(a_codes, a_sf, b_codes, b_sf, nullptr, d, out_dtype, m_p, n_p, k_p, m, n, ldd, opts, status, stream, 0,
+                          nullptr, 0, 0, &scales);
+}
+
+extern "C" int fos_gemm_mxfp4_unscaled(const uint8_t *a_codes, const uint8_t *a_sf, const uint8_t *b_codes, const uint8_t *b_sf,
+                                       void *d, int out_dtype, int64_t m_p, int64_t n_p, int64_t k_p, int64_t m, int64_t n,
+                                       int64_t ldd, const fos_gemm_opts *opts, int32_t *status, void *stream) {
+    const fos::GemmScales scales{nullptr, nullptr, 1.0f, nullptr, false};
+    return gemm_fp4_entry(a_codes, a_sf, b_codes, b_sf, nullptr, d, out_dtype, m_p, n_p, k_p, m, n, ldd, opts, status, stream, 1,
+                          nullptr, 0, 0, &scales);
+}
+
 extern "C" int fos_gemm_nvfp4_fused_a(const void *x, int x_dtype, int64_t x_ld, const float *x_amax, int x_rule,
                                       const uint8_t *b_codes, const uint8_t *b_sf, const float *alpha, void *d,
                                       int out_dtype, int64_t m, int64_t n_p, int64_t k, int64_t n, int64_t ldd,
@@ -1249,8 +1171,12 @@ extern "C" int fos_gemm_nvfp4_fused_a(const void *x, int x_dtype, int64_t x_ld, 
     int dev = 0, sms = 0;
     FOS_CUDA_TRY(cudaGetDevice(&dev));
     FOS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    GemmParams p{nullptr, b_sf, alpha, d, status, m_p, n_p, k, m, n, ldd, out_dtype, 0, 0, x, x_ld, x_amax, x_rule,
-                 x_dtype == FOS_FP16 ? 1 : 0, 0, 0, 0, {}};
+    GemmParams p{};
+    p.b_sf = b_sf; p.alpha = alpha; p.d = d; p.status = status;
+    p.m_p = m_p; p.n_p = n_p; p.k_p = k; p.m = m; p.n = n; p.ldd = ldd;
+    p.out_dtype = out_dtype;
+    p.x = x; p.x_ld = x_ld; p.x_amax = x_amax; p.x_rule = x_rule;
+    p.x_is_fp16 = x_dtype == FOS_FP16 ? 1 : 0;
     if (status) {
         FOS_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int32_t), stream));
     } else {
@@ -1266,15 +1192,15 @@ extern "C" int fos_gemm_nvfp4_fused_a(const void *x, int x_dtype, int64_t x_ld, 
                 : launch_out<128, true>(map_b, map_b, map_sfb, map_sfb, p, sms, stream);
 }
 
-extern "C" int fos_gemm_nvfp4_grouped(const uint8_t *a_codes, const uint8_t *a_sf, const uint8_t *b_codes,
-                                      const uint8_t *b_sf, const float *alpha, void *d, int out_dtype,
-                                      const int32_t *group_start, const int32_t *group_rows, int num_groups,
-                                      int64_t rows_capacity, int64_t n_p, int64_t k_p, int64_t n, int64_t ldd,
-                                      const fos_gemm_opts *opts, int32_t *status, void *stream_) {
+static int gemm_grouped_entry(const uint8_t *a_codes, const uint8_t *a_sf, const uint8_t *b_codes, const uint8_t *b_sf,
+                              const float *alpha, const fos::GemmScales *scales, void *d, int out_dtype,
+                              const int32_t *group_start, const int32_t *group_rows, int num_groups, int64_t rows_capacity,
+                              int64_t n_p, int64_t k_p, int64_t n, int64_t ldd, const fos_gemm_opts *opts, int32_t *status,
+                              void *stream_) {
     using namespace fos;
     const int variant = opts ? opts->variant : 0, max_ctas = opts ? opts->max_ctas : 0;
     if ((variant != 0 && variant != 128 && variant != 256) || max_ctas < 0) return FOS_ERR_INVALID_ARGUMENT;
-    if (!a_codes || !a_sf || !b_codes || !b_sf || !alpha || !d || !group_start || !group_rows) return FOS_ERR_INVALID_ARGUMENT;
+    if (!a_codes || !a_sf || !b_codes || !b_sf || (!alpha && !scales) || !d || !group_start || !group_rows) return FOS_ERR_INVALID_ARGUMENT;
     if (num_groups <= 0 || num_groups > MAX_GROUPS) return FOS_ERR_INVALID_ARGUMENT;
     if (rows_capacity <= 0 || rows_capacity % 128 || n_p <= 0 || n_p % 128 || k_p < 64 || k_p % 64) return FOS_ERR_INVALID_ARGUMENT;
     if (n <= 0 || n > n_p || ldd < n) return FOS_ERR_INVALID_ARGUMENT;
@@ -1291,8 +1217,15 @@ extern "C" int fos_gemm_nvfp4_grouped(const uint8_t *a_codes, const uint8_t *a_s
     FOS_CUDA_TRY(cudaGetDevice(&dev));
     FOS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     if (max_ctas > 0 && max_ctas < sms) sms = max_ctas;
-    GemmParams p{a_sf, b_sf, alpha, d, status, rows_capacity, n_p, k_p, rows_capacity, n, ldd, out_dtype, 0, 0, nullptr, 0,
-                 nullptr, 0, 0, 0, 0, 0, {}};
+    GemmParams p{};
+    p.a_sf = a_sf; p.b_sf = b_sf; p.alpha = alpha; p.d = d; p.status = status;
+    p.m_p = rows_capacity; p.n_p = n_p; p.k_p = k_p; p.m = rows_capacity; p.n = n; p.ldd = ldd;
+    p.out_dtype = out_dtype;
+    if (scales) {
+        p.amax_a = scales->amax_a;
+        p.amax_b = scales->amax_b;
+        p.alpha_denom = scales->denom;
+    }
     p.group_start = group_start;
     p.group_rows = group_rows;
     p.num_groups = num_groups;
@@ -1308,12 +1241,38 @@ extern "C" int fos_gemm_nvfp4_grouped(const uint8_t *a_codes, const uint8_t *a_s
     if (variant == 128) wide = false;
     if (variant == 256 && n_p >= 256) wide = true;
     CUtensorMap map_a, map_b, map_sfa, map_sfb;
+    // 256-row tiles waste half a tile per group on average, 128-row tiles a quarter of that: pairs where groups are long
+    const bool use_pair = variant == 0 && wide && rows_capacity / num_groups >= PAIR_MIN_GROUP_ROWS;
+    if (use_pair) {
+        if ((st = make_operand_map(&map_a, a_codes, rows_capacity, k_p / 2, 128)) != FOS_OK) return st;
+        if ((st = make_operand_map(&map_b, b_codes, b_rows, k_p / 2, 128)) != FOS_OK) return st;
+        if ((st = make_scale_map(&map_sfa, a_sf, rows_capacity / 128, k_p / 64, 1, KB_PER_STAGE)) != FOS_OK) return st;
+        if ((st = make_scale_map(&map_sfb, b_sf, b_rows / 128, k_p / 64, 2, KB_PER_STAGE)) != FOS_OK) return st;
+        return launch_pair_out<false, true>(map_a, map_b, map_sfa, map_sfb, p, max_ctas, stream);
+    }
     if ((st = make_operand_map(&map_a, a_codes, rows_capacity, k_p / 2, BLOCK_M)) != FOS_OK) return st;
     if ((st = make_operand_map(&map_b, b_codes, b_rows, k_p / 2, wide ? 256 : 128)) != FOS_OK) return st;
     if ((st = make_scale_map(&map_sfa, a_sf, rows_capacity / 128, k_p / 64, 1, KB_PER_STAGE)) != FOS_OK) return st;
     if ((st = make_scale_map(&map_sfb, b_sf, b_rows / 128, k_p / 64, wide ? 2 : 1, KB_PER_STAGE)) != FOS_OK) return st;
     return wide ? launch_out<256, false, true>(map_a, map_b, map_sfa, map_sfb, p, sms, stream)
                 : launch_out<128, false, true>(map_a, map_b, map_sfa, map_sfb, p, sms, stream);
+}
+
+extern "C" int fos_gemm_nvfp4_grouped(const uint8_t *a_codes, const uint8_t *a_sf, const uint8_t *b_codes,
+                                      const uint8_t *b_sf, const float *alpha, void *d, int out_dtype,
+                                      const int32_t *group_start, const int32_t *group_rows, int num_groups,
+                                      int64_t rows_capacity, int64_t n_p, int64_t k_p, int64_t n, int64_t ldd,
+                                      const fos_gemm_opts *opts, int32_t *status, void *stream) {
+    return gemm_grouped_entry(a_codes, a_sf, b_codes, b_sf, alpha, nullptr, d, out_dtype, group_start, group_rows, num_groups,
+                              rows_capacity, n_p, k_p, n, ldd, opts, status, stream);
+}
+
+int fos::gemm_nvfp4_grouped_scaled(const uint8_t *a_codes, const uint8_t *a_sf, const uint8_t *b_codes, const uint8_t *b_sf,
+                                   const GemmScales &scales, void *d, int out_dtype, const int32_t *group_start,
+                                   const int32_t *group_rows, int num_groups, int64_t rows_capacity, int64_t n_p, int64_t k_p,
+                                   int64_t n, int64_t ldd, int32_t *status, void *stream) {
+    return gemm_grouped_entry(a_codes, a_sf, b_codes, b_sf, nullptr, &scales, d, out_dtype, group_start, group_rows, num_groups,
+                              rows_capacity, n_p, k_p, n, ldd, nullptr, status, stream);
 }
 
 extern "C" int fos_gemm_mxfp4(const uint8_t *a_codes, const uint8_t *a_sf, const uint8_t *b_codes,

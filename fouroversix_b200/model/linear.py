@@ -205,11 +205,12 @@ class FourOverSixLinear(nn.Linear):
         return dequantize(w, dtype) if isinstance(w, QuantizedTensor) else w.data.to(dtype)
 
     def forward(self, input: torch.Tensor) -> torch.Tensor:
-        if self._one_call_forward_applies(input):
-            return self._forward_one_call(input)
-        return FourOverSixLinearFunction.apply(self.config, input, self.quantized_weight(), self.bias)
+        weight = self.quantized_weight()
+        if self._one_call_forward_applies(input, weight):
+            return self._forward_one_call(input, weight)
+        return FourOverSixLinearFunction.apply(self.config, input, weight, self.bias)
 
-    def _one_call_forward_applies(self, input: torch.Tensor) -> bool:
+    def _one_call_forward_applies(self, input: torch.Tensor, w: QuantizedTensor | nn.Parameter | None = None) -> bool:
         """Inference on a packed NVFP4 weight with the plain activation settings (NVFP4, 1-D blocks, round to
         nearest): the case `fos_linear_forward` covers. Everything else (training, master weights, other formats,
         fake quantization) goes through the autograd function."""
@@ -219,40 +220,39 @@ class FourOverSixLinear(nn.Linear):
                 or cfg.matmul_backend not in (None, MatmulBackend.cutlass)
                 or cfg.quantize_backend not in (None, QuantizeBackend.cuda)):
             return False
-        if (torch.is_grad_enabled() and input.requires_grad) or not input.is_cuda:
+        if (input.requires_grad and torch.is_grad_enabled()) or not input.is_cuda:
             return False
         if input.dtype not in (torch.bfloat16, torch.float16) or input.shape[-1] != self.in_features or input.numel() == 0:
             return False
-        w = self.quantized_weight()
+        w = self.quantized_weight() if w is None else w
         return (isinstance(w, QuantizedTensor) and w.dtype == DataType.nvfp4 and w.scale_factors_are_in_blackwell_layout
                 and w.round_style != RoundStyle.stochastic_unbiased and w.values.is_contiguous()
                 and w.scale_factors.is_contiguous())
 
-    def _forward_one_call(self, input: torch.Tensor) -> torch.Tensor:
-        """`fos_linear_forward`: amax pass, activation quantization, alpha and the GEMM enqueued by one host call
+    def _forward_one_call(self, input: torch.Tensor, w: QuantizedTensor) -> torch.Tensor:
+        """`fos_linear_forward`: amax pass, activation quantization and the GEMM enqueued by one host call
         (the bits of `quantized_matmul(input, weight)`; at decode sizes the call-by-call form is bound by the
         interpreter)."""
-        w = self.quantized_weight()
-        x = input.reshape(-1, self.in_features)
+        x = input if input.dim() == 2 else input.reshape(-1, self.in_features)
         if x.stride(-1) != 1:
             x = x.contiguous()
-        dev, rows = x.device, x.shape[0]
+        dev, rows, out_features = x.device, x.shape[0], self.out_features
         out_dtype = _TORCH_OUT[DataType(self.config.output_dtype)]
         lib = _native.lib()
         need = lib.fos_linear_workspace_bytes(rows, self.in_features)
         workspace = torch.empty(need, dtype=torch.uint8, device=dev)
-        out = torch.empty(rows, self.out_features, dtype=out_dtype, device=dev)
-        def launch() -> None:
-            _native.check(lib.fos_linear_forward(
+        out = torch.empty(rows, out_features, dtype=out_dtype, device=dev)
+        # the GEMM adds the bias where nothing has to be recorded for it and the sum is of the output's type
+        bias = self.bias
+        fused = (bias is not None and bias.dtype == out_dtype != torch.float32 and bias.device == dev
+                 and bias.is_contiguous() and not (bias.requires_grad and torch.is_grad_enabled()))
+        with _native.on_device(dev):
+            _native.check(lib.fos_linear_forward_bias(
                 x.data_ptr(), _native.elem_code(x.dtype), rows, self.in_features, x.stride(0),
                 self.config.activation_scale_rule.cuda_id, w.values.data_ptr(), w.scale_factors.data_ptr(),
-                w.amax.data_ptr(), w.scale_rule.cuda_id, self.out_features, out.data_ptr(), _native.elem_code(out_dtype),
-                out.stride(0), workspace.data_ptr(), need, None, 0, _native.stream_ptr(dev)), "fos_linear_forward")
-
-        if dev.index is None or dev.index == torch.cuda.current_device():
-            launch()                                  # (entering a device context costs microseconds a decode step feels)
-        else:
-            with torch.cuda.device(dev):
-                launch()
-        out = out.reshape(*input.shape[:-1], self.out_features)
-        return out if self.bias is None else out + self.bias
+                w.amax.data_ptr(), w.scale_rule.cuda_id, out_features, bias.data_ptr() if fused else 0, out.data_ptr(),
+                _native.elem_code(out_dtype), out.stride(0), workspace.data_ptr(), need, None, 0, _native.stream_ptr(dev)),
+                "fos_linear_forward_bias")
+        if input.dim() != 2:
+            out = out.reshape(*input.shape[:-1], out_features)
+        return out if bias is None or fused else out + bias

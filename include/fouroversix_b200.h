@@ -189,9 +189,9 @@ int fos_gemm_nvfp4(const uint8_t *a_codes, const uint8_t *a_sf, const uint8_t *b
 /*
  * Per-call options of the FP4 GEMMs (the library keeps no process-wide settings). NULL = all zero.
  *   variant   0 = choose the kernel per problem; 128 / 256 = single-CTA kernel with 128 x 128 /
- *             128 x 256 tiles; 2 = CTA-pair kernel (256 x 256 tiles, cta_group::2) where the padded
- *             M and N are multiples of 256, else the single-CTA kernel. Every variant computes the
- *             same product (fp32 sums in a different order).
+ *             128 x 256 tiles; 2 = CTA-pair kernel (256 x 256 tiles, cta_group::2; any size). Every
+ *             variant computes the same product; at most 32 rows of A take, with 0, a kernel that
+ *             splits K (fp32 sums in a different, fixed order).
  *   max_ctas  0 = one persistent CTA per SM; n > 0 = at most n CTAs, which leaves SMs free for a
  *             kernel that must run beside the GEMM (a collective on another stream: a persistent
  *             grid over every SM would keep it waiting until the GEMM has finished).
@@ -227,12 +227,24 @@ int fos_gemm_nvfp4_fused_a(const void *x, int x_dtype, int64_t x_ld, const float
                            int out_dtype, int64_t m, int64_t n_p, int64_t k, int64_t n, int64_t ldd,
                            int32_t *status, void *stream);
 
+/* fos_gemm_alpha_ex and fos_gemm_nvfp4_ex in one launch: alpha = amax_a * amax_b / denominator(rules) is formed in the
+ * GEMM, by the same operations. */
+int fos_gemm_nvfp4_scaled(const uint8_t *a_codes, const uint8_t *a_sf, const float *amax_a, int rule_a, int unbiased_a,
+                          const uint8_t *b_codes, const uint8_t *b_sf, const float *amax_b, int rule_b, int unbiased_b,
+                          void *d, int out_dtype, int64_t m_p, int64_t n_p, int64_t k_p, int64_t m, int64_t n,
+                          int64_t ldd, const fos_gemm_opts *opts, int32_t *status, void *stream);
+
+/* fos_gemm_mxfp4_ex with alpha = 1, which is what two MXFP4 tensors need (they have no per-tensor scale). */
+int fos_gemm_mxfp4_unscaled(const uint8_t *a_codes, const uint8_t *a_sf, const uint8_t *b_codes, const uint8_t *b_sf,
+                            void *d, int out_dtype, int64_t m_p, int64_t n_p, int64_t k_p, int64_t m, int64_t n,
+                            int64_t ldd, const fos_gemm_opts *opts, int32_t *status, void *stream);
+
 /*
  * A linear layer's forward pass on a packed weight as ONE host call: out[rows, out_features] = Q(x) @ W^T with x
  * [rows, in_features] (bf16 / fp16, row stride ld_x) quantized here (NVFP4, 1-D blocks, `activation_rule`, its amax
  * computed by the library) and W packed beforehand by fos_quantize (NVFP4, tiled scales, `weight_rule`, padded to
- * 128 rows and 64 columns). Enqueues what fos_quantize, fos_gemm_alpha and fos_gemm_nvfp4_ex enqueue, with the
- * packed activation, its amax and alpha in `workspace` (fos_linear_workspace_bytes(rows, in_features) bytes of
+ * 128 rows and 64 columns). Computes what fos_quantize, fos_gemm_alpha and fos_gemm_nvfp4_ex compute, with the
+ * packed activation and its amax in `workspace` (fos_linear_workspace_bytes(rows, in_features) bytes of
  * device memory, 256-byte aligned): same bits as the three calls. opts may be NULL; status as for fos_gemm_nvfp4.
  *
  * Replaces: FourOverSixLinearFunction.forward of src/fouroversix/model/modules/linear.py:40-110 for packed weights
@@ -243,6 +255,14 @@ int fos_linear_forward(const void *x, int x_dtype, int64_t rows, int64_t in_feat
                        const uint8_t *w_codes, const uint8_t *w_sf, const float *w_amax, int weight_rule,
                        int64_t out_features, void *out, int out_dtype, int64_t ld_out, void *workspace,
                        int64_t workspace_bytes, const fos_gemm_opts *opts, int32_t *status, void *stream);
+
+/* The same with the layer's bias [out_features] (of the output's type, bf16 / fp16; NULL: none) added to the rounded
+ * product, as a separate 16-bit addition would. FOS_ERR_UNSUPPORTED for a bias with fp32 output. */
+int fos_linear_forward_bias(const void *x, int x_dtype, int64_t rows, int64_t in_features, int64_t ld_x,
+                            int activation_rule, const uint8_t *w_codes, const uint8_t *w_sf, const float *w_amax,
+                            int weight_rule, int64_t out_features, const void *bias, void *out, int out_dtype,
+                            int64_t ld_out, void *workspace, int64_t workspace_bytes, const fos_gemm_opts *opts,
+                            int32_t *status, void *stream);
 
 /*
  * Grouped problems in one launch: num_groups GEMMs that share n, k and the output type, each with its own A rows,
