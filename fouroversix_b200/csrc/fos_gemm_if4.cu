@@ -19,7 +19,7 @@
 // extra HBM traffic but decodes every element once rather than once per tile that uses it.
 #include <mutex>
 
-#include "fos_tcgen05.cuh"
+#include "fos_pair.cuh"
 
 namespace fos {
 namespace {
@@ -171,8 +171,8 @@ struct F16GemmParams {
 
 // kind::f16 instruction descriptor: fp32 accumulate (1 in bits [4,6)), A and B fp16 (0 in [7,10) and
 // [10,13)), both K-major, N >> 3 in [17,23), M >> 4 in [24,29).
-__device__ __forceinline__ uint32_t f16_idesc(int n) {
-    return (1u << 4) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(BLOCK_M >> 4) << 24);
+__device__ __forceinline__ uint32_t f16_idesc(int n, int m = BLOCK_M) {
+    return (1u << 4) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
 }
 __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                            uint32_t accumulate) {
@@ -274,7 +274,6 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                 const uint32_t s = it % STAGES, ph = (it / STAGES) & 1u;
                 ok = __all_sync(0xffffffffu, mbar_wait(full_bar + 8 * s, ph, abort_flag, p.status, 2));
                 if (!ok) break;
-                tc_fence_after();
                 const uint32_t stage = smem_base + s * STAGE_BYTES;
                 const uint64_t a_desc = smem_desc(stage, 16, 1024, 2), b_desc = smem_desc(stage + A_BYTES, 16, 1024, 2);
                 if (issue) {
@@ -333,17 +332,206 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     }
 }
 
+// ---------------------------------------------------------------------------- fp16 GEMM, CTA pairs
+//
+// The same product with cta_group::2 MMAs: two SMs compute a 256 x 256 tile, each fetching 128 rows of A and 128 rows of B
+// per stage of 64 values (32 KB) where the single-CTA kernel fetches 48 KB for the same work, so seven stages fit
+// instead of four and the loads take a third less of the L2's bandwidth. Roles and barriers are those of the FP4 CTA-pair
+// kernel (fos_gemm_nvfp4.cu) without scales; two whole accumulators fit tensor memory.
+constexpr int PAIR_STAGES = 7;
+constexpr int PAIR_STAGE_BYTES = 2 * A_BYTES;
+constexpr int PAIR_SMEM_BYTES = PAIR_STAGES * PAIR_STAGE_BYTES + 1024 + 256;
+static_assert(PAIR_SMEM_BYTES <= 232448, "more shared memory than a CTA can have");
+
+__device__ __forceinline__ void tc_mma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                                uint32_t accumulate) {
+    asm volatile(
+        "{ .reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p; }\n"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+
 template <typename OUT>
-int launch_f16(const CUtensorMap &ma, const CUtensorMap &mb, const F16GemmParams &p, cudaStream_t stream) {
-    auto kernel = gemm_f16_kernel<OUT>;
-    static OncePerDevice configured;   // per instantiation
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                     const F16GemmParams p) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t *smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem_gen + PAIR_STAGES * PAIR_STAGE_BYTES);
+    const uint32_t full_bar = smem_u32(bars);                              // [PAIR_STAGES], used in the leader only
+    const uint32_t empty_bar = full_bar + 8 * PAIR_STAGES;                 // [PAIR_STAGES]
+    const uint32_t acc_full_bar = empty_bar + 8 * PAIR_STAGES;             // [ACC_STAGES]
+    const uint32_t acc_empty_bar = acc_full_bar + 8 * ACC_STAGES;          // [ACC_STAGES], used in the leader only
+    const uint32_t drain_bar = acc_empty_bar + 8 * ACC_STAGES;             // only used when the leader gives up
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * PAIR_STAGES + 2 * ACC_STAGES + 1);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_cta_rank();                              // 0 = leader
+    const bool leader = rank == 0;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < PAIR_STAGES; ++s) {
+            mbar_init(full_bar + 8 * s, 1);
+            mbar_init(empty_bar + 8 * s, 1);
+        }
+        for (int a = 0; a < ACC_STAGES; ++a) {
+            mbar_init(acc_full_bar + 8 * a, 1);
+            mbar_init(acc_empty_bar + 8 * a, 2 * EPI_WARPS);
+        }
+        mbar_init(drain_bar, 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 1) {
+        __syncwarp();
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
+                     ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();            // both CTAs have initialised their barriers and tensor memory
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    // (the second half of a tile may lie beyond the operands: zero-filled by the copies, not stored)
+    const int64_t num_m = (p.m_p + 255) / 256, num_n = (p.n_p + 255) / 256;
+    const int64_t num_tiles = num_m * num_n;
+    const int k_tiles = static_cast<int>(p.k_p / 64);
+    const int64_t pair_id = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
+
+    if (warp == 0) {
+        // ------------------------------------------------------------------ TMA producer (both CTAs)
+        const bool issue = elect_one();
+        const uint32_t leader_full = map_to_cta(full_bar, 0);
+        asm volatile("griddepcontrol.wait;" ::: "memory");     // the expanded operands
+        uint32_t s = 0, ph = 0;
+        bool ok = true;
+        for (int64_t t = pair_id; t < num_tiles && ok; t += num_pairs) {
+            int64_t mb, nb;
+            tile_coords(t, num_m, num_n, mb, nb);
+            const int m0 = static_cast<int>(mb * 256 + rank * 128), n0 = static_cast<int>(nb * 256 + rank * 128);
+            for (int kt = 0; kt < k_tiles; ++kt) {
+                ok = __all_sync(0xffffffffu, mbar_wait(empty_bar + 8 * s, ph ^ 1u, abort_flag, p.status, 1));
+                if (!ok) break;
+                const uint32_t stage = smem_base + s * PAIR_STAGE_BYTES, bar = leader_full + 8 * s;
+                if (issue) {
+                    if (leader) mbar_expect_tx(full_bar + 8 * s, 2 * PAIR_STAGE_BYTES);      // the bytes of both CTAs
+                    pair::tma_load_2d_pair(stage, &map_a, kt * BLOCK_K_BYTES, m0, bar);
+                    pair::tma_load_2d_pair(stage + A_BYTES, &map_b, kt * BLOCK_K_BYTES, n0, bar);
+                }
+                __syncwarp();
+                if (++s == PAIR_STAGES) { s = 0; ph ^= 1u; }
+            }
+        }
+        // the leader's last releases arrive in both CTAs' shared memory: stay until they have
+        for (int i = 0; i < PAIR_STAGES && ok; ++i) {
+            ok = __all_sync(0xffffffffu, mbar_wait(empty_bar + 8 * s, ph ^ 1u, abort_flag, p.status, 7));
+            if (++s == PAIR_STAGES) { s = 0; ph ^= 1u; }
+        }
+        if (!ok) {
+            const unsigned long long t0 = global_timer_ns();
+            while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
+        }
+    } else if (warp == 1 && leader) {
+        // ------------------------------------------------------------------ MMA issuer, for both CTAs
+        const bool issue = elect_one();
+        const uint32_t idesc = f16_idesc(256, 256);
+        uint32_t s = 0, ph = 0, tile_i = 0;
+        bool ok = true;
+        for (int64_t t = pair_id; t < num_tiles && ok; t += num_pairs, ++tile_i) {
+            const uint32_t acc = tile_i % ACC_STAGES, acc_ph = (tile_i / ACC_STAGES) & 1u;
+            ok = __all_sync(0xffffffffu, mbar_wait(acc_empty_bar + 8 * acc, acc_ph ^ 1u, abort_flag, p.status, 3));
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t d_tmem = tmem_base + acc * 256;
+            for (int kt = 0; kt < k_tiles; ++kt) {
+                ok = __all_sync(0xffffffffu, mbar_wait(full_bar + 8 * s, ph, abort_flag, p.status, 2));
+                if (!ok) break;
+                const uint32_t stage = smem_base + s * PAIR_STAGE_BYTES;
+                const uint64_t a_desc = smem_desc(stage, 16, 1024, 2), b_desc = smem_desc(stage + A_BYTES, 16, 1024, 2);
+                if (issue) {
+#pragma unroll
+                    for (int j = 0; j < MMAS_PER_STAGE; ++j)
+                        tc_mma_f16_pair(d_tmem, a_desc + 2 * j, b_desc + 2 * j, idesc, (kt > 0 || j > 0) ? 1u : 0u);
+                    tc_commit_pair(empty_bar + 8 * s);
+                }
+                __syncwarp();
+                if (++s == PAIR_STAGES) { s = 0; ph ^= 1u; }
+            }
+            if (ok && issue) tc_commit_pair(acc_full_bar + 8 * acc);
+        }
+        if (!ok) {
+            // giving up: the MMAs already issued must have finished before tensor memory is released
+            if (issue) pair::tc_commit_pair_local(drain_bar);
+            __syncwarp();
+            const long long t0 = clock64();
+            while (!mbar_try_wait(drain_bar, 0) && clock64() - t0 < 20000000ll) {}   // about 10 ms
+        }
+    } else if (warp >= 2) {
+        // ------------------------------------------------------------------ epilogue (both CTAs)
+        const int quad = warp & 3, half = (warp - 2) >> 2;
+        asm volatile("griddepcontrol.wait;" ::: "memory");     // alpha, and whoever still reads d
+        const float alpha = __ldg(p.alpha);
+        OUT *out = static_cast<OUT *>(p.d);
+        const bool vec16 = (reinterpret_cast<uintptr_t>(out) % 16 == 0) && ((p.ldd * sizeof(OUT)) % 16 == 0);
+        const bool vec32 = (reinterpret_cast<uintptr_t>(out) % 32 == 0) && ((p.ldd * sizeof(OUT)) % 32 == 0);
+        const uint32_t leader_acc_empty = map_to_cta(acc_empty_bar, 0);
+        uint32_t tile_i = 0;
+        bool ok = true;
+        for (int64_t t = pair_id; t < num_tiles && ok; t += num_pairs, ++tile_i) {
+            int64_t mb, nb;
+            tile_coords(t, num_m, num_n, mb, nb);
+            const int64_t row = mb * 256 + rank * 128 + quad * 32 + lane, n0 = nb * 256 + half * 128;
+            const uint32_t acc = tile_i % ACC_STAGES, acc_ph = (tile_i / ACC_STAGES) & 1u;
+            // (in the peer this barrier is arrived on from the leader's SM: one lane polls for the warp)
+            if (lane == 0) ok = mbar_wait_poll(acc_full_bar + 8 * acc, acc_ph, abort_flag, p.status, 4);
+            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * 256 + half * 128;
+            OUT *dst = out + row * p.ldd + n0;
+            const int64_t left = row < p.m ? p.n - n0 : 0;
+#pragma unroll
+            for (int c = 0; c < 128; c += 32) {
+                uint32_t v[32];
+                tc_load_32cols_sync(t_acc + c, v);
+                if (c == 96) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(leader_acc_empty + 8 * acc);
+                }
+                pair::store_columns<OUT, 32>(dst + c, v, alpha, nullptr, left - c, vec32, vec16);
+            }
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();            // nobody leaves while the peer may still touch this CTA's memory
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    }
+}
+
+template <typename OUT>
+int launch_f16(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mb_pair, const F16GemmParams &p, cudaStream_t stream) {
     int dev = 0, sms = 0;
     FOS_CUDA_TRY(cudaGetDevice(&dev));
+    FOS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const int64_t tiles = (p.m_p / BLOCK_M) * ((p.n_p + BLOCK_N - 1) / BLOCK_N);
+    const int64_t pair_tiles = ((p.m_p + 255) / 256) * ((p.n_p + 255) / 256);
+    if (pairs_pay(tiles, pair_tiles, sms))
+        return pair::launch(gemm_f16_pair_kernel<OUT>, THREADS, PAIR_SMEM_BYTES, pair_tiles, 0, stream, ma, mb_pair, p);
+    auto kernel = gemm_f16_kernel<OUT>;
+    static OncePerDevice configured;   // per instantiation
     FOS_CUDA_TRY(configured.run(dev, [&] {
         return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     }));
-    FOS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    const int64_t tiles = (p.m_p / BLOCK_M) * ((p.n_p + BLOCK_N - 1) / BLOCK_N);
     const unsigned grid = static_cast<unsigned>(tiles < sms ? tiles : sms);
     kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(ma, mb, p);
     FOS_CUDA_TRY(cudaGetLastError());
@@ -390,18 +578,19 @@ int gemm_if4_impl(const uint8_t *a_codes, const uint8_t *a_sf, int a_format, int
     int st;
     if ((st = launch_expand(a_codes, a_sf, a_format, a_sf_layout, m_p, k_p, a16, stream)) != FOS_OK) return st;
     if ((st = launch_expand(b_codes, b_sf, b_format, b_sf_layout, n_p, k_p, b16, stream)) != FOS_OK) return st;
-    CUtensorMap map_a, map_b;
+    CUtensorMap map_a, map_b, map_b_pair;
     if ((st = make_operand_map(&map_a, a16, m_p, k_p * 2, BLOCK_M)) != FOS_OK) return st;
     if ((st = make_operand_map(&map_b, b16, n_p, k_p * 2, BLOCK_N)) != FOS_OK) return st;
+    if ((st = make_operand_map(&map_b_pair, b16, n_p, k_p * 2, 128)) != FOS_OK) return st;
     if (status) {
         FOS_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int32_t), stream));
     } else {
         FOS_CUDA_TRY(wait_failures_ptr(&status));   // the library's sticky word
     }
     F16GemmParams p{alpha, d, status, m_p, n_p, k_p, m, n, ldd};
-    if (out_dtype == FOS_BF16) return launch_f16<__nv_bfloat16>(map_a, map_b, p, stream);
-    if (out_dtype == FOS_FP16) return launch_f16<__half>(map_a, map_b, p, stream);
-    return launch_f16<float>(map_a, map_b, p, stream);
+    if (out_dtype == FOS_BF16) return launch_f16<__nv_bfloat16>(map_a, map_b, map_b_pair, p, stream);
+    if (out_dtype == FOS_FP16) return launch_f16<__half>(map_a, map_b, map_b_pair, p, stream);
+    return launch_f16<float>(map_a, map_b, map_b_pair, p, stream);
 }
 
 int check_gemm_if4_args(const uint8_t *a_codes, const uint8_t *a_sf, int a_format, int a_sf_layout,
