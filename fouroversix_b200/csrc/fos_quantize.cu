@@ -54,6 +54,7 @@ struct QuantParams {
     float fake_divisor;
     // grouped launch (TMA-fed row kernels, grid.y = group): group g is rows group_start[g] .. group_start[g + 1]
     // (device values, multiples of 128) of x and of the outputs, quantized as a tensor of its own with amax[g]
+    const int32_t *rows_in_use;   // of each group: its rows beyond these may be left alone (quantize_rows_mse_kernel); or nullptr
     const int32_t *group_start;
     int num_groups;
 };
@@ -1189,8 +1190,8 @@ constexpr int FEED_SMEM_BYTES = FEED_STAGES * FEED_STAGE_BYTES + 1024;
 // EXTRAS: the instantiation that can rotate blocks (random Hadamard transform) and round
 // stochastically; the plain one carries neither code path, which keeps its register count down.
 // Grouped launch: the tile rows of group blockIdx.y and its amax word. (The row ranges come from device
-// memory that earlier work in the stream wrote; grouped launches are ordinary launches, not programmatic
-// dependents, so that work is complete.) Ranges are clipped to the buffers.
+// memory that earlier work in the stream wrote: a grouped launch waits for it before anything else.) Ranges are clipped to
+// the buffers.
 __device__ __forceinline__ void group_tiles(const QuantParams &p, int &tile_r0, int &tiles_r, const float *&amax_ptr) {
     const int all = static_cast<int>(p.rows_p >> 7);
     int t0 = __ldg(p.group_start + blockIdx.y) >> 7, t1 = __ldg(p.group_start + blockIdx.y + 1) >> 7;
@@ -1218,7 +1219,10 @@ quantize_rows_tma_kernel(const __grid_constant__ CUtensorMap map_x, const QuantP
     const int tiles_c = static_cast<int>(p.cols_p >> 6);
     int tiles_r = static_cast<int>(p.rows_p >> 7), tile_r0 = 0;
     const float *amax_ptr = p.amax;
-    if (!FAKE && p.group_start != nullptr) group_tiles(p, tile_r0, tiles_r, amax_ptr);
+    if (!FAKE && p.group_start != nullptr) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");      // the row ranges, x and amax come from earlier kernels
+        group_tiles(p, tile_r0, tiles_r, amax_ptr);
+    }
     const int64_t n_tiles = static_cast<int64_t>(tiles_c) * tiles_r;
 
     if (threadIdx.x == 0) {
@@ -1469,7 +1473,14 @@ template <typename T> __device__ __forceinline__ void unpack2_fma(uint32_t w, fl
     hi = f.y;
 }
 
-template <typename T>
+__device__ __forceinline__ int rows_in_use_at(const int *tile_rows, uint32_t stage) {
+    int rows;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(rows) : "r"(smem_u32(tile_rows) + 4 * stage));
+    return rows;
+}
+
+// IN_USE: a grouped launch whose rows beyond the group's rows in use come out as anything; warps without others skip them.
+template <typename T, bool IN_USE = false>
 __global__ void __launch_bounds__(FEED_THREADS, FOS_FEED_CTAS)
 quantize_rows_mse_kernel(const __grid_constant__ CUtensorMap map_x, const QuantParams p) {
     extern __shared__ uint8_t feed_smem_raw[];
@@ -1477,6 +1488,7 @@ quantize_rows_mse_kernel(const __grid_constant__ CUtensorMap map_x, const QuantP
     __shared__ __align__(16) float coop[FEED_CONSUMERS / 32][20];
     __shared__ __align__(16) longlong2 tile_meta[FEED_STAGES];     // per stage: byte offsets of the tile's codes and scales
     __shared__ __align__(8) uint64_t full_bar[FEED_STAGES], empty_bar[FEED_STAGES];
+    __shared__ int tile_rows[IN_USE ? FEED_STAGES : 1];            // rows in use from the tile's first on
     __shared__ int abort_flag;
 
     const uint32_t stage0 = (smem_u32(feed_smem_raw) + 1023u) & ~1023u;
@@ -1484,7 +1496,10 @@ quantize_rows_mse_kernel(const __grid_constant__ CUtensorMap map_x, const QuantP
     const int tiles_c = static_cast<int>(p.cols_p >> 6);
     int tiles_r = static_cast<int>(p.rows_p >> 7), tile_r0 = 0;
     const float *amax_ptr = p.amax;
-    if (p.group_start != nullptr) group_tiles(p, tile_r0, tiles_r, amax_ptr);
+    if (p.group_start != nullptr) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");      // the row ranges, x and amax come from earlier kernels
+        group_tiles(p, tile_r0, tiles_r, amax_ptr);
+    }
     const int64_t n_tiles = static_cast<int64_t>(tiles_c) * tiles_r;
     const int64_t code_ld = p.cols_p >> 1, n_cb = p.cols_p >> 4;
 
@@ -1517,6 +1532,7 @@ quantize_rows_mse_kernel(const __grid_constant__ CUtensorMap map_x, const QuantP
             // (the arrive below releases this store to the consumers that acquire the barrier's phase)
             tile_meta[s] = make_longlong2(static_cast<int64_t>(tr) * 128 * code_ld + tc_ * 32,
                                           p.sf_tiled ? tile * 512 : static_cast<int64_t>(tr) * 128 * n_cb + tc_ * 4);
+            if constexpr (IN_USE) tile_rows[s] = __ldg(p.rows_in_use + blockIdx.y) - (tr - tile_r0) * FEED_TILE_ROWS;
             mbar_expect_tx(smem_u32(&full_bar[s]), FEED_STAGE_BYTES);
             tma_load_2d(stage0 + s * FEED_STAGE_BYTES, &map_x, tc_ * 128, tr * FEED_TILE_ROWS, smem_u32(&full_bar[s]));
             if (++s == FEED_STAGES) { s = 0; parity ^= 1u; }
@@ -1563,8 +1579,10 @@ quantize_rows_mse_kernel(const __grid_constant__ CUtensorMap map_x, const QuantP
         asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(code_off), "=l"(sf_off) : "r"(meta_addr + 16 * s_idx));
         uint8_t *codes = code_ptr + code_off;
         uint8_t *sf = sf_ptr + sf_off;
+        // (the tile's rows in use are read where they are needed: a register kept for them would spill)
+        const bool any_in_use = !IN_USE || warp * 8 < rows_in_use_at(tile_rows, s_idx);
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
+        for (int j = 0; j < 2 && any_in_use; ++j) {
             const uint4 a = lds_16(piece0 + s_off + j * 64 * 128);
             const uint4 b = lds_16(piece1 + s_off + j * 64 * 128);
             const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
@@ -1606,7 +1624,9 @@ quantize_rows_mse_kernel(const __grid_constant__ CUtensorMap map_x, const QuantP
             const bool pick_fast = diff < 0.0f;
             uint32_t lo = pick_fast ? cbk[0] : ca[0], hi = pick_fast ? cbk[1] : ca[1];
             uint32_t sf_byte = pick_fast ? both >> 8 : both & 0xffu;
-            const bool undecided = !(fabsf(diff) > tau);
+            bool undecided = !(fabsf(diff) > tau);
+            // (whatever a row beyond holds, it must not send the warp through the exact sequence)
+            if constexpr (IN_USE) undecided = undecided && row_in_tile + 64 * j < rows_in_use_at(tile_rows, s_idx);
             if (__any_sync(FULL, undecided)) {
                 // Undecided blocks whose scales the pre-filter accepts (two normal E4M3 numbers) are
                 // re-decided exactly by the whole warp, one block at a time; the others (zero or
@@ -1793,7 +1813,7 @@ inline bool make_x_map(CUtensorMap *map, const QuantParams &p, bool transposed) 
 }
 
 // Launches the TMA-fed kernel when x qualifies; *launched tells whether it did.
-template <typename T, int KIND, bool TRANSPOSED, bool FAKE, bool TWO_D, bool EXTRAS, bool LEAN = false>
+template <typename T, int KIND, bool TRANSPOSED, bool FAKE, bool TWO_D, bool EXTRAS, int LEAN = 0>
 cudaError_t launch_rows_tma_impl(const QuantParams &p, cudaStream_t stream, bool *launched) {
     *launched = false;
     if (reinterpret_cast<uintptr_t>(p.x) % 16 != 0 || (p.ld * 2) % 16 != 0) return cudaSuccess;
@@ -1802,7 +1822,8 @@ cudaError_t launch_rows_tma_impl(const QuantParams &p, cudaStream_t stream, bool
     if (p.cols * 2 >= (int64_t(1) << 31) || p.rows >= (int64_t(1) << 31) || p.ld * 2 >= (int64_t(1) << 40)) return cudaSuccess;
     CUtensorMap map;
     if (!make_x_map(&map, p, TRANSPOSED)) return cudaSuccess;
-    auto kernel = LEAN ? quantize_rows_mse_kernel<T>
+    // LEAN: 1 = the kernel of the default configuration, 2 = that for grouped launches that pack the rows in use only
+    auto kernel = LEAN ? quantize_rows_mse_kernel<T, LEAN == 2>
                        : (TRANSPOSED ? quantize_cols_tma_kernel<T, KIND, TWO_D, EXTRAS> : quantize_rows_tma_kernel<T, KIND, FAKE, TWO_D, EXTRAS>);
     static int ctas_per_sm[64] = {};
     static int sm_count[64] = {};
@@ -1840,7 +1861,7 @@ cudaError_t launch_rows_tma_impl(const QuantParams &p, cudaStream_t stream, bool
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = grouped ? 0 : 1;      // (a grouped launch reads row ranges written by earlier work: a full dependency)
+    cfg.numAttrs = 1;
     e = cudaLaunchKernelEx(&cfg, kernel, map, p);
     if (e == cudaSuccess) *launched = true;
     return e;
@@ -1861,7 +1882,7 @@ cudaError_t launch_rows(const QuantParams &p, cudaStream_t stream) {
         if constexpr (KIND == KIND_ADAPTIVE) {
             // the default configuration (mean-squared error, round to nearest, no rotation) has a kernel of its own
             if (p.rule == FOS_RULE_MSE && !p.rht && !p.stochastic && p.variant != 2) {
-                const cudaError_t e = launch_rows_tma_impl<T, KIND, false, false, false, false, true>(p, stream, &launched);
+                const cudaError_t e = launch_rows_tma_impl<T, KIND, false, false, false, false, 1>(p, stream, &launched);
                 if (e != cudaSuccess || launched) return e;
             }
         }
@@ -1897,6 +1918,143 @@ cudaError_t launch_rows(const QuantParams &p, cudaStream_t stream) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, p);
+}
+
+// ------------------------------------------------------------------------------------
+// small tensors: amax and quantization in one launch
+// ------------------------------------------------------------------------------------
+//
+// A decoding step packs a few rows (16 x 8192: 256 KB), and the three launches of the general chain (zero the amax
+// word, amax pass, quantize kernel) cost more than the work. Here one cluster of 16 CTAs holds the whole tensor in
+// shared memory: every thread loads its blocks of 16 values once, the CTAs exchange their maxima through distributed
+// shared memory, and the blocks are quantized from shared memory; then the padding is filled in. Bound by latency
+// (one round trip to memory, one cluster barrier, at most SMALL_BLOCKS blocks per thread in sequence); the limit on
+// the size is where the general chain, which has the whole chip, gets ahead.
+
+constexpr int SMALL_CTAS = 16, SMALL_THREADS = 512, SMALL_BLOCKS = 2;
+constexpr int64_t SMALL_MAX_BLOCKS = static_cast<int64_t>(SMALL_CTAS) * SMALL_THREADS * SMALL_BLOCKS;
+
+template <typename T, int KIND>
+__global__ void __launch_bounds__(SMALL_THREADS)
+quantize_small_kernel(const QuantParams p, float *amax_out) {
+    __shared__ __align__(16) uint4 words[SMALL_BLOCKS][2][SMALL_THREADS];
+    __shared__ float4 lut[128];
+    __shared__ __align__(16) float coop[SMALL_THREADS / 32][20];
+    __shared__ float warp_max[SMALL_THREADS / 32], cta_max[SMALL_CTAS];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t rank = cluster_cta_rank();
+    const int first = static_cast<int>(rank) * SMALL_THREADS + tid;
+    constexpr int STEP = SMALL_CTAS * SMALL_THREADS;
+    const int n_cb = static_cast<int>(p.cols_p >> 4), total = static_cast<int>(p.out_rows) * n_cb;
+
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // this CTA runs: its peers may write to it
+    // x, and whatever still reads the outputs of an earlier call; only then may the kernel behind this one start
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    float m = 0.0f;
+#pragma unroll
+    for (int j = 0; j < SMALL_BLOCKS; ++j) {
+        const int i = first + j * STEP;
+        uint32_t w[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+        if (i < total) load_block_words<T>(p, i / n_cb, i % n_cb, w);
+        const uint4 a = make_uint4(w[0], w[1], w[2], w[3]), b = make_uint4(w[4], w[5], w[6], w[7]);
+        words[j][0][tid] = a;
+        words[j][1][tid] = b;
+        m = fmaxf(m, fmaxf(abs_max8<T>(a), abs_max8<T>(b)));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(FULL, m, o));
+    if (lane == 0) warp_max[warp] = m;
+    __syncthreads();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (tid < SMALL_CTAS) {
+        m = warp_max[0];
+#pragma unroll
+        for (int w = 1; w < SMALL_THREADS / 32; ++w) m = fmaxf(m, warp_max[w]);
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(map_to_cta(smem_u32(&cta_max[rank]), tid)), "f"(m) : "memory");
+    }
+    cluster_sync_all();
+    m = cta_max[0];
+#pragma unroll
+    for (int c = 1; c < SMALL_CTAS; ++c) m = fmaxf(m, cta_max[c]);
+    const TensorConsts tc = tensor_consts<KIND>(m, p.rule);
+    if (rank == 0 && tid == 0) *amax_out = m;
+    if (tid < 128) lut[tid] = scale_entry(tid, tc, rule_has_filter<KIND, false>(p.rule) && !p.exact_only && tc.filter_ok);
+    __syncthreads();
+
+#pragma unroll 1
+    for (int j = 0; j < SMALL_BLOCKS; ++j) {
+        const int i = first + j * STEP;
+        if (i - lane >= total) break;                     // (whole warps: the undecided blocks are a warp's work)
+        const uint4 a = words[j][0][tid], b = words[j][1][tid];
+        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        float v[16];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const float2 f = unpack2<T>(w[k]);
+            v[2 * k] = f.x;
+            v[2 * k + 1] = f.y;
+        }
+        uint32_t lo, hi, sf_byte;
+        quantize_block<KIND, false, false>(v, tc, p.rule, p.exact_only != 0, nullptr, lane, lut, coop[warp], lo, hi, sf_byte);
+        if (i < total) {
+            const int64_t row = i / n_cb, cb = i % n_cb;
+            *reinterpret_cast<uint2 *>(p.codes + row * (p.cols_p >> 1) + cb * 8) = make_uint2(lo, hi);
+            p.sf[sf_offset(row, cb, n_cb, p.sf_tiled != 0)] = static_cast<uint8_t>(sf_byte);
+        }
+    }
+    // the padding rows: zero codes, zero scales
+    const int pad_rows = static_cast<int>(p.rows_p - p.out_rows);
+    uint8_t *pad = p.codes + p.out_rows * (p.cols_p >> 1);
+    for (int i = first; i < pad_rows * n_cb; i += STEP) *reinterpret_cast<uint2 *>(pad + static_cast<int64_t>(i) * 8) = make_uint2(0u, 0u);
+    const int quads = n_cb >> 2;
+    for (int i = first; i < pad_rows * quads; i += STEP) {
+        // four scales of a row lie side by side in either layout
+        uint8_t *at = p.sf + sf_offset(p.out_rows + i / quads, (i % quads) * 4, n_cb, p.sf_tiled != 0);
+        at[0] = at[1] = at[2] = at[3] = 0;
+    }
+}
+
+// True when the tensor qualifies (plain 1-D blocks whose amax this call computes, at most SMALL_MAX_BLOCKS blocks with
+// every thread's blocks in shared memory) and the device takes a cluster of 16 CTAs.
+template <typename T, int KIND>
+cudaError_t launch_small(const QuantParams &p, float *amax_out, cudaStream_t stream, bool *launched) {
+    *launched = false;
+    if (p.out_rows * (p.cols_p >> 4) > SMALL_MAX_BLOCKS) return cudaSuccess;
+    auto kernel = quantize_small_kernel<T, KIND>;
+    static OncePerDevice configured;
+    static int fits[64] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64) return cudaSuccess;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(SMALL_CTAS);
+    cfg.blockDim = dim3(SMALL_THREADS);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = SMALL_CTAS;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e = configured.run(dev, [&] {
+        cudaError_t r = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (r != cudaSuccess) return r;
+        int n = 0;
+        r = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
+        fits[dev] = r == cudaSuccess && n > 0;
+        return r;
+    });
+    if (e != cudaSuccess) return e;
+    if (!fits[dev]) return cudaSuccess;
+    cfg.numAttrs = 2;
+    e = cudaLaunchKernelEx(&cfg, kernel, p, amax_out);
+    if (e == cudaSuccess) *launched = true;
+    return e;
 }
 
 template <typename T, int KIND>
@@ -1951,6 +2109,13 @@ inline cudaLaunchConfig_t dependent_launch_config(unsigned grid, unsigned block,
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cfg;
+}
+
+template <typename T>
+cudaError_t launch_small_kind(const QuantParams &p, int kind, float *amax_out, cudaStream_t stream, bool *launched) {
+    if (kind == KIND_STATIC) return launch_small<T, KIND_STATIC>(p, amax_out, stream, launched);
+    if (kind == KIND_ADAPTIVE) return launch_small<T, KIND_ADAPTIVE>(p, amax_out, stream, launched);
+    return launch_small<T, KIND_IF4>(p, amax_out, stream, launched);
 }
 
 template <typename T>
@@ -2124,7 +2289,14 @@ static int quantize_entry(const void *x, int x_dtype, int64_t rows, int64_t cols
     const int64_t ld_bytes = ld * 2;
     p.vec_bytes = (addr % 32 == 0 && ld_bytes % 32 == 0) ? 32 : ((addr % 16 == 0 && ld_bytes % 16 == 0) ? 16 : 0);
     const bool vec16 = p.vec_bytes != 0 && cols % 8 == 0;
+    const int kind = format == FOS_IF4 ? KIND_IF4 : (is_static ? KIND_STATIC : KIND_ADAPTIVE);
 
+    if (!amax_in && !block_2d && !transpose && !p.rht && !stochastic && p.variant == 0) {
+        bool launched = false;
+        FOS_CUDA_TRY(x_dtype == FOS_BF16 ? launch_small_kind<__nv_bfloat16>(p, kind, amax_out, stream, &launched)
+                                         : launch_small_kind<__half>(p, kind, amax_out, stream, &launched));
+        if (launched) return FOS_OK;
+    }
     if (amax_in) {
         // the quantize kernel copies the value over: no separate copy operation in the stream
         p.amax = amax_in;
@@ -2140,7 +2312,6 @@ static int quantize_entry(const void *x, int x_dtype, int64_t rows, int64_t cols
     // pass: it does not write x, so x can be fetched while it drains.
     p.x_is_ready = amax_in == nullptr;
 
-    const int kind = format == FOS_IF4 ? KIND_IF4 : (is_static ? KIND_STATIC : KIND_ADAPTIVE);
     FOS_CUDA_TRY(x_dtype == FOS_BF16
                      ? launch_all<__nv_bfloat16>(p, kind, block_2d != 0, transpose != 0, stream)
                      : launch_all<__half>(p, kind, block_2d != 0, transpose != 0, stream));
@@ -2168,15 +2339,17 @@ template <typename T, int KIND>
 cudaError_t launch_rows_grouped(const fos::QuantParams &p, cudaStream_t stream, bool *launched) {
     using namespace fos;
     if constexpr (KIND == KIND_ADAPTIVE) {
-        if (p.rule == FOS_RULE_MSE && p.variant != 2) return launch_rows_tma_impl<T, KIND, false, false, false, false, true>(p, stream, launched);
+        if (p.rule == FOS_RULE_MSE && p.variant != 2)
+            return p.rows_in_use ? launch_rows_tma_impl<T, KIND, false, false, false, false, 2>(p, stream, launched)
+                                 : launch_rows_tma_impl<T, KIND, false, false, false, false, 1>(p, stream, launched);
     }
     return launch_rows_tma_impl<T, KIND, false, false, false, false>(p, stream, launched);
 }
 
-extern "C" int fos_quantize_grouped(const void *x, int x_dtype, int64_t rows_capacity, int64_t cols, int64_t ld, int format,
-                                    int scale_rule, const int32_t *group_start, const int32_t *group_rows, int num_groups,
-                                    const float *amax_in, uint8_t *codes, uint8_t *sf, float *amax_out, int flags,
-                                    void *stream_) {
+static int quantize_grouped_entry(const void *x, int x_dtype, int64_t rows_capacity, int64_t cols, int64_t ld, int format,
+                                  int scale_rule, const int32_t *group_start, const int32_t *group_rows, int num_groups,
+                                  const float *amax_in, uint8_t *codes, uint8_t *sf, float *amax_out, int flags, bool in_use_only,
+                                  void *stream_) {
     using namespace fos;
     if (!x || !codes || !sf || !amax_out || !group_start || !group_rows) return FOS_ERR_INVALID_ARGUMENT;
     if (num_groups <= 0 || num_groups > 65535) return FOS_ERR_INVALID_ARGUMENT;
@@ -2208,6 +2381,7 @@ extern "C" int fos_quantize_grouped(const void *x, int x_dtype, int64_t rows_cap
     p.vec_bytes = (reinterpret_cast<uintptr_t>(x) % 32 == 0 && (ld * 2) % 32 == 0) ? 32 : 16;
     p.x_is_ready = 1;
     p.group_start = group_start;
+    p.rows_in_use = in_use_only ? group_rows : nullptr;
     p.num_groups = num_groups;
     if (amax_in) {
         if (amax_in != amax_out)
@@ -2244,6 +2418,21 @@ extern "C" int fos_quantize_grouped(const void *x, int x_dtype, int64_t rows_cap
                                   : launch_rows_grouped<__half, KIND_ADAPTIVE>(p, stream, &launched);
     FOS_CUDA_TRY(e);
     return launched ? FOS_OK : FOS_ERR_UNSUPPORTED;
+}
+
+extern "C" int fos_quantize_grouped(const void *x, int x_dtype, int64_t rows_capacity, int64_t cols, int64_t ld, int format,
+                                    int scale_rule, const int32_t *group_start, const int32_t *group_rows, int num_groups,
+                                    const float *amax_in, uint8_t *codes, uint8_t *sf, float *amax_out, int flags,
+                                    void *stream) {
+    return quantize_grouped_entry(x, x_dtype, rows_capacity, cols, ld, format, scale_rule, group_start, group_rows, num_groups,
+                                  amax_in, codes, sf, amax_out, flags, false, stream);
+}
+
+int fos::quantize_grouped_rows_in_use(const void *x, int x_dtype, int64_t rows_capacity, int64_t cols, int64_t ld, int format,
+                                      int scale_rule, const int32_t *group_start, const int32_t *group_rows, int num_groups,
+                                      const float *amax_in, uint8_t *codes, uint8_t *sf, float *amax_out, int flags, void *stream) {
+    return quantize_grouped_entry(x, x_dtype, rows_capacity, cols, ld, format, scale_rule, group_start, group_rows, num_groups,
+                                  amax_in, codes, sf, amax_out, flags, true, stream);
 }
 
 extern "C" int fos_quantize(const void *x, int x_dtype, int64_t rows, int64_t cols, int64_t ld, int format,
