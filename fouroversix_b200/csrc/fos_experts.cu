@@ -38,6 +38,17 @@ template <> struct Half16<__half> {
         return *reinterpret_cast<uint32_t *>(&p);
     }
 };
+// Every kernel of the layer starts here. In the one-call form each is launched as the programmatic dependent of the one
+// before it: its CTAs may be placed while that one drains, and wait here before they touch memory. What came before
+// THAT one is then complete too, because it waited the same way. (Ordinary launches: both instructions do nothing.)
+__device__ __forceinline__ void chain_begin() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+constexpr int ROW_THREADS = 256;         // of the kernels that give a row to a warp
+constexpr int GATHER_CTAS = 6, GLU_CTAS = 4;     // their CTAs per SM (one wave: a warp takes rows in turn)
+
 template <typename P> __device__ __forceinline__ P as_pair(uint32_t w) { return *reinterpret_cast<P *>(&w); }
 template <typename P> __device__ __forceinline__ uint32_t as_word(P p) { return *reinterpret_cast<uint32_t *>(&p); }
 
@@ -57,50 +68,84 @@ template <typename P> __device__ __forceinline__ P fold_abs_max(P m, uint4 v) {
     return __hmax2(m, __habs2(as_pair<P>(v.w)));
 }
 
-// The CTA's maximum of the threads' packed running maxima, raised into amax[0] (a non-negative float, zeroed by the
+// The warp's maximum of the lanes' packed running maxima, raised into amax[0] (a non-negative float, zeroed by the
 // caller before the launch, compared as an integer). The words written are the ones the grouped amax pass would
-// write: the largest magnitude of the group's values, exactly, as a float. Called by all threads of the CTA.
+// write: the largest magnitude of the group's values, exactly, as a float. Called by all lanes of the warp.
 template <typename T>
-__device__ __forceinline__ void raise_amax(typename Half16<T>::Pair m2, float *amax, float *warp_max) {
+__device__ __forceinline__ void raise_amax(typename Half16<T>::Pair m2, float *amax, int lane) {
     using H = Half16<T>;
     float m = fmaxf(H::lo(as_word(m2)), H::hi(as_word(m2)));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    __syncthreads();                                      // the previous row's values have been read
-    if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < static_cast<int>(blockDim.x >> 5); ++w) m = fmaxf(m, warp_max[w]);
-        // (a stale smaller value read here only costs an atomic that changes nothing)
-        if (m > 0.0f && m > *reinterpret_cast<volatile float *>(amax)) atomicMax(reinterpret_cast<int *>(amax), __float_as_int(m));
-    }
+    // (a stale smaller value read here only costs an atomic that changes nothing)
+    if (lane == 0 && m > 0.0f && m > *reinterpret_cast<volatile float *>(amax)) atomicMax(reinterpret_cast<int *>(amax), __float_as_int(m));
 }
 
-// out[r] = x[row_token[r]], or zeros where row_token[r] < 0. One CTA per row at a time, 16 bytes per thread.
+// The two row kernels below give a warp a row, or (few rows) a segment of one: a row is a few KB, so its own latency (look
+// up the row, fetch it, reduce) dominates, and warps that do not wait for one another overlap theirs. A unit of work is
+// (row, segment); in the one-call form of the layer the rows are taken in the order of the (token, slot) pairs, which
+// visits the rows in use only - of 256 tokens over 32 experts a quarter of the padded buffer - and leaves the padding
+// rows as they are: no row of a product depends on another, and nobody reads those.
+struct RowUnits {
+    int rows, segs, seg_chunks;            // rows (or pairs), segments per row, 16-byte pieces per segment
+    const int32_t *pair_row, *pair_expert; // pair order: the pairs' rows (-1: none) and experts; nullptr: row order
+    int top_k;
+};
+
+// out[r] = x[row_token[r]], or zeros where row_token[r] < 0, 16 bytes per lane and piece.
 // With amax != nullptr also amax[row_expert[r]] = max(amax[..], max |out[r]|): the per-expert maxima the grouped
 // quantization of `out` needs, so that it can skip its own pass over the buffer.
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(ROW_THREADS, GATHER_CTAS)
 gather_rows_kernel(const uint8_t *__restrict__ x, int64_t ld_x_bytes, const int32_t *__restrict__ row_token,
-                   uint8_t *__restrict__ out, int64_t ld_out_bytes, int rows, int chunks,
+                   uint8_t *__restrict__ out, int64_t ld_out_bytes, const RowUnits units, int chunks,
                    const int32_t *__restrict__ row_expert, float *__restrict__ amax) {
+    chain_begin();
     using P = typename Half16<T>::Pair;
-    __shared__ float warp_max[8];
-    for (int r = blockIdx.x; r < rows; r += gridDim.x) {
-        const int t = __ldg(row_token + r);
-        const uint4 *src = reinterpret_cast<const uint4 *>(x + static_cast<int64_t>(t < 0 ? 0 : t) * ld_x_bytes);
+    const int lane = threadIdx.x & 31, warps = gridDim.x * (ROW_THREADS / 32), total = units.rows * units.segs;
+    for (int i = (blockIdx.x * ROW_THREADS + threadIdx.x) >> 5; i < total; i += warps) {
+        const int at = units.segs == 1 ? i : i / units.segs, seg = i - at * units.segs;
+        const int c_begin = seg * units.seg_chunks, c_end = min(chunks, c_begin + units.seg_chunks);
+        const int r = units.pair_row ? __ldg(units.pair_row + at) : at;
+        if (r < 0) continue;
+        const int t = units.pair_row ? at / units.top_k : __ldg(row_token + r);
         uint4 *dst = reinterpret_cast<uint4 *>(out + r * ld_out_bytes);
-        P m2 = as_pair<P>(0u);
-        for (int c = threadIdx.x; c < chunks; c += blockDim.x) {
-            const uint4 v = t < 0 ? make_uint4(0u, 0u, 0u, 0u) : __ldg(src + c);
-            dst[c] = v;
-            m2 = fold_abs_max<P>(m2, v);
+        if (t < 0) {
+            for (int c = c_begin + lane; c < c_end; c += 32) dst[c] = make_uint4(0u, 0u, 0u, 0u);
+            continue;
         }
-        if (amax != nullptr && t >= 0) raise_amax<T>(m2, amax + __ldg(row_expert + r), warp_max);
+        const uint4 *src = reinterpret_cast<const uint4 *>(x + static_cast<int64_t>(t) * ld_x_bytes);
+        P m2 = as_pair<P>(0u);
+        for (int c0 = c_begin + lane; c0 < c_end; c0 += 32 * 4) {             // four loads in flight per lane
+            uint4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = c0 + 32 * u < c_end ? __ldg(src + c0 + 32 * u) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (c0 + 32 * u < c_end) dst[c0 + 32 * u] = v[u];
+                m2 = fold_abs_max<P>(m2, v[u]);
+            }
+        }
+        __syncwarp();
+        if (amax != nullptr) raise_amax<T>(m2, amax + __ldg(units.pair_row ? units.pair_expert + at : row_expert + r), lane);
     }
 }
 
-// The reference's chain on one (gate, up) pair, every intermediate rounded to the 16-bit type:
+// 1 / (1 + expf(-t)) of two numbers, rounded to the 16-bit type (a packed pair). The fast functions give the quotient to
+// within (12 + 1.5 |t|) units of 2^-23 for |t| <= 64 (__expf: 2 + 1.173 |t| units in the last place by CUDA's own bound, the
+// addition and __fdividef 3, and the binary32 sequence itself is within 4 of the true value); where both ends of that
+// interval round to the same number, the binary32 sequence does too. The rest - a value within the interval of a
+// rounding boundary (one in 500 in bf16, one in 60 in fp16), a large |t|, NaN - runs the sequence itself.
+template <typename T> __device__ __forceinline__ uint32_t sigmoid16x2(float t0, float t1) {
+    using H = Half16<T>;
+    const float s0 = __fdividef(1.0f, 1.0f + __expf(-t0)), s1 = __fdividef(1.0f, 1.0f + __expf(-t1));
+    const float w0 = s0 * fmaf(fabsf(t0), 0x1.8p-23f, 0x1.8p-20f), w1 = s1 * fmaf(fabsf(t1), 0x1.8p-23f, 0x1.8p-20f);
+    const uint32_t low = H::pack(s0 - w0, s1 - w1), high = H::pack(s0 + w0, s1 + w1);
+    if (low == high && fmaxf(fabsf(t0), fabsf(t1)) <= 64.0f) return low;
+    return H::pack(1.0f / (1.0f + expf(-t0)), 1.0f / (1.0f + expf(-t1)));
+}
+
+// The reference's chain on two (gate, up) pairs, every intermediate rounded to the 16-bit type:
 //   g = gate + bias_g; u = up + bias_u; g = min(g, limit); u = min(max(u, -limit), limit)   (NaN passes through)
 //   out = (u + 1) * (g * sigmoid(g * alpha))
 // A (gate, up) pair is one 32-bit word, and a packed 16-bit addition, multiplication or fused multiply-add
@@ -112,57 +157,70 @@ gather_rows_kernel(const uint8_t *__restrict__ x, int64_t ld_x_bytes, const int3
 // comparing with r selects the same values as comparing with the limit itself, because no number of the type
 // lies between the two. Returns the output in the low half.
 template <typename T>
-__device__ __forceinline__ uint32_t glu_word(uint32_t gate_up, uint32_t bias, float alpha,
-                                             typename Half16<T>::Pair limit2, typename Half16<T>::Pair floor2,
-                                             typename Half16<T>::Pair tail2) {
+__device__ __forceinline__ uint32_t glu_words(uint32_t gate_up0, uint32_t gate_up1, uint32_t bias0, uint32_t bias1, float alpha,
+                                              typename Half16<T>::Pair limit2, typename Half16<T>::Pair floor2,
+                                              typename Half16<T>::Pair one2) {
     using H = Half16<T>;
     using P = typename H::Pair;
-    P v = __hadd2_rn(as_pair<P>(gate_up), as_pair<P>(bias));
-    v = __hmax2_nan(__hmin2_nan(v, limit2), floor2);
-    const float t = H::r16(H::lo(as_word(v)) * alpha);
-    const float s = 1.0f / (1.0f + expf(-t));
-    // (g, u) * (s, 1) + (-0, 1) = (g * s, u + 1): adding -0 keeps the sign of a zero product
-    const uint32_t s1 = (H::pack(s, 0.0f) & 0xffffu) | (as_word(tail2) & 0xffff0000u);
-    const P w = __hfma2(v, as_pair<P>(s1), as_pair<P>((as_word(tail2) & 0xffff0000u) | 0x8000u));
-    return as_word(__hmul2_rn(w, __lowhigh2highlow(w)));
+    P v0 = __hadd2_rn(as_pair<P>(gate_up0), as_pair<P>(bias0)), v1 = __hadd2_rn(as_pair<P>(gate_up1), as_pair<P>(bias1));
+    v0 = __hmax2_nan(__hmin2_nan(v0, limit2), floor2);
+    v1 = __hmax2_nan(__hmin2_nan(v1, limit2), floor2);
+    const uint32_t g2 = __byte_perm(as_word(v0), as_word(v1), 0x5410), u2 = __byte_perm(as_word(v0), as_word(v1), 0x7632);
+    const uint32_t t2 = H::pack(H::lo(g2) * alpha, H::hi(g2) * alpha);
+    const P w = __hmul2_rn(as_pair<P>(g2), as_pair<P>(sigmoid16x2<T>(H::lo(t2), H::hi(t2))));
+    return as_word(__hmul2_rn(__hadd2_rn(as_pair<P>(u2), one2), w));
 }
 
 // gate_up [rows][2 * inter] with gate in the even and up in the odd columns; bias [experts][2 * inter];
-// out [rows][inter]. A thread makes 8 outputs from 32 bytes of gate_up and 32 bytes of bias.
+// out [rows][inter]. A lane makes 8 outputs from 32 bytes of gate_up and 32 bytes of bias, two such pieces at a time.
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(ROW_THREADS, GLU_CTAS)
 glu_kernel(const uint8_t *__restrict__ gate_up, int64_t ld_gu_bytes, const uint8_t *__restrict__ bias, int64_t ld_bias_bytes,
-           const int32_t *__restrict__ row_expert, uint8_t *__restrict__ out, int64_t ld_out_bytes, int rows, int chunks,
+           const int32_t *__restrict__ row_expert, uint8_t *__restrict__ out, int64_t ld_out_bytes, const RowUnits units, int chunks,
            float alpha, float limit, float *__restrict__ amax) {
+    chain_begin();
     using H = Half16<T>;
     using P = typename H::Pair;
-    __shared__ float warp_max[8];
-    const float r = H::r16(limit);
-    const P limit2 = as_pair<P>(H::pack(r, r)), floor2 = as_pair<P>(H::pack(-INFINITY, -r)), tail2 = as_pair<P>(H::pack(1.0f, 1.0f));
-    for (int row = blockIdx.x; row < rows; row += gridDim.x) {
-        const int e = __ldg(row_expert + row);
+    const float l = H::r16(limit);
+    const P limit2 = as_pair<P>(H::pack(l, l)), floor2 = as_pair<P>(H::pack(-INFINITY, -l)), one2 = as_pair<P>(H::pack(1.0f, 1.0f));
+    const int lane = threadIdx.x & 31, warps = gridDim.x * (ROW_THREADS / 32), total = units.rows * units.segs;
+    for (int i = (blockIdx.x * ROW_THREADS + threadIdx.x) >> 5; i < total; i += warps) {
+        const int at = units.segs == 1 ? i : i / units.segs, seg = i - at * units.segs;
+        const int c_begin = seg * units.seg_chunks, c_end = min(chunks, c_begin + units.seg_chunks);
+        const int row = units.pair_row ? __ldg(units.pair_row + at) : at;
+        if (row < 0) continue;
+        const int e = __ldg(units.pair_row ? units.pair_expert + at : row_expert + row);
         uint4 *dst = reinterpret_cast<uint4 *>(out + row * ld_out_bytes);
         if (e < 0) {
-            for (int c = threadIdx.x; c < chunks; c += blockDim.x) dst[c] = make_uint4(0u, 0u, 0u, 0u);
+            for (int c = c_begin + lane; c < c_end; c += 32) dst[c] = make_uint4(0u, 0u, 0u, 0u);
             continue;
         }
         const uint4 *src = reinterpret_cast<const uint4 *>(gate_up + row * ld_gu_bytes);
         const uint4 *b = reinterpret_cast<const uint4 *>(bias + e * ld_bias_bytes);
         P m2 = as_pair<P>(0u);
-        for (int c = threadIdx.x; c < chunks; c += blockDim.x) {
-            const uint4 v0 = ldg_stream(src + 2 * c), v1 = ldg_stream(src + 2 * c + 1);
-            const uint4 b0 = __ldg(b + 2 * c), b1 = __ldg(b + 2 * c + 1);
-            const uint32_t v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-            const uint32_t bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-            uint32_t o[8];
+        for (int c0 = c_begin + lane; c0 < c_end; c0 += 64) {
+            uint4 g[2][2], w[2][2];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) o[i] = glu_word<T>(v[i], bb[i], alpha, limit2, floor2, tail2);
-            const uint4 packed = make_uint4(__byte_perm(o[0], o[1], 0x5410), __byte_perm(o[2], o[3], 0x5410),
-                                            __byte_perm(o[4], o[5], 0x5410), __byte_perm(o[6], o[7], 0x5410));
-            dst[c] = packed;
-            m2 = fold_abs_max<P>(m2, packed);
+            for (int u = 0; u < 2; ++u) {
+                const int c = c0 + 32 * u < c_end ? c0 + 32 * u : c0;
+                g[u][0] = ldg_stream(src + 2 * c);
+                g[u][1] = ldg_stream(src + 2 * c + 1);
+                w[u][0] = __ldg(b + 2 * c);
+                w[u][1] = __ldg(b + 2 * c + 1);
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                if (c0 + 32 * u >= c_end) break;
+                const uint4 packed = make_uint4(glu_words<T>(g[u][0].x, g[u][0].y, w[u][0].x, w[u][0].y, alpha, limit2, floor2, one2),
+                                                glu_words<T>(g[u][0].z, g[u][0].w, w[u][0].z, w[u][0].w, alpha, limit2, floor2, one2),
+                                                glu_words<T>(g[u][1].x, g[u][1].y, w[u][1].x, w[u][1].y, alpha, limit2, floor2, one2),
+                                                glu_words<T>(g[u][1].z, g[u][1].w, w[u][1].z, w[u][1].w, alpha, limit2, floor2, one2));
+                dst[c0 + 32 * u] = packed;
+                m2 = fold_abs_max<P>(m2, packed);
+            }
         }
-        if (amax != nullptr) raise_amax<T>(m2, amax + e, warp_max);     // (e is the same for the whole CTA: no divergence)
+        __syncwarp();
+        if (amax != nullptr) raise_amax<T>(m2, amax + e, lane);     // (e is the same for the whole warp)
     }
 }
 
@@ -177,6 +235,7 @@ combine_kernel(const uint8_t *__restrict__ y, int64_t ld_y_bytes, const uint8_t 
                const int32_t *__restrict__ pair_row, const int32_t *__restrict__ pair_expert,
                const uint16_t *__restrict__ pair_weight, int top_k, uint8_t *__restrict__ out, int64_t ld_out_bytes, int tokens,
                int chunks) {
+    chain_begin();
     using P = typename Half16<T>::Pair;
     __shared__ int s_row[MAX_TOP_K], s_ex[MAX_TOP_K];
     __shared__ uint32_t s_w[MAX_TOP_K];
@@ -234,7 +293,12 @@ __device__ __forceinline__ int route_expert_of(const IDX *__restrict__ routing, 
 template <typename IDX>
 __global__ void __launch_bounds__(ROUTE_THREADS)
 route_count_kernel(const IDX *__restrict__ routing, int pairs, int seg, int experts, int rows_capacity,
-                   int32_t *__restrict__ seg_count, int32_t *__restrict__ row_token, int32_t *__restrict__ row_expert) {
+                   int32_t *__restrict__ seg_count, int32_t *__restrict__ row_token, int32_t *__restrict__ row_expert,
+                   float *__restrict__ amax) {
+    chain_begin();
+    if (amax != nullptr && blockIdx.x == 0 && threadIdx.x < 2 * experts) {        // (the one-call form: both projections' maxima)
+        for (int i = threadIdx.x; i < 2 * experts; i += ROUTE_THREADS) amax[i] = 0.0f;
+    }
     __shared__ int s_count[ROUTE_MAX_EXPERTS];
     const int tid = threadIdx.x;
     s_count[tid] = 0;
@@ -262,6 +326,7 @@ route_place_kernel(const IDX *__restrict__ routing, int pairs, int seg, int top_
                    const int32_t *__restrict__ seg_count, int32_t *__restrict__ group_start,
                    int32_t *__restrict__ group_rows, int32_t *__restrict__ row_token, int32_t *__restrict__ row_expert,
                    int32_t *__restrict__ pair_row, int32_t *__restrict__ pair_expert) {
+    chain_begin();
     __shared__ int s_at[ROUTE_WARPS][ROUTE_MAX_EXPERTS];     // counts, then next rows, per (warp, expert)
     __shared__ int s_total[ROUTE_MAX_EXPERTS], s_first[ROUTE_MAX_EXPERTS];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -351,17 +416,31 @@ inline bool aligned16(const void *p, int64_t ld_bytes) {
     return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld_bytes % 16 == 0;
 }
 
-inline unsigned grid_for(int64_t rows) {
-    const int64_t cap = 148 * 8;
-    return static_cast<unsigned>(rows < cap ? rows : cap);
+// The units of `rows` rows of `chunks` 16-byte pieces: whole rows where those occupy every resident warp, else segments of
+// at least 128 pieces (shorter ones only meet at the per-expert maxima); at most one wave of CTAs (a warp takes units in turn).
+inline RowUnits row_units(int64_t rows, int chunks, int ctas_per_sm, unsigned *grid) {
+    const int64_t warps = 148 * static_cast<int64_t>(ctas_per_sm) * (ROW_THREADS / 32);
+    int64_t segs = (warps + rows - 1) / rows;
+    const int64_t most = (chunks + 127) / 128;
+    segs = segs < 1 ? 1 : (segs > most ? most : segs);
+    RowUnits u{};
+    u.rows = static_cast<int>(rows);
+    u.seg_chunks = static_cast<int>(((chunks + segs - 1) / segs + 31) / 32 * 32);
+    u.segs = (chunks + u.seg_chunks - 1) / u.seg_chunks;
+    const int64_t ctas = (rows * u.segs + ROW_THREADS / 32 - 1) / (ROW_THREADS / 32), cap = 148 * static_cast<int64_t>(ctas_per_sm);
+    *grid = static_cast<unsigned>(ctas < cap ? ctas : cap);
+    return u;
 }
+
+// The (token, slot) pairs in whose order the one-call form visits the rows in use.
+struct PairOrder { const int32_t *row, *expert; int64_t pairs; int top_k; };
 
 }  // namespace
 }  // namespace fos
 
-extern "C" int fos_experts_gather_rows(const void *x, int dtype, int64_t ld_x, const int32_t *row_token, void *out,
-                                       int64_t ld_out, int64_t rows_capacity, int64_t cols, const int32_t *row_expert,
-                                       float *amax, void *stream_) {
+static int gather_rows(const void *x, int dtype, int64_t ld_x, const int32_t *row_token, void *out, int64_t ld_out,
+                       int64_t rows_capacity, int64_t cols, const int32_t *row_expert, float *amax,
+                       const fos::PairOrder *order, void *stream_) {
     using namespace fos;
     if (!x || !row_token || !out || rows_capacity <= 0 || cols <= 0 || ld_x < cols || ld_out < cols) return FOS_ERR_INVALID_ARGUMENT;
     if ((amax != nullptr) != (row_expert != nullptr)) return FOS_ERR_INVALID_ARGUMENT;
@@ -371,22 +450,31 @@ extern "C" int fos_experts_gather_rows(const void *x, int dtype, int64_t ld_x, c
     const int st = check_device();
     if (st != FOS_OK) return st;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-    const unsigned g = grid_for(rows_capacity), threads = threads_for(static_cast<int>(cols / 8));
+    unsigned g = 0;
+    RowUnits units = row_units(order ? order->pairs : rows_capacity, static_cast<int>(cols / 8), GATHER_CTAS, &g);
+    if (order) { units.pair_row = order->row; units.pair_expert = order->expert; units.top_k = order->top_k; }
     if (dtype == FOS_BF16)
-        gather_rows_kernel<__nv_bfloat16><<<g, threads, 0, stream>>>(static_cast<const uint8_t *>(x), ld_x * 2, row_token,
-                                                                     static_cast<uint8_t *>(out), ld_out * 2, static_cast<int>(rows_capacity),
-                                                                     static_cast<int>(cols / 8), row_expert, amax);
+        FOS_CUDA_TRY(launch_dependent(gather_rows_kernel<__nv_bfloat16>, dim3(g), ROW_THREADS, 0, stream,
+            static_cast<const uint8_t *>(x), ld_x * 2, row_token,
+            static_cast<uint8_t *>(out), ld_out * 2, units,
+            static_cast<int>(cols / 8), row_expert, amax));
     else
-        gather_rows_kernel<__half><<<g, threads, 0, stream>>>(static_cast<const uint8_t *>(x), ld_x * 2, row_token,
-                                                              static_cast<uint8_t *>(out), ld_out * 2, static_cast<int>(rows_capacity),
-                                                              static_cast<int>(cols / 8), row_expert, amax);
-    FOS_CUDA_TRY(cudaGetLastError());
+        FOS_CUDA_TRY(launch_dependent(gather_rows_kernel<__half>, dim3(g), ROW_THREADS, 0, stream,
+            static_cast<const uint8_t *>(x), ld_x * 2, row_token,
+            static_cast<uint8_t *>(out), ld_out * 2, units,
+            static_cast<int>(cols / 8), row_expert, amax));
     return FOS_OK;
 }
 
-extern "C" int fos_experts_glu(const void *gate_up, int dtype, int64_t ld_gate_up, const void *bias, const int32_t *row_expert,
-                               void *out, int64_t ld_out, int64_t rows_capacity, int64_t intermediate, float alpha,
-                               float limit, float *amax, void *stream_) {
+extern "C" int fos_experts_gather_rows(const void *x, int dtype, int64_t ld_x, const int32_t *row_token, void *out,
+                                       int64_t ld_out, int64_t rows_capacity, int64_t cols, const int32_t *row_expert,
+                                       float *amax, void *stream) {
+    return gather_rows(x, dtype, ld_x, row_token, out, ld_out, rows_capacity, cols, row_expert, amax, nullptr, stream);
+}
+
+static int experts_glu(const void *gate_up, int dtype, int64_t ld_gate_up, const void *bias, const int32_t *row_expert, void *out,
+                       int64_t ld_out, int64_t rows_capacity, int64_t intermediate, float alpha, float limit, float *amax,
+                       const fos::PairOrder *order, void *stream_) {
     using namespace fos;
     if (!gate_up || !bias || !row_expert || !out || rows_capacity <= 0 || intermediate <= 0 ||
         ld_gate_up < 2 * intermediate || ld_out < intermediate)
@@ -398,18 +486,28 @@ extern "C" int fos_experts_glu(const void *gate_up, int dtype, int64_t ld_gate_u
     const int st = check_device();
     if (st != FOS_OK) return st;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-    const unsigned g = grid_for(rows_capacity);
-    const int rows = static_cast<int>(rows_capacity), chunks = static_cast<int>(intermediate / 8);
+    unsigned g = 0;
+    const int chunks = static_cast<int>(intermediate / 8);
+    RowUnits units = row_units(order ? order->pairs : rows_capacity, chunks, GLU_CTAS, &g);
+    if (order) { units.pair_row = order->row; units.pair_expert = order->expert; units.top_k = order->top_k; }
     if (dtype == FOS_BF16)
-        glu_kernel<__nv_bfloat16><<<g, threads_for(chunks), 0, stream>>>(static_cast<const uint8_t *>(gate_up), ld_gate_up * 2,
-                                                           static_cast<const uint8_t *>(bias), 2 * intermediate * 2, row_expert,
-                                                           static_cast<uint8_t *>(out), ld_out * 2, rows, chunks, alpha, limit, amax);
+        FOS_CUDA_TRY(launch_dependent(glu_kernel<__nv_bfloat16>, dim3(g), ROW_THREADS, 0, stream,
+            static_cast<const uint8_t *>(gate_up), ld_gate_up * 2,
+            static_cast<const uint8_t *>(bias), 2 * intermediate * 2, row_expert,
+            static_cast<uint8_t *>(out), ld_out * 2, units, chunks, alpha, limit, amax));
     else
-        glu_kernel<__half><<<g, threads_for(chunks), 0, stream>>>(static_cast<const uint8_t *>(gate_up), ld_gate_up * 2,
-                                                    static_cast<const uint8_t *>(bias), 2 * intermediate * 2, row_expert,
-                                                    static_cast<uint8_t *>(out), ld_out * 2, rows, chunks, alpha, limit, amax);
-    FOS_CUDA_TRY(cudaGetLastError());
+        FOS_CUDA_TRY(launch_dependent(glu_kernel<__half>, dim3(g), ROW_THREADS, 0, stream,
+            static_cast<const uint8_t *>(gate_up), ld_gate_up * 2,
+            static_cast<const uint8_t *>(bias), 2 * intermediate * 2, row_expert,
+            static_cast<uint8_t *>(out), ld_out * 2, units, chunks, alpha, limit, amax));
     return FOS_OK;
+}
+
+extern "C" int fos_experts_glu(const void *gate_up, int dtype, int64_t ld_gate_up, const void *bias, const int32_t *row_expert,
+                               void *out, int64_t ld_out, int64_t rows_capacity, int64_t intermediate, float alpha,
+                               float limit, float *amax, void *stream) {
+    return experts_glu(gate_up, dtype, ld_gate_up, bias, row_expert, out, ld_out, rows_capacity, intermediate, alpha, limit, amax,
+                       nullptr, stream);
 }
 
 extern "C" int fos_experts_combine(const void *y, int dtype, int64_t ld_y, const void *bias, const int32_t *pair_row,
@@ -425,26 +523,28 @@ extern "C" int fos_experts_combine(const void *y, int dtype, int64_t ld_y, const
     const int st = check_device();
     if (st != FOS_OK) return st;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-    const unsigned g = grid_for(tokens);
+    const unsigned g = static_cast<unsigned>(tokens < 148 * 8 ? tokens : 148 * 8);
     const int n = static_cast<int>(tokens), chunks = static_cast<int>(hidden / 8);
     if (dtype == FOS_BF16)
-        combine_kernel<__nv_bfloat16><<<g, threads_for(chunks), 0, stream>>>(static_cast<const uint8_t *>(y), ld_y * 2,
-                                                               static_cast<const uint8_t *>(bias), hidden * 2, pair_row, pair_expert,
-                                                               static_cast<const uint16_t *>(pair_weight), top_k,
-                                                               static_cast<uint8_t *>(out), ld_out * 2, n, chunks);
+        FOS_CUDA_TRY(launch_dependent(combine_kernel<__nv_bfloat16>, dim3(g), threads_for(chunks), 0, stream,
+            static_cast<const uint8_t *>(y), ld_y * 2,
+            static_cast<const uint8_t *>(bias), hidden * 2, pair_row, pair_expert,
+            static_cast<const uint16_t *>(pair_weight), top_k,
+            static_cast<uint8_t *>(out), ld_out * 2, n, chunks));
     else
-        combine_kernel<__half><<<g, threads_for(chunks), 0, stream>>>(static_cast<const uint8_t *>(y), ld_y * 2,
-                                                        static_cast<const uint8_t *>(bias), hidden * 2, pair_row, pair_expert,
-                                                        static_cast<const uint16_t *>(pair_weight), top_k,
-                                                        static_cast<uint8_t *>(out), ld_out * 2, n, chunks);
-    FOS_CUDA_TRY(cudaGetLastError());
+        FOS_CUDA_TRY(launch_dependent(combine_kernel<__half>, dim3(g), threads_for(chunks), 0, stream,
+            static_cast<const uint8_t *>(y), ld_y * 2,
+            static_cast<const uint8_t *>(bias), hidden * 2, pair_row, pair_expert,
+            static_cast<const uint16_t *>(pair_weight), top_k,
+            static_cast<uint8_t *>(out), ld_out * 2, n, chunks));
     return FOS_OK;
 }
 
-extern "C" int fos_experts_route(const void *routing_indices, int index_bytes, int64_t tokens, int top_k, int num_experts,
-                                 int64_t rows_capacity, int32_t *group_start, int32_t *group_rows, int32_t *row_token,
-                                 int32_t *row_expert, int32_t *pair_row, int32_t *pair_expert, int32_t *workspace,
-                                 void *stream_) {
+// fos_experts_route; with `amax` also zeroes amax[0 .. 2 * num_experts).
+static int experts_route(const void *routing_indices, int index_bytes, int64_t tokens, int top_k, int num_experts,
+                         int64_t rows_capacity, int32_t *group_start, int32_t *group_rows, int32_t *row_token,
+                         int32_t *row_expert, int32_t *pair_row, int32_t *pair_expert, int32_t *workspace, float *amax,
+                         void *stream_) {
     using namespace fos;
     if (!routing_indices || !group_start || !group_rows || !row_token || !row_expert || !pair_row || !pair_expert ||
         !workspace || tokens <= 0 || top_k <= 0 || num_experts <= 0 || (index_bytes != 4 && index_bytes != 8))
@@ -465,17 +565,28 @@ extern "C" int fos_experts_route(const void *routing_indices, int index_bytes, i
     segments = (pairs + seg - 1) / seg;
     if (index_bytes == 8) {
         const int64_t *idx = static_cast<const int64_t *>(routing_indices);
-        route_count_kernel<int64_t><<<segments, ROUTE_THREADS, 0, stream>>>(idx, pairs, seg, num_experts, cap, workspace, row_token, row_expert);
-        route_place_kernel<int64_t><<<segments, ROUTE_THREADS, 0, stream>>>(idx, pairs, seg, top_k, num_experts, workspace, group_start,
-                                                                            group_rows, row_token, row_expert, pair_row, pair_expert);
+        FOS_CUDA_TRY(launch_dependent(route_count_kernel<int64_t>, dim3(segments), ROUTE_THREADS, 0, stream,
+            idx, pairs, seg, num_experts, cap, workspace, row_token, row_expert, amax));
+        FOS_CUDA_TRY(launch_dependent(route_place_kernel<int64_t>, dim3(segments), ROUTE_THREADS, 0, stream,
+            idx, pairs, seg, top_k, num_experts, workspace, group_start,
+            group_rows, row_token, row_expert, pair_row, pair_expert));
     } else {
         const int32_t *idx = static_cast<const int32_t *>(routing_indices);
-        route_count_kernel<int32_t><<<segments, ROUTE_THREADS, 0, stream>>>(idx, pairs, seg, num_experts, cap, workspace, row_token, row_expert);
-        route_place_kernel<int32_t><<<segments, ROUTE_THREADS, 0, stream>>>(idx, pairs, seg, top_k, num_experts, workspace, group_start,
-                                                                            group_rows, row_token, row_expert, pair_row, pair_expert);
+        FOS_CUDA_TRY(launch_dependent(route_count_kernel<int32_t>, dim3(segments), ROUTE_THREADS, 0, stream,
+            idx, pairs, seg, num_experts, cap, workspace, row_token, row_expert, amax));
+        FOS_CUDA_TRY(launch_dependent(route_place_kernel<int32_t>, dim3(segments), ROUTE_THREADS, 0, stream,
+            idx, pairs, seg, top_k, num_experts, workspace, group_start,
+            group_rows, row_token, row_expert, pair_row, pair_expert));
     }
-    FOS_CUDA_TRY(cudaGetLastError());
     return FOS_OK;
+}
+
+extern "C" int fos_experts_route(const void *routing_indices, int index_bytes, int64_t tokens, int top_k, int num_experts,
+                                 int64_t rows_capacity, int32_t *group_start, int32_t *group_rows, int32_t *row_token,
+                                 int32_t *row_expert, int32_t *pair_row, int32_t *pair_expert, int32_t *workspace,
+                                 void *stream) {
+    return experts_route(routing_indices, index_bytes, tokens, top_k, num_experts, rows_capacity, group_start, group_rows,
+                         row_token, row_expert, pair_row, pair_expert, workspace, nullptr, stream);
 }
 
 // ---------------------------------------------------------------------------- the whole layer in one call
@@ -546,40 +657,35 @@ extern "C" int fos_experts_forward(const void *x, int dtype, int64_t tokens, int
     if (workspace_bytes < w.total) return FOS_ERR_INVALID_ARGUMENT;
     uint8_t *base = static_cast<uint8_t *>(workspace);
     auto ints = [&](int64_t off) { return reinterpret_cast<int32_t *>(base + off); };
-    float *amax = reinterpret_cast<float *>(base + w.amax), *alphas = reinterpret_cast<float *>(base + w.alpha);
-    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    float *amax = reinterpret_cast<float *>(base + w.amax);
     const int64_t gate_up_rows = round_up64(2 * intermediate, 128), down_rows = round_up64(hidden, 128);
 
-    int st = fos_experts_route(routing_indices, index_bytes, tokens, top_k, num_experts, w.capacity, ints(w.group_start),
-                               ints(w.group_rows), ints(w.row_token), ints(w.row_expert), ints(w.pair_row),
-                               ints(w.pair_expert), ints(w.route_work), stream_);
+    int st = experts_route(routing_indices, index_bytes, tokens, top_k, num_experts, w.capacity, ints(w.group_start),
+                           ints(w.group_rows), ints(w.row_token), ints(w.row_expert), ints(w.pair_row), ints(w.pair_expert),
+                           ints(w.route_work), amax, stream_);
     if (st != FOS_OK) return st;
-    FOS_CUDA_TRY(cudaMemsetAsync(amax, 0, sizeof(float) * 2 * num_experts, stream));
-    st = fos_experts_gather_rows(x, dtype, ld_x, ints(w.row_token), base + w.rows_x, hidden, w.capacity, hidden,
-                                 ints(w.row_expert), amax, stream_);
+    const PairOrder order{ints(w.pair_row), ints(w.pair_expert), w.pairs, top_k};
+    st = gather_rows(x, dtype, ld_x, ints(w.row_token), base + w.rows_x, hidden, w.capacity, hidden, ints(w.row_expert), amax,
+                     &order, stream_);
     if (st != FOS_OK) return st;
-    st = fos_quantize_grouped(base + w.rows_x, dtype, w.capacity, hidden, hidden, FOS_NVFP4, activation_rule, ints(w.group_start),
+    st = quantize_grouped_rows_in_use(base + w.rows_x, dtype, w.capacity, hidden, hidden, FOS_NVFP4, activation_rule, ints(w.group_start),
                               ints(w.group_rows), num_experts, amax, base + w.codes_x, base + w.sf_x, amax, 0, stream_);
     if (st != FOS_OK) return st;
-    st = fos_gemm_alpha_grouped(amax, FOS_NVFP4, activation_rule, 0, gate_up_amax, FOS_NVFP4, weight_rule, 0, alphas, num_experts, stream_);
+    const float denom = alpha_divisor(FOS_NVFP4, activation_rule, FOS_NVFP4, weight_rule);
+    st = gemm_nvfp4_grouped_scaled(base + w.codes_x, base + w.sf_x, gate_up_codes, gate_up_sf, {amax, gate_up_amax, denom, nullptr, true},
+                                   base + w.gate_up, dtype, ints(w.group_start), ints(w.group_rows), num_experts, w.capacity,
+                                   gate_up_rows, hidden, 2 * intermediate, 2 * intermediate, status, stream_);
     if (st != FOS_OK) return st;
-    st = fos_gemm_nvfp4_grouped(base + w.codes_x, base + w.sf_x, gate_up_codes, gate_up_sf, alphas, base + w.gate_up, dtype,
-                                ints(w.group_start), ints(w.group_rows), num_experts, w.capacity, gate_up_rows, hidden,
-                                2 * intermediate, 2 * intermediate, nullptr, status, stream_);
+    st = experts_glu(base + w.gate_up, dtype, 2 * intermediate, gate_up_bias, ints(w.row_expert), base + w.gated, intermediate,
+                     w.capacity, intermediate, alpha, limit, amax + num_experts, &order, stream_);
     if (st != FOS_OK) return st;
-    st = fos_experts_glu(base + w.gate_up, dtype, 2 * intermediate, gate_up_bias, ints(w.row_expert), base + w.gated, intermediate,
-                         w.capacity, intermediate, alpha, limit, amax + num_experts, stream_);
-    if (st != FOS_OK) return st;
-    st = fos_quantize_grouped(base + w.gated, dtype, w.capacity, intermediate, intermediate, FOS_NVFP4, activation_rule,
+    st = quantize_grouped_rows_in_use(base + w.gated, dtype, w.capacity, intermediate, intermediate, FOS_NVFP4, activation_rule,
                               ints(w.group_start), ints(w.group_rows), num_experts, amax + num_experts, base + w.codes_g,
                               base + w.sf_g, amax + num_experts, 0, stream_);
     if (st != FOS_OK) return st;
-    st = fos_gemm_alpha_grouped(amax + num_experts, FOS_NVFP4, activation_rule, 0, down_amax, FOS_NVFP4, weight_rule, 0,
-                                alphas + num_experts, num_experts, stream_);
-    if (st != FOS_OK) return st;
-    st = fos_gemm_nvfp4_grouped(base + w.codes_g, base + w.sf_g, down_codes, down_sf, alphas + num_experts, base + w.y, dtype,
-                                ints(w.group_start), ints(w.group_rows), num_experts, w.capacity, down_rows, intermediate,
-                                hidden, hidden, nullptr, status, stream_);
+    st = gemm_nvfp4_grouped_scaled(base + w.codes_g, base + w.sf_g, down_codes, down_sf, {amax + num_experts, down_amax, denom, nullptr, true},
+                                   base + w.y, dtype, ints(w.group_start), ints(w.group_rows), num_experts, w.capacity,
+                                   down_rows, intermediate, hidden, hidden, status, stream_);
     if (st != FOS_OK) return st;
     return fos_experts_combine(base + w.y, dtype, hidden, down_bias, ints(w.pair_row), ints(w.pair_expert), routing_weights,
                                top_k, out, ld_out, tokens, hidden, stream_);
