@@ -70,6 +70,14 @@ class B200MatmulBackend:
         reason = cls.unsupported_reason(input, other, out_dtype=out_dtype)
         if reason is not None:
             raise ValueError(f"B200 matmul: {reason}")
+        return cls._quantized_matmul(input, other, out_dtype=out_dtype, out=out, check_status=check_status, variant=variant,
+                                     max_ctas=max_ctas)
+
+    @classmethod
+    def _quantized_matmul(cls, input: QuantizedTensor, other: QuantizedTensor, *, out_dtype: DataType,
+                          out: torch.Tensor | None = None, check_status: bool = False, variant: int = 0,
+                          max_ctas: int = 0) -> torch.Tensor:
+        """`quantized_matmul` of a request that `unsupported_reason` has accepted."""
         dev = input.device
         m, n = input.original_shape[0], other.original_shape[0]
         m_p, k_p = input.padded_shape
@@ -81,7 +89,6 @@ class B200MatmulBackend:
             out = torch.empty(m, n, dtype=torch_out, device=dev)
         elif out.shape != (m, n) or out.dtype != torch_out or out.stride(1) != 1:
             raise ValueError("B200 matmul: `out` has the wrong shape, dtype or layout")
-        alpha = torch.empty(1, dtype=torch.float32, device=dev)
         status = torch.zeros(1, dtype=torch.int32, device=dev) if check_status else None
         a_vals, b_vals = input.values.contiguous(), other.values.contiguous()
         a_sf, b_sf = input.scale_factors.contiguous(), other.scale_factors.contiguous()
@@ -89,30 +96,30 @@ class B200MatmulBackend:
         # block-scaled FP4 tensor cores when both operands are NVFP4 in the tile layout; otherwise
         # (IF4, or row-major scales) the fp16 path, which needs a scratch buffer for the expanded operands
         native_fp4 = (fa == fb == _native.FOS_NVFP4 and _layout(input) == _layout(other) == _native.FOS_SF_TILED)
-        with torch.cuda.device(dev):
+        with _native.on_device(dev):
             lib, stream = _native.lib(), _native.stream_ptr(dev)
             status_ptr = 0 if status is None else status.data_ptr()
             opts = _native.gemm_opts(variant, max_ctas)
             if fa == _native.FOS_MXFP4:
-                alpha.fill_(1.0)
-                _native.check(lib.fos_gemm_mxfp4_ex(
-                    a_vals.data_ptr(), a_sf.data_ptr(), b_vals.data_ptr(), b_sf.data_ptr(), alpha.data_ptr(),
-                    out.data_ptr(), _native.elem_code(torch_out), m_p, n_p, k_p, m, n, out.stride(0),
+                _native.check(lib.fos_gemm_mxfp4_unscaled(
+                    a_vals.data_ptr(), a_sf.data_ptr(), b_vals.data_ptr(), b_sf.data_ptr(), out.data_ptr(), _native.elem_code(torch_out), m_p, n_p, k_p, m, n, out.stride(0),
                     opts, status_ptr, stream), "fos_gemm_mxfp4")
                 if status is not None and int(status.item()) != 0:
                     raise _native.NativeLibraryError(
                         f"fos_gemm_mxfp4: a bounded device-side wait timed out (site {int(status.item())})")
                 return out
-            _native.check(lib.fos_gemm_alpha_ex(
-                input.amax.data_ptr(), fa, input.scale_rule.cuda_id, int(input.round_style == RoundStyle.stochastic_unbiased),
-                other.amax.data_ptr(), fb, other.scale_rule.cuda_id, int(other.round_style == RoundStyle.stochastic_unbiased),
-                alpha.data_ptr(), stream), "fos_gemm_alpha")
+            unbiased_a, unbiased_b = (int(t.round_style is RoundStyle.stochastic_unbiased) for t in (input, other))
             if native_fp4:
-                _native.check(lib.fos_gemm_nvfp4_ex(
-                    a_vals.data_ptr(), a_sf.data_ptr(), b_vals.data_ptr(), b_sf.data_ptr(), alpha.data_ptr(),
+                _native.check(lib.fos_gemm_nvfp4_scaled(
+                    a_vals.data_ptr(), a_sf.data_ptr(), input.amax.data_ptr(), input.scale_rule.cuda_id, unbiased_a,
+                    b_vals.data_ptr(), b_sf.data_ptr(), other.amax.data_ptr(), other.scale_rule.cuda_id, unbiased_b,
                     out.data_ptr(), _native.elem_code(torch_out), m_p, n_p, k_p, m, n, out.stride(0),
                     opts, status_ptr, stream), "fos_gemm_nvfp4")
             else:
+                alpha = torch.empty(1, dtype=torch.float32, device=dev)
+                _native.check(lib.fos_gemm_alpha_ex(
+                    input.amax.data_ptr(), fa, input.scale_rule.cuda_id, unbiased_a, other.amax.data_ptr(), fb,
+                    other.scale_rule.cuda_id, unbiased_b, alpha.data_ptr(), stream), "fos_gemm_alpha")
                 nbytes = int(lib.fos_gemm_if4_workspace_bytes(m_p, n_p, k_p))
                 workspace = torch.empty(nbytes, dtype=torch.uint8, device=dev)
                 _native.check(lib.fos_gemm_if4(
@@ -168,7 +175,7 @@ class B200MatmulBackend:
         alpha = torch.empty(1, dtype=torch.float32, device=dev)
         status = torch.zeros(1, dtype=torch.int32, device=dev) if check_status else None
         rule = ScaleRule(config.scale_rule).cuda_id
-        with torch.cuda.device(dev):
+        with _native.on_device(dev):
             lib, stream = _native.lib(), _native.stream_ptr(dev)
             _native.check(lib.fos_gemm_alpha(amax.data_ptr(), _native.FOS_NVFP4, rule, other.amax.data_ptr(), _native.FOS_NVFP4,
                                              other.scale_rule.cuda_id, alpha.data_ptr(), stream), "fos_gemm_alpha")
@@ -204,7 +211,7 @@ class B200MatmulBackend:
         alpha = torch.empty(1, dtype=torch.float32, device=dev)
         a_vals, b_vals = input.values.contiguous(), other.values.contiguous()
         a_sf, b_sf = input.scale_factors.contiguous(), other.scale_factors.contiguous()
-        with torch.cuda.device(dev):
+        with _native.on_device(dev):
             lib, stream = _native.lib(), _native.stream_ptr(dev)
             _native.check(lib.fos_gemm_alpha(
                 input.amax.data_ptr(), _native.FOS_NVFP4, input.scale_rule.cuda_id,

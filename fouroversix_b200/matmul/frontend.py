@@ -55,4 +55,4 @@ def quantized_matmul(
         if backend is None:
             raise ValueError(f"No backend found that supports the given parameters ({reason})")
         raise ValueError(f"Backend {backend} does not support the given parameters ({reason})")
-    return impl.quantized_matmul(input, other, out_dtype=DataType(out_dtype), **kwargs)
+    return impl._quantized_matmul(input, other, out_dtype=DataType(out_dtype), **kwargs)

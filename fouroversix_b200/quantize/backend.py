@@ -23,15 +23,13 @@ from .quantized_tensor import QuantizedTensor, padded_shape_for
 _FORMATS = {DataType.nvfp4: _native.FOS_NVFP4, DataType.if4: _native.FOS_IF4, DataType.mxfp4: _native.FOS_MXFP4}
 
 
+_KERNEL_FLAGS = {"auto": 0, "no_tma": _native.FOS_QUANTIZE_NO_TMA, "general": _native.FOS_QUANTIZE_GENERAL_KERNEL}
+
+
 def _is_tiled(dtype: DataType) -> bool:
     # like the reference's PyTorch back end, IF4 keeps its scales row-major
     # (src/fouroversix/quantize/pytorch/backend.py:107-120)
     return dtype in (DataType.nvfp4, DataType.mxfp4)
-
-
-def _scale_view(scales: torch.Tensor, dtype: DataType) -> torch.Tensor:
-    """The scale bytes typed as the reference types them: E4M3, or E8M0 for the MX formats."""
-    return scales.view(torch.float8_e8m0fnu if dtype.scale_type == ScaleType.mx else torch.float8_e4m3fn)
 
 
 class B200QuantizeBackend:
@@ -52,7 +50,7 @@ class B200QuantizeBackend:
             return "input must be 2-D"
         if config.dtype not in _FORMATS:
             return f"dtype {config.dtype.value} is not implemented (nvfp4, if4 and mxfp4 are)"
-        if config.scale_rule not in config.dtype.supported_scale_rules:
+        if not config.dtype.supports_scale_rule(config.scale_rule):
             return f"scale rule {config.scale_rule.value} is not defined for {config.dtype.value}"
         if config.round_style.is_stochastic:
             if config.block_scale_2d or config.dtype not in (DataType.nvfp4, DataType.if4):
@@ -85,6 +83,12 @@ class B200QuantizeBackend:
         reason = cls.unsupported_reason(x, config)
         if reason is not None:
             raise ValueError(f"B200 quantize: {reason}")
+        return cls._quantize(x, config, amax, exact_only, seed, kernel)
+
+    @classmethod
+    def _quantize(cls, x: torch.Tensor, config: QuantizationConfig, amax: torch.Tensor | None = None,
+                  exact_only: bool = False, seed: int | None = None, kernel: str = "auto") -> QuantizedTensor:
+        """`quantize` of a request that `unsupported_reason` has accepted."""
         if x.stride(1) != 1:
             x = x.contiguous()
         rows, cols = x.shape
@@ -92,7 +96,7 @@ class B200QuantizeBackend:
         rows_p, cols_p = padded_shape_for(out_shape, config.dtype)
         dev = x.device
         values = torch.empty(rows_p, cols_p // 2, dtype=torch.uint8, device=dev)
-        scales = torch.empty(rows_p * cols_p // config.dtype.block_size, dtype=torch.uint8, device=dev)
+        scales = torch.empty(rows_p * cols_p // config.dtype.block_size, dtype=config.dtype.scale_type.torch_dtype, device=dev)
         amax_out = torch.empty(1, dtype=torch.float32, device=dev)
         if amax is not None:
             amax = amax.detach().reshape(1).to(device=dev, dtype=torch.float32)
@@ -103,9 +107,9 @@ class B200QuantizeBackend:
                 0 if amax is None else amax.data_ptr(), values.data_ptr(), scales.data_ptr(),
                 amax_out.data_ptr(),
                 (_native.FOS_QUANTIZE_EXACT_ONLY if exact_only else 0) | (_native.FOS_QUANTIZE_RHT if config.rht else 0)
-                | {"auto": 0, "no_tma": _native.FOS_QUANTIZE_NO_TMA, "general": _native.FOS_QUANTIZE_GENERAL_KERNEL}[kernel]
+                | _KERNEL_FLAGS[kernel]
                 | (_native.FOS_QUANTIZE_UNBIASED if config.round_style == RoundStyle.stochastic_unbiased else 0))
-        with torch.cuda.device(dev):
+        with _native.on_device(dev):
             if config.round_style.is_stochastic:
                 if seed is None:
                     seed = int(torch.randint(0, 2 ** 62, (1,)).item())
@@ -116,7 +120,7 @@ class B200QuantizeBackend:
                 status = _native.lib().fos_quantize(*args, _native.stream_ptr(dev))
         _native.check(status, "fos_quantize")
         return QuantizedTensor(
-            values, _scale_view(scales, config.dtype), amax_out, config.dtype, out_shape,
+            values, scales, amax_out, config.dtype, out_shape,
             config.scale_rule, config.round_style, (rows_p, cols_p),
             scale_factors_are_in_blackwell_layout=tiled)
 
@@ -129,7 +133,7 @@ class B200QuantizeBackend:
         if x.stride(1) != 1:
             x = x.contiguous()
         out = torch.empty(1, dtype=torch.float32, device=x.device)
-        with torch.cuda.device(x.device):
+        with _native.on_device(x.device):
             _native.check(_native.lib().fos_amax(x.data_ptr(), _native.elem_code(x.dtype), x.shape[0], x.shape[1],
                                                  x.stride(0), out.data_ptr(), _native.stream_ptr(x.device)), "fos_amax")
         return out
@@ -158,7 +162,7 @@ class B200QuantizeBackend:
         values = tensor.values.contiguous()
         scales = tensor.scale_factors.contiguous()
         amax = None if tensor.amax is None else tensor.amax.to(device=dev, dtype=torch.float32)
-        with torch.cuda.device(dev):
+        with _native.on_device(dev):
             status = _native.lib().fos_dequantize_ex(
                 values.data_ptr(), scales.data_ptr(), 0 if amax is None else amax.data_ptr(), _FORMATS[tensor.dtype],
                 tensor.scale_rule.cuda_id,
@@ -182,7 +186,7 @@ class B200QuantizeBackend:
         rows_p, cols_p = tensor.padded_shape
         dev = tensor.device
         out = torch.empty(rows_p, cols_p, dtype=dtype, device=dev)
-        with torch.cuda.device(dev):
+        with _native.on_device(dev):
             status = _native.lib().fos_dequantize_ex(
                 tensor.values.contiguous().data_ptr(), tensor.scale_factors.contiguous().data_ptr(), 0,
                 _FORMATS[tensor.dtype], tensor.scale_rule.cuda_id,
@@ -206,7 +210,7 @@ class B200QuantizeBackend:
             rows, cols = x.shape
             out = torch.empty(rows, cols, dtype=x.dtype, device=x.device)
             amax_out = torch.empty(1, dtype=torch.float32, device=x.device)
-            with torch.cuda.device(x.device):
+            with _native.on_device(x.device):
                 status = _native.lib().fos_pseudo_quantize(
                     x.data_ptr(), _native.elem_code(x.dtype), rows, cols, x.stride(0), _FORMATS[config.dtype],
                     config.scale_rule.cuda_id, 0, out.data_ptr(), out.stride(0), amax_out.data_ptr(), 0,

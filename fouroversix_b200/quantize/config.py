@@ -6,12 +6,12 @@ Field names, defaults and string coercion follow the reference's dataclass
 
 from __future__ import annotations
 
-from dataclasses import dataclass, field, fields
+from dataclasses import dataclass, field
 from typing import Any
 
 from fouroversix_b200.utils import DataType, QuantizeBackend, RoundStyle, ScaleRule
 
-_ENUM_FIELDS = {"backend": QuantizeBackend, "dtype": DataType, "round_style": RoundStyle, "scale_rule": ScaleRule}
+_ENUM_FIELDS = (("backend", QuantizeBackend), ("dtype", DataType), ("round_style", RoundStyle), ("scale_rule", ScaleRule))
 
 
 @dataclass
@@ -41,8 +41,7 @@ class QuantizationConfig:
     transpose: bool = False
 
     def __post_init__(self) -> None:
-        for f in fields(self):
-            enum_cls = _ENUM_FIELDS.get(f.name)
-            value = getattr(self, f.name)
-            if enum_cls is not None and isinstance(value, str) and not isinstance(value, enum_cls):
-                setattr(self, f.name, enum_cls(value))
+        for name, enum_cls in _ENUM_FIELDS:
+            value = getattr(self, name)
+            if value is not None and not isinstance(value, enum_cls) and isinstance(value, str):
+                setattr(self, name, enum_cls(value))

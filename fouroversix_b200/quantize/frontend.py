@@ -46,7 +46,7 @@ def quantize(x: torch.Tensor, config: QuantizationConfig | None = None) -> Quant
         raise ValueError(f"Backend {config.backend} does not support the given parameters ({reason})")
     if config.pseudo_quantize:
         return impl.pseudo_quantize(x, config)
-    return impl.quantize(x, config)
+    return impl._quantize(x, config)
 
 
 def dequantize(tensor: QuantizedTensor, dtype: torch.dtype = torch.bfloat16, *,

@@ -38,10 +38,10 @@ class QuantizedTensor:
         *,
         scale_factors_are_in_blackwell_layout: bool = True,
     ) -> None:
-        self.dtype = DataType(dtype)
+        self.dtype = dtype if type(dtype) is DataType else DataType(dtype)
         self.original_shape = tuple(original_shape)
-        self.scale_rule = ScaleRule(scale_rule)
-        self.round_style = RoundStyle(round_style)
+        self.scale_rule = scale_rule if type(scale_rule) is ScaleRule else ScaleRule(scale_rule)
+        self.round_style = round_style if type(round_style) is RoundStyle else RoundStyle(round_style)
         self.scale_factors_are_in_blackwell_layout = bool(scale_factors_are_in_blackwell_layout)
 
         if padded_shape is not None:

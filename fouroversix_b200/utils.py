@@ -33,11 +33,11 @@ class ScaleRule(str, Enum):
     @property
     def cuda_id(self) -> int:
         """Number of the rule in the native interface (FOS_RULE_* in the C header)."""
-        return _RULE_IDS[self.value]
+        return _RULE_IDS[self._value_]
 
     @property
     def is_static(self) -> bool:
-        return self.value.startswith("static")
+        return self._value_.startswith("static")
 
 
 _RULE_IDS = {"static_6": 0, "static_4": 1, "mae": 2, "mse": 3, "abs_max": 4}
@@ -146,21 +146,7 @@ class DataType(str, Enum):
 
     def _parts(self) -> tuple[str, str, int] | None:
         """(family, value type, block size) of a block-scaled format, else None."""
-        name = self.value
-        family = next((f for f in ("mx", "nv", "if") if name.startswith(f)), None)
-        if family is None:
-            return None
-        body = name[2:]
-        small = body.endswith("_bs8")
-        body = body.removesuffix("_bs8")
-        if family == "if":
-            value = "if" + body
-        elif body.startswith("int"):
-            value = body
-        else:
-            value = body  # fp3, fp4, fp6_e2m3 ...
-        block = 8 if small else (32 if family == "mx" else 16)
-        return family, value, block
+        return _FORMAT_PARTS[self._value_]
 
     @property
     def block_size(self) -> int | None:
@@ -177,25 +163,43 @@ class DataType(str, Enum):
         parts = self._parts()
         if parts is None:
             return None
-        return {"mx": ScaleType.mx, "nv": ScaleType.nv, "if": ScaleType.nv_if}[parts[0]]
+        return _FAMILY_SCALES[parts[0]]
 
     @property
     def supported_scale_rules(self) -> set[ScaleRule]:
-        parts = self._parts()
-        if parts is None:
-            return set()
-        family, value, _ = parts
-        if family == "if":
-            return {r for r in ScaleRule if not r.is_static}
-        if family == "mx":
-            return {r for r in ScaleRule if r.is_static}
-        if value == "fp4":
-            return set(ScaleRule)
-        return {ScaleRule.static_6}
+        return set(_FORMAT_RULES[self._value_])
+
+    def supports_scale_rule(self, rule: ScaleRule) -> bool:
+        return rule in _FORMAT_RULES[self._value_]
 
     @property
     def torch_dtype(self) -> torch.dtype | None:
         return {"bfloat16": torch.bfloat16, "float16": torch.float16, "float32": torch.float32}.get(self.value)
+
+
+def _parse_format(name: str) -> tuple[str, str, int] | None:
+    family = next((f for f in ("mx", "nv", "if") if name.startswith(f)), None)
+    if family is None:
+        return None
+    small = name.endswith("_bs8")
+    body = name[2:].removesuffix("_bs8")                 # fp3, fp4, fp6_e2m3, int4 ...; 3, 4 ... of an if format
+    return family, "if" + body if family == "if" else body, 8 if small else (32 if family == "mx" else 16)
+
+
+def _rules_of(parts: tuple[str, str, int] | None) -> tuple[ScaleRule, ...]:
+    if parts is None:
+        return ()
+    if parts[0] == "if":
+        return tuple(r for r in ScaleRule if not r.is_static)
+    if parts[0] == "mx":
+        return tuple(r for r in ScaleRule if r.is_static)
+    return tuple(ScaleRule) if parts[1] == "fp4" else (ScaleRule.static_6,)
+
+
+# looked up several times by every call: what a format's name says, worked out once per member
+_FORMAT_PARTS = {d.value: _parse_format(d.value) for d in DataType}
+_FORMAT_RULES = {name: _rules_of(parts) for name, parts in _FORMAT_PARTS.items()}
+_FAMILY_SCALES = {"mx": ScaleType.mx, "nv": ScaleType.nv, "if": ScaleType.nv_if}
 
 
 class QuantizeBackend(str, Enum):
