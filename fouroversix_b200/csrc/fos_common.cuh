@@ -32,6 +32,10 @@ int quantize_mxfp4(const void *x, int x_dtype, int64_t rows, int64_t cols, int64
 int dequantize_mxfp4(const uint8_t *codes, const uint8_t *sf, int sf_layout, int64_t rows_p, int64_t cols_p, int64_t rows,
                      int64_t cols, void *out, int out_dtype, int64_t ld_out, cudaStream_t stream);
 
+// fos_quantize (NVFP4, 1-D blocks, tiled scales, amax computed) for a GEMM's A operand: the padding rows may be left alone,
+// because no row of a product depends on another.
+int quantize_activation(const void *x, int x_dtype, int64_t rows, int64_t cols, int64_t ld, int scale_rule, uint8_t *codes,
+                        uint8_t *sf, float *amax_out, void *stream);
 // fos_quantize_grouped for callers that read no product of a padding row: what comes out there is not defined.
 int quantize_grouped_rows_in_use(const void *x, int x_dtype, int64_t rows_capacity, int64_t cols, int64_t ld, int format,
                                  int scale_rule, const int32_t *group_start, const int32_t *group_rows, int num_groups,

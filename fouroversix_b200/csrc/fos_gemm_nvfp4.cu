@@ -58,7 +58,9 @@ constexpr int SF_LEAD = FOS_GEMM_SF_LEAD;   // 0 or 1: how many stages the scale
 
 constexpr int SF_CP_WARPS = 2;                     // warps 10 and 11 issue the scale copies, taking stages in turn
 constexpr int NUM_THREADS = 384;                   // warps: 0 TMA, 1 MMA, 2-9 epilogue (FUSED_A: also the A operand), 10-11 scale copies
-constexpr int PAIR_MIN_GROUP_ROWS = 640;           // grouped launches: CTA pairs from this many rows of the buffer per group
+// Grouped launches: CTA pairs from this many rows of the buffer per group (us, pairs / 128-row tiles: 1152 rows, 32 groups of
+// K 2880, N 5760 300 / 324, N 2880 155 / 192; 640 rows, 8 groups of K 1024, N 2048 11.7 / 11.7).
+constexpr int PAIR_MIN_GROUP_ROWS = 640;
 constexpr int MAX_GROUPS = 256;                    // of a grouped launch (their row ranges are kept in shared memory)
 constexpr int SF_COL0 = 256;                       // tensor-memory columns: accumulators first, then per
                                                    // stage 16 columns of A scales and N/8 of B scales
@@ -1067,7 +1069,7 @@ static int gemm_fp4_entry(const uint8_t *a_codes, const uint8_t *a_sf, const uin
     }
     CUtensorMap map_a, map_b;
 
-    if (m <= skinny::MAX_TOKENS && variant == 0 && max_ctas == 0 && !d_peers && n_p / 128 <= INT32_MAX / skinny::MAX_SPLIT) {
+    if (variant == 0 && max_ctas == 0 && !d_peers && skinny::pays(m, n_p, k_p, sms)) {
         skinny::Params q{};
         q.alpha = alpha;
         q.amax_a = p.amax_a; q.amax_b = p.amax_b; q.denom = p.alpha_denom;

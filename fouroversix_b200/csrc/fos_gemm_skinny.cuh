@@ -285,6 +285,17 @@ inline int split_for(int64_t tiles, int k_tiles, int sms) {
     return split;
 }
 
+// Where the kernel is taken (measured against the 128 x 128 tiles of the single-CTA kernel, in a graph, us): K split over a
+// cluster, 16 x 8192 -> 8192 11.5 / 13.0, 8 x 4096 -> 2048 7.1 / 7.5, 32 x 14336 -> 4096 12.5 / 19.4, but with 32 tokens the
+// exchange of the partial sums wants a long K (32 x 8192 -> 8192 12.3 / 13.0; 32 x 4096 -> 4096 8.7 / 7.8); or more tiles than
+// SMs, 32 x 4096 -> 28672 14.9 / 15.6. Short K without a split: 24 x 2880 -> 2880 7.7 / 6.8, not taken.
+inline bool pays(int64_t m, int64_t n_p, int64_t k_p, int sms) {
+    const int k_tiles = static_cast<int>((k_p / 64 + KB_PER_STAGE - 1) / KB_PER_STAGE);
+    const int64_t tiles = n_p / 128;
+    return m <= MAX_TOKENS && tiles <= INT32_MAX / MAX_SPLIT &&
+           (tiles >= sms || (split_for(tiles, k_tiles, sms) > 1 && (m <= 16 || k_tiles >= 32)));
+}
+
 template <int N, typename OUT, bool MX>
 int launch(const CUtensorMap &mw, const CUtensorMap &mx, const CUtensorMap &mws, const CUtensorMap &mxs, const Params &p,
            int64_t tiles, bool dependent, cudaStream_t stream) {

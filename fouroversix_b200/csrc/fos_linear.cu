@@ -57,8 +57,7 @@ extern "C" int fos_linear_forward_bias(const void *x, int x_dtype, int64_t rows,
     if (workspace_bytes < w.total) return FOS_ERR_INVALID_ARGUMENT;
     uint8_t *base = static_cast<uint8_t *>(workspace);
     float *amax = reinterpret_cast<float *>(base + w.amax);
-    const int st = fos_quantize(x, x_dtype, rows, in_features, ld_x, FOS_NVFP4, activation_rule, 0, 0, FOS_SF_TILED, nullptr,
-                                base + w.codes, base + w.sf, amax, 0, stream);
+    const int st = quantize_activation(x, x_dtype, rows, in_features, ld_x, activation_rule, base + w.codes, base + w.sf, amax, stream);
     if (st != FOS_OK) return st;
     const GemmScales scales{amax, w_amax, alpha_divisor(FOS_NVFP4, activation_rule, FOS_NVFP4, weight_rule), bias, true};
     return gemm_nvfp4_chained(base + w.codes, base + w.sf, w_codes, w_sf, scales, out, out_dtype, w.rows_p,

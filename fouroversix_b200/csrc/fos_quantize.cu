@@ -54,6 +54,7 @@ struct QuantParams {
     float fake_divisor;
     // grouped launch (TMA-fed row kernels, grid.y = group): group g is rows group_start[g] .. group_start[g + 1]
     // (device values, multiples of 128) of x and of the outputs, quantized as a tensor of its own with amax[g]
+    int no_padding;               // quantize_small_kernel: the rows beyond out_rows may be left alone
     const int32_t *rows_in_use;   // of each group: its rows beyond these may be left alone (quantize_rows_mse_kernel); or nullptr
     const int32_t *group_start;
     int num_groups;
@@ -1954,9 +1955,12 @@ cudaError_t launch_rows(const QuantParams &p, cudaStream_t stream) {
 // A decoding step packs a few rows (16 x 8192: 256 KB), and the three launches of the general chain (zero the amax
 // word, amax pass, quantize kernel) cost more than the work. Here one cluster of 16 CTAs holds the whole tensor in
 // shared memory: every thread loads its blocks of 16 values once, the CTAs exchange their maxima through distributed
-// shared memory, and the blocks are quantized from shared memory; then the padding is filled in. Bound by latency
-// (one round trip to memory, one cluster barrier, at most SMALL_BLOCKS blocks per thread in sequence); the limit on
-// the size is where the general chain, which has the whole chip, gets ahead.
+// shared memory, and the blocks are quantized from shared memory; the padding is filled in while the maxima travel. Bound
+// by latency (one round trip to memory, two cluster barriers, at most SMALL_BLOCKS blocks per thread in sequence). In a
+// graph (us, this kernel / the general chain, mse): 1 x 1024 3.2 / 3.8, 16 x 2048 4.1 / 4.7, 16 x 8192 4.5 / 4.8,
+// 128 x 2048 4.6 / 5.0, 256 x 1024 4.9 / 5.2; but 32 x 8192 5.7 / 5.1 and 16 x 16384 6.8 / 5.7, where the padding of 16 SMs' worth of
+// threads takes as long as the blocks: two blocks per thread only where no padding is written. Launched one by one, a call
+// is two launches (some 5 us of the host) shorter.
 
 constexpr int SMALL_CTAS = 16, SMALL_THREADS = 512, SMALL_BLOCKS = 2;
 constexpr int64_t SMALL_MAX_BLOCKS = static_cast<int64_t>(SMALL_CTAS) * SMALL_THREADS * SMALL_BLOCKS;
@@ -2000,7 +2004,27 @@ quantize_small_kernel(const QuantParams p, float *amax_out) {
         for (int w = 1; w < SMALL_THREADS / 32; ++w) m = fmaxf(m, warp_max[w]);
         asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(map_to_cta(smem_u32(&cta_max[rank]), tid)), "f"(m) : "memory");
     }
-    cluster_sync_all();
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    // while the maxima travel: the padding rows, zero codes and zero scales (16 bytes and 4 at a time where aligned)
+    if (!p.no_padding) {
+        const int pad_rows = static_cast<int>(p.rows_p - p.out_rows), quads = n_cb >> 2;
+        uint8_t *pad = p.codes + p.out_rows * (p.cols_p >> 1);
+        if (reinterpret_cast<uintptr_t>(pad) % 16 == 0) {
+            for (int i = first; i < pad_rows * (n_cb >> 1); i += STEP) reinterpret_cast<uint4 *>(pad)[i] = make_uint4(0u, 0u, 0u, 0u);
+        } else {
+            for (int i = first; i < pad_rows * n_cb; i += STEP) reinterpret_cast<uint2 *>(pad)[i] = make_uint2(0u, 0u);
+        }
+        const bool words_ok = reinterpret_cast<uintptr_t>(p.sf) % 4 == 0;
+        for (int i = first; i < pad_rows * quads; i += STEP) {
+            // four scales of a row lie side by side in either layout
+            uint8_t *at = p.sf + sf_offset(p.out_rows + i / quads, (i % quads) * 4, n_cb, p.sf_tiled != 0);
+            if (words_ok) *reinterpret_cast<uint32_t *>(at) = 0u;
+            else at[0] = at[1] = at[2] = at[3] = 0;
+        }
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     m = cta_max[0];
 #pragma unroll
     for (int c = 1; c < SMALL_CTAS; ++c) m = fmaxf(m, cta_max[c]);
@@ -2030,24 +2054,15 @@ quantize_small_kernel(const QuantParams p, float *amax_out) {
             p.sf[sf_offset(row, cb, n_cb, p.sf_tiled != 0)] = static_cast<uint8_t>(sf_byte);
         }
     }
-    // the padding rows: zero codes, zero scales
-    const int pad_rows = static_cast<int>(p.rows_p - p.out_rows);
-    uint8_t *pad = p.codes + p.out_rows * (p.cols_p >> 1);
-    for (int i = first; i < pad_rows * n_cb; i += STEP) *reinterpret_cast<uint2 *>(pad + static_cast<int64_t>(i) * 8) = make_uint2(0u, 0u);
-    const int quads = n_cb >> 2;
-    for (int i = first; i < pad_rows * quads; i += STEP) {
-        // four scales of a row lie side by side in either layout
-        uint8_t *at = p.sf + sf_offset(p.out_rows + i / quads, (i % quads) * 4, n_cb, p.sf_tiled != 0);
-        at[0] = at[1] = at[2] = at[3] = 0;
-    }
 }
 
-// True when the tensor qualifies (plain 1-D blocks whose amax this call computes, at most SMALL_MAX_BLOCKS blocks with
-// every thread's blocks in shared memory) and the device takes a cluster of 16 CTAs.
+// True when the tensor qualifies (plain 1-D blocks whose amax this call computes, every thread's blocks in shared memory)
+// and the device takes a cluster of 16 CTAs.
 template <typename T, int KIND>
 cudaError_t launch_small(const QuantParams &p, float *amax_out, cudaStream_t stream, bool *launched) {
     *launched = false;
-    if (p.out_rows * (p.cols_p >> 4) > SMALL_MAX_BLOCKS) return cudaSuccess;
+    const bool pads = !p.no_padding && p.rows_p != p.out_rows;
+    if (p.out_rows * (p.cols_p >> 4) > (pads ? SMALL_MAX_BLOCKS / SMALL_BLOCKS : SMALL_MAX_BLOCKS)) return cudaSuccess;
     auto kernel = quantize_small_kernel<T, KIND>;
     static OncePerDevice configured;
     static int fits[64] = {};
@@ -2263,7 +2278,7 @@ extern "C" int fos_pseudo_quantize(const void *x, int x_dtype, int64_t rows, int
 static int quantize_entry(const void *x, int x_dtype, int64_t rows, int64_t cols, int64_t ld, int format,
                           int scale_rule, int block_2d, int transpose, int sf_layout, const float *amax_in,
                           uint8_t *codes, uint8_t *sf, float *amax_out, int flags, void *stream_, int stochastic,
-                          uint64_t seed) {
+                          uint64_t seed, bool no_padding = false) {
     using namespace fos;
     if (stochastic) {
         // stochastic rounding lives in the TMA-fed kernels only: NVFP4, 1-D blocks, aligned input
@@ -2312,6 +2327,7 @@ static int quantize_entry(const void *x, int x_dtype, int64_t rows, int64_t cols
     p.rht = (flags & FOS_QUANTIZE_RHT) != 0;
     if (p.rht && p.out_cols % 16 != 0) return FOS_ERR_INVALID_ARGUMENT;   // blocks of 16 along the quantized axis
     p.stochastic = stochastic;
+    p.no_padding = no_padding;
     p.unbiased = stochastic && (flags & FOS_QUANTIZE_UNBIASED) != 0;
     p.seed_lo = static_cast<uint32_t>(seed);
     p.seed_hi = static_cast<uint32_t>(seed >> 32);
@@ -2470,6 +2486,12 @@ extern "C" int fos_quantize(const void *x, int x_dtype, int64_t rows, int64_t co
                             uint8_t *codes, uint8_t *sf, float *amax_out, int flags, void *stream) {
     return quantize_entry(x, x_dtype, rows, cols, ld, format, scale_rule, block_2d, transpose, sf_layout, amax_in, codes, sf,
                           amax_out, flags, stream, 0, 0);
+}
+
+int fos::quantize_activation(const void *x, int x_dtype, int64_t rows, int64_t cols, int64_t ld, int scale_rule, uint8_t *codes,
+                             uint8_t *sf, float *amax_out, void *stream) {
+    return quantize_entry(x, x_dtype, rows, cols, ld, FOS_NVFP4, scale_rule, 0, 0, FOS_SF_TILED, nullptr, codes, sf, amax_out, 0, stream,
+                          0, 0, true);
 }
 
 extern "C" int fos_quantize_stochastic(const void *x, int x_dtype, int64_t rows, int64_t cols, int64_t ld, int format,
