@@ -320,7 +320,7 @@ def run_ours(args, rank: int, world: int, local_rank: int) -> None:
     t = time_graphs(lambda i: fos.quantized_matmul(a_sets[i % N_ROTATE], b_dev), N_ROTATE, max(args.steps, 10), 3)
     pipeline["quantize_both_and_multiply"] = {
         "ms": t, "shape": "A 8192x4096 @ B(4096x4096)^T",
-        "note": "fouroversix_b200.quantized_matmul on two bf16 tensors: 2 x (zero, amax, quantize) + alpha + GEMM"}
+        "note": "fouroversix_b200.quantized_matmul on two bf16 tensors: 2 x (zero, amax, quantize) + GEMM"}
     qb = fos.quantize(b_dev)
     t = time_graphs(lambda i: fos.quantized_matmul(a_sets[i % N_ROTATE], qb), N_ROTATE, max(args.steps, 10), 3)
     pipeline["quantize_activation_and_multiply"] = {"ms": t, "note": "weight quantized once, outside the timed region"}
@@ -730,7 +730,7 @@ def run_case(args) -> None:
 
 def experts_pipeline(dev, steps: int) -> dict:
     """The grouped experts layer (32 experts of GPT-OSS-20B shape, 4 per token, uniformly random routing) as CUDA-graph
-    replays: routing tables (2 kernels), gather, 2 x (quantize, alpha, grouped GEMM), SwiGLU, combine - eleven kernels of the
+    replays: routing tables (2 kernels), gather, 2 x (quantize, grouped GEMM), SwiGLU, combine - nine kernels of the
     library and no read-back."""
     from fouroversix_b200.model import FourOverSixExperts
 

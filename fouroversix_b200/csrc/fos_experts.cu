@@ -597,7 +597,7 @@ namespace {
 struct ExpertsWorkspace {
     int64_t capacity, pairs;
     // byte offsets into the workspace, each a multiple of 256
-    int64_t group_start, group_rows, row_token, row_expert, pair_row, pair_expert, route_work, amax, alpha;
+    int64_t group_start, group_rows, row_token, row_expert, pair_row, pair_expert, route_work, amax;
     int64_t rows_x, codes_x, sf_x, gate_up, gated, codes_g, sf_g, y, total;
 };
 
@@ -615,7 +615,6 @@ ExpertsWorkspace experts_workspace(int64_t tokens, int top_k, int num_experts, i
     w.pair_expert = take(4 * w.pairs);
     w.route_work = take(4 * static_cast<int64_t>(FOS_EXPERTS_ROUTE_WORKSPACE_INTS) * num_experts);
     w.amax = take(4 * 2 * num_experts);
-    w.alpha = take(4 * 2 * num_experts);
     w.rows_x = take(2 * w.capacity * hidden);
     w.codes_x = take(w.capacity * hidden / 2);
     w.sf_x = take(w.capacity * hidden / 16);
