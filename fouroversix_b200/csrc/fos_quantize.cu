@@ -1144,7 +1144,8 @@ quantize_rows_kernel(const QuantParams p) {
     uint32_t w[8];
     load_block_words<T>(p, static_cast<int64_t>(tr) * 64 + r_in_tile, tc_ * 4 + cb_in_tile, w);
     // amax comes from the previous kernel in the stream; nothing above needed it. With
-    // programmatic dependent launch this CTA may be running before that kernel has finished.
+    // programmatic dependent launch (behind the amax pass only, see launch_rows) this CTA may be running before that
+    // kernel has finished.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const TensorConsts tc = tensor_consts<KIND>(*reinterpret_cast<const volatile float *>(p.amax), p.rule);
     if (p.amax_store != nullptr && threadIdx.x == 0 && blockIdx.x == 0) *p.amax_store = tc.amax;
@@ -1944,7 +1945,8 @@ cudaError_t launch_rows(const QuantParams &p, cudaStream_t stream) {
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    // (the kernel reads x before it waits, and by read-only loads: only where the kernel before it cannot be x's writer)
+    cfg.numAttrs = p.x_is_ready ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, p);
 }
 
