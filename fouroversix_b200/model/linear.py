@@ -242,10 +242,12 @@ class FourOverSixLinear(nn.Linear):
         need = lib.fos_linear_workspace_bytes(rows, self.in_features)
         workspace = torch.empty(need, dtype=torch.uint8, device=dev)
         out = torch.empty(rows, out_features, dtype=out_dtype, device=dev)
-        # the GEMM adds the bias where nothing has to be recorded for it and the sum is of the output's type
+        # the GEMM adds the bias where nothing has to be recorded for it, the sum is of the output's type and there is one
+        # element per output feature (any other shape is broadcast or refused by the addition)
         bias = self.bias
         fused = (bias is not None and bias.dtype == out_dtype != torch.float32 and bias.device == dev
-                 and bias.is_contiguous() and not (bias.requires_grad and torch.is_grad_enabled()))
+                 and bias.shape == (out_features,) and bias.is_contiguous()
+                 and not (bias.requires_grad and torch.is_grad_enabled()))
         with _native.on_device(dev):
             _native.check(lib.fos_linear_forward_bias(
                 x.data_ptr(), _native.elem_code(x.dtype), rows, self.in_features, x.stride(0),
