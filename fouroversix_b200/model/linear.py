@@ -24,6 +24,7 @@ from typing import Any
 
 import torch
 import torch.nn as nn
+from torch.autograd import forward_ad
 
 from fouroversix_b200 import _native
 from fouroversix_b200.matmul import quantized_matmul
@@ -34,6 +35,13 @@ _TORCH_OUT = {DataType.bfloat16: torch.bfloat16, DataType.float16: torch.float16
 
 from .config import ModuleQuantizationConfig
 from .quantize import QuantizedModule
+
+
+def _is_only_memory(t: torch.Tensor) -> bool:
+    """Whether the elements at the tensor's address are all there is to it: not a subclass with operations of its own, not
+    wrapped by vmap, jvp or another function transform, no forward-mode tangent, no pending negation."""
+    return (type(t) in (nn.Parameter, torch.Tensor) and not torch._C._functorch.is_functorch_wrapped_tensor(t)
+            and forward_ad.unpack_dual(t).tangent is None and not t.is_neg())
 
 
 class FourOverSixLinearFunction(torch.autograd.Function):
@@ -247,7 +255,7 @@ class FourOverSixLinear(nn.Linear):
         bias = self.bias
         fused = (bias is not None and bias.dtype == out_dtype != torch.float32 and bias.device == dev
                  and bias.shape == (out_features,) and bias.is_contiguous()
-                 and not (bias.requires_grad and torch.is_grad_enabled()))
+                 and not (bias.requires_grad and torch.is_grad_enabled()) and _is_only_memory(bias))
         with _native.on_device(dev):
             _native.check(lib.fos_linear_forward_bias(
                 x.data_ptr(), _native.elem_code(x.dtype), rows, self.in_features, x.stride(0),

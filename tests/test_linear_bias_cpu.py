@@ -8,6 +8,7 @@ import ctypes
 import pytest
 import torch
 import torch.nn as nn
+from torch.autograd import forward_ad
 
 import fouroversix_b200 as fos
 from fouroversix_b200 import _native
@@ -63,3 +64,28 @@ def test_a_bias_of_a_wrong_length_is_refused(layer, length):
     _, forward = layer
     with pytest.raises(RuntimeError):
         forward(torch.zeros(length, dtype=torch.bfloat16))
+
+
+def test_a_tangent_of_the_bias_reaches_the_output(layer):
+    entry, forward = layer
+    bias, tangent = torch.randn(24).bfloat16(), torch.randn(24).bfloat16()
+    with forward_ad.dual_level():
+        y, dy = forward_ad.unpack_dual(forward(forward_ad.make_dual(bias, tangent)))
+        assert torch.equal(y, bias.expand(3, 24)) and torch.equal(dy, tangent.expand(3, 24)) and entry.bias == 0
+
+
+def test_a_batch_of_biases(layer):
+    _, forward = layer
+    biases = torch.randn(5, 24).bfloat16()
+    assert torch.equal(torch.func.vmap(forward)(biases), biases[:, None].expand(5, 3, 24))
+
+
+def test_a_bias_with_a_pending_negation_and_one_of_a_subclass(layer):
+    entry, forward = layer
+
+    class Own(torch.Tensor):
+        pass
+
+    bias = torch.randn(24).bfloat16()
+    assert torch.equal(forward(torch._neg_view(bias)), -bias.expand(3, 24)) and entry.bias == 0
+    assert type(forward(bias.as_subclass(Own))) is Own and entry.bias == 0
