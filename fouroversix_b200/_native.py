@@ -89,6 +89,7 @@ SIGNATURES = {
                                      _c_i64, _c_ptr]),
     "fos_gemm_mxfp4": (_c_int, [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_i64, _c_i64, _c_i64,
                                 _c_i64, _c_i64, _c_i64, _c_ptr, _c_ptr]),
+    "fos_gemm_fp4_kernel": (_c_int, [_c_i64, _c_i64, _c_i64, _c_int, _c_ptr, _c_int, _c_ptr]),
     "fos_gemm_nvfp4_ex": (_c_int, [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_i64, _c_i64, _c_i64,
                                    _c_i64, _c_i64, _c_i64, _c_ptr, _c_ptr, _c_ptr]),
     "fos_gemm_mxfp4_ex": (_c_int, [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_i64, _c_i64, _c_i64,

@@ -987,6 +987,35 @@ int launch_out(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &
     return launch<BLOCK_N, float, FUSED_A, GROUPED>(ma, mb, msa, msb, p, sms, stream);
 }
 
+// Which kernel a problem takes (`sms`: the device's; max_ctas as in fos_gemm_opts).
+constexpr int GEMM_SKINNY = 1, GEMM_PAIR = 2, GEMM_128 = 128, GEMM_256 = 256;
+
+inline int sms_allowed(int sms, int max_ctas) { return max_ctas > 0 && max_ctas < sms ? max_ctas : sms; }
+
+// 128 x 256 tiles unless they would fill less than half of the SMs (a 128 x 128 tile takes nine tenths of the
+// time of a 128 x 256 one, so the narrow kernel only pays when it doubles the number of busy SMs); in place of
+// the wide ones 256 x 256 tiles on CTA pairs wherever those need no more rounds (see pairs_pay), unless one CTA is all
+// that is allowed
+inline int gemm_kernel_for(int64_t m, int64_t m_p, int64_t n_p, int64_t k_p, int variant, int max_ctas, bool scatter, int sms) {
+    if (variant == 128 || variant == 256) return variant;
+    if (variant == 0 && max_ctas == 0 && !scatter && skinny::pays(m, n_p, k_p, sms)) return GEMM_SKINNY;
+    sms = sms_allowed(sms, max_ctas);
+    const int64_t tiles_256 = (m_p / BLOCK_M) * ((n_p + 255) / 256), pair_tiles = ((m_p + 255) / 256) * ((n_p + 255) / 256);
+    const bool wide = n_p >= 256 && tiles_256 * 2 > sms;
+    if (!scatter && max_ctas != 1 && (variant == 2 || (wide && pairs_pay(tiles_256, pair_tiles, sms)))) return GEMM_PAIR;
+    return wide ? GEMM_256 : GEMM_128;
+}
+
+// 256-row tiles waste half a tile per group on average, 128-row tiles a quarter of that: pairs where groups are long
+inline int grouped_kernel_for(int64_t rows_capacity, int num_groups, int64_t n_p, int variant, int max_ctas, int sms) {
+    if (variant == 128) return GEMM_128;
+    sms = sms_allowed(sms, max_ctas);
+    const int64_t tiles_256 = (rows_capacity / BLOCK_M) * ((n_p + 255) / 256);
+    const bool wide = n_p >= 256 && (tiles_256 * 2 > sms || variant == 256);
+    if (variant == 0 && wide && max_ctas != 1 && rows_capacity / num_groups >= PAIR_MIN_GROUP_ROWS) return GEMM_PAIR;
+    return wide ? GEMM_256 : GEMM_128;
+}
+
 #ifdef FOS_GEMM_DEBUG
 int g_gemm_debug = 0;     // timing experiments of a debug build (fos_gemm_debug_set)
 #endif
@@ -1002,6 +1031,20 @@ extern "C" int fos_gemm_debug_set(int bits) {
     return FOS_OK;
 }
 #endif
+
+extern "C" int fos_gemm_fp4_kernel(int64_t m, int64_t n, int64_t k, int num_groups, const fos_gemm_opts *opts, int sms, int *k_split) {
+    using namespace fos;
+    const int variant = opts ? opts->variant : 0, max_ctas = opts ? opts->max_ctas : 0;
+    if ((variant != 0 && variant != 128 && variant != 256 && (variant != 2 || num_groups > 0)) || max_ctas < 0 || m <= 0 || n <= 0 ||
+        k <= 0 || num_groups < 0 || sms <= 0)
+        return FOS_ERR_INVALID_ARGUMENT;
+    const int64_t m_p = round_up64(m, 128), n_p = round_up64(n, 128), k_p = round_up64(k, 64);
+    const int kernel = num_groups > 0 ? grouped_kernel_for(m_p, num_groups, n_p, variant, max_ctas, sms)
+                                      : gemm_kernel_for(m, m_p, n_p, k_p, variant, max_ctas, false, sms);
+    if (k_split)
+        *k_split = kernel == GEMM_SKINNY ? skinny::split_for(n_p / 128, static_cast<int>((k_p / 64 + KB_PER_STAGE - 1) / KB_PER_STAGE), sms) : 1;
+    return kernel;
+}
 
 static int gemm_fp4_entry(const uint8_t *a_codes, const uint8_t *a_sf, const uint8_t *b_codes,
                           const uint8_t *b_sf, const float *alpha, void *d, int out_dtype, int64_t m_p,
@@ -1035,7 +1078,7 @@ static int gemm_fp4_entry(const uint8_t *a_codes, const uint8_t *a_sf, const uin
     int dev = 0, sms = 0;
     FOS_CUDA_TRY(cudaGetDevice(&dev));
     FOS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (max_ctas > 0 && max_ctas < sms) sms = max_ctas;   // leave SMs to concurrent kernels
+    const int choice = gemm_kernel_for(m, m_p, n_p, k_p, variant, max_ctas, d_peers != nullptr, sms);
 
 #ifdef FOS_GEMM_DEBUG
     const int debug_bits = g_gemm_debug;
@@ -1069,7 +1112,7 @@ static int gemm_fp4_entry(const uint8_t *a_codes, const uint8_t *a_sf, const uin
     }
     CUtensorMap map_a, map_b;
 
-    if (variant == 0 && max_ctas == 0 && !d_peers && skinny::pays(m, n_p, k_p, sms)) {
+    if (choice == GEMM_SKINNY) {
         skinny::Params q{};
         q.alpha = alpha;
         q.amax_a = p.amax_a; q.amax_b = p.amax_b; q.denom = p.alpha_denom;
@@ -1080,15 +1123,7 @@ static int gemm_fp4_entry(const uint8_t *a_codes, const uint8_t *a_sf, const uin
                   : skinny::launch_n<false>(a_codes, a_sf, b_codes, b_sf, q, out_dtype, m_p, n_p, k_p, sms, scales && scales->chained, stream);
     }
 
-    // 128 x 256 tiles unless they would fill less than half of the SMs (a 128 x 128 tile takes nine tenths of the
-    // time of a 128 x 256 one, so the narrow kernel only pays when it doubles the number of busy SMs); in place of
-    // the wide ones 256 x 256 tiles on CTA pairs wherever those need no more rounds (see pairs_pay)
-    const int64_t tiles_256 = (m_p / BLOCK_M) * ((n_p + 255) / 256), pair_tiles = ((m_p + 255) / 256) * ((n_p + 255) / 256);
-    bool wide = n_p >= 256 && tiles_256 * 2 > sms;
-    const bool use_pair = !d_peers && (variant == 2 || (variant == 0 && wide && pairs_pay(tiles_256, pair_tiles, sms)));
-    if (variant == 128) wide = false;
-    if (variant == 256) wide = true;
-    if (use_pair) {
+    if (choice == GEMM_PAIR) {
         CUtensorMap map_sfa, map_sfb;
         const int tiles = mx ? KB_PER_STAGE / 2 : KB_PER_STAGE;
         if ((st = make_operand_map(&map_a, a_codes, m_p, k_p / 2, 128)) != FOS_OK) return st;
@@ -1098,6 +1133,8 @@ static int gemm_fp4_entry(const uint8_t *a_codes, const uint8_t *a_sf, const uin
         return mx ? launch_pair_out<true>(map_a, map_b, map_sfa, map_sfb, p, max_ctas, stream)
                   : launch_pair_out<false>(map_a, map_b, map_sfa, map_sfb, p, max_ctas, stream);
     }
+    const bool wide = choice == GEMM_256;
+    sms = sms_allowed(sms, max_ctas);                       // leave SMs to concurrent kernels
     if ((st = make_operand_map(&map_a, a_codes, m_p, k_p / 2, BLOCK_M)) != FOS_OK) return st;
     if ((st = make_operand_map(&map_b, b_codes, n_p, k_p / 2, wide ? 256 : 128)) != FOS_OK) return st;
     CUtensorMap map_sfa, map_sfb;
@@ -1218,7 +1255,6 @@ static int gemm_grouped_entry(const uint8_t *a_codes, const uint8_t *a_sf, const
     int dev = 0, sms = 0;
     FOS_CUDA_TRY(cudaGetDevice(&dev));
     FOS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (max_ctas > 0 && max_ctas < sms) sms = max_ctas;
     GemmParams p{};
     p.a_sf = a_sf; p.b_sf = b_sf; p.alpha = alpha; p.d = d; p.status = status;
     p.m_p = rows_capacity; p.n_p = n_p; p.k_p = k_p; p.m = rows_capacity; p.n = n; p.ldd = ldd;
@@ -1238,20 +1274,17 @@ static int gemm_grouped_entry(const uint8_t *a_codes, const uint8_t *a_sf, const
     }
     // how many row blocks are in use is known on the device only: the grid is sized for the buffers, and
     // CTAs that find no tile leave at once
-    const int64_t tiles_256 = (rows_capacity / BLOCK_M) * ((n_p + 255) / 256);
-    bool wide = n_p >= 256 && tiles_256 * 2 > sms;
-    if (variant == 128) wide = false;
-    if (variant == 256 && n_p >= 256) wide = true;
+    const int choice = grouped_kernel_for(rows_capacity, num_groups, n_p, variant, max_ctas, sms);
     CUtensorMap map_a, map_b, map_sfa, map_sfb;
-    // 256-row tiles waste half a tile per group on average, 128-row tiles a quarter of that: pairs where groups are long
-    const bool use_pair = variant == 0 && wide && rows_capacity / num_groups >= PAIR_MIN_GROUP_ROWS;
-    if (use_pair) {
+    if (choice == GEMM_PAIR) {
         if ((st = make_operand_map(&map_a, a_codes, rows_capacity, k_p / 2, 128)) != FOS_OK) return st;
         if ((st = make_operand_map(&map_b, b_codes, b_rows, k_p / 2, 128)) != FOS_OK) return st;
         if ((st = make_scale_map(&map_sfa, a_sf, rows_capacity / 128, k_p / 64, 1, KB_PER_STAGE)) != FOS_OK) return st;
         if ((st = make_scale_map(&map_sfb, b_sf, b_rows / 128, k_p / 64, 2, KB_PER_STAGE)) != FOS_OK) return st;
         return launch_pair_out<false, true>(map_a, map_b, map_sfa, map_sfb, p, max_ctas, stream);
     }
+    const bool wide = choice == GEMM_256;
+    sms = sms_allowed(sms, max_ctas);
     if ((st = make_operand_map(&map_a, a_codes, rows_capacity, k_p / 2, BLOCK_M)) != FOS_OK) return st;
     if ((st = make_operand_map(&map_b, b_codes, b_rows, k_p / 2, wide ? 256 : 128)) != FOS_OK) return st;
     if ((st = make_scale_map(&map_sfa, a_sf, rows_capacity / 128, k_p / 64, 1, KB_PER_STAGE)) != FOS_OK) return st;

@@ -99,7 +99,8 @@ __device__ __forceinline__ void store_columns(OUT *dst, const uint32_t *acc, flo
 }
 
 // Persistent launch of clusters of two CTAs: one pair per `tiles` at most, as many as can be resident, max_ctas CTAs at
-// most (0: no limit); a programmatic dependent of the kernel before it in the stream (see launch_dependent).
+// most (0: no limit; never 1, which leaves no room for a pair); a programmatic dependent of the kernel before it in the
+// stream (see launch_dependent).
 template <typename... Args>
 int launch(void (*kernel)(Args...), int threads, int smem_bytes, int64_t tiles, int max_ctas,
            cudaStream_t stream, const std::decay_t<Args> &...args) {
@@ -137,7 +138,7 @@ int launch(void (*kernel)(Args...), int threads, int smem_bytes, int64_t tiles, 
         }
     }
     int64_t pairs = tiles < clusters ? tiles : clusters;
-    if (max_ctas > 0 && pairs > max_ctas / 2) pairs = max_ctas > 1 ? max_ctas / 2 : 1;
+    if (max_ctas > 0 && pairs > max_ctas / 2) pairs = max_ctas / 2;
     cfg.gridDim = dim3(static_cast<unsigned>(2 * pairs));
     cfg.numAttrs = 2;
     FOS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, args...));

@@ -188,13 +188,15 @@ int fos_gemm_nvfp4(const uint8_t *a_codes, const uint8_t *a_sf, const uint8_t *b
 
 /*
  * Per-call options of the FP4 GEMMs (the library keeps no process-wide settings). NULL = all zero.
- *   variant   0 = choose the kernel per problem; 128 / 256 = single-CTA kernel with 128 x 128 /
- *             128 x 256 tiles; 2 = CTA-pair kernel (256 x 256 tiles, cta_group::2; any size). Every
- *             variant computes the same product; at most 32 rows of A take, with 0, a kernel that
- *             splits K (fp32 sums in a different, fixed order).
+ *   variant   0 = choose the kernel per problem (fos_gemm_fp4_kernel tells which); 128 / 256 =
+ *             single-CTA kernel with 128 x 128 / 128 x 256 tiles; 2 = CTA-pair kernel (256 x 256 tiles,
+ *             cta_group::2; any size; the single-CTA kernel where max_ctas is 1). Every variant
+ *             computes the same product, and those three the same bits.
  *   max_ctas  0 = one persistent CTA per SM; n > 0 = at most n CTAs, which leaves SMs free for a
  *             kernel that must run beside the GEMM (a collective on another stream: a persistent
  *             grid over every SM would keep it waiting until the GEMM has finished).
+ * With both 0, some problems of at most 32 rows of A take a kernel that may split K: fp32 sums in another,
+ * fixed order. Any other variant or limit keeps them on the kernels above, and on their order.
  * No counterpart in the reference (its CUTLASS kernel has one tile shape and takes the whole GPU,
  * src/fouroversix/csrc/fp4_gemm.cu:166-172).
  */
@@ -202,6 +204,13 @@ typedef struct fos_gemm_opts {
     int32_t variant;
     int32_t max_ctas;
 } fos_gemm_opts;
+
+/* The kernel that a problem of m x n x k values takes on a device of `sms` SMs (host arithmetic, no CUDA call): 128 or
+ * 256 = single-CTA kernel of that tile width, 2 = CTA pairs, 1 = the kernel for few rows, with the number of CTAs that share
+ * a tile's K in *k_split (1 for every other kernel; may be NULL). num_groups > 0: fos_gemm_nvfp4_grouped with m rows of capacity. Negative:
+ * status. Both formats and every output type choose alike. No counterpart in the reference. */
+int fos_gemm_fp4_kernel(int64_t m, int64_t n, int64_t k, int num_groups, const fos_gemm_opts *opts, int sms, int *k_split);
+
 int fos_gemm_nvfp4_ex(const uint8_t *a_codes, const uint8_t *a_sf, const uint8_t *b_codes,
                       const uint8_t *b_sf, const float *alpha, void *d, int out_dtype,
                       int64_t m_p, int64_t n_p, int64_t k_p, int64_t m, int64_t n, int64_t ldd,

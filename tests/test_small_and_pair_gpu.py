@@ -125,3 +125,9 @@ def test_grouped_problems_on_cta_pairs(counts, n, k):
         canvas = torch.full((layout.capacity, n), 7.0, dtype=torch.bfloat16, device=DEV)
         outs[variant] = grouped_quantized_matmul(gq, stacked, out_dtype=fos.DataType.bfloat16, out=canvas, variant=variant)
     assert torch.equal(outs[0], outs[256])
+
+
+@pytest.mark.parametrize("variant", [0, 2])
+def test_a_limit_of_one_cta(variant):
+    qx, qw = _operands(300, 600, 320, "nvfp4")
+    assert torch.equal(_run(qx, qw, variant=variant, max_ctas=1), _run(qx, qw, variant=256))
