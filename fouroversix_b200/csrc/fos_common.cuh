@@ -260,6 +260,37 @@ __device__ __forceinline__ void ldg_nc_32(const void *p, uint32_t (&v)[8]) {
                  : "l"(p));
 }
 
+// Loads, behind griddepcontrol.wait, of what the kernel before this one in the stream may still have been writing when
+// this one was launched (a programmatic dependent). __ldg and ld.global.nc promise memory that nobody writes while the
+// kernel runs, and the compiler may move them above the wait; these are coherent, and volatile statements keep their order.
+__device__ __forceinline__ uint32_t ld_b32(const void *p) {
+    uint32_t v;
+    asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint32_t ld_b16(const void *p) {
+    uint16_t v;
+    asm volatile("ld.global.b16 %0, [%1];" : "=h"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ int32_t ld_int(const int32_t *p) { return static_cast<int32_t>(ld_b32(p)); }
+__device__ __forceinline__ float ld_float(const float *p) { return __uint_as_float(ld_b32(p)); }
+__device__ __forceinline__ uint4 ld_16(const void *p) {                        // `p` 16-byte aligned
+    uint4 v;
+    asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint4 ld_16_stream(const void *p) {                 // the same for what is read once
+    uint4 v;
+    asm volatile("ld.global.L1::no_allocate.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void ld_32_stream(const void *p, uint32_t (&v)[8]) {   // `p` 32-byte aligned
+    asm volatile("ld.global.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "l"(p));
+}
+
 // 32-byte store (sm_100 and later); `p` must be 32-byte aligned.
 __device__ __forceinline__ void stg_32(void *p, const uint32_t *v) {
     asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"

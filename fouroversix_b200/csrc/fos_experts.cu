@@ -52,13 +52,6 @@ constexpr int GATHER_CTAS = 6, GLU_CTAS = 4;     // their CTAs per SM (one wave:
 template <typename P> __device__ __forceinline__ P as_pair(uint32_t w) { return *reinterpret_cast<P *>(&w); }
 template <typename P> __device__ __forceinline__ uint32_t as_word(P p) { return *reinterpret_cast<uint32_t *>(&p); }
 
-__device__ __forceinline__ uint4 ldg_stream(const uint4 *p) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
-
 // max |value| of the eight 16-bit numbers of a 16-byte piece, folded into a running packed maximum
 // (NaNs are skipped, as fmaxf skips them in the amax pass of the quantization).
 template <typename P> __device__ __forceinline__ P fold_abs_max(P m, uint4 v) {
@@ -106,9 +99,9 @@ gather_rows_kernel(const uint8_t *__restrict__ x, int64_t ld_x_bytes, const int3
     for (int i = (blockIdx.x * ROW_THREADS + threadIdx.x) >> 5; i < total; i += warps) {
         const int at = units.segs == 1 ? i : i / units.segs, seg = i - at * units.segs;
         const int c_begin = seg * units.seg_chunks, c_end = min(chunks, c_begin + units.seg_chunks);
-        const int r = units.pair_row ? __ldg(units.pair_row + at) : at;
+        const int r = units.pair_row ? ld_int(units.pair_row + at) : at;
         if (r < 0) continue;
-        const int t = units.pair_row ? at / units.top_k : __ldg(row_token + r);
+        const int t = units.pair_row ? at / units.top_k : ld_int(row_token + r);
         uint4 *dst = reinterpret_cast<uint4 *>(out + r * ld_out_bytes);
         if (t < 0) {
             for (int c = c_begin + lane; c < c_end; c += 32) dst[c] = make_uint4(0u, 0u, 0u, 0u);
@@ -119,7 +112,7 @@ gather_rows_kernel(const uint8_t *__restrict__ x, int64_t ld_x_bytes, const int3
         for (int c0 = c_begin + lane; c0 < c_end; c0 += 32 * 4) {             // four loads in flight per lane
             uint4 v[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) v[u] = c0 + 32 * u < c_end ? __ldg(src + c0 + 32 * u) : make_uint4(0u, 0u, 0u, 0u);
+            for (int u = 0; u < 4; ++u) v[u] = c0 + 32 * u < c_end ? ld_16(src + c0 + 32 * u) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 if (c0 + 32 * u < c_end) dst[c0 + 32 * u] = v[u];
@@ -127,7 +120,7 @@ gather_rows_kernel(const uint8_t *__restrict__ x, int64_t ld_x_bytes, const int3
             }
         }
         __syncwarp();
-        if (amax != nullptr) raise_amax<T>(m2, amax + __ldg(units.pair_row ? units.pair_expert + at : row_expert + r), lane);
+        if (amax != nullptr) raise_amax<T>(m2, amax + ld_int(units.pair_row ? units.pair_expert + at : row_expert + r), lane);
     }
 }
 
@@ -187,9 +180,9 @@ glu_kernel(const uint8_t *__restrict__ gate_up, int64_t ld_gu_bytes, const uint8
     for (int i = (blockIdx.x * ROW_THREADS + threadIdx.x) >> 5; i < total; i += warps) {
         const int at = units.segs == 1 ? i : i / units.segs, seg = i - at * units.segs;
         const int c_begin = seg * units.seg_chunks, c_end = min(chunks, c_begin + units.seg_chunks);
-        const int row = units.pair_row ? __ldg(units.pair_row + at) : at;
+        const int row = units.pair_row ? ld_int(units.pair_row + at) : at;
         if (row < 0) continue;
-        const int e = __ldg(units.pair_row ? units.pair_expert + at : row_expert + row);
+        const int e = ld_int(units.pair_row ? units.pair_expert + at : row_expert + row);
         uint4 *dst = reinterpret_cast<uint4 *>(out + row * ld_out_bytes);
         if (e < 0) {
             for (int c = c_begin + lane; c < c_end; c += 32) dst[c] = make_uint4(0u, 0u, 0u, 0u);
@@ -203,10 +196,10 @@ glu_kernel(const uint8_t *__restrict__ gate_up, int64_t ld_gu_bytes, const uint8
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 const int c = c0 + 32 * u < c_end ? c0 + 32 * u : c0;
-                g[u][0] = ldg_stream(src + 2 * c);
-                g[u][1] = ldg_stream(src + 2 * c + 1);
-                w[u][0] = __ldg(b + 2 * c);
-                w[u][1] = __ldg(b + 2 * c + 1);
+                g[u][0] = ld_16_stream(src + 2 * c);
+                g[u][1] = ld_16_stream(src + 2 * c + 1);
+                w[u][0] = ld_16(b + 2 * c);
+                w[u][1] = ld_16(b + 2 * c + 1);
             }
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
@@ -244,8 +237,8 @@ combine_kernel(const uint8_t *__restrict__ y, int64_t ld_y_bytes, const uint8_t 
         if (threadIdx.x == 0) {                           // insertion sort of the token's slots by expert
             for (int k = 0; k < top_k; ++k) {
                 const int64_t i = static_cast<int64_t>(t) * top_k + k;
-                const int e = __ldg(pair_expert + i), r = __ldg(pair_row + i);
-                const uint32_t w = __ldg(pair_weight + i);
+                const int e = ld_int(pair_expert + i), r = ld_int(pair_row + i);
+                const uint32_t w = ld_b16(pair_weight + i);
                 int j = k;
                 for (; j > 0 && s_ex[j - 1] > e; --j) { s_ex[j] = s_ex[j - 1]; s_row[j] = s_row[j - 1]; s_w[j] = s_w[j - 1]; }
                 s_ex[j] = e; s_row[j] = r; s_w[j] = w | (w << 16);
@@ -257,8 +250,8 @@ combine_kernel(const uint8_t *__restrict__ y, int64_t ld_y_bytes, const uint8_t 
             uint32_t acc[4] = {0u, 0u, 0u, 0u};
             for (int k = 0; k < top_k; ++k) {
                 if (s_row[k] < 0) continue;               // a slot whose expert index was out of range
-                const uint4 v = ldg_stream(reinterpret_cast<const uint4 *>(y + s_row[k] * ld_y_bytes) + c);
-                const uint4 b = __ldg(reinterpret_cast<const uint4 *>(bias + s_ex[k] * ld_bias_bytes) + c);
+                const uint4 v = ld_16_stream(reinterpret_cast<const uint4 *>(y + s_row[k] * ld_y_bytes) + c);
+                const uint4 b = ld_16(reinterpret_cast<const uint4 *>(bias + s_ex[k] * ld_bias_bytes) + c);
                 const P w2 = as_pair<P>(s_w[k]);
                 const uint32_t vv[4] = {v.x, v.y, v.z, v.w}, bb[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
@@ -286,7 +279,9 @@ constexpr int ROUTE_THREADS = 256, ROUTE_WARPS = ROUTE_THREADS / 32, ROUTE_MAX_E
 template <typename IDX>
 __device__ __forceinline__ int route_expert_of(const IDX *__restrict__ routing, int p, int end, int experts) {
     if (p >= end) return -1;
-    const long long e = static_cast<long long>(routing[p]);
+    long long e;
+    if constexpr (sizeof(IDX) == 8) asm volatile("ld.global.b64 %0, [%1];" : "=l"(e) : "l"(routing + p));
+    else e = ld_int(reinterpret_cast<const int32_t *>(routing + p));
     return (e >= 0 && e < experts) ? static_cast<int>(e) : -1;
 }
 
@@ -335,7 +330,7 @@ route_place_kernel(const IDX *__restrict__ routing, int pairs, int seg, int top_
     if (tid < experts) {
         int total = 0;
         for (int sgm = 0; sgm < static_cast<int>(gridDim.x); ++sgm) {
-            const int n = __ldg(seg_count + sgm * experts + tid);
+            const int n = ld_int(seg_count + sgm * experts + tid);
             total += n;
             if (sgm < static_cast<int>(blockIdx.x)) before += n;
         }

@@ -475,7 +475,7 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         // ------------------------------------------------------------------ epilogue (both CTAs)
         const int quad = warp & 3, half = (warp - 2) >> 2;
         asm volatile("griddepcontrol.wait;" ::: "memory");     // alpha, and whoever still reads d
-        const float alpha = __ldg(p.alpha);
+        const float alpha = ld_float(p.alpha);
         OUT *out = static_cast<OUT *>(p.d);
         const bool vec16 = (reinterpret_cast<uintptr_t>(out) % 16 == 0) && ((p.ldd * sizeof(OUT)) % 16 == 0);
         const bool vec32 = (reinterpret_cast<uintptr_t>(out) % 32 == 0) && ((p.ldd * sizeof(OUT)) % 32 == 0);

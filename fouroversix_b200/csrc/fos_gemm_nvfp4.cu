@@ -129,9 +129,9 @@ struct GemmParams {
 };
 
 __device__ __forceinline__ float gemm_alpha(const GemmParams &p, int group = 0) {
-    if (p.alpha) return __ldg(p.alpha + group);
+    if (p.alpha) return ld_float(p.alpha + group);
     if (!p.amax_a) return 1.0f;
-    return __fdiv_rn(__fmul_rn(*static_cast<const volatile float *>(p.amax_a + group), __ldg(p.amax_b + group)), p.alpha_denom);
+    return __fdiv_rn(__fmul_rn(ld_float(p.amax_a + group), ld_float(p.amax_b + group)), p.alpha_denom);
 }
 
 // GROUPED: first row of every group (and one past the last group), and one past each group's last valid row.
@@ -148,14 +148,14 @@ template <int THREADS> __device__ __forceinline__ void load_groups(const GemmPar
     for (int g0 = 0; g0 <= p.num_groups; g0 += THREADS) {
         const int g = g0 + static_cast<int>(threadIdx.x);
         if (g <= p.num_groups) {
-            int32_t s0 = __ldg(p.group_start + g);
+            int32_t s0 = ld_int(p.group_start + g);
             s0 = (s0 < 0 ? 0 : (s0 > cap ? cap : s0)) & ~127;             // never beyond the buffers
             groups.start[g] = s0;
             if (g < p.num_groups) {
                 // valid rows end inside the group's own range, whatever group_rows claims
-                int32_t s1 = __ldg(p.group_start + g + 1);
+                int32_t s1 = ld_int(p.group_start + g + 1);
                 s1 = (s1 < s0 ? s0 : (s1 > cap ? cap : s1)) & ~127;
-                const int32_t r = __ldg(p.group_rows + g), e = s0 + (r < 0 ? 0 : r);
+                const int32_t r = ld_int(p.group_rows + g), e = s0 + (r < 0 ? 0 : r);
                 groups.end[g] = e > s1 ? s1 : e;
             }
         }
@@ -412,7 +412,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         uint32_t a_s = 0, a_ph = 0, a_j = 0, a_w = 0;
         const int e_tid = static_cast<int>(threadIdx.x) - 64, a_row = e_tid >> 1, a_half = e_tid & 1;
         if constexpr (FUSED_A) {
-            qc = static_quant_consts(__ldg(p.x_amax), p.x_rule);
+            qc = static_quant_consts(ld_float(p.x_amax), p.x_rule);
             if (e_tid < 128) a_lut[e_tid] = static_scale_entry(e_tid, qc.decode);
             asm volatile("bar.sync 1, 256;" ::: "memory");
         }
@@ -429,7 +429,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     for (int b = 0; b < 8; ++b) {
                         const int64_t col = col0 + 16 * b;
                         if (x_row < p.m && col < p.k_p) {
-                            ldg_nc_32(static_cast<const uint16_t *>(p.x) + x_row * p.x_ld + col, w[b]);
+                            ld_32_stream(static_cast<const uint16_t *>(p.x) + x_row * p.x_ld + col, w[b]);
                         } else {
 #pragma unroll
                             for (int i = 0; i < 8; ++i) w[b][i] = 0u;

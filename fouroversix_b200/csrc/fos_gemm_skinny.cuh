@@ -237,9 +237,9 @@ gemm_fp4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         cluster_sync_all();       // all partial sums have arrived
     }
     if (warp >= 2 && ok) {
-        const float alpha = p.alpha ? __ldg(p.alpha)
+        const float alpha = p.alpha ? ld_float(p.alpha)
                             : !p.amax_a ? 1.0f
-                                        : __fdiv_rn(__fmul_rn(*static_cast<const volatile float *>(p.amax_a), __ldg(p.amax_b)), p.denom);
+                                        : __fdiv_rn(__fmul_rn(ld_float(p.amax_a), ld_float(p.amax_b)), p.denom);
         const int f = tile * 128 + feature;
         const bool f_ok = f < p.n;
         const OUT *bias = static_cast<const OUT *>(p.bias);

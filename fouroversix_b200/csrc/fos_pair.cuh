@@ -13,7 +13,7 @@ namespace {
 // rounds once from the exact sum, which is what adding in binary32 and rounding gives for two 16-bit numbers.
 template <typename OUT> __device__ __forceinline__ uint32_t add_bias(uint32_t word, const OUT *bias, int64_t left) {
     const uint16_t *b = reinterpret_cast<const uint16_t *>(bias);
-    const uint32_t lo = left > 0 ? __ldg(b) : 0u, hi = left > 1 ? __ldg(b + 1) : 0u, both = lo | (hi << 16);
+    const uint32_t lo = left > 0 ? ld_b16(b) : 0u, hi = left > 1 ? ld_b16(b + 1) : 0u, both = lo | (hi << 16);
     if constexpr (std::is_same<OUT, __half>::value) {
         const __half2 r = __hadd2_rn(*reinterpret_cast<const __half2 *>(&word), *reinterpret_cast<const __half2 *>(&both));
         return *reinterpret_cast<const uint32_t *>(&r);
@@ -73,7 +73,7 @@ __device__ __forceinline__ void store_columns(OUT *dst, const uint32_t *acc, flo
                 if constexpr (sizeof(OUT) == 2) {
                     if (i % 2 == 0) pk[i / 2] = add_bias<OUT>(pk[i / 2], bias + c + i, here - i);
                 } else {
-                    if (i < here) pk[i] = __float_as_uint(__uint_as_float(pk[i]) + __ldg(bias + c + i));
+                    if (i < here) pk[i] = __float_as_uint(__uint_as_float(pk[i]) + ld_float(bias + c + i));
                 }
             }
         }

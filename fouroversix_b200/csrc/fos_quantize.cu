@@ -1098,28 +1098,31 @@ __global__ void __launch_bounds__(CTA_THREADS) quantize_kernel(const QuantParams
 
 constexpr int ROWS_CTA_THREADS = 256;
 
-// The 16 values of block (row, cb) as eight words of two 16-bit elements; zeros outside x.
-template <typename T>
+// The 16 values of block (row, cb) as eight words of two 16-bit elements; zeros outside x. COHERENT: x may have been written
+// while this kernel was already resident (see ld_b32).
+template <typename T, bool COHERENT = false>
 __device__ __forceinline__ void load_block_words(const QuantParams &p, int64_t row, int64_t cb, uint32_t (&w)[8]) {
     const T *x = static_cast<const T *>(p.x);
     const int64_t col0 = cb * 16;
     if (row < p.out_rows && col0 + 16 <= p.out_cols && p.vec_bytes != 0) {
         const T *src = x + row * p.ld + col0;
         if (p.vec_bytes == 32) {
-            ldg_nc_32(src, w);
+            if constexpr (COHERENT) ld_32_stream(src, w);
+            else ldg_nc_32(src, w);
         } else {
-            const uint4 a = ldg_nc_16(src), b = ldg_nc_16(src + 8);
+            const uint4 a = COHERENT ? ld_16_stream(src) : ldg_nc_16(src), b = COHERENT ? ld_16_stream(src + 8) : ldg_nc_16(src + 8);
             w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
             w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
         }
     } else {
         const uint16_t *xs = reinterpret_cast<const uint16_t *>(x);
+        auto at = [&](int64_t i) -> uint32_t { return COHERENT ? ld_b16(xs + i) : xs[i]; };
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             uint32_t lo = 0u, hi = 0u;
             if (row < p.out_rows) {
-                if (col0 + 2 * k < p.out_cols) lo = xs[row * p.ld + col0 + 2 * k];
-                if (col0 + 2 * k + 1 < p.out_cols) hi = xs[row * p.ld + col0 + 2 * k + 1];
+                if (col0 + 2 * k < p.out_cols) lo = at(row * p.ld + col0 + 2 * k);
+                if (col0 + 2 * k + 1 < p.out_cols) hi = at(row * p.ld + col0 + 2 * k + 1);
             }
             w[k] = lo | (hi << 16);
         }
@@ -1223,7 +1226,7 @@ constexpr int FEED_SMEM_BYTES = FEED_STAGES * FEED_STAGE_BYTES + 1024;
 // the buffers.
 __device__ __forceinline__ void group_tiles(const QuantParams &p, int &tile_r0, int &tiles_r, const float *&amax_ptr) {
     const int all = static_cast<int>(p.rows_p >> 7);
-    int t0 = __ldg(p.group_start + blockIdx.y) >> 7, t1 = __ldg(p.group_start + blockIdx.y + 1) >> 7;
+    int t0 = ld_int(p.group_start + blockIdx.y) >> 7, t1 = ld_int(p.group_start + blockIdx.y + 1) >> 7;
     t0 = t0 < 0 ? 0 : (t0 > all ? all : t0);
     t1 = t1 < t0 ? t0 : (t1 > all ? all : t1);
     tile_r0 = t0;
@@ -1561,7 +1564,7 @@ quantize_rows_mse_kernel(const __grid_constant__ CUtensorMap map_x, const QuantP
             // (the arrive below releases this store to the consumers that acquire the barrier's phase)
             tile_meta[s] = make_longlong2(static_cast<int64_t>(tr) * 128 * code_ld + tc_ * 32,
                                           p.sf_tiled ? tile * 512 : static_cast<int64_t>(tr) * 128 * n_cb + tc_ * 4);
-            if constexpr (IN_USE) tile_rows[s] = __ldg(p.rows_in_use + blockIdx.y) - (tr - tile_r0) * FEED_TILE_ROWS;
+            if constexpr (IN_USE) tile_rows[s] = ld_int(p.rows_in_use + blockIdx.y) - (tr - tile_r0) * FEED_TILE_ROWS;
             mbar_expect_tx(smem_u32(&full_bar[s]), FEED_STAGE_BYTES);
             tma_load_2d(stage0 + s * FEED_STAGE_BYTES, &map_x, tc_ * 128, tr * FEED_TILE_ROWS, smem_u32(&full_bar[s]));
             if (++s == FEED_STAGES) { s = 0; parity ^= 1u; }
@@ -1989,7 +1992,7 @@ quantize_small_kernel(const QuantParams p, float *amax_out) {
     for (int j = 0; j < SMALL_BLOCKS; ++j) {
         const int i = first + j * STEP;
         uint32_t w[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-        if (i < total) load_block_words<T>(p, i / n_cb, i % n_cb, w);
+        if (i < total) load_block_words<T, true>(p, i / n_cb, i % n_cb, w);
         const uint4 a = make_uint4(w[0], w[1], w[2], w[3]), b = make_uint4(w[4], w[5], w[6], w[7]);
         words[j][0][tid] = a;
         words[j][1][tid] = b;

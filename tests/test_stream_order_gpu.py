@@ -46,3 +46,53 @@ def test_quantize_with_a_given_amax_behind_the_writer_of_its_input(first_column,
             want = B200QuantizeBackend.quantize(view, cfg, amax=amax, kernel=kernel)
         else:
             assert _same(B200QuantizeBackend.quantize(view, cfg, amax=amax, kernel=kernel), want)
+
+
+def test_product_right_behind_the_kernel_that_packs_its_second_operand():
+    """The amax word of a small second operand is written at the end of the kernel before the GEMM."""
+    g = torch.Generator(device=DEV).manual_seed(5)
+    qx = fos.quantize(torch.randn(256, 512, generator=g, device=DEV).bfloat16())
+    ws = [(torch.randn(256, 512, generator=g, device=DEV) * 2.0 ** i).bfloat16() for i in range(-4, 4)]
+    want = []
+    for w in ws:
+        qw = fos.quantize(w)
+        torch.cuda.synchronize()
+        want.append(fos.quantized_matmul(qx, qw))
+    for w, y in zip(ws, want, strict=True):
+        assert torch.equal(fos.quantized_matmul(qx, w), y)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16], ids=["bf16", "fp16"])
+@pytest.mark.parametrize("columns", [512, 509])
+def test_small_tensor_right_behind_its_writer(columns, dtype):
+    g = torch.Generator(device=DEV).manual_seed(columns)
+    x = torch.randn(64, 512, generator=g, device=DEV).to(dtype)
+    for i in range(8):
+        rows = torch.randint(64, (128,), generator=g, device=DEV, dtype=torch.int32)
+        out = torch.full((128, 512), 3.0, dtype=dtype, device=DEV)
+        _gather(x, rows, out)
+        got = fos.quantize(out[:, :columns])
+        torch.cuda.synchronize()
+        assert _same(got, fos.quantize(out[:, :columns])), i
+
+
+def test_experts_layer_with_another_routing_each_time():
+    from fouroversix_b200.model.experts import FourOverSixExperts
+
+    g = torch.Generator(device=DEV).manual_seed(8)
+    e, h, i, tokens = 8, 512, 256, 96
+    weights = [torch.randn(*s, generator=g, device=DEV).mul(0.05).bfloat16() for s in ((e, 2 * i, h), (e, 2 * i), (e, h, i), (e, h))]
+    layer = FourOverSixExperts(*weights)
+    calls = []
+    with torch.no_grad():
+        for _ in range(6):
+            x = torch.randn(tokens, h, generator=g, device=DEV).bfloat16()
+            scores, indices = torch.randn(tokens, e, generator=g, device=DEV).topk(2)
+            calls.append((x, indices, scores.softmax(-1).bfloat16()))
+        want = []
+        for c in calls:
+            want.append(layer(*c))
+            torch.cuda.synchronize()
+        got = [layer(*c) for c in calls]
+    for y, z in zip(got, want, strict=True):
+        assert torch.equal(y, z)
