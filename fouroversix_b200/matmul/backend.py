@@ -108,7 +108,7 @@ class B200MatmulBackend:
                     raise _native.NativeLibraryError(
                         f"fos_gemm_mxfp4: a bounded device-side wait timed out (site {int(status.item())})")
                 return out
-            unbiased_a, unbiased_b = (int(t.round_style is RoundStyle.stochastic_unbiased) for t in (input, other))
+            unbiased_a, unbiased_b = (int(t.round_style == RoundStyle.stochastic_unbiased) for t in (input, other))
             if native_fp4:
                 _native.check(lib.fos_gemm_nvfp4_scaled(
                     a_vals.data_ptr(), a_sf.data_ptr(), input.amax.data_ptr(), input.scale_rule.cuda_id, unbiased_a,

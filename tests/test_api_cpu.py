@@ -188,3 +188,24 @@ def test_experts_routing_tables_on_the_host():
     for e in range(6):
         mine, pairs = rows[expert == e], order[expert == e]
         assert (mine[1:] > mine[:-1]).all() and (pairs[1:] > pairs[:-1]).all()
+
+
+@pytest.mark.parametrize("style", ["stochastic_unbiased", fos.RoundStyle.stochastic_unbiased, "nearest"])
+def test_product_knows_an_unbiased_operand_by_the_value_of_its_round_style(monkeypatch, style):
+    """The 16/17 factor in alpha; the attribute may have been set to the style's name."""
+    from fouroversix_b200.matmul import B200MatmulBackend
+
+    seen = {}
+
+    class Entry:
+        def fos_gemm_nvfp4_scaled(self, *args):
+            seen["unbiased"] = args[4], args[9]
+            return 0
+
+    monkeypatch.setattr(_native, "lib", Entry)
+    monkeypatch.setattr(_native, "stream_ptr", lambda device: 0)
+    q, r = (fos.QuantizedTensor(torch.zeros(128, 32, dtype=torch.uint8), torch.zeros(512).to(torch.float8_e4m3fn), torch.ones(1), "nvfp4",
+                                (128, 64), "mse", "nearest", (128, 64)) for _ in range(2))
+    q.round_style = style
+    B200MatmulBackend._quantized_matmul(q, r, out_dtype=fos.DataType.bfloat16)
+    assert seen["unbiased"] == (int(style != "nearest"), 0)
