@@ -526,7 +526,7 @@ int launch_f16(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &
     const int64_t tiles = (p.m_p / BLOCK_M) * ((p.n_p + BLOCK_N - 1) / BLOCK_N);
     const int64_t pair_tiles = ((p.m_p + 255) / 256) * ((p.n_p + 255) / 256);
     if (pairs_pay(tiles, pair_tiles, sms))
-        return pair::launch(gemm_f16_pair_kernel<OUT>, THREADS, PAIR_SMEM_BYTES, pair_tiles, 0, stream, ma, mb_pair, p);
+        return pair::launch<gemm_f16_pair_kernel<OUT>>(THREADS, PAIR_SMEM_BYTES, pair_tiles, 0, stream, ma, mb_pair, p);
     auto kernel = gemm_f16_kernel<OUT>;
     static OncePerDevice configured;   // per instantiation
     FOS_CUDA_TRY(configured.run(dev, [&] {

@@ -950,8 +950,9 @@ int launch_pair(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap 
                 const GemmParams &p, int max_ctas, cudaStream_t stream) {
     // (grouped: at most one more row tile per group than the buffer has)
     const int64_t row_tiles = (p.m_p + 255) / 256 + (GROUPED ? p.num_groups : 0);
-    return pair::launch(pair::gemm_fp4_pair_kernel<OUT, MX, GROUPED>, pair::THREADS, pair::PairCfg<MX>::SMEM_BYTES,
-                        row_tiles * ((p.n_p + 255) / 256), max_ctas, stream, ma, mb, msa, msb, p);
+    return pair::launch<pair::gemm_fp4_pair_kernel<OUT, MX, GROUPED>>(pair::THREADS, pair::PairCfg<MX>::SMEM_BYTES,
+                                                                      row_tiles * ((p.n_p + 255) / 256), max_ctas, stream,
+                                                                      ma, mb, msa, msb, p);
 }
 
 template <bool MX, bool GROUPED = false>

@@ -2,8 +2,6 @@
 // an epilogue, the launch (sm_100a).
 #pragma once
 
-#include <vector>
-
 #include "fos_tcgen05.cuh"
 
 namespace fos {
@@ -101,13 +99,11 @@ __device__ __forceinline__ void store_columns(OUT *dst, const uint32_t *acc, flo
 // Persistent launch of clusters of two CTAs: one pair per `tiles` at most, as many as can be resident, max_ctas CTAs at
 // most (0: no limit; never 1, which leaves no room for a pair); a programmatic dependent of the kernel before it in the
 // stream (see launch_dependent).
-template <typename... Args>
-int launch(void (*kernel)(Args...), int threads, int smem_bytes, int64_t tiles, int max_ctas,
-           cudaStream_t stream, const std::decay_t<Args> &...args) {
-    struct Resident { void (*kernel)(Args...); int device, clusters; };
-    static std::vector<Resident> resident;     // per kernel and device: how many pairs can be resident at once
-    static std::mutex mu;
-    int dev = 0;
+template <auto KERNEL, typename... Args>
+int launch(int threads, int smem_bytes, int64_t tiles, int max_ctas, cudaStream_t stream, const Args &...args) {
+    static OncePerDevice configured;           // per kernel
+    static int resident[64] = {};              // pairs that can be resident at once
+    int dev = 0, clusters = 0;
     FOS_CUDA_TRY(cudaGetDevice(&dev));
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(static_cast<unsigned>(threads));
@@ -122,26 +118,23 @@ int launch(void (*kernel)(Args...), int threads, int smem_bytes, int64_t tiles, 
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    int clusters = 0;
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        for (const Resident &r : resident)
-            if (r.kernel == kernel && r.device == dev) clusters = r.clusters;
-        if (clusters == 0) {
-            FOS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
-            int sms = 0;
-            FOS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-            cfg.gridDim = dim3(static_cast<unsigned>(sms & ~1));
-            FOS_CUDA_TRY(cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg));
-            if (clusters < 1) clusters = 1;
-            resident.push_back({kernel, dev, clusters});
-        }
-    }
+    const bool kept = dev >= 0 && dev < 64;
+    FOS_CUDA_TRY(configured.run(dev, [&] {
+        cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
+        int sms = 0;
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cfg.gridDim = dim3(static_cast<unsigned>(sms & ~1));
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, KERNEL, &cfg);
+        if (e == cudaSuccess && kept) resident[dev] = clusters;
+        return e;
+    }));
+    if (kept) clusters = resident[dev];
+    if (clusters < 1) clusters = 1;
     int64_t pairs = tiles < clusters ? tiles : clusters;
     if (max_ctas > 0 && pairs > max_ctas / 2) pairs = max_ctas / 2;
     cfg.gridDim = dim3(static_cast<unsigned>(2 * pairs));
     cfg.numAttrs = 2;
-    FOS_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, args...));
+    FOS_CUDA_TRY(cudaLaunchKernelEx(&cfg, KERNEL, args...));
     return FOS_OK;
 }
 
