@@ -2089,12 +2089,15 @@ cudaError_t launch_small(const QuantParams &p, float *amax_out, cudaStream_t str
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     e = configured.run(dev, [&] {
-        cudaError_t r = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (r != cudaSuccess) return r;
+        // (a device that takes no such cluster says so by zero or by an error: either way the general kernels run)
         int n = 0;
-        r = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
-        fits[dev] = r == cudaSuccess && n > 0;
-        return r;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+            (void)cudaGetLastError();
+            n = 0;
+        }
+        fits[dev] = n > 0;
+        return cudaSuccess;
     });
     if (e != cudaSuccess) return e;
     if (!fits[dev]) return cudaSuccess;
