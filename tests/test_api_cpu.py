@@ -56,6 +56,15 @@ def test_argument_validation_needs_no_gpu():
     assert lib.fos_experts_workspace_bytes(0, 4, 32, 2880, 2880) == -1
     # a linear layer as one call: NULL buffers; the workspace holds the packed activation of the padded shape
     assert lib.fos_linear_forward(0, 0, 16, 8192, 8192, 3, 0, 0, 0, 3, 8192, 0, 0, 8192, 0, 0, None, 0, 0) == -1
+    for out_type, bias, status in ((0, 0, -1), (2, 256, -2)):     # a bias with fp32 output is not an option
+        assert lib.fos_linear_forward_bias(*([256] if bias else [0]), 0, 16, 8192, 8192, 3, *([256] * 3 if bias else [0] * 3), 3, 8192, bias,
+                                           256 if bias else 0, out_type, 8192, 256 if bias else 0, 0, None, 0, 0) == status
+    # products that form alpha themselves: NULL operands, NULL amax words, a K that is no multiple of its block
+    gemm = [128, 128, 64, 128, 128, 128]                         # m_p, n_p, k_p, m, n, ldd
+    assert lib.fos_gemm_nvfp4_scaled(0, 0, 0, 3, 0, 0, 0, 0, 3, 0, 0, 0, *gemm, None, 0, 0) == -1
+    assert lib.fos_gemm_nvfp4_scaled(256, 256, 256, 3, 0, 256, 256, 0, 3, 0, 256, 0, *gemm, None, 0, 0) == -1
+    assert lib.fos_gemm_mxfp4_unscaled(0, 0, 0, 0, 0, 0, *gemm, None, 0, 0) == -1
+    assert lib.fos_gemm_mxfp4_unscaled(256, 256, 256, 256, 256, 0, *gemm, None, 0, 0) == -1          # 64: half a scale tile
     need = lib.fos_linear_workspace_bytes(16, 8200)
     assert need % 256 == 0 and need >= 128 * 8256 // 2 + 128 * 8256 // 16 + 8
     assert lib.fos_linear_workspace_bytes(16, 0) == -1

@@ -34,3 +34,15 @@ def test_a_named_variant_is_taken():
     for m, n, k in ((1, 8192, 8192), (4096, 10240, 8192), (100, 100, 64)):
         assert [choice(m, n, k, variant=v)[0] for v in (128, 256, 2)] == [NARROW, WIDE, PAIRS]
     assert choice(100, 100, 64, variant=3)[0] == -1 and choice(0, 100, 64)[0] == -1 and choice(512, 512, 64, 2, variant=2)[0] == -1
+
+
+def test_where_the_kernel_for_few_rows_is_taken():
+    """Up to 16 rows from 16 stages of K (256 values each), 17 to 32 from 32; any K where there are more tiles than SMs."""
+    for m, n, k, kernel in ((16, 1000, 3841, FEW_ROWS), (16, 1000, 3840, NARROW), (17, 1000, 7937, FEW_ROWS), (17, 1000, 7936, NARROW),
+                            (32, 1000, 7937, FEW_ROWS), (33, 1000, 16384, NARROW), (32, 128 * SMS, 64, FEW_ROWS),
+                            (32, 128 * (SMS - 1), 64, NARROW)):
+        assert choice(m, n, k)[0] == kernel, (m, n, k)
+        assert choice(m, n, k, max_ctas=SMS)[0] != FEW_ROWS and choice(m, n, k, variant=128)[0] != FEW_ROWS
+    # K is shared by as many CTAs as are resident at once (two per SM), each keeping eight stages, eight at most
+    assert [choice(16, n, 16384)[1] for n in (8, 128 * 37, 128 * 38, 128 * 74, 128 * 75, 128 * SMS)] == [8, 8, 4, 4, 2, 2]
+    assert [choice(16, 8, k)[1] for k in (4096, 8191, 8192, 16384, 1 << 20)] == [2, 4, 4, 8, 8]

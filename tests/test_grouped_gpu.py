@@ -198,9 +198,10 @@ def test_glu_kernel_keeps_every_rounding_of_the_operation_chain(dtype):
     gu = torch.stack([gates, ups], dim=1).reshape(rows, 2 * inter).contiguous()
     bias = (torch.randn(3, 2 * inter, generator=g) * 0.5).to(dtype).to(DEV)
     bias[0] = 0
-    row_expert = (torch.arange(rows, device=DEV) % 4 - 1).to(torch.int32)          # -1: a padding row
-    # alpha = 1 with no bias and no effective limit feeds every 16-bit pattern to the sigmoid itself (expert 0)
-    for alpha, limit in ((1.702, 7.0), (0.3333, 2.7182818), (1.0, 3.0e38)):
+    # -1: a padding row, every fourth; shifted by one row the second time, so that every pattern lies in a row in use once
+    # alpha = 1 with no bias and no effective limit feeds every 16-bit pattern to the sigmoid itself
+    for alpha, limit, shift in ((1.702, 7.0, 0), (0.3333, 2.7182818, 0), (0.3333, 2.7182818, 1), (1.0, 3.0e38, 0), (1.0, 3.0e38, 1)):
+        row_expert = ((torch.arange(rows, device=DEV) + shift) % 4 - 1).to(torch.int32)
         if alpha == 1.0:
             bias.zero_()
         out = torch.full((rows, inter), 9, dtype=dtype, device=DEV)

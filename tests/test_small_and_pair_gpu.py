@@ -4,11 +4,14 @@ reference."""
 
 from __future__ import annotations
 
+import ctypes
+
 import pytest
 import torch
 import torch.nn as nn
 
 import fouroversix_b200 as fos
+from fouroversix_b200 import _native
 from fouroversix_b200.matmul import B200MatmulBackend
 from fouroversix_b200.quantize.backend import B200QuantizeBackend
 
@@ -36,10 +39,29 @@ def _run(qx, qw, out_dtype="float32", **kw):
     return B200MatmulBackend.quantized_matmul(qx, qw, out_dtype=fos.DataType(out_dtype), check_status=True, **kw)
 
 
+FEW_ROWS, PAIRS, SINGLE_128 = 1, 2, 128
+
+
+def _kernel(m, n, k):
+    """(kernel, CTAs that share a tile's K) of a problem on this device."""
+    split = ctypes.c_int(0)
+    sms = torch.cuda.get_device_properties(DEV).multi_processor_count
+    return _native.lib().fos_gemm_fp4_kernel(m, n, k, 0, None, sms, ctypes.byref(split)), split.value
+
+
 @pytest.mark.parametrize("fmt", ["nvfp4", "mxfp4"])
-@pytest.mark.parametrize("m,n,k", [(1, 8, 64), (16, 130, 1984), (17, 1000, 2048), (32, 264, 4096), (33, 128, 4160), (64, 384, 8192),
-                                   (65, 1024, 4032), (128, 136, 16384)])
-def test_few_tokens(m, n, k, fmt):
+@pytest.mark.parametrize("m,n,k,kernel", [
+    # the kernel for few rows: 16 and 32 token columns, splits of 2, 4 and 8 and none (more tiles than SMs), features and K
+    # that end inside a tile and a stage
+    (1, 8, 4096, (FEW_ROWS, 2)), (1, 136, 4160, (FEW_ROWS, 2)), (16, 392, 4032, (FEW_ROWS, 2)), (16, 130, 8128, (FEW_ROWS, 4)),
+    (16, 1000, 8192, (FEW_ROWS, 4)), (7, 264, 16384, (FEW_ROWS, 8)), (17, 520, 8256, (FEW_ROWS, 4)), (32, 1032, 14336, (FEW_ROWS, 4)),
+    (31, 264, 16448, (FEW_ROWS, 8)), (16, 18952, 1088, (FEW_ROWS, 1)), (32, 19000, 1024, (FEW_ROWS, 1)), (3, 18945, 64, (FEW_ROWS, 1)),
+    # the 128 x 128 tiles of the single-CTA kernel
+    (1, 8, 64, (SINGLE_128, 1)), (16, 130, 1984, (SINGLE_128, 1)), (17, 1000, 2048, (SINGLE_128, 1)), (32, 264, 4096, (SINGLE_128, 1)),
+    (33, 128, 4160, (SINGLE_128, 1)), (64, 384, 8192, (SINGLE_128, 1)), (65, 1024, 4032, (SINGLE_128, 1)),
+    (128, 136, 16384, (SINGLE_128, 1))])
+def test_few_tokens(m, n, k, kernel, fmt):
+    assert _kernel(m, n, k) == kernel
     qx, qw = _operands(m, n, k, fmt)
     want = _exact(qx, qw)
     canvas = torch.full((m + 1, n + 8), 7.0, device=DEV)
@@ -49,6 +71,7 @@ def test_few_tokens(m, n, k, fmt):
     for t in ("bfloat16", "float16"):
         assert torch.equal(_run(qx, qw, t), out.to(getattr(torch, t)))
     assert torch.equal(_run(qx, qw), out)                                  # the partial sums are added in a fixed order
+    assert ((_run(qx, qw, variant=128) - out).abs().max() / want.abs().max()).item() < SUM_ORDER
 
 
 @pytest.mark.parametrize("fmt", ["nvfp4", "mxfp4"])
@@ -94,18 +117,24 @@ def test_small_tensors_equal_the_general_kernels(rows, cols, dtype, rule):
         assert torch.equal(got.scale_factors.view(torch.uint8), want.scale_factors.view(torch.uint8))
 
 
-@pytest.mark.parametrize("tokens", [5, 100, 333])
+@pytest.mark.parametrize("tokens,k,kernel", [(5, 8192, (FEW_ROWS, 4)), (32, 8192, (FEW_ROWS, 4)), (5, 2880, (SINGLE_128, 1)),
+                                             (100, 2880, (SINGLE_128, 1)), (333, 2880, (SINGLE_128, 1)), (2100, 1024, (PAIRS, 1))])
 @pytest.mark.parametrize("dtype", ["bfloat16", "float16"])
-def test_bias_added_by_the_gemm(tokens, dtype):
+def test_bias_added_by_the_gemm(tokens, k, kernel, dtype):
+    """5000 features: the last tile of every kernel ends inside a piece of its columns."""
+    assert _kernel(tokens, 5000, k) == kernel
     t = getattr(torch, dtype)
     torch.manual_seed(tokens)
-    layer = nn.Linear(2880, 5000, bias=True, device=DEV, dtype=t)
+    layer = nn.Linear(k, 5000, bias=True, device=DEV, dtype=t)
     fl = fos.FourOverSixLinear(layer, fos.ModuleQuantizationConfig(output_dtype=dtype)).quantize_weight_()
-    x = torch.randn(tokens, 2880, device=DEV, dtype=t)
+    x = torch.randn(tokens, k, device=DEV, dtype=t)
     recorded = fl(x)                                       # the bias wants a gradient: added outside
     assert recorded.requires_grad
     with torch.no_grad():
-        assert torch.equal(fl(x), recorded.detach())
+        fused = fl(x)
+        assert torch.equal(fused, recorded.detach())
+        fl.bias, bias = None, fl.bias
+        assert torch.equal(fused, fl(x) + bias)
 
 
 @pytest.mark.parametrize("counts", [(1000, 0, 1281, 127, 1792, 1), (640, 900)])
