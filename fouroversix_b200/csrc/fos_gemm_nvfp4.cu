@@ -27,15 +27,19 @@
 //               32x128b.warpx4 (a 512-byte tile is 32 rows of 16 bytes, which every 32-lane
 //               quadrant of tensor memory needs: the copy broadcasts it) into a ring of scale
 //               columns, one slot per scale stage, taking stages in turn, and tcgen05.commit
-//               the slot's `ready` barrier. Issued from the MMA warp the copies queue up in
-//               line with the MMAs (372 us at 8192^3); from warps of their own they overlap
-//               them, and two warps issue them faster than one (235 -> 219 us).
+//               the slot's `ready` barrier. Issued from this kernel's MMA warp, behind a wait
+//               per stage, the copies queued up in line with the MMAs (372 us at 8192^3); from warps
+//               of their own they overlap them, and two warps issue them faster than one (235 ->
+//               219 us). (The CTA-pair kernel below does issue them from its MMA warp: two SMs share
+//               that warp's waits, and its barriers are probed a stage ahead.)
 //
-// What bounds the kernel (8192^3, parts switched off in a -DFOS_GEMM_DEBUG build): MMAs alone
-// 150 us, loads alone 148, loads + MMAs 176, everything 219. The scale copies are the largest
-// single cost: twelve per stage, each about 30 ns of the copying warp and about 14 cycles of the
-// tensor pipe that no MMA gets. Loads and MMAs together lose 26 us to the round trip of a stage
-// (four 48 KB stages cannot cover it) and to the shared-memory port both use.
+// What bounds the kernel: 218 us at 8192^3 (K 8192, 128 x 256 tiles). Parts switched off in a
+// -DFOS_GEMM_DEBUG build, before the MMA warp probed its barriers a stage ahead: MMAs alone 150 us,
+// loads alone 148, loads + MMAs 176, everything 219. The scale copies are the largest single cost: twelve per stage, each
+// about 30 ns of the copying warp and about 14 cycles of the tensor pipe that no MMA gets.
+// Loads and MMAs together lose 26 us to the round trip of a stage (four 48 KB stages cannot cover
+// it) and to the shared-memory port both use. The probes gain where few stages are in flight per tile:
+// 16 x 8192 -> 8192 with 128 x 128 tiles 15.5 -> 13.0 us.
 //
 // Every mbarrier wait is bounded (in SM cycles). A wait that gives up records where
 // in *status, raises a CTA-wide abort flag, and all roles fall through to the common exit,
@@ -58,8 +62,15 @@ constexpr int SF_LEAD = FOS_GEMM_SF_LEAD;   // 0 or 1: how many stages the scale
 
 constexpr int SF_CP_WARPS = 2;                     // warps 10 and 11 issue the scale copies, taking stages in turn
 constexpr int NUM_THREADS = 384;                   // warps: 0 TMA, 1 MMA, 2-9 epilogue (FUSED_A: also the A operand), 10-11 scale copies
-// Grouped launches: CTA pairs from this many rows of the buffer per group (us, pairs / 128-row tiles: 1152 rows, 32 groups of
-// K 2880, N 5760 300 / 324, N 2880 155 / 192; 640 rows, 8 groups of K 1024, N 2048 11.7 / 11.7).
+// Grouped launches: CTA pairs from this many rows of the buffer per group (padding included: the host knows no other number; a
+// group's own share of it is 127 rows on average). In a graph, random routing, us, pairs / the better of the 128-row tiles:
+//   buffer rows                 192    256    320    384    448    512    576    640    768    896    1152   1664
+//   32 groups, 2880 -> 5760   72/59  76/74  79/87 106/109 137/124 140/152 143/158 168/181 203/219 231/252 292/325 412/465
+//   32 groups, 2880 -> 2880   50/43  46/50  48/60  57/68  73/75  75/86  77/94  92/108 107/129 123/146 155/193 215/277
+//    8 groups, 4096 -> 4096   26/22  25/27  25/27  30/33  35/33  36/38  36/40  41/41  48/48  55/56  65/72  92/99
+//   16 groups, 1024 -> 2048   12/9   12/12  12/12  15/15  17/15  18/16  17/19  18/19  23/23  23/26  28/33  38/42
+// From 640 on pairs are never behind by more than 2 %; below, it depends on how the groups' own rows fall (a group of 257 to
+// 384 rows leaves half a pair idle), which the host does not know.
 constexpr int PAIR_MIN_GROUP_ROWS = 640;
 constexpr int MAX_GROUPS = 256;                    // of a grouped launch (their row ranges are kept in shared memory)
 constexpr int SF_COL0 = 256;                       // tensor-memory columns: accumulators first, then per

@@ -1,12 +1,12 @@
-// FP4 GEMM for at most 128 tokens (decoding): D[t, f] = alpha * sum_k X[t, k] * W[f, k] (+ bias[f]).
+// FP4 GEMM for at most 32 tokens (decoding; which problems: pays()): D[t, f] = alpha * sum_k X[t, k] * W[f, k] (+ bias[f]).
 //
 // What bounds it is the weight's way out of HBM, so the weight is the M operand (128 rows of a tile, nothing of it
-// padding) and the tokens are the N operand (16 / 32 / 64 / 128 columns): per stage a CTA fetches 16 KB of weight,
-// 2 KB of its scales and 1/8 to 1/1 of that for the tokens, where the general kernel would fetch and multiply a
-// 128-row tile of padding for 16 tokens. Two CTAs per SM keep about 200 KB of loads in flight.
+// padding) and the tokens are the N operand (16 or 32 columns): per stage a CTA fetches 16 KB of weight, 2 KB of its
+// scales and 4 to 6 KB for the tokens, where the general kernel would fetch and multiply a 128-row tile of padding
+// for 16 tokens. Two CTAs per SM keep about 200 KB of loads in flight.
 // A projection has few 128-row tiles (64 at 8192 features), so K is split over the S CTAs of a cluster, which add up
 // their partial sums through distributed shared memory in the order of K: no atomics, no workspace, the same bits
-// every time. S = 1 when K is short (every CTA keeps at least SKINNY_MIN_STAGES stages).
+// every time. S = 1 when K is short (every CTA keeps at least MIN_STAGES stages; see split_for).
 // Launched as the programmatic dependent of the kernel that packs the tokens, the CTAs fetch their first
 // stages of weight while that kernel still runs, and wait for it before they touch anything it writes.
 //
@@ -64,19 +64,10 @@ __device__ __forceinline__ float lds_f32(uint32_t addr) {
     return v;
 }
 
-template <typename OUT> __device__ __forceinline__ float out_value(float v) {
-    if constexpr (std::is_same<OUT, __half>::value) return __half2float(__float2half_rn(v));
-    else if constexpr (std::is_same<OUT, __nv_bfloat16>::value) return __bfloat162float(__float2bfloat16_rn(v));
-    else return v;
-}
 template <typename OUT> __device__ __forceinline__ OUT to_out(float v) {
     if constexpr (std::is_same<OUT, __half>::value) return __float2half_rn(v);
     else if constexpr (std::is_same<OUT, __nv_bfloat16>::value) return __float2bfloat16_rn(v);
     else return v;
-}
-template <typename OUT> __device__ __forceinline__ float from_out(OUT v) {
-    if constexpr (std::is_same<OUT, float>::value) return v;
-    else return elem_to_float<OUT>(v);
 }
 
 template <int N, typename OUT, bool MX>
@@ -243,15 +234,21 @@ gemm_fp4_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         const int f = tile * 128 + feature;
         const bool f_ok = f < p.n;
         const OUT *bias = static_cast<const OUT *>(p.bias);
-        const float b = bias && f_ok ? from_out<OUT>(bias[f]) : 0.0f;
+        float b = 0.0f;
+        if constexpr (sizeof(OUT) == 2) {                     // (no entry takes a bias with fp32 output)
+            if (bias && f_ok) b = elem_to_float<OUT>(bias[f]);
+        }
         OUT *out = static_cast<OUT *>(p.d) + f;
         const int t0 = split > 1 ? part * n_part : 0;
         auto put = [&](int c, float sum) {
             const int t = t0 + c;
             if (!f_ok || t >= p.m) return;
-            const float v = alpha * sum;
-            // the bias is added to the value rounded to the output's type, as a separate addition would
-            out[t * p.ldd] = to_out<OUT>(bias ? out_value<OUT>(v) + b : v);
+            OUT v = to_out<OUT>(alpha * sum);
+            if constexpr (sizeof(OUT) == 2) {
+                // the bias is added to the value rounded to the output's type, as a separate addition would
+                if (bias) v = to_out<OUT>(elem_to_float<OUT>(v) + b);
+            }
+            out[t * p.ldd] = v;
         };
         if (split > 1) {
             for (int c = 0; c < n_part; ++c) {

@@ -46,8 +46,8 @@ __device__ __forceinline__ void tc_commit_pair_local(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// `N` columns (a multiple of 16) of the accumulator row of this lane, scaled, converted and stored: 16 columns
-// (32 or 64 bytes) at a time.
+// `N` columns (a multiple of 16) of the accumulator row of this lane, scaled, converted, a 16-bit bias added, and stored: 16
+// columns (32 or 64 bytes) at a time.
 template <typename OUT, int N>
 __device__ __forceinline__ void store_columns(OUT *dst, const uint32_t *acc, float alpha, const OUT *bias, int64_t left, bool vec32,
                                               bool vec16) {
@@ -65,14 +65,10 @@ __device__ __forceinline__ void store_columns(OUT *dst, const uint32_t *acc, flo
                 pk[i] = __float_as_uint(alpha * __uint_as_float(acc[c + i]));
             }
         }
-        if (bias) {
+        if constexpr (sizeof(OUT) == 2) {                     // (no entry takes a bias with fp32 output)
+            if (bias) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                if constexpr (sizeof(OUT) == 2) {
-                    if (i % 2 == 0) pk[i / 2] = add_bias<OUT>(pk[i / 2], bias + c + i, here - i);
-                } else {
-                    if (i < here) pk[i] = __float_as_uint(__uint_as_float(pk[i]) + ld_float(bias + c + i));
-                }
+                for (int i = 0; i < 8; ++i) pk[i] = add_bias<OUT>(pk[i], bias + c + 2 * i, here - 2 * i);
             }
         }
         OUT *at = dst + c;

@@ -1611,7 +1611,7 @@ quantize_rows_mse_kernel(const __grid_constant__ CUtensorMap map_x, const QuantP
         asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(code_off), "=l"(sf_off) : "r"(meta_addr + 16 * s_idx));
         uint8_t *codes = code_ptr + code_off;
         uint8_t *sf = sf_ptr + sf_off;
-        // (the tile's rows in use are read where they are needed: a register kept for them would spill)
+        // (the tile's rows in use are read where they are needed: kept in a register they spill 16 bytes, read here 12)
         const bool any_in_use = !IN_USE || warp * 8 < rows_in_use_at(tile_rows, s_idx);
 #pragma unroll
         for (int j = 0; j < 2 && any_in_use; ++j) {

@@ -224,7 +224,7 @@ class FourOverSixLinear(nn.Linear):
 
     def _one_call_forward_applies(self, input: torch.Tensor, w: QuantizedTensor | nn.Parameter | None = None) -> bool:
         """Inference on a packed NVFP4 weight with the plain activation settings (NVFP4, 1-D blocks, round to
-        nearest): the case `fos_linear_forward` covers. Everything else (training, master weights, other formats,
+        nearest): the case `fos_linear_forward_bias` covers. Everything else (training, master weights, other formats,
         fake quantization) goes through the autograd function."""
         cfg = self.config
         if (cfg.keep_master_weights or cfg.disable_fprop_quantization or cfg.pseudo_quantize
@@ -242,7 +242,7 @@ class FourOverSixLinear(nn.Linear):
                 and w.scale_factors.is_contiguous())
 
     def _forward_one_call(self, input: torch.Tensor, w: QuantizedTensor) -> torch.Tensor:
-        """`fos_linear_forward`: amax pass, activation quantization and the GEMM enqueued by one host call
+        """`fos_linear_forward_bias`: amax pass, activation quantization and the GEMM enqueued by one host call
         (the bits of `quantized_matmul(input, weight)`; at decode sizes the call-by-call form is bound by the
         interpreter)."""
         x = input if input.dim() == 2 else input.reshape(-1, self.in_features)

@@ -346,8 +346,9 @@ int fos_gemm_nvfp4_grouped(const uint8_t *a_codes, const uint8_t *a_sf, const ui
  * routing mask and its per-expert read-back of lines 286-303.
  */
 /*
- * fos_experts_forward: the whole layer in one host call - the four calls above around two fos_quantize_grouped /
- * fos_gemm_alpha_grouped / fos_gemm_nvfp4_grouped chains, eleven kernels enqueued on `stream` without a read-back:
+ * fos_experts_forward: the whole layer in one host call - what the four calls above compute around two
+ * fos_quantize_grouped / fos_gemm_nvfp4_grouped chains (alpha formed in the GEMM), nine kernels enqueued on `stream`
+ * without a read-back:
  *   out[t] = sum over the token's experts e (ascending) of
  *            (glu(x[t] @ gate_up[e]^T + gate_up_bias[e]) @ down[e]^T + down_bias[e]) * routing_weights[t][slot]
  * with both products in NVFP4 (activations quantized per expert with `activation_rule`, the weights packed

@@ -52,7 +52,7 @@ def test_ptq_linear_forward_matches_dequantized_matmul():
 @pytest.mark.parametrize("shape,k,n,rule,out", [((16,), 8192, 8192, "mse", "bfloat16"), ((3, 41), 520, 392, "static_6", "float16"),
                                                 ((300,), 1024, 2880, "mae", "float32")])
 def test_one_call_forward_equals_the_call_by_call_forward(shape, k, n, rule, out):
-    """Inference on a packed weight takes `fos_linear_forward` (one host call); the autograd function quantizes and
+    """Inference on a packed weight takes `fos_linear_forward_bias` (one host call); the autograd function quantizes and
     multiplies call by call. Same kernels, same bits - ragged rows, a width that is not a multiple of 64, a bias."""
     from fouroversix_b200.model.linear import FourOverSixLinearFunction
 
