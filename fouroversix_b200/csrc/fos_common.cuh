@@ -36,6 +36,20 @@ int dequantize_mxfp4(const uint8_t *codes, const uint8_t *sf, int sf_layout, int
 // because no row of a product depends on another.
 int quantize_activation(const void *x, int x_dtype, int64_t rows, int64_t cols, int64_t ld, int scale_rule, uint8_t *codes,
                         uint8_t *sf, float *amax_out, void *stream);
+// The steps of a chain over tensors that were complete before its first kernel: the maxima of up to three 16-byte aligned
+// tensors (row stride and columns multiples of 8) of one type in one launch, into words[0 .. n_words) which are zeroed first
+// (a job's words lie among them), then fos_quantize / fos_quantize_stochastic (NVFP4, tiled scales) of one of them at a
+// time with its word. Every kernel of the chain waits for the one before it, so x is not waited for again.
+struct AmaxJob {
+    const void *x;
+    int64_t rows, cols, ld;
+    float *plain;            // max |x|, or nullptr
+    float *rotated;          // max |x^T rotated along x's rows| (rows % 16 == 0), or nullptr
+};
+int amax_of_tensors(const AmaxJob *jobs, int count, int x_dtype, float *words, int n_words, void *stream);
+int quantize_in_chain(const void *x, int x_dtype, int64_t rows, int64_t cols, int64_t ld, int scale_rule, int block_2d,
+                      int transpose, int flags, int stochastic, uint64_t seed, float *amax, uint8_t *codes, uint8_t *sf,
+                      void *stream);
 // fos_quantize_grouped for callers that read no product of a padding row: what comes out there is not defined.
 int quantize_grouped_rows_in_use(const void *x, int x_dtype, int64_t rows_capacity, int64_t cols, int64_t ld, int format,
                                  int scale_rule, const int32_t *group_start, const int32_t *group_rows, int num_groups,

@@ -72,14 +72,14 @@ __device__ __forceinline__ float abs_max8(uint4 w) {
                  fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fmaxf(fabsf(d.x), fabsf(d.y))));
 }
 
-// Sets the amax word to zero. A kernel rather than a memset so that the chain "previous kernel ->
+// Sets the amax word (of a training step: words, at most 32) to zero. A kernel rather than a memset so that the chain "previous kernel ->
 // this -> amax pass -> quantize kernel" consists of kernels only and every link can be a
 // programmatic dependent launch: this kernel may be scheduled while the previous one drains, it
 // waits for that kernel's completion (amax_out may still be read by it, and x may be written by
 // it), and only then lets the amax pass start.
-__global__ void zero_amax_kernel(float *amax) {
+__global__ void zero_amax_kernel(float *amax, int words) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (threadIdx.x == 0) *amax = 0.0f;
+    if (threadIdx.x < words) amax[threadIdx.x] = 0.0f;
 }
 
 // max |x| of the chunks (VB bytes each) that one thread owns: 128 bytes per thread in flight per
@@ -315,10 +315,11 @@ template <typename T> __device__ __forceinline__ float rotated_max(float m) {
 }
 
 // max |rotated x^T| before the last factor and rounding, the rotation running along x's rows: a thread takes the blocks of two
-// neighbouring columns (4-byte loads, coalesced over a row) of units tid, tid + stride, ...
-template <typename T>
+// neighbouring columns (4-byte loads, coalesced over a row) of units tid, tid + stride, ... With PLAIN also max |x| of
+// what it reads, in `plain`.
+template <typename T, bool PLAIN>
 __device__ __forceinline__ float rotated_column_pairs(const T *__restrict__ x, int64_t rows, int64_t cols, int64_t ld, int64_t tid,
-                                                      int64_t stride) {
+                                                      int64_t stride, float &plain) {
     const int64_t per_row = cols >> 1, step_r = stride / per_row, step_c = stride - step_r * per_row, bands = rows >> 4;
     int64_t r = tid / per_row, c = tid - r * per_row;
     float m = 0.0f;
@@ -327,6 +328,10 @@ __device__ __forceinline__ float rotated_column_pairs(const T *__restrict__ x, i
         uint32_t p[16], w0[8], w1[8];
 #pragma unroll
         for (int i = 0; i < 16; ++i) p[i] = __ldg(src + i * (ld >> 1));
+        if constexpr (PLAIN) {
+#pragma unroll
+            for (int i = 0; i < 16; i += 4) plain = fmaxf(plain, abs_max8<T>(make_uint4(p[i], p[i + 1], p[i + 2], p[i + 3])));
+        }
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             w0[k] = __byte_perm(p[2 * k], p[2 * k + 1], 0x5410);
@@ -364,7 +369,8 @@ __global__ void __launch_bounds__(256, 4) amax_rht_kernel(const T *__restrict__ 
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     if (transposed && wide) {
-        m = rotated_column_pairs<T>(x, rows, cols, ld, tid, stride);
+        float unused = 0.0f;
+        m = rotated_column_pairs<T, false>(x, rows, cols, ld, tid, stride, unused);
     } else {
         const int64_t per_row = transposed ? cols : cols >> 4, step = transposed ? ld : 1;
         const int64_t units = (transposed ? rows >> 4 : rows) * per_row;
@@ -386,6 +392,47 @@ __global__ void __launch_bounds__(256, 4) amax_rht_kernel(const T *__restrict__ 
     __shared__ float warp_max[8];
     m = cta_max_of(m, warp_max);
     if (threadIdx.x == 0) atomicMax(reinterpret_cast<int *>(amax), __float_as_int(rotated_max<T>(m)));
+}
+
+// The maxima of several tensors in one launch (a training step quantizes two or three tensors at a time, one of them in two
+// forms): CTAs first_cta[j] .. first_cta[j + 1] share job j, the grid is one wave. `rotated`: max |rotated x^T|, the rotation
+// running along x's rows (rotated_column_pairs); a tensor that is also wanted as it is, in `plain`, is read once
+// for both. Same launch chain as amax_kernel. Vector width 16 bytes (32 where x allows).
+constexpr int MAX_AMAX_JOBS = 3;
+struct AmaxJobs {
+    AmaxJob job[MAX_AMAX_JOBS];
+    int first_cta[MAX_AMAX_JOBS + 1];
+};
+
+template <typename T>
+__global__ void __launch_bounds__(256, 4) amax_jobs_kernel(const AmaxJobs jobs) {
+    int j = 0;
+#pragma unroll
+    for (int i = 1; i < MAX_AMAX_JOBS; ++i) j += static_cast<int>(blockIdx.x) >= jobs.first_cta[i] ? 1 : 0;
+    const AmaxJob job = jobs.job[j];
+    const T *x = static_cast<const T *>(job.x);
+    const int64_t tid = (static_cast<int>(blockIdx.x) - jobs.first_cta[j]) * static_cast<int64_t>(256) + threadIdx.x;
+    const int64_t stride = (jobs.first_cta[j + 1] - jobs.first_cta[j]) * static_cast<int64_t>(256);
+    float plain = 0.0f, rotated = 0.0f;
+    if (job.rotated != nullptr) {
+        rotated = job.plain != nullptr ? rotated_column_pairs<T, true>(x, job.rows, job.cols, job.ld, tid, stride, plain)
+                                       : rotated_column_pairs<T, false>(x, job.rows, job.cols, job.ld, tid, stride, plain);
+    } else if (reinterpret_cast<uintptr_t>(x) % 32 == 0 && job.ld % 16 == 0 && job.cols % 16 == 0) {
+        plain = amax_chunks<T, 32>(x, job.rows, job.cols, job.ld, tid, stride);
+    } else {
+        plain = amax_chunks<T, 16>(x, job.rows, job.cols, job.ld, tid, stride);
+    }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    __shared__ float warp_max[8];
+    if (job.plain != nullptr) {
+        plain = cta_max_of(plain, warp_max);
+        if (threadIdx.x == 0) atomicMax(reinterpret_cast<int *>(job.plain), __float_as_int(plain));
+    }
+    if (job.rotated != nullptr) {
+        rotated = cta_max_of(rotated, warp_max);
+        if (threadIdx.x == 0) atomicMax(reinterpret_cast<int *>(job.rotated), __float_as_int(rotated_max<T>(rotated)));
+    }
 }
 
 // ------------------------------------------------------------------------------------
@@ -2334,7 +2381,7 @@ cudaError_t launch_amax(const void *x, int64_t rows, int64_t cols, int64_t ld, b
                         cudaStream_t stream, bool rht = false, bool transposed = false) {
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg = dependent_launch_config(1, 32, stream, attr);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, zero_amax_kernel, amax);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, zero_amax_kernel, amax, 1);
     if (e != cudaSuccess) return e;
     if (rht) {
         // amax of the ROTATED tensor: one wave of the four CTAs per SM
@@ -2382,6 +2429,34 @@ cudaError_t launch_amax(const void *x, int64_t rows, int64_t cols, int64_t ld, b
     if (blocks < 1) blocks = 1;
     cfg = dependent_launch_config(static_cast<unsigned>(blocks), 256, stream, attr);
     return cudaLaunchKernelEx(&cfg, amax_kernel<T>, static_cast<const T *>(x), rows, cols, ld, vec, amax);
+}
+
+template <typename T>
+cudaError_t launch_amax_jobs(const AmaxJob *jobs, int count, float *words, int n_words, cudaStream_t stream) {
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    AmaxJobs a{};
+    int64_t total = 0;
+    for (int j = 0; j < count; ++j) total += jobs[j].rows * jobs[j].cols;
+    // CTAs by size; a thread takes 64 values at a time, so no job gets more CTAs than it has such pieces
+    int at = 0;
+    for (int j = 0; j < count; ++j) {
+        a.job[j] = jobs[j];
+        a.first_cta[j] = at;
+        const int64_t values = jobs[j].rows * jobs[j].cols, most = (values + 256 * 64 - 1) / (256 * 64);
+        const int64_t share = static_cast<int64_t>(static_cast<double>(values) / static_cast<double>(total) * (4 * sms));
+        at += static_cast<int>(share < 1 ? 1 : (share < most ? share : most));
+    }
+    for (int j = count; j <= MAX_AMAX_JOBS; ++j) a.first_cta[j] = at;
+    cudaLaunchAttribute attr[1];
+    cudaLaunchConfig_t cfg = dependent_launch_config(1, 32, stream, attr);
+    e = cudaLaunchKernelEx(&cfg, zero_amax_kernel, words, n_words);
+    if (e != cudaSuccess) return e;
+    cfg = dependent_launch_config(static_cast<unsigned>(at), 256, stream, attr);
+    return cudaLaunchKernelEx(&cfg, amax_jobs_kernel<T>, a);
 }
 
 template <typename T>
@@ -2447,7 +2522,7 @@ extern "C" int fos_pseudo_quantize(const void *x, int x_dtype, int64_t rows, int
 static int quantize_entry(const void *x, int x_dtype, int64_t rows, int64_t cols, int64_t ld, int format,
                           int scale_rule, int block_2d, int transpose, int sf_layout, const float *amax_in,
                           uint8_t *codes, uint8_t *sf, float *amax_out, int flags, void *stream_, int stochastic,
-                          uint64_t seed, bool no_padding = false) {
+                          uint64_t seed, bool no_padding = false, bool x_is_ready = false) {
     using namespace fos;
     if (stochastic) {
         // stochastic rounding lives in the TMA-fed kernels only: NVFP4, 1-D blocks, aligned input
@@ -2525,7 +2600,7 @@ static int quantize_entry(const void *x, int x_dtype, int64_t rows, int64_t cols
     }
     // When this call launched the amax pass itself, the kernel before the quantize kernel is that
     // pass: it does not write x, so x can be fetched while it drains.
-    p.x_is_ready = amax_in == nullptr;
+    p.x_is_ready = amax_in == nullptr || x_is_ready;
 
     FOS_CUDA_TRY(x_dtype == FOS_BF16
                      ? launch_all<__nv_bfloat16>(p, kind, block_2d != 0, transpose != 0, stream)
@@ -2661,6 +2736,21 @@ int fos::quantize_activation(const void *x, int x_dtype, int64_t rows, int64_t c
                              uint8_t *sf, float *amax_out, void *stream) {
     return quantize_entry(x, x_dtype, rows, cols, ld, FOS_NVFP4, scale_rule, 0, 0, FOS_SF_TILED, nullptr, codes, sf, amax_out, 0, stream,
                           0, 0, true);
+}
+
+int fos::amax_of_tensors(const AmaxJob *jobs, int count, int x_dtype, float *words, int n_words, void *stream_) {
+    if (count < 1 || count > MAX_AMAX_JOBS || n_words > 32) return FOS_ERR_INVALID_ARGUMENT;
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    FOS_CUDA_TRY(x_dtype == FOS_BF16 ? launch_amax_jobs<__nv_bfloat16>(jobs, count, words, n_words, stream)
+                                     : launch_amax_jobs<__half>(jobs, count, words, n_words, stream));
+    return FOS_OK;
+}
+
+int fos::quantize_in_chain(const void *x, int x_dtype, int64_t rows, int64_t cols, int64_t ld, int scale_rule, int block_2d,
+                           int transpose, int flags, int stochastic, uint64_t seed, float *amax, uint8_t *codes, uint8_t *sf,
+                           void *stream) {
+    return quantize_entry(x, x_dtype, rows, cols, ld, FOS_NVFP4, scale_rule, block_2d, transpose, FOS_SF_TILED, amax, codes, sf, amax,
+                          flags, stream, stochastic, seed, false, true);
 }
 
 extern "C" int fos_quantize_stochastic(const void *x, int x_dtype, int64_t rows, int64_t cols, int64_t ld, int format,

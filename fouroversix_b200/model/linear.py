@@ -29,7 +29,7 @@ from torch.autograd import forward_ad
 from fouroversix_b200 import _native
 from fouroversix_b200.matmul import quantized_matmul
 from fouroversix_b200.quantize import QuantizedTensor, dequantize, quantize
-from fouroversix_b200.utils import DataType, MatmulBackend, QuantizeBackend, RoundStyle
+from fouroversix_b200.utils import DataType, MatmulBackend, QuantizeBackend, RoundStyle, ScaleRule
 
 _TORCH_OUT = {DataType.bfloat16: torch.bfloat16, DataType.float16: torch.float16, DataType.float32: torch.float32}
 
@@ -46,6 +46,31 @@ def _is_only_memory(t: torch.Tensor) -> bool:
     pending negation, and no function transform (vmap, ...) or forward-mode level around, which could have wrapped it
     or given it a tangent. (Asked about the level, not the tensor: a third of the time, which a small call feels.)"""
     return type(t) in _PLAIN_TYPES and forward_ad._current_level < 0 and _transform_level() is None and not t.is_neg()
+
+
+_ROUNDING_CODES = {RoundStyle.nearest: 0, RoundStyle.stochastic: 1, RoundStyle.stochastic_unbiased: 2}
+
+
+def _one_call_training_applies(cfg: ModuleQuantizationConfig, *operands: torch.Tensor) -> bool:
+    """Whether a pass is what `fos_linear_train_forward` / `fos_linear_train_backward` compute in one host call: NVFP4 throughout,
+    activations and weights rounded to nearest, operands of one 16-bit type that the copy engine takes as they are. Everything
+    else goes quantization by quantization, and is refused there where it has to be."""
+    if (cfg.disable_fprop_quantization or cfg.pseudo_quantize or cfg.activation_dtype != DataType.nvfp4
+            or cfg.weight_dtype != DataType.nvfp4 or cfg.gradient_dtype != DataType.nvfp4
+            or cfg.activation_round_style != RoundStyle.nearest or cfg.weight_round_style != RoundStyle.nearest
+            or cfg.gradient_round_style not in _ROUNDING_CODES
+            or cfg.matmul_backend not in (None, MatmulBackend.cutlass) or cfg.quantize_backend not in (None, QuantizeBackend.cuda)):
+        return False
+    first = operands[0]
+    if first.dtype not in (torch.bfloat16, torch.float16):
+        return False
+    for t in operands:
+        rows, cols = t.shape
+        ld = t.stride(0)
+        if (not t.is_cuda or t.device != first.device or t.dtype != first.dtype or t.stride(1) != 1 or rows == 0 or cols == 0
+                or cols % 8 or ld % 8 or ld < cols or t.data_ptr() % 16):
+            return False
+    return True
 
 
 class FourOverSixLinearFunction(torch.autograd.Function):
@@ -66,9 +91,14 @@ class FourOverSixLinearFunction(torch.autograd.Function):
             out = x2d @ weight.T
             out_features = weight.shape[0]
         else:
+            w = weight.data if trainable else weight
+            if not isinstance(w, QuantizedTensor) and w.dim() == 2 and x2d.shape[1] == w.shape[1] \
+                    and _one_call_training_applies(config, x2d, w):
+                out = FourOverSixLinearFunction._forward_one_call(config, x2d, w)
+                out = out.reshape(*input.shape[:-1], w.shape[0])
+                return out if bias is None else out + bias
             act_cfg = config.get_activation_config()
             if not isinstance(weight, QuantizedTensor):
-                w = weight.data if trainable else weight
                 weight = quantize(w, config.get_weight_config())
             if config.pseudo_quantize:
                 # both operands fake-quantized, then a high-precision matmul
@@ -80,6 +110,44 @@ class FourOverSixLinearFunction(torch.autograd.Function):
                 out_features = weight.original_shape[0]
         out = out.reshape(*input.shape[:-1], out_features)
         return out if bias is None else out + bias
+
+    @staticmethod
+    def _forward_one_call(config: ModuleQuantizationConfig, x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+        """`quantized_matmul(x, quantize(w))` enqueued by one host call: same bits."""
+        dev, (rows, k), n = x.device, x.shape, w.shape[0]
+        out = torch.empty(rows, n, dtype=_TORCH_OUT[DataType(config.output_dtype)], device=dev)
+        lib = _native.lib()
+        need = lib.fos_linear_train_workspace_bytes(rows, k, n)
+        workspace = torch.empty(need, dtype=torch.uint8, device=dev)
+        with _native.on_device(dev):
+            _native.check(lib.fos_linear_train_forward(
+                x.data_ptr(), w.data_ptr(), _native.elem_code(x.dtype), rows, k, n, x.stride(0), w.stride(0),
+                ScaleRule(config.activation_scale_rule).cuda_id, ScaleRule(config.weight_scale_rule).cuda_id,
+                int(config.weight_scale_2d), out.data_ptr(), _native.elem_code(out.dtype), out.stride(0), workspace.data_ptr(),
+                need, _native.stream_ptr(dev)), "fos_linear_train_forward")
+        return out
+
+    @staticmethod
+    def _backward_one_call(cfg: ModuleQuantizationConfig, dy: torch.Tensor, x: torch.Tensor,
+                           w: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+        """Both products of the backward pass enqueued by one host call: same bits, and the same seeds drawn in the same order."""
+        dev, (rows, k), n = dy.device, x.shape, w.shape[0]
+        torch_out = _TORCH_OUT[DataType(cfg.output_dtype)]
+        dx = torch.empty(rows, k, dtype=torch_out, device=dev)
+        dw = torch.empty(n, k, dtype=torch_out, device=dev)
+        rounding = _ROUNDING_CODES[cfg.gradient_round_style]
+        seeds = [int(torch.randint(0, 2 ** 62, (1,)).item()) for _ in range(2)] if rounding else [0, 0]
+        lib = _native.lib()
+        need = lib.fos_linear_train_workspace_bytes(rows, k, n)
+        workspace = torch.empty(need, dtype=torch.uint8, device=dev)
+        with _native.on_device(dev):
+            _native.check(lib.fos_linear_train_backward(
+                dy.data_ptr(), x.data_ptr(), w.data_ptr(), _native.elem_code(dy.dtype), rows, k, n, dy.stride(0), x.stride(0), w.stride(0),
+                ScaleRule(cfg.gradient_scale_rule).cuda_id, rounding, seeds[0], seeds[1], ScaleRule(cfg.activation_scale_rule).cuda_id,
+                ScaleRule(cfg.weight_scale_rule).cuda_id, int(cfg.weight_scale_2d), dx.data_ptr(), dw.data_ptr(),
+                _native.elem_code(torch_out), dx.stride(0), dw.stride(0), workspace.data_ptr(), need, _native.stream_ptr(dev)),
+                "fos_linear_train_backward")
+        return dx, dw
 
     @staticmethod
     def backward(ctx, grad_output: torch.Tensor):
@@ -98,6 +166,12 @@ class FourOverSixLinearFunction(torch.autograd.Function):
         dy = grad_output.reshape(-1, grad_output.shape[-1])     # [tokens, out]
         x = input.reshape(-1, input.shape[-1])                   # [tokens, in]
         w = weight.data                                          # [out, in]
+
+        if (not cfg.disable_dgrad_quantization and not cfg.disable_wgrad_quantization and dy.shape[0] % 16 == 0
+                and _one_call_training_applies(cfg, dy, x, w)):
+            dx, dw = FourOverSixLinearFunction._backward_one_call(cfg, dy, x, w)
+            db = dy.sum(0) if bias is not None and ctx.needs_input_grad[3] else None
+            return None, dx.reshape(*grad_output.shape[:-1], w.shape[1]), dw.to(w.dtype), db
 
         # dgrad: dx[tokens, in] = dy @ W = q(dy) @ q(W^T)^T
         if cfg.disable_dgrad_quantization:

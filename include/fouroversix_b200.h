@@ -260,6 +260,31 @@ int fos_gemm_mxfp4_unscaled(const uint8_t *a_codes, const uint8_t *a_sf, const u
  * (quantize the input, quantized_matmul), without its bias addition.
  */
 int64_t fos_linear_workspace_bytes(int64_t rows, int64_t in_features);
+
+/*
+ * A training step's forward and backward pass with a high-precision weight W [out_features, in_features], each as ONE host
+ * call; x [rows, in_features], dy [rows, out_features] and W share one 16-bit type `dtype`.
+ *   forward   out[rows, out] = Q(x) @ Q(W)^T
+ *   backward  dx[rows, in]   = Q(dy) @ Q(W^T)^T
+ *             dw[out, in]    = Q(rot(dy^T)) @ Q(rot(x^T))^T, both rotated (FOS_QUANTIZE_RHT) along the rows
+ * NVFP4, round to nearest, W in 16 x 16 blocks with weight_2d; dy is rounded as gradient_rounding says: 0 to nearest, 1
+ * stochastically, 2 stochastically with the 16/17 maxima, with the given seeds. Same bits as fos_quantize /
+ * fos_quantize_stochastic and fos_gemm_nvfp4_scaled call by call. Base addresses 16-byte aligned, row strides and
+ * feature counts multiples of 8, backward also rows a multiple of 16: FOS_ERR_UNSUPPORTED otherwise.
+ * `workspace`: fos_linear_train_workspace_bytes(...) bytes of device memory, 256-byte aligned, for either pass.
+ *
+ * Replaces: FourOverSixLinearFunction.forward / .backward of src/fouroversix/model/modules/linear.py:40-372 in their default
+ * configuration, without the bias.
+ */
+int64_t fos_linear_train_workspace_bytes(int64_t rows, int64_t in_features, int64_t out_features);
+int fos_linear_train_forward(const void *x, const void *w, int dtype, int64_t rows, int64_t in_features, int64_t out_features,
+                             int64_t ld_x, int64_t ld_w, int activation_rule, int weight_rule, int weight_2d, void *out,
+                             int out_dtype, int64_t ld_out, void *workspace, int64_t workspace_bytes, void *stream);
+int fos_linear_train_backward(const void *dy, const void *x, const void *w, int dtype, int64_t rows, int64_t in_features,
+                              int64_t out_features, int64_t ld_dy, int64_t ld_x, int64_t ld_w, int gradient_rule,
+                              int gradient_rounding, uint64_t seed_dgrad, uint64_t seed_wgrad, int activation_rule, int weight_rule,
+                              int weight_2d, void *dx, void *dw, int out_dtype, int64_t ld_dx, int64_t ld_dw, void *workspace,
+                              int64_t workspace_bytes, void *stream);
 int fos_linear_forward(const void *x, int x_dtype, int64_t rows, int64_t in_features, int64_t ld_x, int activation_rule,
                        const uint8_t *w_codes, const uint8_t *w_sf, const float *w_amax, int weight_rule,
                        int64_t out_features, void *out, int out_dtype, int64_t ld_out, void *workspace,
