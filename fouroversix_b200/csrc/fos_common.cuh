@@ -75,6 +75,20 @@ int gemm_nvfp4_grouped_scaled(const uint8_t *a_codes, const uint8_t *a_sf, const
                               const int32_t *group_rows, int num_groups, int64_t rows_capacity, int64_t n_p, int64_t k_p,
                               int64_t n, int64_t ldd, int32_t *status, void *stream);
 
+// The same for the gate-up projection of an experts layer, gate in the even and up in the odd of its n columns: d is not the
+// product but its clamped SwiGLU with the bias [groups][n] of the output's type (16 bits), n / 2 columns wide, and
+// amax[group] is raised to the largest magnitude written for the group. FOS_ERR_UNSUPPORTED (nothing launched) where the
+// problem is not one for the kernel on CTA pairs.
+struct GluEpilogue {
+    const void *bias;
+    float alpha, limit;
+    float *amax;
+};
+int gemm_nvfp4_grouped_glu(const uint8_t *a_codes, const uint8_t *a_sf, const uint8_t *b_codes, const uint8_t *b_sf,
+                           const GemmScales &scales, const GluEpilogue &glu, void *d, int out_dtype, const int32_t *group_start,
+                           const int32_t *group_rows, int num_groups, int64_t rows_capacity, int64_t n_p, int64_t k_p,
+                           int64_t n, int64_t ldd, int32_t *status, void *stream);
+
 #define FOS_CUDA_TRY(expr)                                         \
     do {                                                           \
         cudaError_t fos_e_ = (expr);                               \

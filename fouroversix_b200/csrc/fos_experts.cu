@@ -12,32 +12,11 @@
 // chain; what they save is its memory traffic (each operation reads and writes the whole tensor, the
 // gathers materialise the bias per row) and its launches. Gather and combine are bound by HBM, the SwiGLU
 // by its arithmetic (a sigmoid with an IEEE division and six roundings per output).
-#include "fos_common.cuh"
+#include "fos_glu.cuh"
 
 namespace fos {
 namespace {
 
-template <typename T> struct Half16;
-template <> struct Half16<__nv_bfloat16> {
-    using Pair = __nv_bfloat162;
-    static __device__ __forceinline__ float lo(uint32_t w) { return __uint_as_float(w << 16); }
-    static __device__ __forceinline__ float hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
-    static __device__ __forceinline__ float r16(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
-    static __device__ __forceinline__ uint32_t pack(float lo_v, float hi_v) {   // round and pack
-        Pair p = __floats2bfloat162_rn(lo_v, hi_v);
-        return *reinterpret_cast<uint32_t *>(&p);
-    }
-};
-template <> struct Half16<__half> {
-    using Pair = __half2;
-    static __device__ __forceinline__ float lo(uint32_t w) { return __half2float(__ushort_as_half(static_cast<unsigned short>(w & 0xffffu))); }
-    static __device__ __forceinline__ float hi(uint32_t w) { return __half2float(__ushort_as_half(static_cast<unsigned short>(w >> 16))); }
-    static __device__ __forceinline__ float r16(float v) { return __half2float(__float2half_rn(v)); }
-    static __device__ __forceinline__ uint32_t pack(float lo_v, float hi_v) {
-        Pair p = __floats2half2_rn(lo_v, hi_v);
-        return *reinterpret_cast<uint32_t *>(&p);
-    }
-};
 // Every kernel of the layer starts here. In the one-call form each is launched as the programmatic dependent of the one
 // before it: its CTAs may be placed while that one drains, and wait here before they touch memory. What came before
 // THAT one is then complete too, because it waited the same way. (Ordinary launches: both instructions do nothing.)
@@ -48,31 +27,6 @@ __device__ __forceinline__ void chain_begin() {
 
 constexpr int ROW_THREADS = 256;         // of the kernels that give a row to a warp
 constexpr int GATHER_CTAS = 6, GLU_CTAS = 4;     // their CTAs per SM (one wave: a warp takes rows in turn)
-
-template <typename P> __device__ __forceinline__ P as_pair(uint32_t w) { return *reinterpret_cast<P *>(&w); }
-template <typename P> __device__ __forceinline__ uint32_t as_word(P p) { return *reinterpret_cast<uint32_t *>(&p); }
-
-// max |value| of the eight 16-bit numbers of a 16-byte piece, folded into a running packed maximum
-// (NaNs are skipped, as fmaxf skips them in the amax pass of the quantization).
-template <typename P> __device__ __forceinline__ P fold_abs_max(P m, uint4 v) {
-    m = __hmax2(m, __habs2(as_pair<P>(v.x)));
-    m = __hmax2(m, __habs2(as_pair<P>(v.y)));
-    m = __hmax2(m, __habs2(as_pair<P>(v.z)));
-    return __hmax2(m, __habs2(as_pair<P>(v.w)));
-}
-
-// The warp's maximum of the lanes' packed running maxima, raised into amax[0] (a non-negative float, zeroed by the
-// caller before the launch, compared as an integer). The words written are the ones the grouped amax pass would
-// write: the largest magnitude of the group's values, exactly, as a float. Called by all lanes of the warp.
-template <typename T>
-__device__ __forceinline__ void raise_amax(typename Half16<T>::Pair m2, float *amax, int lane) {
-    using H = Half16<T>;
-    float m = fmaxf(H::lo(as_word(m2)), H::hi(as_word(m2)));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    // (a stale smaller value read here only costs an atomic that changes nothing)
-    if (lane == 0 && m > 0.0f && m > *reinterpret_cast<volatile float *>(amax)) atomicMax(reinterpret_cast<int *>(amax), __float_as_int(m));
-}
 
 // The two row kernels below give a warp a row, or (few rows) a segment of one: a row is a few KB, so its own latency (look
 // up the row, fetch it, reduce) dominates, and warps that do not wait for one another overlap theirs. A unit of work is
@@ -122,46 +76,6 @@ gather_rows_kernel(const uint8_t *__restrict__ x, int64_t ld_x_bytes, const int3
         __syncwarp();
         if (amax != nullptr) raise_amax<T>(m2, amax + ld_int(units.pair_row ? units.pair_expert + at : row_expert + r), lane);
     }
-}
-
-// 1 / (1 + expf(-t)) of two numbers, rounded to the 16-bit type (a packed pair). The fast functions give the quotient to
-// within (12 + 1.5 |t|) units of 2^-23 for |t| <= 64 (__expf: 2 + 1.173 |t| units in the last place by CUDA's own bound, the
-// addition and __fdividef 3, and the binary32 sequence itself is within 4 of the true value); where both ends of that
-// interval round to the same number, the binary32 sequence does too. The rest - a value within the interval of a
-// rounding boundary (one in 500 in bf16, one in 60 in fp16), a large |t|, NaN - runs the sequence itself.
-template <typename T> __device__ __forceinline__ uint32_t sigmoid16x2(float t0, float t1) {
-    using H = Half16<T>;
-    const float s0 = __fdividef(1.0f, 1.0f + __expf(-t0)), s1 = __fdividef(1.0f, 1.0f + __expf(-t1));
-    const float w0 = s0 * fmaf(fabsf(t0), 0x1.8p-23f, 0x1.8p-20f), w1 = s1 * fmaf(fabsf(t1), 0x1.8p-23f, 0x1.8p-20f);
-    const uint32_t low = H::pack(s0 - w0, s1 - w1), high = H::pack(s0 + w0, s1 + w1);
-    if (low == high && fmaxf(fabsf(t0), fabsf(t1)) <= 64.0f) return low;
-    return H::pack(1.0f / (1.0f + expf(-t0)), 1.0f / (1.0f + expf(-t1)));
-}
-
-// The reference's chain on two (gate, up) pairs, every intermediate rounded to the 16-bit type:
-//   g = gate + bias_g; u = up + bias_u; g = min(g, limit); u = min(max(u, -limit), limit)   (NaN passes through)
-//   out = (u + 1) * (g * sigmoid(g * alpha))
-// A (gate, up) pair is one 32-bit word, and a packed 16-bit addition, multiplication or fused multiply-add
-// rounds once from the exact result, which is what "compute in binary32, round to the type" gives for sums and
-// products of 16-bit numbers (their exact value fits binary32, or lies so far from a rounding boundary of the
-// 16-bit type that the first rounding cannot move it across). Only g * alpha (alpha is a binary32 number) and
-// the sigmoid run in binary32. The _rn forms of the packed operations keep the compiler from contracting a
-// multiplication and the addition after it into one fused operation, which would drop a rounding. limit2 = (r, r), floor2 = (-inf, -r) with r the limit rounded to the type:
-// comparing with r selects the same values as comparing with the limit itself, because no number of the type
-// lies between the two. Returns the output in the low half.
-template <typename T>
-__device__ __forceinline__ uint32_t glu_words(uint32_t gate_up0, uint32_t gate_up1, uint32_t bias0, uint32_t bias1, float alpha,
-                                              typename Half16<T>::Pair limit2, typename Half16<T>::Pair floor2,
-                                              typename Half16<T>::Pair one2) {
-    using H = Half16<T>;
-    using P = typename H::Pair;
-    P v0 = __hadd2_rn(as_pair<P>(gate_up0), as_pair<P>(bias0)), v1 = __hadd2_rn(as_pair<P>(gate_up1), as_pair<P>(bias1));
-    v0 = __hmax2_nan(__hmin2_nan(v0, limit2), floor2);
-    v1 = __hmax2_nan(__hmin2_nan(v1, limit2), floor2);
-    const uint32_t g2 = __byte_perm(as_word(v0), as_word(v1), 0x5410), u2 = __byte_perm(as_word(v0), as_word(v1), 0x7632);
-    const uint32_t t2 = H::pack(H::lo(g2) * alpha, H::hi(g2) * alpha);
-    const P w = __hmul2_rn(as_pair<P>(g2), as_pair<P>(sigmoid16x2<T>(H::lo(t2), H::hi(t2))));
-    return as_word(__hmul2_rn(__hadd2_rn(as_pair<P>(u2), one2), w));
 }
 
 // gate_up [rows][2 * inter] with gate in the even and up in the odd columns; bias [experts][2 * inter];
@@ -666,12 +580,20 @@ extern "C" int fos_experts_forward(const void *x, int dtype, int64_t tokens, int
                               ints(w.group_rows), num_experts, amax, base + w.codes_x, base + w.sf_x, amax, 0, stream_);
     if (st != FOS_OK) return st;
     const float denom = alpha_divisor(FOS_NVFP4, activation_rule, FOS_NVFP4, weight_rule);
-    st = gemm_nvfp4_grouped_scaled(base + w.codes_x, base + w.sf_x, gate_up_codes, gate_up_sf, {amax, gate_up_amax, denom, nullptr, true},
-                                   base + w.gate_up, dtype, ints(w.group_start), ints(w.group_rows), num_experts, w.capacity,
-                                   gate_up_rows, hidden, 2 * intermediate, 2 * intermediate, status, stream_);
-    if (st != FOS_OK) return st;
-    st = experts_glu(base + w.gate_up, dtype, 2 * intermediate, gate_up_bias, ints(w.row_expert), base + w.gated, intermediate,
-                     w.capacity, intermediate, alpha, limit, amax + num_experts, &order, stream_);
+    // the SwiGLU in the GEMM's epilogue where that GEMM runs on CTA pairs, else in a kernel of its own
+    const GemmScales gate_up_scales{amax, gate_up_amax, denom, nullptr, true};
+    const GluEpilogue glu{gate_up_bias, alpha, limit, amax + num_experts};
+    st = gemm_nvfp4_grouped_glu(base + w.codes_x, base + w.sf_x, gate_up_codes, gate_up_sf, gate_up_scales, glu, base + w.gated, dtype,
+                                ints(w.group_start), ints(w.group_rows), num_experts, w.capacity, gate_up_rows, hidden,
+                                2 * intermediate, intermediate, status, stream_);
+    if (st == FOS_ERR_UNSUPPORTED) {
+        st = gemm_nvfp4_grouped_scaled(base + w.codes_x, base + w.sf_x, gate_up_codes, gate_up_sf, gate_up_scales, base + w.gate_up, dtype,
+                                       ints(w.group_start), ints(w.group_rows), num_experts, w.capacity, gate_up_rows, hidden,
+                                       2 * intermediate, 2 * intermediate, status, stream_);
+        if (st != FOS_OK) return st;
+        st = experts_glu(base + w.gate_up, dtype, 2 * intermediate, gate_up_bias, ints(w.row_expert), base + w.gated, intermediate,
+                         w.capacity, intermediate, alpha, limit, amax + num_experts, &order, stream_);
+    }
     if (st != FOS_OK) return st;
     st = quantize_grouped_rows_in_use(base + w.gated, dtype, w.capacity, intermediate, intermediate, FOS_NVFP4, activation_rule,
                               ints(w.group_start), ints(w.group_rows), num_experts, amax + num_experts, base + w.codes_g,

@@ -45,6 +45,7 @@
 // in *status, raises a CTA-wide abort flag, and all roles fall through to the common exit,
 // which lets in-flight copies land, releases tensor memory and returns.
 #include "fos_gemm_skinny.cuh"
+#include "fos_glu.cuh"
 #include "fos_pair.cuh"
 
 namespace fos {
@@ -106,6 +107,7 @@ struct GemmParams {
     const float *amax_b;
     float alpha_denom;
     const void *bias;        // [n] of the output's type, added to the rounded product, or nullptr
+    GluEpilogue glu;         // gemm_fp4_pair_kernel<.., GLU>: d is [rows][n / 2]
     void *d;
     int32_t *status;         // where a bounded wait that gives up records its site: the caller's word, or the sticky one
     int64_t m_p, n_p, k_p;   // padded problem (k_p in values)
@@ -696,7 +698,39 @@ template <bool MX> struct PairCfg {
 
 // GROUPED: row tiles run through each group's rows in steps of 256, so a tile never computes two groups' rows (its second
 // half may reach into the next group's, or beyond the last: not stored).
-template <typename OUT, bool MX, bool GROUPED = false>
+//
+// GLU (with GROUPED): the columns are (gate, up) pairs and what is stored is their SwiGLU, so the product itself never
+// reaches memory (32768 x 5760: 377 MB less written and read, and the kernel that did it, 125 us). A lane holds
+// a row of the tile, so a pair lies in neighbouring registers of one lane, and the bias is the same for all lanes.
+// The accumulators overlap by 96 columns only, so the arithmetic (about 25 instructions per output, 64 outputs per thread
+// and tile) runs while the next tile's MMAs do: at K 2880 a tile's MMAs take some 7000 cycles, the epilogue half of that.
+template <typename OUT, int N>
+__device__ __forceinline__ void glu_columns(OUT *dst, const uint32_t *acc, float alpha, const OUT *bias, int64_t cols_left, bool row_ok,
+                                            const GluEpilogue &glu, typename Half16<OUT>::Pair limit2,
+                                            typename Half16<OUT>::Pair floor2, typename Half16<OUT>::Pair one2,
+                                            typename Half16<OUT>::Pair &max2) {
+    using H = Half16<OUT>;
+#pragma unroll
+    for (int c = 0; c < N; c += 16) {
+        if (c >= cols_left) break;                           // (the product's width is a multiple of 16)
+        const uint4 b0 = ld_16(bias + c), b1 = ld_16(bias + c + 8);
+        const uint32_t b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+        uint32_t o[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t *v = acc + c + 4 * i;
+            o[i] = glu_words<OUT>(H::pack(alpha * __uint_as_float(v[0]), alpha * __uint_as_float(v[1])),
+                                  H::pack(alpha * __uint_as_float(v[2]), alpha * __uint_as_float(v[3])), b[2 * i], b[2 * i + 1],
+                                  glu.alpha, limit2, floor2, one2);
+        }
+        if (!row_ok) continue;
+        const uint4 packed = make_uint4(o[0], o[1], o[2], o[3]);
+        *reinterpret_cast<uint4 *>(dst + c / 2) = packed;
+        max2 = fold_abs_max(max2, packed);
+    }
+}
+
+template <typename OUT, bool MX, bool GROUPED = false, bool GLU = false>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                      const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_sfb,
@@ -898,6 +932,17 @@ gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         const bool vec16 = (reinterpret_cast<uintptr_t>(out) % 16 == 0) && ((p.ldd * sizeof(OUT)) % 16 == 0);
         const bool vec32 = (reinterpret_cast<uintptr_t>(out) % 32 == 0) && ((p.ldd * sizeof(OUT)) % 32 == 0);
         const uint32_t leader_acc_empty = map_to_cta(acc_empty_bar, 0);
+        using GluType = std::conditional_t<GLU, OUT, __half>;                  // (fp32 products have no SwiGLU)
+        using GluPair = typename Half16<GluType>::Pair;
+        [[maybe_unused]] GluPair limit2, floor2, one2, max2;
+        if constexpr (GLU) {
+            using H = Half16<GluType>;
+            const float l = H::r16(p.glu.limit);
+            limit2 = as_pair<GluPair>(H::pack(l, l));
+            floor2 = as_pair<GluPair>(H::pack(-INFINITY, -l));
+            one2 = as_pair<GluPair>(H::pack(1.0f, 1.0f));
+            max2 = as_pair<GluPair>(0u);
+        }
         uint32_t tile_i = 0;
         bool ok = true;
         for (int64_t t = pair_id; t < num_tiles && ok; t += num_pairs, ++tile_i) {
@@ -923,7 +968,13 @@ gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             const OUT *bias = p.bias ? static_cast<const OUT *>(p.bias) + nb * TILE_N : nullptr;
             const int64_t left = row < row_end ? p.n - nb * TILE_N : 0;
             auto store = [&](const uint32_t *acc, int col, auto n) {
-                store_columns<OUT, decltype(n)::value>(dst + col, acc, alpha, bias ? bias + col : nullptr, left - col, vec32, vec16);
+                if constexpr (GLU) {
+                    glu_columns<OUT, decltype(n)::value>(out + row * p.ldd + (nb * TILE_N + col) / 2, acc, alpha,
+                                                         static_cast<const OUT *>(p.glu.bias) + group * p.n + nb * TILE_N + col,
+                                                         p.n - nb * TILE_N - col, row < row_end, p.glu, limit2, floor2, one2, max2);
+                } else {
+                    store_columns<OUT, decltype(n)::value>(dst + col, acc, alpha, bias ? bias + col : nullptr, left - col, vec32, vec16);
+                }
             };
             uint32_t v[FIRST / 48][48];
 #pragma unroll
@@ -940,6 +991,11 @@ gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
             uint32_t w[32];
             tc_load_32cols_sync(t_acc + second + (SECOND - 32), w);
             store(w, second + (SECOND - 32), std::integral_constant<int, 32>{});
+            if constexpr (GLU) {
+                __syncwarp();
+                raise_amax<OUT>(max2, p.glu.amax + group, lane);
+                max2 = as_pair<GluPair>(0u);
+            }
         }
     }
 
@@ -956,14 +1012,14 @@ gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 
 // ---------------------------------------------------------------------------- host side
 
-template <typename OUT, bool MX, bool GROUPED>
+template <typename OUT, bool MX, bool GROUPED, bool GLU = false>
 int launch_pair(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &msa, const CUtensorMap &msb,
                 const GemmParams &p, int max_ctas, cudaStream_t stream) {
     // (grouped: at most one more row tile per group than the buffer has)
     const int64_t row_tiles = (p.m_p + 255) / 256 + (GROUPED ? p.num_groups : 0);
-    return pair::launch<pair::gemm_fp4_pair_kernel<OUT, MX, GROUPED>>(pair::THREADS, pair::PairCfg<MX>::SMEM_BYTES,
-                                                                      row_tiles * ((p.n_p + 255) / 256), max_ctas, stream,
-                                                                      ma, mb, msa, msb, p);
+    return pair::launch<pair::gemm_fp4_pair_kernel<OUT, MX, GROUPED, GLU>>(pair::THREADS, pair::PairCfg<MX>::SMEM_BYTES,
+                                                                           row_tiles * ((p.n_p + 255) / 256), max_ctas, stream,
+                                                                           ma, mb, msa, msb, p);
 }
 
 template <bool MX, bool GROUPED = false>
@@ -1247,15 +1303,18 @@ static int gemm_grouped_entry(const uint8_t *a_codes, const uint8_t *a_sf, const
                               const float *alpha, const fos::GemmScales *scales, void *d, int out_dtype,
                               const int32_t *group_start, const int32_t *group_rows, int num_groups, int64_t rows_capacity,
                               int64_t n_p, int64_t k_p, int64_t n, int64_t ldd, const fos_gemm_opts *opts, int32_t *status,
-                              void *stream_) {
+                              void *stream_, const fos::GluEpilogue *glu = nullptr) {
     using namespace fos;
     const int variant = opts ? opts->variant : 0, max_ctas = opts ? opts->max_ctas : 0;
     if ((variant != 0 && variant != 128 && variant != 256) || max_ctas < 0) return FOS_ERR_INVALID_ARGUMENT;
     if (!a_codes || !a_sf || !b_codes || !b_sf || (!alpha && !scales) || !d || !group_start || !group_rows) return FOS_ERR_INVALID_ARGUMENT;
     if (num_groups <= 0 || num_groups > MAX_GROUPS) return FOS_ERR_INVALID_ARGUMENT;
     if (rows_capacity <= 0 || rows_capacity % 128 || n_p <= 0 || n_p % 128 || k_p < 64 || k_p % 64) return FOS_ERR_INVALID_ARGUMENT;
-    if (n <= 0 || n > n_p || ldd < n) return FOS_ERR_INVALID_ARGUMENT;
+    if (n <= 0 || n > n_p || ldd < (glu ? n / 2 : n)) return FOS_ERR_INVALID_ARGUMENT;
     if (out_dtype != FOS_BF16 && out_dtype != FOS_FP16 && out_dtype != FOS_FP32) return FOS_ERR_INVALID_ARGUMENT;
+    // (the epilogue's stores are 8 outputs of a row, its loads 8 numbers of the bias)
+    if (glu && (out_dtype == FOS_FP32 || n % 16 || ldd % 8 || reinterpret_cast<uintptr_t>(d) % 16 || reinterpret_cast<uintptr_t>(glu->bias) % 16))
+        return FOS_ERR_UNSUPPORTED;
     if (reinterpret_cast<uintptr_t>(a_codes) % 16 || reinterpret_cast<uintptr_t>(b_codes) % 16 ||
         reinterpret_cast<uintptr_t>(a_sf) % 16 || reinterpret_cast<uintptr_t>(b_sf) % 16)
         return FOS_ERR_MISALIGNED;
@@ -1279,20 +1338,27 @@ static int gemm_grouped_entry(const uint8_t *a_codes, const uint8_t *a_sf, const
     p.group_start = group_start;
     p.group_rows = group_rows;
     p.num_groups = num_groups;
+    // how many row blocks are in use is known on the device only: the grid is sized for the buffers, and
+    // CTAs that find no tile leave at once
+    const int choice = grouped_kernel_for(rows_capacity, num_groups, n_p, variant, max_ctas, sms);
+    if (glu) {
+        if (choice != GEMM_PAIR) return FOS_ERR_UNSUPPORTED;
+        p.glu = *glu;
+    }
     if (status) {
         FOS_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int32_t), stream));
     } else {
         FOS_CUDA_TRY(wait_failures_ptr(&p.status));
     }
-    // how many row blocks are in use is known on the device only: the grid is sized for the buffers, and
-    // CTAs that find no tile leave at once
-    const int choice = grouped_kernel_for(rows_capacity, num_groups, n_p, variant, max_ctas, sms);
     CUtensorMap map_a, map_b, map_sfa, map_sfb;
     if (choice == GEMM_PAIR) {
         if ((st = make_operand_map(&map_a, a_codes, rows_capacity, k_p / 2, 128)) != FOS_OK) return st;
         if ((st = make_operand_map(&map_b, b_codes, b_rows, k_p / 2, 128)) != FOS_OK) return st;
         if ((st = make_scale_map(&map_sfa, a_sf, rows_capacity / 128, k_p / 64, 1, KB_PER_STAGE)) != FOS_OK) return st;
         if ((st = make_scale_map(&map_sfb, b_sf, b_rows / 128, k_p / 64, 2, KB_PER_STAGE)) != FOS_OK) return st;
+        if (glu)
+            return out_dtype == FOS_BF16 ? launch_pair<__nv_bfloat16, false, true, true>(map_a, map_b, map_sfa, map_sfb, p, max_ctas, stream)
+                                         : launch_pair<__half, false, true, true>(map_a, map_b, map_sfa, map_sfb, p, max_ctas, stream);
         return launch_pair_out<false, true>(map_a, map_b, map_sfa, map_sfb, p, max_ctas, stream);
     }
     const bool wide = choice == GEMM_256;
@@ -1320,6 +1386,14 @@ int fos::gemm_nvfp4_grouped_scaled(const uint8_t *a_codes, const uint8_t *a_sf, 
                                    int64_t n, int64_t ldd, int32_t *status, void *stream) {
     return gemm_grouped_entry(a_codes, a_sf, b_codes, b_sf, nullptr, &scales, d, out_dtype, group_start, group_rows, num_groups,
                               rows_capacity, n_p, k_p, n, ldd, nullptr, status, stream);
+}
+
+int fos::gemm_nvfp4_grouped_glu(const uint8_t *a_codes, const uint8_t *a_sf, const uint8_t *b_codes, const uint8_t *b_sf,
+                                const GemmScales &scales, const GluEpilogue &glu, void *d, int out_dtype, const int32_t *group_start,
+                                const int32_t *group_rows, int num_groups, int64_t rows_capacity, int64_t n_p, int64_t k_p,
+                                int64_t n, int64_t ldd, int32_t *status, void *stream) {
+    return gemm_grouped_entry(a_codes, a_sf, b_codes, b_sf, nullptr, &scales, d, out_dtype, group_start, group_rows, num_groups,
+                              rows_capacity, n_p, k_p, n, ldd, nullptr, status, stream, &glu);
 }
 
 extern "C" int fos_gemm_mxfp4(const uint8_t *a_codes, const uint8_t *a_sf, const uint8_t *b_codes,
