@@ -55,6 +55,12 @@ int quantize_grouped_rows_in_use(const void *x, int x_dtype, int64_t rows_capaci
                                  int scale_rule, const int32_t *group_start, const int32_t *group_rows, int num_groups,
                                  const float *amax_in, uint8_t *codes, uint8_t *sf, float *amax_out, int flags, void *stream);
 
+// The same where row r of the groups' buffer is a copy of row row_source[r] of x (rows in use; others: anything), which the kernel
+// fetches from there. NVFP4, rule mse, the groups' maxima given; FOS_ERR_UNSUPPORTED (nothing launched) for anything else.
+int quantize_grouped_gathered(const void *x, int x_dtype, int64_t x_rows, int64_t cols, int64_t ld, const int32_t *row_source,
+                              int64_t rows_capacity, int scale_rule, const int32_t *group_start, const int32_t *group_rows,
+                              int num_groups, float *amax, uint8_t *codes, uint8_t *sf, void *stream);
+
 // How a GEMM's output is scaled without an alpha word: alpha = amax_a * amax_b / denom is formed in the GEMM (the same
 // operations as fos_gemm_alpha; amax_a == nullptr: 1), bias [n] of the output's type (or nullptr) is added to the
 // rounded product. `chained`: the kernel before the GEMM in the stream is this library's, packs A, and lets its

@@ -213,11 +213,13 @@ constexpr int ROUTE_THREADS = 256, ROUTE_WARPS = ROUTE_THREADS / 32, ROUTE_MAX_E
 //   pair_row[p]     the row pair p was given (ascending in p within an expert), -1 for an index outside [0, experts)
 //   row_token[r], row_expert[r]   the token and the expert of row r, -1 for padding rows
 // route_count_kernel: every CTA counts its segment per expert into seg_count[segment][expert], and the CTAs
-// together fill the row tables with -1. route_place_kernel: every CTA adds up the counts of all segments (totals,
+// together fill the row tables with -1; CTAs beyond the segments (the one-call form) take a warp per token for its largest
+// magnitude. route_place_kernel: every CTA adds up the counts of all segments (totals,
 // hence the experts' first rows) and of the segments before its own (hence its own first row per expert), splits
 // its segment over its warps the same way (count, running sum), and then each warp walks its pairs 32 at a
 // time, ranks the pairs of one expert among themselves with match_any and advances its own counters. Rows
-// ascend with the pair index because segments, warps and lanes do.
+// ascend with the pair index because segments, warps and lanes do. With the tokens' maxima it also raises the experts', which
+// the grouped quantization needs: 8192 tokens are read once for it (47 MB), not the 32768 rows that their experts get.
 template <typename IDX>
 __device__ __forceinline__ int route_expert_of(const IDX *__restrict__ routing, int p, int end, int experts) {
     if (p >= end) return -1;
@@ -227,19 +229,51 @@ __device__ __forceinline__ int route_expert_of(const IDX *__restrict__ routing, 
     return (e >= 0 && e < experts) ? static_cast<int>(e) : -1;
 }
 
-template <typename IDX>
+struct TokenMaxima {
+    const uint8_t *x;                      // [tokens] rows of `chunks` 16-byte pieces, or nullptr: no maxima
+    int64_t ld_bytes;
+    int tokens, chunks;
+    float *of_token;                       // [tokens]
+};
+
+template <typename T> __device__ __forceinline__ void token_maxima(const TokenMaxima &m, int first_warp, int warps, int lane) {
+    using P = typename Half16<T>::Pair;
+    for (int t = first_warp; t < m.tokens; t += warps) {
+        const uint4 *src = reinterpret_cast<const uint4 *>(m.x + t * m.ld_bytes);
+        P m2 = as_pair<P>(0u);
+        for (int c0 = lane; c0 < m.chunks; c0 += 32 * 4) {                    // four loads in flight per lane
+            uint4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = c0 + 32 * u < m.chunks ? ld_16(src + c0 + 32 * u) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) m2 = fold_abs_max<P>(m2, v[u]);
+        }
+        __syncwarp();
+        float largest = fmaxf(Half16<T>::lo(as_word(m2)), Half16<T>::hi(as_word(m2)));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) largest = fmaxf(largest, __shfl_xor_sync(0xffffffffu, largest, o));
+        if (lane == 0) m.of_token[t] = largest;
+    }
+}
+
+template <typename IDX, typename T>
 __global__ void __launch_bounds__(ROUTE_THREADS)
-route_count_kernel(const IDX *__restrict__ routing, int pairs, int seg, int experts, int rows_capacity,
+route_count_kernel(const IDX *__restrict__ routing, int pairs, int seg, int segments, int experts, int rows_capacity,
                    int32_t *__restrict__ seg_count, int32_t *__restrict__ row_token, int32_t *__restrict__ row_expert,
-                   float *__restrict__ amax) {
+                   float *__restrict__ amax, const TokenMaxima maxima) {
     chain_begin();
+    if (static_cast<int>(blockIdx.x) >= segments) {
+        const int first = ((blockIdx.x - segments) * ROUTE_THREADS + threadIdx.x) >> 5;
+        token_maxima<T>(maxima, first, (gridDim.x - segments) * ROUTE_WARPS, threadIdx.x & 31);
+        return;
+    }
     if (amax != nullptr && blockIdx.x == 0 && threadIdx.x < 2 * experts) {        // (the one-call form: both projections' maxima)
         for (int i = threadIdx.x; i < 2 * experts; i += ROUTE_THREADS) amax[i] = 0.0f;
     }
     __shared__ int s_count[ROUTE_MAX_EXPERTS];
     const int tid = threadIdx.x;
     s_count[tid] = 0;
-    for (int r = blockIdx.x * ROUTE_THREADS + tid; r < rows_capacity; r += gridDim.x * ROUTE_THREADS) {
+    for (int r = blockIdx.x * ROUTE_THREADS + tid; r < rows_capacity; r += segments * ROUTE_THREADS) {
         row_token[r] = -1;
         row_expert[r] = -1;
     }
@@ -262,8 +296,11 @@ __global__ void __launch_bounds__(ROUTE_THREADS)
 route_place_kernel(const IDX *__restrict__ routing, int pairs, int seg, int top_k, int experts,
                    const int32_t *__restrict__ seg_count, int32_t *__restrict__ group_start,
                    int32_t *__restrict__ group_rows, int32_t *__restrict__ row_token, int32_t *__restrict__ row_expert,
-                   int32_t *__restrict__ pair_row, int32_t *__restrict__ pair_expert) {
+                   int32_t *__restrict__ pair_row, int32_t *__restrict__ pair_expert, const float *__restrict__ token_max,
+                   float *__restrict__ amax) {
     chain_begin();
+    __shared__ int s_max[ROUTE_MAX_EXPERTS];                 // the segment's largest magnitude per expert
+    s_max[threadIdx.x] = 0;
     __shared__ int s_at[ROUTE_WARPS][ROUTE_MAX_EXPERTS];     // counts, then next rows, per (warp, expert)
     __shared__ int s_total[ROUTE_MAX_EXPERTS], s_first[ROUTE_MAX_EXPERTS];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -330,10 +367,17 @@ route_place_kernel(const IDX *__restrict__ routing, int pairs, int seg, int top_
             pair_row[p] = row;
             pair_expert[p] = e;
             if (e >= 0) {
-                row_token[row] = p / top_k;
+                const int t = p / top_k;
+                row_token[row] = t;
                 row_expert[row] = e;
+                // (non-negative floats order like their bit patterns)
+                if (token_max != nullptr) atomicMax(&s_max[e], __float_as_int(ld_float(token_max + t)));
             }
         }
+    }
+    if (token_max != nullptr) {
+        __syncthreads();
+        if (tid < experts && s_max[tid] > 0) atomicMax(reinterpret_cast<int *>(amax + tid), s_max[tid]);
     }
 }
 
@@ -466,11 +510,12 @@ extern "C" int fos_experts_combine(const void *y, int dtype, int64_t ld_y, const
     return FOS_OK;
 }
 
-// fos_experts_route; with `amax` also zeroes amax[0 .. 2 * num_experts).
+// fos_experts_route; with `amax` also zeroes amax[0 .. 2 * num_experts), and with `maxima` then raises the first num_experts to the
+// largest magnitudes of the experts' tokens.
 static int experts_route(const void *routing_indices, int index_bytes, int64_t tokens, int top_k, int num_experts,
                          int64_t rows_capacity, int32_t *group_start, int32_t *group_rows, int32_t *row_token,
                          int32_t *row_expert, int32_t *pair_row, int32_t *pair_expert, int32_t *workspace, float *amax,
-                         void *stream_) {
+                         const fos::TokenMaxima &maxima, int x_dtype, void *stream_) {
     using namespace fos;
     if (!routing_indices || !group_start || !group_rows || !row_token || !row_expert || !pair_row || !pair_expert ||
         !workspace || tokens <= 0 || top_k <= 0 || num_experts <= 0 || (index_bytes != 4 && index_bytes != 8))
@@ -489,22 +534,21 @@ static int experts_route(const void *routing_indices, int index_bytes, int64_t t
     if (segments > ROUTE_MAX_SEGMENTS) segments = ROUTE_MAX_SEGMENTS;
     const int seg = (pairs + segments - 1) / segments;
     segments = (pairs + seg - 1) / seg;
-    if (index_bytes == 8) {
-        const int64_t *idx = static_cast<const int64_t *>(routing_indices);
-        FOS_CUDA_TRY(launch_dependent(route_count_kernel<int64_t>, dim3(segments), ROUTE_THREADS, 0, stream,
-            idx, pairs, seg, num_experts, cap, workspace, row_token, row_expert, amax));
-        FOS_CUDA_TRY(launch_dependent(route_place_kernel<int64_t>, dim3(segments), ROUTE_THREADS, 0, stream,
-            idx, pairs, seg, top_k, num_experts, workspace, group_start,
-            group_rows, row_token, row_expert, pair_row, pair_expert));
-    } else {
-        const int32_t *idx = static_cast<const int32_t *>(routing_indices);
-        FOS_CUDA_TRY(launch_dependent(route_count_kernel<int32_t>, dim3(segments), ROUTE_THREADS, 0, stream,
-            idx, pairs, seg, num_experts, cap, workspace, row_token, row_expert, amax));
-        FOS_CUDA_TRY(launch_dependent(route_place_kernel<int32_t>, dim3(segments), ROUTE_THREADS, 0, stream,
-            idx, pairs, seg, top_k, num_experts, workspace, group_start,
-            group_rows, row_token, row_expert, pair_row, pair_expert));
-    }
-    return FOS_OK;
+    // (the tokens' maxima: a warp each, one wave at most)
+    const int token_ctas = !maxima.x ? 0 : (maxima.tokens < 148 * 6 * ROUTE_WARPS ? (maxima.tokens + ROUTE_WARPS - 1) / ROUTE_WARPS : 148 * 6);
+    auto launch = [&](auto *idx, auto element) -> int {
+        using IDX = std::remove_const_t<std::remove_pointer_t<decltype(idx)>>;
+        using T = decltype(element);
+        FOS_CUDA_TRY(launch_dependent(route_count_kernel<IDX, T>, dim3(segments + token_ctas), ROUTE_THREADS, 0, stream, idx, pairs, seg,
+                                      segments, num_experts, cap, workspace, row_token, row_expert, amax, maxima));
+        FOS_CUDA_TRY(launch_dependent(route_place_kernel<IDX>, dim3(segments), ROUTE_THREADS, 0, stream, idx, pairs, seg, top_k,
+                                      num_experts, workspace, group_start, group_rows, row_token, row_expert, pair_row,
+                                      pair_expert, maxima.of_token, amax));
+        return FOS_OK;
+    };
+    auto launch_index = [&](auto *idx) { return x_dtype == FOS_FP16 ? launch(idx, __half{}) : launch(idx, __nv_bfloat16{}); };
+    return index_bytes == 8 ? launch_index(static_cast<const int64_t *>(routing_indices))
+                            : launch_index(static_cast<const int32_t *>(routing_indices));
 }
 
 extern "C" int fos_experts_route(const void *routing_indices, int index_bytes, int64_t tokens, int top_k, int num_experts,
@@ -512,7 +556,7 @@ extern "C" int fos_experts_route(const void *routing_indices, int index_bytes, i
                                  int32_t *row_expert, int32_t *pair_row, int32_t *pair_expert, int32_t *workspace,
                                  void *stream) {
     return experts_route(routing_indices, index_bytes, tokens, top_k, num_experts, rows_capacity, group_start, group_rows,
-                         row_token, row_expert, pair_row, pair_expert, workspace, nullptr, stream);
+                         row_token, row_expert, pair_row, pair_expert, workspace, nullptr, fos::TokenMaxima{}, FOS_BF16, stream);
 }
 
 // ---------------------------------------------------------------------------- the whole layer in one call
@@ -523,7 +567,7 @@ namespace {
 struct ExpertsWorkspace {
     int64_t capacity, pairs;
     // byte offsets into the workspace, each a multiple of 256
-    int64_t group_start, group_rows, row_token, row_expert, pair_row, pair_expert, route_work, amax;
+    int64_t group_start, group_rows, row_token, row_expert, pair_row, pair_expert, route_work, amax, token_max;
     int64_t rows_x, codes_x, sf_x, gate_up, gated, codes_g, sf_g, y, total;
 };
 
@@ -541,6 +585,7 @@ ExpertsWorkspace experts_workspace(int64_t tokens, int top_k, int num_experts, i
     w.pair_expert = take(4 * w.pairs);
     w.route_work = take(4 * static_cast<int64_t>(FOS_EXPERTS_ROUTE_WORKSPACE_INTS) * num_experts);
     w.amax = take(4 * 2 * num_experts);
+    w.token_max = take(4 * tokens);
     w.rows_x = take(2 * w.capacity * hidden);
     w.codes_x = take(w.capacity * hidden / 2);
     w.sf_x = take(w.capacity * hidden / 16);
@@ -585,16 +630,29 @@ extern "C" int fos_experts_forward(const void *x, int dtype, int64_t tokens, int
     float *amax = reinterpret_cast<float *>(base + w.amax);
     const int64_t gate_up_rows = round_up64(2 * intermediate, 128), down_rows = round_up64(hidden, 128);
 
+    if (ld_x < hidden || ld_out < hidden) return FOS_ERR_INVALID_ARGUMENT;
+    if (!aligned16(x, ld_x * 2)) return FOS_ERR_MISALIGNED;
+    // the rows are gathered by the quantization where the default rule lets it; then the maxima are the tokens'
+    const bool gathered = activation_rule == FOS_RULE_MSE;
+    const TokenMaxima maxima = gathered ? TokenMaxima{static_cast<const uint8_t *>(x), ld_x * 2, static_cast<int>(tokens),
+                                                      static_cast<int>(hidden / 8), reinterpret_cast<float *>(base + w.token_max)}
+                                        : TokenMaxima{};
     int st = experts_route(routing_indices, index_bytes, tokens, top_k, num_experts, w.capacity, ints(w.group_start),
                            ints(w.group_rows), ints(w.row_token), ints(w.row_expert), ints(w.pair_row), ints(w.pair_expert),
-                           ints(w.route_work), amax, stream_);
+                           ints(w.route_work), amax, maxima, dtype, stream_);
     if (st != FOS_OK) return st;
     const PairOrder order{ints(w.pair_row), ints(w.pair_expert), w.pairs, top_k};
-    st = gather_rows(x, dtype, ld_x, ints(w.row_token), base + w.rows_x, hidden, w.capacity, hidden, ints(w.row_expert), amax,
-                     &order, stream_);
-    if (st != FOS_OK) return st;
-    st = quantize_grouped_rows_in_use(base + w.rows_x, dtype, w.capacity, hidden, hidden, FOS_NVFP4, activation_rule, ints(w.group_start),
-                              ints(w.group_rows), num_experts, amax, base + w.codes_x, base + w.sf_x, amax, 0, stream_);
+    st = gathered ? quantize_grouped_gathered(x, dtype, tokens, hidden, ld_x, ints(w.row_token), w.capacity, activation_rule,
+                                              ints(w.group_start), ints(w.group_rows), num_experts, amax, base + w.codes_x,
+                                              base + w.sf_x, stream_)
+                  : FOS_ERR_UNSUPPORTED;
+    if (st == FOS_ERR_UNSUPPORTED) {
+        st = gather_rows(x, dtype, ld_x, ints(w.row_token), base + w.rows_x, hidden, w.capacity, hidden, ints(w.row_expert), amax,
+                         &order, stream_);
+        if (st != FOS_OK) return st;
+        st = quantize_grouped_rows_in_use(base + w.rows_x, dtype, w.capacity, hidden, hidden, FOS_NVFP4, activation_rule, ints(w.group_start),
+                                          ints(w.group_rows), num_experts, amax, base + w.codes_x, base + w.sf_x, amax, 0, stream_);
+    }
     if (st != FOS_OK) return st;
     const float denom = alpha_divisor(FOS_NVFP4, activation_rule, FOS_NVFP4, weight_rule);
     // the SwiGLU in the GEMM's epilogue where that GEMM runs on CTA pairs, else in a kernel of its own

@@ -58,6 +58,8 @@ struct QuantParams {
     const int32_t *rows_in_use;   // of each group: its rows beyond these may be left alone (quantize_rows_mse_kernel); or nullptr
     const int32_t *group_start;
     int num_groups;
+    const int32_t *row_source;    // of each row in use the row of x it is a copy of (quantize_rows_mse_kernel<.., true, true>)
+    int64_t source_rows;          // of x
 };
 
 
@@ -1713,7 +1715,10 @@ __device__ __forceinline__ int rows_in_use_at(const int *tile_rows, uint32_t sta
 }
 
 // IN_USE: a grouped launch whose rows beyond the group's rows in use come out as anything; warps without others skip them.
-template <typename T, bool IN_USE = false>
+// GATHER (with IN_USE): row r of the groups' buffer is row row_source[r] of x and the buffer itself does not exist: the
+// producer warp fetches a tile four rows per lane (tile::gather4), the quads with rows in use only. An experts layer's tokens
+// (8192 x 2880 to 4 experts each: 47 MB that stay in L2) are then not written out and read back as 189 MB.
+template <typename T, bool IN_USE = false, bool GATHER = false>
 __global__ void __launch_bounds__(FEED_THREADS, FOS_FEED_CTAS)
 quantize_rows_mse_kernel(const __grid_constant__ CUtensorMap map_x, const QuantParams p) {
     extern __shared__ uint8_t feed_smem_raw[];
@@ -1752,7 +1757,7 @@ quantize_rows_mse_kernel(const __grid_constant__ CUtensorMap map_x, const QuantP
 
     if (warp == FEED_CONSUMERS / 32) {
         // ---------------- producer ----------------
-        if (lane != 0) return;
+        if (!GATHER && lane != 0) return;
         const int step_r = static_cast<int>(gridDim.x) / tiles_c, step_c = static_cast<int>(gridDim.x) % tiles_c;
         int tr = tile_r0 + static_cast<int>(blockIdx.x) / tiles_c, tc_ = static_cast<int>(blockIdx.x) % tiles_c;
         int64_t tile = static_cast<int64_t>(tile_r0) * tiles_c + blockIdx.x;
@@ -1760,14 +1765,35 @@ quantize_rows_mse_kernel(const __grid_constant__ CUtensorMap map_x, const QuantP
         int issued = 0, s = 0;
         uint32_t parity = 1;   // of the "stage is free" barrier; the first round finds every stage free
         for (; issued < my_tiles; ++issued) {
-            if (issued >= FEED_STAGES && !mbar_wait(smem_u32(&empty_bar[s]), parity, &abort_flag, &g_wait_failures, 8))
-                break;
-            // (the arrive below releases this store to the consumers that acquire the barrier's phase)
-            tile_meta[s] = make_longlong2(static_cast<int64_t>(tr) * 128 * code_ld + tc_ * 32,
-                                          p.sf_tiled ? tile * 512 : static_cast<int64_t>(tr) * 128 * n_cb + tc_ * 4);
-            if constexpr (IN_USE) tile_rows[s] = ld_int(p.rows_in_use + blockIdx.y) - (tr - tile_r0) * FEED_TILE_ROWS;
-            mbar_expect_tx(smem_u32(&full_bar[s]), FEED_STAGE_BYTES);
-            tma_load_2d(stage0 + s * FEED_STAGE_BYTES, &map_x, tc_ * 128, tr * FEED_TILE_ROWS, smem_u32(&full_bar[s]));
+            bool free = issued < FEED_STAGES;
+            if (!free && lane == 0) free = mbar_wait(smem_u32(&empty_bar[s]), parity, &abort_flag, &g_wait_failures, 8);
+            if constexpr (GATHER) free = __shfl_sync(FULL, free ? 1 : 0, 0) != 0;
+            if (!free) break;
+            int rows = 0;
+            if constexpr (IN_USE) rows = ld_int(p.rows_in_use + blockIdx.y) - (tr - tile_r0) * FEED_TILE_ROWS;
+            if (lane == 0) {
+                // (the arrive below releases these stores to the consumers that acquire the barrier's phase)
+                tile_meta[s] = make_longlong2(static_cast<int64_t>(tr) * 128 * code_ld + tc_ * 32,
+                                              p.sf_tiled ? tile * 512 : static_cast<int64_t>(tr) * 128 * n_cb + tc_ * 4);
+                if constexpr (IN_USE) tile_rows[s] = rows;
+            }
+            if constexpr (GATHER) {
+                const int quads = rows <= 0 ? 0 : (rows >= FEED_TILE_ROWS ? FEED_TILE_ROWS / 4 : (rows + 3) / 4);
+                if (lane == 0) mbar_expect_tx(smem_u32(&full_bar[s]), quads * 512);
+                __syncwarp();
+                if (lane < quads) {
+                    const uint4 src = ld_16(p.row_source + tr * FEED_TILE_ROWS + lane * 4);
+                    int4 r = make_int4(static_cast<int>(src.x), static_cast<int>(src.y), static_cast<int>(src.z), static_cast<int>(src.w));
+                    // (the first row of a quad is in use; the others may be padding: any row does)
+                    r.y = r.y < 0 ? r.x : r.y;
+                    r.z = r.z < 0 ? r.x : r.z;
+                    r.w = r.w < 0 ? r.x : r.w;
+                    tma_gather4(stage0 + s * FEED_STAGE_BYTES + lane * 512, &map_x, tc_ * 128, r, smem_u32(&full_bar[s]));
+                }
+            } else {
+                mbar_expect_tx(smem_u32(&full_bar[s]), FEED_STAGE_BYTES);
+                tma_load_2d(stage0 + s * FEED_STAGE_BYTES, &map_x, tc_ * 128, tr * FEED_TILE_ROWS, smem_u32(&full_bar[s]));
+            }
             if (++s == FEED_STAGES) { s = 0; parity ^= 1u; }
             tile += gridDim.x;
             tr += step_r;
@@ -2039,13 +2065,14 @@ quantize_cols_tma_kernel(const __grid_constant__ CUtensorMap map_x, const QuantP
 }
 
 // Tensor map over x as bytes: [rows][cols * 2] with a row pitch of ld * 2, boxes of 128 rows x 128 bytes.
-inline bool make_x_map(CUtensorMap *map, const QuantParams &p, bool transposed) {
+// (`gather`: of one row.)
+inline bool make_x_map(CUtensorMap *map, const QuantParams &p, bool transposed, bool gather) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return false;
-    cuuint64_t dims[2] = {static_cast<cuuint64_t>(p.cols * 2), static_cast<cuuint64_t>(p.rows)};
+    cuuint64_t dims[2] = {static_cast<cuuint64_t>(p.cols * 2), static_cast<cuuint64_t>(gather ? p.source_rows : p.rows)};
     cuuint64_t strides[1] = {static_cast<cuuint64_t>(p.ld * 2)};
     cuuint32_t box[2] = {transposed ? static_cast<cuuint32_t>(COLS_BOX_BYTES) : 128u,
-                         static_cast<cuuint32_t>(transposed ? COLS_BOX_ROWS : FEED_TILE_ROWS)};
+                         static_cast<cuuint32_t>(gather ? 1 : (transposed ? COLS_BOX_ROWS : FEED_TILE_ROWS))};
     cuuint32_t estr[2] = {1, 1};
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(p.x), dims, strides, box, estr,
               CU_TENSOR_MAP_INTERLEAVE_NONE, transposed ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
@@ -2061,9 +2088,10 @@ cudaError_t launch_rows_tma_impl(const QuantParams &p, cudaStream_t stream, bool
     if (TRANSPOSED && (reinterpret_cast<uintptr_t>(p.codes) % 16 != 0 || reinterpret_cast<uintptr_t>(p.sf) % 2 != 0)) return cudaSuccess;
     if (p.cols * 2 >= (int64_t(1) << 31) || p.rows >= (int64_t(1) << 31) || p.ld * 2 >= (int64_t(1) << 40)) return cudaSuccess;
     CUtensorMap map;
-    if (!make_x_map(&map, p, TRANSPOSED)) return cudaSuccess;
-    // LEAN: 1 = the kernel of the default configuration, 2 = that for grouped launches that pack the rows in use only
-    auto kernel = LEAN ? quantize_rows_mse_kernel<T, LEAN == 2>
+    if (!make_x_map(&map, p, TRANSPOSED, LEAN == 3)) return cudaSuccess;
+    // LEAN: 1 = the kernel of the default configuration, 2 = that for grouped launches that pack the rows in use only, 3 =
+    // the same whose rows are gathered
+    auto kernel = LEAN ? quantize_rows_mse_kernel<T, LEAN >= 2, LEAN == 3>
                        : (TRANSPOSED ? quantize_cols_tma_kernel<T, KIND, TWO_D, EXTRAS> : quantize_rows_tma_kernel<T, KIND, FAKE, TWO_D, EXTRAS>);
     static int ctas_per_sm[64] = {};
     static int sm_count[64] = {};
@@ -2629,6 +2657,7 @@ template <typename T, int KIND>
 cudaError_t launch_rows_grouped(const fos::QuantParams &p, cudaStream_t stream, bool *launched) {
     using namespace fos;
     if constexpr (KIND == KIND_ADAPTIVE) {
+        if (p.row_source) return launch_rows_tma_impl<T, KIND, false, false, false, false, 3>(p, stream, launched);
         if (p.rule == FOS_RULE_MSE && p.variant != 2)
             return p.rows_in_use ? launch_rows_tma_impl<T, KIND, false, false, false, false, 2>(p, stream, launched)
                                  : launch_rows_tma_impl<T, KIND, false, false, false, false, 1>(p, stream, launched);
@@ -2639,7 +2668,7 @@ cudaError_t launch_rows_grouped(const fos::QuantParams &p, cudaStream_t stream, 
 static int quantize_grouped_entry(const void *x, int x_dtype, int64_t rows_capacity, int64_t cols, int64_t ld, int format,
                                   int scale_rule, const int32_t *group_start, const int32_t *group_rows, int num_groups,
                                   const float *amax_in, uint8_t *codes, uint8_t *sf, float *amax_out, int flags, bool in_use_only,
-                                  void *stream_) {
+                                  void *stream_, const int32_t *row_source = nullptr, int64_t source_rows = 0) {
     using namespace fos;
     if (!x || !codes || !sf || !amax_out || !group_start || !group_rows) return FOS_ERR_INVALID_ARGUMENT;
     if (num_groups <= 0 || num_groups > 65535) return FOS_ERR_INVALID_ARGUMENT;
@@ -2649,6 +2678,10 @@ static int quantize_grouped_entry(const void *x, int x_dtype, int64_t rows_capac
     if (format != FOS_NVFP4 && format != FOS_IF4) return format == FOS_MXFP4 ? FOS_ERR_UNSUPPORTED : FOS_ERR_INVALID_ARGUMENT;
     const bool is_static = scale_rule == FOS_RULE_STATIC_6 || scale_rule == FOS_RULE_STATIC_4;
     if (format == FOS_IF4 && is_static) return FOS_ERR_UNSUPPORTED;
+    // (gathered rows: one kernel, 16-byte loads of their sources, int32 row numbers)
+    if (row_source && (format != FOS_NVFP4 || scale_rule != FOS_RULE_MSE || !amax_in || !in_use_only ||
+                       reinterpret_cast<uintptr_t>(row_source) % 16 != 0 || source_rows <= 0 || source_rows >= (int64_t(1) << 31)))
+        return FOS_ERR_UNSUPPORTED;
     if (flags & (FOS_QUANTIZE_RHT | FOS_QUANTIZE_NO_TMA | FOS_QUANTIZE_UNBIASED)) return FOS_ERR_UNSUPPORTED;
     // the TMA-fed kernels only: whole 64-value scale tiles per row, 16-byte aligned rows
     if (cols % 64 != 0 || reinterpret_cast<uintptr_t>(x) % 16 != 0 || (ld * 2) % 16 != 0) return FOS_ERR_UNSUPPORTED;
@@ -2672,6 +2705,8 @@ static int quantize_grouped_entry(const void *x, int x_dtype, int64_t rows_capac
     p.x_is_ready = 1;
     p.group_start = group_start;
     p.rows_in_use = in_use_only ? group_rows : nullptr;
+    p.row_source = row_source;
+    p.source_rows = source_rows;
     p.num_groups = num_groups;
     if (amax_in) {
         if (amax_in != amax_out)
@@ -2723,6 +2758,13 @@ int fos::quantize_grouped_rows_in_use(const void *x, int x_dtype, int64_t rows_c
                                       const float *amax_in, uint8_t *codes, uint8_t *sf, float *amax_out, int flags, void *stream) {
     return quantize_grouped_entry(x, x_dtype, rows_capacity, cols, ld, format, scale_rule, group_start, group_rows, num_groups,
                                   amax_in, codes, sf, amax_out, flags, true, stream);
+}
+
+int fos::quantize_grouped_gathered(const void *x, int x_dtype, int64_t x_rows, int64_t cols, int64_t ld, const int32_t *row_source,
+                                   int64_t rows_capacity, int scale_rule, const int32_t *group_start, const int32_t *group_rows,
+                                   int num_groups, float *amax, uint8_t *codes, uint8_t *sf, void *stream) {
+    return quantize_grouped_entry(x, x_dtype, rows_capacity, cols, ld, FOS_NVFP4, scale_rule, group_start, group_rows, num_groups,
+                                  amax, codes, sf, amax, 0, true, stream, row_source, x_rows);
 }
 
 extern "C" int fos_quantize(const void *x, int x_dtype, int64_t rows, int64_t cols, int64_t ld, int format,
