@@ -33,9 +33,10 @@ int dequantize_mxfp4(const uint8_t *codes, const uint8_t *sf, int sf_layout, int
                      int64_t cols, void *out, int out_dtype, int64_t ld_out, cudaStream_t stream);
 
 // fos_quantize (NVFP4, 1-D blocks, tiled scales, amax computed) for a GEMM's A operand: the padding rows may be left alone,
-// because no row of a product depends on another.
+// because no row of a product depends on another. amax_parts: scratch of AMAX_PARTS_WORDS words.
+constexpr int AMAX_PARTS_WORDS = 1024;
 int quantize_activation(const void *x, int x_dtype, int64_t rows, int64_t cols, int64_t ld, int scale_rule, uint8_t *codes,
-                        uint8_t *sf, float *amax_out, void *stream);
+                        uint8_t *sf, float *amax_out, float *amax_parts, void *stream);
 // The steps of a chain over tensors that were complete before its first kernel: the maxima of up to three 16-byte aligned
 // tensors (row stride and columns multiples of 8) of one type in one launch, into words[0 .. n_words) which are zeroed first
 // (a job's words lie among them), then fos_quantize / fos_quantize_stochastic (NVFP4, tiled scales) of one of them at a

@@ -9,7 +9,7 @@ namespace fos {
 namespace {
 
 struct LinearWorkspace {
-    int64_t rows_p, k_p, codes, sf, amax, total;    // byte offsets, multiples of 256
+    int64_t rows_p, k_p, codes, sf, amax, amax_parts, total;    // byte offsets, multiples of 256
 };
 
 LinearWorkspace linear_workspace(int64_t rows, int64_t k) {
@@ -19,6 +19,7 @@ LinearWorkspace linear_workspace(int64_t rows, int64_t k) {
     int64_t at = 0;
     auto take = [&](int64_t bytes) { const int64_t here = at; at += round_up64(bytes, 256); return here; };
     w.amax = take(4);
+    w.amax_parts = take(4 * AMAX_PARTS_WORDS);
     w.codes = take(w.rows_p * w.k_p / 2);
     w.sf = take(w.rows_p * w.k_p / 16);
     w.total = at;
@@ -57,7 +58,8 @@ extern "C" int fos_linear_forward_bias(const void *x, int x_dtype, int64_t rows,
     if (workspace_bytes < w.total) return FOS_ERR_INVALID_ARGUMENT;
     uint8_t *base = static_cast<uint8_t *>(workspace);
     float *amax = reinterpret_cast<float *>(base + w.amax);
-    const int st = quantize_activation(x, x_dtype, rows, in_features, ld_x, activation_rule, base + w.codes, base + w.sf, amax, stream);
+    const int st = quantize_activation(x, x_dtype, rows, in_features, ld_x, activation_rule, base + w.codes, base + w.sf, amax,
+                                       reinterpret_cast<float *>(base + w.amax_parts), stream);
     if (st != FOS_OK) return st;
     const GemmScales scales{amax, w_amax, alpha_divisor(FOS_NVFP4, activation_rule, FOS_NVFP4, weight_rule), bias, true};
     return gemm_nvfp4_chained(base + w.codes, base + w.sf, w_codes, w_sf, scales, out, out_dtype, w.rows_p,

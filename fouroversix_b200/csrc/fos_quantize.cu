@@ -35,6 +35,8 @@ struct QuantParams {
     int64_t rows_p, cols_p;      // Y after padding
     const float *amax;           // device, final by the time the quantize kernel reads it
     float *amax_store;           // where the quantize kernel copies amax to, or null
+    const float *amax_parts;     // amax is the maximum of these (amax_parts_kernel), or nullptr: it is at `amax`
+    int num_amax_parts;          // at most MAX_AMAX_PARTS
     uint8_t *codes;
     uint8_t *sf;
     int rule;
@@ -67,11 +69,19 @@ struct QuantParams {
 // per-tensor amax
 // ------------------------------------------------------------------------------------
 
-template <typename T>
-__device__ __forceinline__ float abs_max8(uint4 w) {
-    float2 a = unpack2<T>(w.x), b = unpack2<T>(w.y), c = unpack2<T>(w.z), d = unpack2<T>(w.w);
-    return fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y))),
-                 fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fmaxf(fabsf(d.x), fabsf(d.y))));
+template <typename T> struct PairOf { using Type = __nv_bfloat162; };
+template <> struct PairOf<__half> { using Type = __half2; };
+
+// The larger magnitudes of two pairs of 16-bit numbers, packed (NaNs are skipped as fmaxf skips them): a quarter of the
+// instructions of unpacking to binary32.
+template <typename T> __device__ __forceinline__ uint32_t abs_max2(uint32_t m, uint32_t w) {
+    using P = typename PairOf<T>::Type;
+    const P r = __hmax2(reinterpret_cast<const P &>(m), __habs2(reinterpret_cast<const P &>(w)));
+    return reinterpret_cast<const uint32_t &>(r);
+}
+template <typename T> __device__ __forceinline__ float larger_half(uint32_t m) {
+    const float2 f = unpack2<T>(m);
+    return fmaxf(f.x, f.y);
 }
 
 // Sets the amax word (of a training step: words, at most 32) to zero. A kernel rather than a memset so that the chain "previous kernel ->
@@ -86,14 +96,15 @@ __global__ void zero_amax_kernel(float *amax, int words) {
 
 // max |x| of the chunks (VB bytes each) that one thread owns: 128 bytes per thread in flight per
 // round, every load of a round predicated (a chunk past the end contributes 0), so that there is
-// no serial tail of single loads, each of which would cost a full memory latency.
-template <typename T, int VB>
+// no serial tail of single loads, each of which would cost a full memory latency. COHERENT: x may have been written while this
+// kernel was already resident (see ld_b32).
+template <typename T, int VB, bool COHERENT = false>
 __device__ __forceinline__ float amax_chunks(const T *__restrict__ x, int64_t rows, int64_t cols, int64_t ld,
                                              int64_t tid, int64_t stride) {
     constexpr int EL = VB / 2, N = 128 / VB;
     const int64_t chunks_per_row = cols / EL, total = rows * chunks_per_row;
     const bool flat = ld == cols;
-    float m = 0.0f;
+    uint32_t m[2] = {0u, 0u};
     for (int64_t i = tid; i < total; i += N * stride) {
         uint32_t w[N][VB / 4];
 #pragma unroll
@@ -105,9 +116,10 @@ __device__ __forceinline__ float amax_chunks(const T *__restrict__ x, int64_t ro
                 const int64_t r = flat ? 0 : idx / chunks_per_row;
                 const T *ptr = flat ? x + idx * EL : x + r * ld + (idx - r * chunks_per_row) * EL;
                 if constexpr (VB == 32) {
-                    ldg_nc_32(ptr, w[k]);
+                    if constexpr (COHERENT) ld_32_stream(ptr, w[k]);
+                    else ldg_nc_32(ptr, w[k]);
                 } else {
-                    const uint4 v = ldg_nc_16(ptr);
+                    const uint4 v = COHERENT ? ld_16_stream(ptr) : ldg_nc_16(ptr);
                     w[k][0] = v.x; w[k][1] = v.y; w[k][2] = v.z; w[k][3] = v.w;
                 }
             }
@@ -115,10 +127,9 @@ __device__ __forceinline__ float amax_chunks(const T *__restrict__ x, int64_t ro
 #pragma unroll
         for (int k = 0; k < N; ++k)
 #pragma unroll
-            for (int j = 0; j < VB / 16; ++j)
-                m = fmaxf(m, abs_max8<T>(make_uint4(w[k][4 * j], w[k][4 * j + 1], w[k][4 * j + 2], w[k][4 * j + 3])));
+            for (int j = 0; j < VB / 4; ++j) m[j & 1] = abs_max2<T>(m[j & 1], w[k][j]);
     }
-    return m;
+    return fmaxf(larger_half<T>(m[0]), larger_half<T>(m[1]));
 }
 
 // max |x| with 32-byte (or 16-byte) loads, 128 bytes in flight per thread, then one atomicMax per CTA.
@@ -158,6 +169,59 @@ __global__ void __launch_bounds__(256) amax_kernel(const T *__restrict__ x, int6
         // non-negative floats order like their bit patterns
         atomicMax(reinterpret_cast<int *>(amax), __float_as_int(m));
     }
+}
+
+// The same for a caller with room for a word per CTA: no word to zero, so no launch before it (1.5 us, and 2.5 us of the
+// host), and no atomics. The kernel that takes the words finds their maximum itself (amax_of). Launched as the dependent
+// of whatever may be writing x, which it waits for, so its loads are coherent ones.
+constexpr int MAX_AMAX_PARTS = 1024;
+
+template <typename T>
+__global__ void __launch_bounds__(256) amax_parts_kernel(const T *__restrict__ x, int64_t rows, int64_t cols, int64_t ld, int vec,
+                                                         float *parts) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    float m = 0.0f;
+    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    if (vec == 32) {
+        m = amax_chunks<T, 32, true>(x, rows, cols, ld, tid, stride);
+    } else if (vec == 16) {
+        m = amax_chunks<T, 16, true>(x, rows, cols, ld, tid, stride);
+    } else {
+        const int64_t total = rows * cols;
+        for (int64_t i = tid; i < total; i += stride) {
+            const int64_t r = i / cols, c = i - r * cols;
+            m = fmaxf(m, larger_half<T>(abs_max2<T>(0u, ld_b16(x + r * ld + c))));
+        }
+    }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(FULL, m, o));
+    __shared__ float warp_max[8];
+    if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) m = fmaxf(m, warp_max[w]);
+        parts[blockIdx.x] = m;
+    }
+}
+
+// The tensor's amax for the 256 threads (whole warps, barrier 1) of a quantize kernel that call this, behind their wait.
+__device__ __forceinline__ float amax_of(const QuantParams &p, const float *amax, float (&warp_max)[8]) {
+    if (p.amax_parts == nullptr) return *reinterpret_cast<const volatile float *>(amax);
+    float m = 0.0f;
+#pragma unroll
+    for (int i = 0; i < MAX_AMAX_PARTS / 256; ++i) {
+        const int at = i * 256 + static_cast<int>(threadIdx.x);
+        if (at < p.num_amax_parts) m = fmaxf(m, ld_float(p.amax_parts + at));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(FULL, m, o));
+    if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = m;
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+#pragma unroll
+    for (int w = 0; w < 8; ++w) m = fmaxf(m, warp_max[w]);
+    return m;
 }
 
 // One amax per group of rows: CTA (x, g) takes a share of rows group_start[g] .. + group_rows[g] and ends with an
@@ -322,6 +386,7 @@ template <typename T> __device__ __forceinline__ float rotated_max(float m) {
 template <typename T, bool PLAIN>
 __device__ __forceinline__ float rotated_column_pairs(const T *__restrict__ x, int64_t rows, int64_t cols, int64_t ld, int64_t tid,
                                                       int64_t stride, float &plain) {
+    uint32_t largest = 0u;
     const int64_t per_row = cols >> 1, step_r = stride / per_row, step_c = stride - step_r * per_row, bands = rows >> 4;
     int64_t r = tid / per_row, c = tid - r * per_row;
     float m = 0.0f;
@@ -332,7 +397,7 @@ __device__ __forceinline__ float rotated_column_pairs(const T *__restrict__ x, i
         for (int i = 0; i < 16; ++i) p[i] = __ldg(src + i * (ld >> 1));
         if constexpr (PLAIN) {
 #pragma unroll
-            for (int i = 0; i < 16; i += 4) plain = fmaxf(plain, abs_max8<T>(make_uint4(p[i], p[i + 1], p[i + 2], p[i + 3])));
+            for (int i = 0; i < 16; ++i) largest = abs_max2<T>(largest, p[i]);
         }
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
@@ -344,6 +409,7 @@ __device__ __forceinline__ float rotated_column_pairs(const T *__restrict__ x, i
         c += step_c;
         if (c >= per_row) { c -= per_row; ++r; }
     }
+    if constexpr (PLAIN) plain = larger_half<T>(largest);
     return m;
 }
 
@@ -1377,7 +1443,8 @@ quantize_rows_kernel(const QuantParams p) {
     // programmatic dependent launch (behind the amax pass only, see launch_rows) this CTA may be running before that
     // kernel has finished.
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const TensorConsts tc = tensor_consts<KIND>(*reinterpret_cast<const volatile float *>(p.amax), p.rule);
+    __shared__ float warp_max[8];
+    const TensorConsts tc = tensor_consts<KIND>(amax_of(p, p.amax, warp_max), p.rule);
     if (p.amax_store != nullptr && threadIdx.x == 0 && blockIdx.x == 0) *p.amax_store = tc.amax;
     if (threadIdx.x < 128)
         lut[threadIdx.x] = scale_entry(threadIdx.x, tc, rule_has_filter<KIND, false>(p.rule) && !p.exact_only && tc.filter_ok);
@@ -1527,7 +1594,8 @@ quantize_rows_tma_kernel(const __grid_constant__ CUtensorMap map_x, const QuantP
     // amax comes from the previous kernel in the stream; with programmatic dependent launch this
     // CTA may be running before that kernel has finished.
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const TensorConsts tc = tensor_consts<KIND>(*reinterpret_cast<const volatile float *>(amax_ptr), p.rule, EXTRAS && p.unbiased);
+    __shared__ float warp_max[8];
+    const TensorConsts tc = tensor_consts<KIND>(amax_of(p, amax_ptr, warp_max), p.rule, EXTRAS && p.unbiased);
     if (p.amax_store != nullptr && threadIdx.x == 0 && blockIdx.x == 0) *p.amax_store = tc.amax;
     if (threadIdx.x < 128)
         lut[threadIdx.x] = scale_entry(threadIdx.x, tc, rule_has_filter<KIND, TWO_D>(p.rule) && !p.exact_only && tc.filter_ok);
@@ -1812,7 +1880,8 @@ quantize_rows_mse_kernel(const __grid_constant__ CUtensorMap map_x, const QuantP
 
     // ---------------- consumers ----------------
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const TensorConsts tc = tensor_consts<KIND_ADAPTIVE>(*reinterpret_cast<const volatile float *>(amax_ptr), p.rule);
+    __shared__ float warp_max[8];
+    const TensorConsts tc = tensor_consts<KIND_ADAPTIVE>(amax_of(p, amax_ptr, warp_max), p.rule);
     if (p.amax_store != nullptr && threadIdx.x == 0 && blockIdx.x == 0) *p.amax_store = tc.amax;
     if (threadIdx.x < 128)
         lut[threadIdx.x] = scale_entry(threadIdx.x, tc, p.rule == FOS_RULE_MSE && !p.exact_only && tc.filter_ok);
@@ -2223,7 +2292,7 @@ quantize_small_kernel(const QuantParams p, float *amax_out) {
     // x, and whatever still reads the outputs of an earlier call; only then may the kernel behind this one start
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    float m = 0.0f;
+    uint32_t m2 = 0u;
 #pragma unroll
     for (int j = 0; j < SMALL_BLOCKS; ++j) {
         const int i = first + j * STEP;
@@ -2232,8 +2301,10 @@ quantize_small_kernel(const QuantParams p, float *amax_out) {
         const uint4 a = make_uint4(w[0], w[1], w[2], w[3]), b = make_uint4(w[4], w[5], w[6], w[7]);
         words[j][0][tid] = a;
         words[j][1][tid] = b;
-        m = fmaxf(m, fmaxf(abs_max8<T>(a), abs_max8<T>(b)));
+#pragma unroll
+        for (int k = 0; k < 8; ++k) m2 = abs_max2<T>(m2, w[k]);
     }
+    float m = larger_half<T>(m2);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(FULL, m, o));
     if (lane == 0) warp_max[warp] = m;
@@ -2404,12 +2475,13 @@ cudaError_t launch_small_kind(const QuantParams &p, int kind, float *amax_out, c
     return launch_small<T, KIND_IF4>(p, amax_out, stream, launched);
 }
 
+// With `parts` (room for MAX_AMAX_PARTS words) one word per CTA there, their number in *num_parts, instead of the maximum at amax.
 template <typename T>
 cudaError_t launch_amax(const void *x, int64_t rows, int64_t cols, int64_t ld, bool vec16, float *amax,
-                        cudaStream_t stream, bool rht = false, bool transposed = false) {
+                        cudaStream_t stream, bool rht = false, bool transposed = false, float *parts = nullptr, int *num_parts = nullptr) {
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg = dependent_launch_config(1, 32, stream, attr);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, zero_amax_kernel, amax, 1);
+    cudaError_t e = parts ? cudaSuccess : cudaLaunchKernelEx(&cfg, zero_amax_kernel, amax, 1);
     if (e != cudaSuccess) return e;
     if (rht) {
         // amax of the ROTATED tensor: one wave of the four CTAs per SM
@@ -2455,6 +2527,12 @@ cudaError_t launch_amax(const void *x, int64_t rows, int64_t cols, int64_t ld, b
         if (even >= resident[slot] / 2) blocks = even;                   // (tiny inputs keep one CTA per 256 chunks)
     }
     if (blocks < 1) blocks = 1;
+    if (parts) {
+        if (blocks > MAX_AMAX_PARTS) blocks = MAX_AMAX_PARTS;
+        *num_parts = static_cast<int>(blocks);
+        cfg = dependent_launch_config(static_cast<unsigned>(blocks), 256, stream, attr);
+        return cudaLaunchKernelEx(&cfg, amax_parts_kernel<T>, static_cast<const T *>(x), rows, cols, ld, vec, parts);
+    }
     cfg = dependent_launch_config(static_cast<unsigned>(blocks), 256, stream, attr);
     return cudaLaunchKernelEx(&cfg, amax_kernel<T>, static_cast<const T *>(x), rows, cols, ld, vec, amax);
 }
@@ -2550,7 +2628,7 @@ extern "C" int fos_pseudo_quantize(const void *x, int x_dtype, int64_t rows, int
 static int quantize_entry(const void *x, int x_dtype, int64_t rows, int64_t cols, int64_t ld, int format,
                           int scale_rule, int block_2d, int transpose, int sf_layout, const float *amax_in,
                           uint8_t *codes, uint8_t *sf, float *amax_out, int flags, void *stream_, int stochastic,
-                          uint64_t seed, bool no_padding = false, bool x_is_ready = false) {
+                          uint64_t seed, bool no_padding = false, bool x_is_ready = false, float *amax_parts = nullptr) {
     using namespace fos;
     if (stochastic) {
         // stochastic rounding lives in the TMA-fed kernels only: NVFP4, 1-D blocks, aligned input
@@ -2621,10 +2699,11 @@ static int quantize_entry(const void *x, int x_dtype, int64_t rows, int64_t cols
         p.amax_store = amax_in != amax_out ? amax_out : nullptr;
     } else {
         FOS_CUDA_TRY(x_dtype == FOS_BF16
-                         ? launch_amax<__nv_bfloat16>(x, rows, cols, ld, vec16, amax_out, stream, p.rht != 0, transpose != 0)
-                         : launch_amax<__half>(x, rows, cols, ld, vec16, amax_out, stream, p.rht != 0, transpose != 0));
+                         ? launch_amax<__nv_bfloat16>(x, rows, cols, ld, vec16, amax_out, stream, p.rht != 0, transpose != 0, amax_parts, &p.num_amax_parts)
+                         : launch_amax<__half>(x, rows, cols, ld, vec16, amax_out, stream, p.rht != 0, transpose != 0, amax_parts, &p.num_amax_parts));
         p.amax = amax_out;
-        p.amax_store = nullptr;
+        p.amax_parts = amax_parts;
+        p.amax_store = amax_parts ? amax_out : nullptr;
     }
     // When this call launched the amax pass itself, the kernel before the quantize kernel is that
     // pass: it does not write x, so x can be fetched while it drains.
@@ -2774,10 +2853,12 @@ extern "C" int fos_quantize(const void *x, int x_dtype, int64_t rows, int64_t co
                           amax_out, flags, stream, 0, 0);
 }
 
+static_assert(fos::AMAX_PARTS_WORDS == fos::MAX_AMAX_PARTS, "the callers' room for the parts");
+
 int fos::quantize_activation(const void *x, int x_dtype, int64_t rows, int64_t cols, int64_t ld, int scale_rule, uint8_t *codes,
-                             uint8_t *sf, float *amax_out, void *stream) {
+                             uint8_t *sf, float *amax_out, float *amax_parts, void *stream) {
     return quantize_entry(x, x_dtype, rows, cols, ld, FOS_NVFP4, scale_rule, 0, 0, FOS_SF_TILED, nullptr, codes, sf, amax_out, 0, stream,
-                          0, 0, true);
+                          0, 0, true, false, amax_parts);
 }
 
 int fos::amax_of_tensors(const AmaxJob *jobs, int count, int x_dtype, float *words, int n_words, void *stream_) {
