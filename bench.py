@@ -529,7 +529,7 @@ def gemm_section(args, fos, B200MatmulBackend, dev, rank, world, peaks):
             "sm_mhz": None if clocks is None else clocks["sm_mhz"],
             "ms_x_mhz": None if clocks is None or clocks["sm_mhz"] is None else ms * clocks["sm_mhz"],
             "clock_reasons": None if clocks is None else clocks["reasons"],
-            "gpu_launches_per_step": 4 if is_if4 else 2, "l2": "operands + output exceed L2",
+            "gpu_launches_per_step": 2, "l2": "operands + output exceed L2",
         }
         del qa, qb, d
         torch.cuda.empty_cache()

@@ -303,6 +303,16 @@ __device__ __forceinline__ uint32_t ld_b32(const void *p) {
     asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
+__device__ __forceinline__ uint32_t ld_b8(const void *p) {
+    uint32_t v;
+    asm volatile("ld.global.u8 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint2 ld_8(const void *p) {                         // `p` 8-byte aligned
+    uint2 v;
+    asm volatile("ld.global.v2.b32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
 __device__ __forceinline__ uint32_t ld_b16(const void *p) {
     uint16_t v;
     asm volatile("ld.global.b16 %0, [%1];" : "=h"(v) : "l"(p));

@@ -9,7 +9,7 @@
 // multiplied with fp32 accumulation. Two kernels:
 //
 //   expand_kernel    packed codes + scales -> fp16 [rows_p, k_p] in a caller-provided workspace
-//                    (one pass per operand, HBM-bound, 0.5625 B read + 2 B written per element)
+//                    (one launch for both operands, HBM-bound, 0.5625 B read + 2 B written per element)
 //   gemm_f16_kernel  tcgen05.mma kind::f16 (M 128, N 256, K 16) over the two fp16 matrices: the
 //                    pipeline of the NVFP4 kernel without scale factors, which leaves room in
 //                    tensor memory for two accumulators, so the epilogue of one tile overlaps the
@@ -27,11 +27,13 @@ namespace {
 // ---------------------------------------------------------------------------- expand
 
 struct ExpandParams {
-    const uint8_t *codes;
-    const uint8_t *sf;
-    __half *out;
-    int64_t rows_p, cols_p;
-    int format, sf_tiled;
+    struct Operand {
+        const uint8_t *codes, *sf;
+        int format, sf_tiled;
+    } operand[2];
+    __half *out;                 // the first operand's rows, then the second's
+    int64_t first, total;        // blocks of the first operand, of both
+    int64_t n_cb;                // blocks per row
 };
 
 __device__ __forceinline__ float as_fp16_value(float v) { return __half2float(__float2half_rn(v)); }
@@ -90,44 +92,44 @@ __device__ __forceinline__ bool expand_block_packed(uint2 c, uint32_t sfb, bool 
 }
 
 // One thread per 16-value block: 8 bytes of codes + 1 scale byte -> 32 bytes of fp16. Four blocks per thread and
-// round, their loads issued before the first is decoded.
+// round, their loads issued before the first is decoded. Both operands are one range of blocks, in which codes and outputs
+// (and row-major scales, IF4's) lie one after the other: no row and column to be found. Launched as the dependent of the
+// kernel that packs an operand, so what it reads is loaded coherently.
 constexpr int EXPAND_DEPTH = 4;
 __global__ void __launch_bounds__(256) expand_kernel(const ExpandParams p) {
-    const int64_t n_cb = p.cols_p >> 4;
-    const int64_t total = p.rows_p * n_cb;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    const bool small = total < (int64_t(1) << 31);
-    for (int64_t i0 = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i0 < total; i0 += stride * EXPAND_DEPTH) {
+    for (int64_t i0 = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i0 < p.total; i0 += stride * EXPAND_DEPTH) {
         uint2 c[EXPAND_DEPTH];
         uint32_t sfbs[EXPAND_DEPTH];
-        int64_t offs[EXPAND_DEPTH];
 #pragma unroll
         for (int d = 0; d < EXPAND_DEPTH; ++d) {
             const int64_t i = i0 + d * stride;
-            offs[d] = -1;
             c[d] = make_uint2(0u, 0u);
             sfbs[d] = 0u;
-            if (i < total) {
-                // (a 64-bit division costs about as much as decoding the block)
-                const int64_t r = small ? static_cast<int64_t>(static_cast<uint32_t>(i) / static_cast<uint32_t>(n_cb)) : i / n_cb;
-                const int64_t cb = i - r * n_cb;
-                c[d] = *reinterpret_cast<const uint2 *>(p.codes + r * (p.cols_p >> 1) + cb * 8);
-                sfbs[d] = p.sf[sf_offset(r, cb, n_cb, p.sf_tiled != 0)];
-                offs[d] = r * p.cols_p + cb * 16;
+            if (i < p.total) {
+                const bool second = i >= p.first;
+                const ExpandParams::Operand &op = p.operand[second ? 1 : 0];
+                const int64_t j = second ? i - p.first : i;
+                c[d] = ld_8(op.codes + j * 8);
+                sfbs[d] = ld_b8(op.sf + (op.sf_tiled ? sf_offset(j / p.n_cb, j % p.n_cb, p.n_cb, true) : j));
             }
         }
 #pragma unroll
         for (int d = 0; d < EXPAND_DEPTH; ++d) {
-            if (offs[d] < 0) continue;
-            uint4 *dst = reinterpret_cast<uint4 *>(p.out + offs[d]);
+            const int64_t i = i0 + d * stride;
+            if (i >= p.total) continue;
+            const bool if4 = p.operand[i >= p.first ? 1 : 0].format == FOS_IF4;
+            uint4 *dst = reinterpret_cast<uint4 *>(p.out + i * 16);
             uint32_t o[8];
-            if (expand_block_packed(c[d], sfbs[d], p.format == FOS_IF4, o)) {
+            if (expand_block_packed(c[d], sfbs[d], if4, o)) {
                 stg_32(dst, o);
                 continue;
             }
             uint32_t sfb = sfbs[d];
-            const bool is_int = p.format == FOS_IF4 && (sfb & 0x80u);
-            if (p.format == FOS_IF4) sfb &= 0x7fu;
+            const bool is_int = if4 && (sfb & 0x80u);
+            if (if4) sfb &= 0x7fu;
             const float s16 = e4m3_to_float(sfb);
             __align__(16) __half h[16];
 #pragma unroll
@@ -163,11 +165,17 @@ constexpr int THREADS = 64 + 32 * EPI_WARPS;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
 
 struct F16GemmParams {
-    const float *alpha;
+    const float *alpha;                   // the product's factor, or nullptr:
+    const float *amax_a, *amax_b;         // then it is amax_a * amax_b / denom (what fos_gemm_alpha computes)
+    float denom;
     void *d;
     int32_t *status;
     int64_t m_p, n_p, k_p, m, n, ldd;
 };
+
+__device__ __forceinline__ float f16_alpha(const F16GemmParams &p) {
+    return p.alpha ? ld_float(p.alpha) : __fdiv_rn(__fmul_rn(ld_float(p.amax_a), ld_float(p.amax_b)), p.denom);
+}
 
 // kind::f16 instruction descriptor: fp32 accumulate (1 in bits [4,6)), A and B fp16 (0 in [7,10) and
 // [10,13)), both K-major, N >> 3 in [17,23), M >> 4 in [24,29).
@@ -290,7 +298,7 @@ gemm_f16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         // ------------------------------------------------------------------ epilogue
         const int quad = warp & 3, half = (warp - 2) >> 2;
         constexpr int COLS = BLOCK_N / 2;
-        const float alpha = __ldg(p.alpha);
+        const float alpha = f16_alpha(p);
         OUT *out = static_cast<OUT *>(p.d);
         const bool vec_ok = (reinterpret_cast<uintptr_t>(out) % 16 == 0) && ((p.ldd * sizeof(OUT)) % 16 == 0);
         uint32_t tile_i = 0;
@@ -475,7 +483,7 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         // ------------------------------------------------------------------ epilogue (both CTAs)
         const int quad = warp & 3, half = (warp - 2) >> 2;
         asm volatile("griddepcontrol.wait;" ::: "memory");     // alpha, and whoever still reads d
-        const float alpha = ld_float(p.alpha);
+        const float alpha = f16_alpha(p);
         OUT *out = static_cast<OUT *>(p.d);
         const bool vec16 = (reinterpret_cast<uintptr_t>(out) % 16 == 0) && ((p.ldd * sizeof(OUT)) % 16 == 0);
         const bool vec32 = (reinterpret_cast<uintptr_t>(out) % 32 == 0) && ((p.ldd * sizeof(OUT)) % 32 == 0);
@@ -538,14 +546,10 @@ int launch_f16(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &
     return FOS_OK;
 }
 
-int launch_expand(const uint8_t *codes, const uint8_t *sf, int format, int sf_layout, int64_t rows_p, int64_t cols_p,
-                  __half *out, cudaStream_t stream) {
-    ExpandParams p{codes, sf, out, rows_p, cols_p, format, sf_layout == FOS_SF_TILED};
-    const int64_t total = rows_p * (cols_p / 16);
-    int64_t blocks = (total + 255) / 256;
+int launch_expand(const ExpandParams &p, cudaStream_t stream) {
+    int64_t blocks = (p.total + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    expand_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(p);
-    FOS_CUDA_TRY(cudaGetLastError());
+    FOS_CUDA_TRY(launch_dependent(expand_kernel, dim3(static_cast<unsigned>(blocks)), 256, 0, stream, p));
     return FOS_OK;
 }
 
@@ -567,17 +571,20 @@ namespace {
 constexpr int64_t STATIC_WORKSPACE_BYTES = int64_t(FOS_GEMM_IF4_STATIC_WORKSPACE_BYTES);
 static __device__ __align__(256) unsigned char g_static_workspace[STATIC_WORKSPACE_BYTES];
 
-// Validates the arguments shared by both entry points, expands both operands into `workspace`
-// and runs the fp16 GEMM. Allocates nothing.
+// The product's factor: a word, or the two maxima it is formed from.
+struct F16Alpha { const float *alpha, *amax_a, *amax_b; float denom; };
+
+// Expands both operands into `workspace` and runs the fp16 GEMM. Allocates nothing.
 int gemm_if4_impl(const uint8_t *a_codes, const uint8_t *a_sf, int a_format, int a_sf_layout, const uint8_t *b_codes,
-                  const uint8_t *b_sf, int b_format, int b_sf_layout, const float *alpha, void *d, int out_dtype,
+                  const uint8_t *b_sf, int b_format, int b_sf_layout, const F16Alpha &alpha, void *d, int out_dtype,
                   int64_t m_p, int64_t n_p, int64_t k_p, int64_t m, int64_t n, int64_t ldd, void *workspace,
                   int32_t *status, cudaStream_t stream) {
     __half *a16 = static_cast<__half *>(workspace);
     __half *b16 = a16 + m_p * k_p;
     int st;
-    if ((st = launch_expand(a_codes, a_sf, a_format, a_sf_layout, m_p, k_p, a16, stream)) != FOS_OK) return st;
-    if ((st = launch_expand(b_codes, b_sf, b_format, b_sf_layout, n_p, k_p, b16, stream)) != FOS_OK) return st;
+    ExpandParams x{{{a_codes, a_sf, a_format, a_sf_layout == FOS_SF_TILED}, {b_codes, b_sf, b_format, b_sf_layout == FOS_SF_TILED}},
+                   a16, m_p * (k_p / 16), (m_p + n_p) * (k_p / 16), k_p / 16};
+    if ((st = launch_expand(x, stream)) != FOS_OK) return st;
     CUtensorMap map_a, map_b, map_b_pair;
     if ((st = make_operand_map(&map_a, a16, m_p, k_p * 2, BLOCK_M)) != FOS_OK) return st;
     if ((st = make_operand_map(&map_b, b16, n_p, k_p * 2, BLOCK_N)) != FOS_OK) return st;
@@ -587,7 +594,7 @@ int gemm_if4_impl(const uint8_t *a_codes, const uint8_t *a_sf, int a_format, int
     } else {
         FOS_CUDA_TRY(wait_failures_ptr(&status));   // the library's sticky word
     }
-    F16GemmParams p{alpha, d, status, m_p, n_p, k_p, m, n, ldd};
+    F16GemmParams p{alpha.alpha, alpha.amax_a, alpha.amax_b, alpha.denom, d, status, m_p, n_p, k_p, m, n, ldd};
     if (out_dtype == FOS_BF16) return launch_f16<__nv_bfloat16>(map_a, map_b, map_b_pair, p, stream);
     if (out_dtype == FOS_FP16) return launch_f16<__half>(map_a, map_b, map_b_pair, p, stream);
     return launch_f16<float>(map_a, map_b, map_b_pair, p, stream);
@@ -625,8 +632,28 @@ extern "C" int fos_gemm_if4(const uint8_t *a_codes, const uint8_t *a_sf, int a_f
     if (!workspace || workspace_bytes < fos_gemm_if4_workspace_bytes(m_p, n_p, k_p)) return FOS_ERR_INVALID_ARGUMENT;
     if (reinterpret_cast<uintptr_t>(workspace) % 128) return FOS_ERR_MISALIGNED;
     if ((st = check_device()) != FOS_OK) return st;
-    return gemm_if4_impl(a_codes, a_sf, a_format, a_sf_layout, b_codes, b_sf, b_format, b_sf_layout, alpha, d, out_dtype,
+    return gemm_if4_impl(a_codes, a_sf, a_format, a_sf_layout, b_codes, b_sf, b_format, b_sf_layout, {alpha, nullptr, nullptr, 1.0f}, d, out_dtype,
                          m_p, n_p, k_p, m, n, ldd, workspace, status, static_cast<cudaStream_t>(stream_));
+}
+
+extern "C" int fos_gemm_if4_scaled(const uint8_t *a_codes, const uint8_t *a_sf, const float *amax_a, int a_format, int a_sf_layout,
+                                   int rule_a, int unbiased_a, const uint8_t *b_codes, const uint8_t *b_sf, const float *amax_b,
+                                   int b_format, int b_sf_layout, int rule_b, int unbiased_b, void *d, int out_dtype, int64_t m_p,
+                                   int64_t n_p, int64_t k_p, int64_t m, int64_t n, int64_t ldd, void *workspace,
+                                   int64_t workspace_bytes, int32_t *status, void *stream_) {
+    using namespace fos;
+    if (!amax_b) return FOS_ERR_INVALID_ARGUMENT;
+    int st = check_gemm_if4_args(a_codes, a_sf, a_format, a_sf_layout, b_codes, b_sf, b_format, b_sf_layout, amax_a, d, out_dtype, m_p, n_p,
+                                 k_p, m, n, ldd);
+    if (st != FOS_OK) return st;
+    for (int rule : {rule_a, rule_b})
+        if (rule < FOS_RULE_STATIC_6 || rule > FOS_RULE_ABS_MAX) return FOS_ERR_INVALID_ARGUMENT;
+    if (!workspace || workspace_bytes < fos_gemm_if4_workspace_bytes(m_p, n_p, k_p)) return FOS_ERR_INVALID_ARGUMENT;
+    if (reinterpret_cast<uintptr_t>(workspace) % 128) return FOS_ERR_MISALIGNED;
+    if ((st = check_device()) != FOS_OK) return st;
+    const F16Alpha alpha{nullptr, amax_a, amax_b, alpha_divisor(a_format, rule_a, b_format, rule_b, unbiased_a, unbiased_b)};
+    return gemm_if4_impl(a_codes, a_sf, a_format, a_sf_layout, b_codes, b_sf, b_format, b_sf_layout, alpha, d, out_dtype, m_p, n_p, k_p, m, n,
+                         ldd, workspace, status, static_cast<cudaStream_t>(stream_));
 }
 
 // fos_gemm_if4 for callers that cannot hand over scratch memory: the expanded operands go into
@@ -659,6 +686,6 @@ extern "C" int fos_gemm_if4_static(const uint8_t *a_codes, const uint8_t *a_sf, 
         }
         workspace = device_address[dev];
     }
-    return gemm_if4_impl(a_codes, a_sf, a_format, a_sf_layout, b_codes, b_sf, b_format, b_sf_layout, alpha, d, out_dtype,
+    return gemm_if4_impl(a_codes, a_sf, a_format, a_sf_layout, b_codes, b_sf, b_format, b_sf_layout, {alpha, nullptr, nullptr, 1.0f}, d, out_dtype,
                          m_p, n_p, k_p, m, n, ldd, workspace, status, static_cast<cudaStream_t>(stream_));
 }

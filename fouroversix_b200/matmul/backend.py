@@ -116,15 +116,11 @@ class B200MatmulBackend:
                     out.data_ptr(), _native.elem_code(torch_out), m_p, n_p, k_p, m, n, out.stride(0),
                     opts, status_ptr, stream), "fos_gemm_nvfp4")
             else:
-                alpha = torch.empty(1, dtype=torch.float32, device=dev)
-                _native.check(lib.fos_gemm_alpha_ex(
-                    input.amax.data_ptr(), fa, input.scale_rule.cuda_id, unbiased_a, other.amax.data_ptr(), fb,
-                    other.scale_rule.cuda_id, unbiased_b, alpha.data_ptr(), stream), "fos_gemm_alpha")
                 nbytes = int(lib.fos_gemm_if4_workspace_bytes(m_p, n_p, k_p))
                 workspace = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-                _native.check(lib.fos_gemm_if4(
-                    a_vals.data_ptr(), a_sf.data_ptr(), fa, _layout(input),
-                    b_vals.data_ptr(), b_sf.data_ptr(), fb, _layout(other), alpha.data_ptr(),
+                _native.check(lib.fos_gemm_if4_scaled(
+                    a_vals.data_ptr(), a_sf.data_ptr(), input.amax.data_ptr(), fa, _layout(input), input.scale_rule.cuda_id, unbiased_a,
+                    b_vals.data_ptr(), b_sf.data_ptr(), other.amax.data_ptr(), fb, _layout(other), other.scale_rule.cuda_id, unbiased_b,
                     out.data_ptr(), _native.elem_code(torch_out), m_p, n_p, k_p, m, n, out.stride(0),
                     workspace.data_ptr(), nbytes, status_ptr, stream), "fos_gemm_if4")
         if status is not None and int(status.item()) != 0:

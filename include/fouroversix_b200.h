@@ -509,6 +509,14 @@ int fos_gemm_if4(const uint8_t *a_codes, const uint8_t *a_sf, int a_format, int 
                  int64_t m, int64_t n, int64_t ldd, void *workspace, int64_t workspace_bytes,
                  int32_t *status, void *stream);
 
+/* fos_gemm_alpha_ex and fos_gemm_if4 in one call: alpha = amax_a * amax_b / denominator(formats, rules) is formed in the GEMM, by
+ * the same operations. */
+int fos_gemm_if4_scaled(const uint8_t *a_codes, const uint8_t *a_sf, const float *amax_a, int a_format, int a_sf_layout, int rule_a,
+                        int unbiased_a, const uint8_t *b_codes, const uint8_t *b_sf, const float *amax_b, int b_format,
+                        int b_sf_layout, int rule_b, int unbiased_b, void *d, int out_dtype, int64_t m_p, int64_t n_p,
+                        int64_t k_p, int64_t m, int64_t n, int64_t ldd, void *workspace, int64_t workspace_bytes,
+                        int32_t *status, void *stream);
+
 /*
  * fos_gemm_if4 without a workspace argument, for callers that have no way to obtain device
  * scratch: code that runs where allocating is forbidden or impossible - in another library's
