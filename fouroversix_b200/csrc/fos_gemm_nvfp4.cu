@@ -73,6 +73,11 @@ constexpr int NUM_THREADS = 384;                   // warps: 0 TMA, 1 MMA, 2-9 e
 // From 640 on pairs are never behind by more than 2 %; below, it depends on how the groups' own rows fall (a group of 257 to
 // 384 rows leaves half a pair idle), which the host does not know.
 constexpr int PAIR_MIN_GROUP_ROWS = 640;
+// With the SwiGLU in the epilogue, which only pairs have, they also save the kernel that does it otherwise (10 us and more):
+// from the size where they stop being behind by more than that.
+constexpr int PAIR_MIN_GLU_ROWS = 256;
+// Up to this many rows per group on average a grouped GEMM is bound by the weights (see grouped_kernel_for).
+constexpr int FEW_GROUP_ROWS = 64;
 constexpr int MAX_GROUPS = 256;                    // of a grouped launch (their row ranges are kept in shared memory)
 constexpr int SF_COL0 = 256;                       // tensor-memory columns: accumulators first, then per
                                                    // stage 16 columns of A scales and N/8 of B scales
@@ -1089,13 +1094,23 @@ inline int gemm_kernel_for(int64_t m, int64_t m_p, int64_t n_p, int64_t k_p, int
     return wide ? GEMM_256 : GEMM_128;
 }
 
-// 256-row tiles waste half a tile per group on average, 128-row tiles a quarter of that: pairs where groups are long
-inline int grouped_kernel_for(int64_t rows_capacity, int num_groups, int64_t n_p, int variant, int max_ctas, int sms) {
+// 256-row tiles waste half a tile per group on average, 128-row tiles a quarter of that: pairs where groups are long.
+// Groups of a few rows each (a decoding step) are bound by their weights' way out of HBM: a tile then takes the time of its
+// columns, whatever its width, and the width is the one whose last round is fuller. 32 groups of 32 rows, 2880 columns: 12
+// wide tiles a group are 2.6 rounds, which take 3, 23 narrow ones 4.97 half rounds. `pair_min_rows`: buffer rows per group
+// from which pairs are taken.
+inline int grouped_kernel_for(int64_t rows_capacity, int num_groups, int64_t n_p, int variant, int max_ctas, int sms,
+                              int pair_min_rows = PAIR_MIN_GROUP_ROWS) {
     if (variant == 128) return GEMM_128;
     sms = sms_allowed(sms, max_ctas);
     const int64_t tiles_256 = (rows_capacity / BLOCK_M) * ((n_p + 255) / 256);
     const bool wide = n_p >= 256 && (tiles_256 * 2 > sms || variant == 256);
-    if (variant == 0 && wide && max_ctas != 1 && rows_capacity / num_groups >= PAIR_MIN_GROUP_ROWS) return GEMM_PAIR;
+    if (variant == 0 && wide && max_ctas != 1 && rows_capacity / num_groups >= pair_min_rows) return GEMM_PAIR;
+    // (the buffer has up to 127 rows of padding per group)
+    if (variant == 0 && wide && rows_capacity <= static_cast<int64_t>(num_groups) * (127 + FEW_GROUP_ROWS)) {
+        auto columns = [&](int64_t width) { return (num_groups * ((n_p + width - 1) / width) + sms - 1) / sms * width; };
+        if (columns(128) < columns(256)) return GEMM_128;
+    }
     return wide ? GEMM_256 : GEMM_128;
 }
 
@@ -1356,7 +1371,7 @@ static int gemm_grouped_entry(const uint8_t *a_codes, const uint8_t *a_sf, const
     p.num_groups = num_groups;
     // how many row blocks are in use is known on the device only: the grid is sized for the buffers, and
     // CTAs that find no tile leave at once
-    const int choice = grouped_kernel_for(rows_capacity, num_groups, n_p, variant, max_ctas, sms);
+    const int choice = grouped_kernel_for(rows_capacity, num_groups, n_p, variant, max_ctas, sms, glu ? PAIR_MIN_GLU_ROWS : PAIR_MIN_GROUP_ROWS);
     if (glu) {
         if (choice != GEMM_PAIR) return FOS_ERR_UNSUPPORTED;
         p.glu = *glu;

@@ -2185,7 +2185,8 @@ cudaError_t launch_rows_tma_impl(const QuantParams &p, cudaStream_t stream, bool
     if (grouped) {
         // how the rows are spread over the groups is known on the device only: every group gets twice its even
         // share of the resident CTAs (at least 8), and a CTA whose group has fewer tiles than that leaves at once
-        grid = 2 * grid / p.num_groups;
+        // (few tiles, a decoding step: the even share, so that all CTAs are resident at once)
+        grid = (n_tiles > 6 * grid ? 2 * grid : grid) / p.num_groups;
         if (grid < 8) grid = 8;
     }
     if (grid > n_tiles) grid = n_tiles;
