@@ -26,9 +26,9 @@ __device__ __forceinline__ void chain_begin() {
 }
 
 constexpr int ROW_THREADS = 256;         // of the kernels that give a row to a warp
-constexpr int GATHER_CTAS = 6, GLU_CTAS = 4, COMBINE_CTAS = 4;     // their CTAs per SM (one wave: a warp takes rows in turn)
+constexpr int GATHER_CTAS = 6, GLU_CTAS = 4;     // their CTAs per SM (one wave: a warp takes rows in turn)
 
-// The row kernels below give a warp a row, or (few rows) a segment of one: a row is a few KB, so its own latency (look
+// The two row kernels below give a warp a row, or (few rows) a segment of one: a row is a few KB, so its own latency (look
 // up the row, fetch it, reduce) dominates, and warps that do not wait for one another overlap theirs. A unit of work is
 // (row, segment); in the one-call form of the layer the rows are taken in the order of the (token, slot) pairs, which
 // visits the rows in use only - of 256 tokens over 32 experts a quarter of the padded buffer - and leaves the padding
@@ -135,72 +135,44 @@ constexpr int MAX_TOP_K = 8;
 
 // out[t] = sum over the token's experts, in ascending order of the expert's index (the order in which the
 // reference's host loop adds them into the 16-bit result), of (y[row] + bias[expert]) * weight, every
-// operation rounded to the 16-bit type, the running sum too (packed 16-bit arithmetic: see glu_words).
-// A warp takes a token (or a segment of one, see RowUnits): lane k holds slot k, the slots' order comes from shuffles, and the
-// lanes fetch four slots' pieces at a time. (A CTA per token, whose first thread sorted the slots between two barriers,
-// left the loads of 8 tokens per SM in flight.) Bound by HBM.
+// operation rounded to the 16-bit type, the running sum too (packed 16-bit arithmetic: see glu_word).
 template <typename T>
-__global__ void __launch_bounds__(ROW_THREADS, COMBINE_CTAS)
+__global__ void __launch_bounds__(256)
 combine_kernel(const uint8_t *__restrict__ y, int64_t ld_y_bytes, const uint8_t *__restrict__ bias, int64_t ld_bias_bytes,
                const int32_t *__restrict__ pair_row, const int32_t *__restrict__ pair_expert,
-               const uint16_t *__restrict__ pair_weight, int top_k, uint8_t *__restrict__ out, int64_t ld_out_bytes,
-               const RowUnits units, int chunks) {
+               const uint16_t *__restrict__ pair_weight, int top_k, uint8_t *__restrict__ out, int64_t ld_out_bytes, int tokens,
+               int chunks) {
     chain_begin();
     using P = typename Half16<T>::Pair;
-    constexpr unsigned ALL = 0xffffffffu;
-    const int lane = threadIdx.x & 31, warps = gridDim.x * (ROW_THREADS / 32), total = units.rows * units.segs;
-    for (int i = (blockIdx.x * ROW_THREADS + threadIdx.x) >> 5; i < total; i += warps) {
-        const int t = units.segs == 1 ? i : i / units.segs, seg = i - t * units.segs;
-        const int c_begin = seg * units.seg_chunks, c_end = min(chunks, c_begin + units.seg_chunks);
-        int expert = 0, row = -1;
-        uint32_t weight = 0u;
-        if (lane < top_k) {
-            const int64_t at = static_cast<int64_t>(t) * top_k + lane;
-            expert = ld_int(pair_expert + at);
-            row = ld_int(pair_row + at);                  // (-1: the expert index was out of range)
-            weight = ld_b16(pair_weight + at);
-        }
-        // the place of this lane's slot in the order of the experts (equal ones in the order of the slots) ...
-        int place = 0;
-        for (int k = 0; k < top_k; ++k) {
-            const int other = __shfl_sync(ALL, expert, k);
-            place += other < expert || (other == expert && k < lane) ? 1 : 0;
-        }
-        // ... and the slot whose place is this lane's number
-        int slot = 0;
-        for (int k = 0; k < top_k; ++k) slot = __shfl_sync(ALL, place, k) == lane ? k : slot;
-        expert = __shfl_sync(ALL, expert, slot);
-        row = __shfl_sync(ALL, row, slot);
-        weight = __shfl_sync(ALL, weight, slot) * 0x10001u;
-        uint4 *dst = reinterpret_cast<uint4 *>(out + t * ld_out_bytes);
-        for (int c0 = c_begin; c0 < c_end; c0 += 32) {
-            const int c = c0 + lane;
-            uint32_t acc[4] = {0u, 0u, 0u, 0u};
-            for (int k0 = 0; k0 < top_k; k0 += 4) {
-                uint4 v[4], b[4];
-                uint32_t w[4];
-                bool used[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int r = __shfl_sync(ALL, row, k0 + u), e = __shfl_sync(ALL, expert, k0 + u);
-                    w[u] = __shfl_sync(ALL, weight, k0 + u);
-                    used[u] = k0 + u < top_k && r >= 0;
-                    if (used[u] && c < c_end) {
-                        v[u] = ld_16_stream(reinterpret_cast<const uint4 *>(y + r * ld_y_bytes) + c);
-                        b[u] = ld_16(reinterpret_cast<const uint4 *>(bias + e * ld_bias_bytes) + c);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (!used[u]) continue;
-                    const P w2 = as_pair<P>(w[u]);
-                    const uint32_t vv[4] = {v[u].x, v[u].y, v[u].z, v[u].w}, bb[4] = {b[u].x, b[u].y, b[u].z, b[u].w};
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        acc[j] = as_word(__hadd2_rn(as_pair<P>(acc[j]), __hmul2_rn(__hadd2_rn(as_pair<P>(vv[j]), as_pair<P>(bb[j])), w2)));
-                }
+    __shared__ int s_row[MAX_TOP_K], s_ex[MAX_TOP_K];
+    __shared__ uint32_t s_w[MAX_TOP_K];
+    for (int t = blockIdx.x; t < tokens; t += gridDim.x) {
+        __syncthreads();                                  // the previous token's slots have been read
+        if (threadIdx.x == 0) {                           // insertion sort of the token's slots by expert
+            for (int k = 0; k < top_k; ++k) {
+                const int64_t i = static_cast<int64_t>(t) * top_k + k;
+                const int e = ld_int(pair_expert + i), r = ld_int(pair_row + i);
+                const uint32_t w = ld_b16(pair_weight + i);
+                int j = k;
+                for (; j > 0 && s_ex[j - 1] > e; --j) { s_ex[j] = s_ex[j - 1]; s_row[j] = s_row[j - 1]; s_w[j] = s_w[j - 1]; }
+                s_ex[j] = e; s_row[j] = r; s_w[j] = w | (w << 16);
             }
-            if (c < c_end) dst[c] = make_uint4(acc[0], acc[1], acc[2], acc[3]);
+        }
+        __syncthreads();
+        uint4 *dst = reinterpret_cast<uint4 *>(out + t * ld_out_bytes);
+        for (int c = threadIdx.x; c < chunks; c += blockDim.x) {
+            uint32_t acc[4] = {0u, 0u, 0u, 0u};
+            for (int k = 0; k < top_k; ++k) {
+                if (s_row[k] < 0) continue;               // a slot whose expert index was out of range
+                const uint4 v = ld_16_stream(reinterpret_cast<const uint4 *>(y + s_row[k] * ld_y_bytes) + c);
+                const uint4 b = ld_16(reinterpret_cast<const uint4 *>(bias + s_ex[k] * ld_bias_bytes) + c);
+                const P w2 = as_pair<P>(s_w[k]);
+                const uint32_t vv[4] = {v.x, v.y, v.z, v.w}, bb[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    acc[i] = as_word(__hadd2_rn(as_pair<P>(acc[i]), __hmul2_rn(__hadd2_rn(as_pair<P>(vv[i]), as_pair<P>(bb[i])), w2)));
+            }
+            dst[c] = make_uint4(acc[0], acc[1], acc[2], acc[3]);
         }
     }
 }
@@ -381,6 +353,18 @@ route_place_kernel(const IDX *__restrict__ routing, int pairs, int seg, int top_
     }
 }
 
+// Threads per CTA for rows of `chunks` 16-byte pieces: the multiple of 32 up to 256 that leaves the fewest
+// idle threads in a row's last round (the larger on a tie).
+inline unsigned threads_for(int chunks) {
+    unsigned best = 256;
+    double best_eff = 0.0;
+    for (unsigned t = 64; t <= 256; t += 32) {
+        const double eff = static_cast<double>(chunks) / (static_cast<double>((chunks + t - 1) / t) * t);
+        if (eff >= best_eff) { best_eff = eff; best = t; }
+    }
+    return best;
+}
+
 inline bool aligned16(const void *p, int64_t ld_bytes) {
     return reinterpret_cast<uintptr_t>(p) % 16 == 0 && ld_bytes % 16 == 0;
 }
@@ -492,21 +476,20 @@ extern "C" int fos_experts_combine(const void *y, int dtype, int64_t ld_y, const
     const int st = check_device();
     if (st != FOS_OK) return st;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
-    unsigned g = 0;
-    const int chunks = static_cast<int>(hidden / 8);
-    const RowUnits units = row_units(tokens, chunks, COMBINE_CTAS, &g);
+    const unsigned g = static_cast<unsigned>(tokens < 148 * 8 ? tokens : 148 * 8);
+    const int n = static_cast<int>(tokens), chunks = static_cast<int>(hidden / 8);
     if (dtype == FOS_BF16)
-        FOS_CUDA_TRY(launch_dependent(combine_kernel<__nv_bfloat16>, dim3(g), ROW_THREADS, 0, stream,
+        FOS_CUDA_TRY(launch_dependent(combine_kernel<__nv_bfloat16>, dim3(g), threads_for(chunks), 0, stream,
             static_cast<const uint8_t *>(y), ld_y * 2,
             static_cast<const uint8_t *>(bias), hidden * 2, pair_row, pair_expert,
             static_cast<const uint16_t *>(pair_weight), top_k,
-            static_cast<uint8_t *>(out), ld_out * 2, units, chunks));
+            static_cast<uint8_t *>(out), ld_out * 2, n, chunks));
     else
-        FOS_CUDA_TRY(launch_dependent(combine_kernel<__half>, dim3(g), ROW_THREADS, 0, stream,
+        FOS_CUDA_TRY(launch_dependent(combine_kernel<__half>, dim3(g), threads_for(chunks), 0, stream,
             static_cast<const uint8_t *>(y), ld_y * 2,
             static_cast<const uint8_t *>(bias), hidden * 2, pair_row, pair_expert,
             static_cast<const uint16_t *>(pair_weight), top_k,
-            static_cast<uint8_t *>(out), ld_out * 2, units, chunks));
+            static_cast<uint8_t *>(out), ld_out * 2, n, chunks));
     return FOS_OK;
 }
 
