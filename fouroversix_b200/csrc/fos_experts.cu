@@ -118,10 +118,9 @@ glu_kernel(const uint8_t *__restrict__ gate_up, int64_t ld_gu_bytes, const uint8
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 if (c0 + 32 * u >= c_end) break;
-                const uint4 packed = make_uint4(glu_words<T>(g[u][0].x, g[u][0].y, w[u][0].x, w[u][0].y, alpha, limit2, floor2, one2),
-                                                glu_words<T>(g[u][0].z, g[u][0].w, w[u][0].z, w[u][0].w, alpha, limit2, floor2, one2),
-                                                glu_words<T>(g[u][1].x, g[u][1].y, w[u][1].x, w[u][1].y, alpha, limit2, floor2, one2),
-                                                glu_words<T>(g[u][1].z, g[u][1].w, w[u][1].z, w[u][1].w, alpha, limit2, floor2, one2));
+                const uint32_t gate_up8[8] = {g[u][0].x, g[u][0].y, g[u][0].z, g[u][0].w, g[u][1].x, g[u][1].y, g[u][1].z, g[u][1].w};
+                const uint32_t bias8[8] = {w[u][0].x, w[u][0].y, w[u][0].z, w[u][0].w, w[u][1].x, w[u][1].y, w[u][1].z, w[u][1].w};
+                const uint4 packed = glu_words<T>(gate_up8, bias8, alpha, limit2, floor2, one2);
                 dst[c0 + 32 * u] = packed;
                 m2 = fold_abs_max<P>(m2, packed);
             }

@@ -715,21 +715,26 @@ __device__ __forceinline__ void glu_columns(OUT *dst, const uint32_t *acc, float
                                             typename Half16<OUT>::Pair floor2, typename Half16<OUT>::Pair one2,
                                             typename Half16<OUT>::Pair &max2) {
     using H = Half16<OUT>;
+    uint4 bias0[N / 16], bias1[N / 16];
+#pragma unroll
+    for (int i = 0; i < N / 16; ++i) {
+        bias0[i] = bias1[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (16 * i < cols_left) {                            // (the product's width is a multiple of 16)
+            bias0[i] = ld_16(bias + 16 * i);
+            bias1[i] = ld_16(bias + 16 * i + 8);
+        }
+    }
 #pragma unroll
     for (int c = 0; c < N; c += 16) {
-        if (c >= cols_left) break;                           // (the product's width is a multiple of 16)
-        const uint4 b0 = ld_16(bias + c), b1 = ld_16(bias + c + 8);
+        if (c >= cols_left) break;
+        const uint4 b0 = bias0[c / 16], b1 = bias1[c / 16];
         const uint32_t b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-        uint32_t o[4];
+        uint32_t gate_up[8];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t *v = acc + c + 4 * i;
-            o[i] = glu_words<OUT>(H::pack(alpha * __uint_as_float(v[0]), alpha * __uint_as_float(v[1])),
-                                  H::pack(alpha * __uint_as_float(v[2]), alpha * __uint_as_float(v[3])), b[2 * i], b[2 * i + 1],
-                                  glu.alpha, limit2, floor2, one2);
-        }
+        for (int i = 0; i < 8; ++i)
+            gate_up[i] = H::pack(alpha * __uint_as_float(acc[c + 2 * i]), alpha * __uint_as_float(acc[c + 2 * i + 1]));
+        const uint4 packed = glu_words<OUT>(gate_up, b, glu.alpha, limit2, floor2, one2);
         if (!row_ok) continue;
-        const uint4 packed = make_uint4(o[0], o[1], o[2], o[3]);
         *reinterpret_cast<uint4 *>(dst + c / 2) = packed;
         max2 = fold_abs_max(max2, packed);
     }

@@ -62,16 +62,18 @@ __device__ __forceinline__ void raise_amax(typename Half16<T>::Pair m2, float *a
 template <typename T> __device__ __noinline__ uint32_t sigmoid16x2_sequence(float t0, float t1) {
     return Half16<T>::pack(1.0f / (1.0f + expf(-t0)), 1.0f / (1.0f + expf(-t1)));
 }
-template <typename T> __device__ __forceinline__ uint32_t sigmoid16x2(float t0, float t1) {
+// (`sure`: the result is the sequence's. The callers take the fast path of several pairs before they look: with a branch per
+// pair the chains of one warp, some 300 cycles each, ran one after the other.)
+template <typename T> __device__ __forceinline__ uint32_t sigmoid16x2(float t0, float t1, bool &sure) {
     using H = Half16<T>;
     const float s0 = __fdividef(1.0f, 1.0f + __expf(-t0)), s1 = __fdividef(1.0f, 1.0f + __expf(-t1));
     const float w0 = s0 * fmaf(fabsf(t0), 0x1.8p-23f, 0x1.8p-20f), w1 = s1 * fmaf(fabsf(t1), 0x1.8p-23f, 0x1.8p-20f);
     const uint32_t low = H::pack(s0 - w0, s1 - w1), high = H::pack(s0 + w0, s1 + w1);
-    if (low == high && fmaxf(fabsf(t0), fabsf(t1)) <= 64.0f) return low;
-    return sigmoid16x2_sequence<T>(t0, t1);
+    sure = low == high && fmaxf(fabsf(t0), fabsf(t1)) <= 64.0f;
+    return low;
 }
 
-// The reference's chain on two (gate, up) pairs, every intermediate rounded to the 16-bit type:
+// The reference's chain on eight (gate, up) pairs, two to a word of the output, every intermediate rounded to the 16-bit type:
 //   g = gate + bias_g; u = up + bias_u; g = min(g, limit); u = min(max(u, -limit), limit)   (NaN passes through)
 //   out = (u + 1) * (g * sigmoid(g * alpha))
 // A (gate, up) pair is one 32-bit word, and a packed 16-bit addition, multiplication or fused multiply-add
@@ -81,20 +83,37 @@ template <typename T> __device__ __forceinline__ uint32_t sigmoid16x2(float t0, 
 // the sigmoid run in binary32. The _rn forms of the packed operations keep the compiler from contracting a
 // multiplication and the addition after it into one fused operation, which would drop a rounding. limit2 = (r, r), floor2 = (-inf, -r) with r the limit rounded to the type:
 // comparing with r selects the same values as comparing with the limit itself, because no number of the type
-// lies between the two. Returns the output in the low half.
+// lies between the two.
 template <typename T>
-__device__ __forceinline__ uint32_t glu_words(uint32_t gate_up0, uint32_t gate_up1, uint32_t bias0, uint32_t bias1, float alpha,
-                                              typename Half16<T>::Pair limit2, typename Half16<T>::Pair floor2,
-                                              typename Half16<T>::Pair one2) {
+__device__ __forceinline__ uint4 glu_words(const uint32_t (&gate_up)[8], const uint32_t (&bias)[8], float alpha,
+                                           typename Half16<T>::Pair limit2, typename Half16<T>::Pair floor2,
+                                           typename Half16<T>::Pair one2) {
     using H = Half16<T>;
     using P = typename H::Pair;
-    P v0 = __hadd2_rn(as_pair<P>(gate_up0), as_pair<P>(bias0)), v1 = __hadd2_rn(as_pair<P>(gate_up1), as_pair<P>(bias1));
-    v0 = __hmax2_nan(__hmin2_nan(v0, limit2), floor2);
-    v1 = __hmax2_nan(__hmin2_nan(v1, limit2), floor2);
-    const uint32_t g2 = __byte_perm(as_word(v0), as_word(v1), 0x5410), u2 = __byte_perm(as_word(v0), as_word(v1), 0x7632);
-    const uint32_t t2 = H::pack(H::lo(g2) * alpha, H::hi(g2) * alpha);
-    const P w = __hmul2_rn(as_pair<P>(g2), as_pair<P>(sigmoid16x2<T>(H::lo(t2), H::hi(t2))));
-    return as_word(__hmul2_rn(__hadd2_rn(as_pair<P>(u2), one2), w));
+    uint32_t g2[4], u2[4], t2[4], s2[4], o[4];
+    bool all_sure = true;
+    bool sure[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        P v0 = __hadd2_rn(as_pair<P>(gate_up[2 * i]), as_pair<P>(bias[2 * i]));
+        P v1 = __hadd2_rn(as_pair<P>(gate_up[2 * i + 1]), as_pair<P>(bias[2 * i + 1]));
+        v0 = __hmax2_nan(__hmin2_nan(v0, limit2), floor2);
+        v1 = __hmax2_nan(__hmin2_nan(v1, limit2), floor2);
+        g2[i] = __byte_perm(as_word(v0), as_word(v1), 0x5410);
+        u2[i] = __byte_perm(as_word(v0), as_word(v1), 0x7632);
+        t2[i] = H::pack(H::lo(g2[i]) * alpha, H::hi(g2[i]) * alpha);
+        s2[i] = sigmoid16x2<T>(H::lo(t2[i]), H::hi(t2[i]), sure[i]);
+        all_sure = all_sure && sure[i];
+    }
+    if (!all_sure) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (!sure[i]) s2[i] = sigmoid16x2_sequence<T>(H::lo(t2[i]), H::hi(t2[i]));
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        o[i] = as_word(__hmul2_rn(__hadd2_rn(as_pair<P>(u2[i]), one2), __hmul2_rn(as_pair<P>(g2[i]), as_pair<P>(s2[i]))));
+    return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
 }  // namespace
