@@ -147,14 +147,24 @@ combine_kernel(const uint8_t *__restrict__ y, int64_t ld_y_bytes, const uint8_t 
     __shared__ uint32_t s_w[MAX_TOP_K];
     for (int t = blockIdx.x; t < tokens; t += gridDim.x) {
         __syncthreads();                                  // the previous token's slots have been read
-        if (threadIdx.x == 0) {                           // insertion sort of the token's slots by expert
-            for (int k = 0; k < top_k; ++k) {
-                const int64_t i = static_cast<int64_t>(t) * top_k + k;
-                const int e = ld_int(pair_expert + i), r = ld_int(pair_row + i);
-                const uint32_t w = ld_b16(pair_weight + i);
-                int j = k;
-                for (; j > 0 && s_ex[j - 1] > e; --j) { s_ex[j] = s_ex[j - 1]; s_row[j] = s_row[j - 1]; s_w[j] = s_w[j - 1]; }
-                s_ex[j] = e; s_row[j] = r; s_w[j] = w | (w << 16);
+        if (threadIdx.x < 32) {                           // the token's slots in the order of their experts, a lane each
+            const int lane = static_cast<int>(threadIdx.x);
+            int e = 0, r = -1, place = 0;
+            uint32_t w = 0u;
+            if (lane < top_k) {
+                const int64_t i = static_cast<int64_t>(t) * top_k + lane;
+                e = ld_int(pair_expert + i);
+                r = ld_int(pair_row + i);
+                w = ld_b16(pair_weight + i);
+            }
+            for (int k = 0; k < top_k; ++k) {             // (equal ones in the order of the slots)
+                const int other = __shfl_sync(0xffffffffu, e, k);
+                place += other < e || (other == e && k < lane) ? 1 : 0;
+            }
+            if (lane < top_k) {
+                s_ex[place] = e;
+                s_row[place] = r;
+                s_w[place] = w | (w << 16);
             }
         }
         __syncthreads();
