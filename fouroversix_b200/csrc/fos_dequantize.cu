@@ -17,69 +17,65 @@ struct DequantParams {
     int64_t rows_p, cols_p, rows, cols, ld_out;
     int format, sf_tiled;
     float divisor;
-    int sf_words;             // tiled scales, 16-byte aligned
-    int run_log2;             // blocks of a row that a unit takes, 2^5 .. 2^8
-    uint32_t units;
 };
 
-// One thread per 16-value block: 8 bytes of codes and one scale in, 16 values out. A unit of work is a run of 2^run_log2 blocks
-// (32 to 256, whichever leaves the fewest threads idle) of one block column in the four rows r, r + 32, r + 64, r + 96
-// of a 128-row tile, so a warp reads and writes contiguous pieces of four rows, all loads of a unit are issued before the
-// first block is decoded, and the four rows' scales are one 16-byte load where they are tiled (a tile keeps them side by side;
-// byte by byte a warp touched as many bytes of L2 for the scales as for the codes). One wave of CTAs.
-constexpr int DEQUANT_ROWS = 4, DEQUANT_CTAS = 5;
+// One thread per 16-value block: 8 bytes of codes and one scale in, 16 values out. A CTA takes
+// runs of 256 blocks of one row (contiguous codes in, contiguous values out), DEPTH runs at a time: the
+// loads of all of them are issued before the first block is decoded, so a thread has DEPTH loads in
+// flight instead of one (with one, the kernel waited a memory latency per run: 29 us for 8192 x 4096).
+constexpr int DEQUANT_DEPTH = 4;
 
 // SMALL: every offset (bytes of codes and scales, elements of the output) fits 32 bits, so the address arithmetic
 // of a block is 32-bit (a third of the kernel's instructions were 64-bit multiplies and compares).
 template <typename OUT, bool SMALL>
-__global__ void __launch_bounds__(256, DEQUANT_CTAS) dequantize_kernel(const DequantParams p) {
+__global__ void __launch_bounds__(256) dequantize_kernel(const DequantParams p) {
     using idx_t = typename std::conditional<SMALL, uint32_t, int64_t>::type;
-    const uint32_t n_cb = static_cast<uint32_t>(p.cols_p >> 4);
-    const uint32_t cb_used = static_cast<uint32_t>((p.cols + 15) >> 4), chunks = (cb_used + (1u << p.run_log2) - 1u) >> p.run_log2;
-    const uint32_t tx = threadIdx.x & ((1u << p.run_log2) - 1u), ty = threadIdx.x >> p.run_log2;
-    const uint32_t per_cta = 256u >> p.run_log2;                           // row groups per unit; a divisor of 32
+    const int n_cb = static_cast<int>(p.cols_p >> 4);
+    const int cb_used = static_cast<int>((p.cols + 15) >> 4);
+    const int chunks = (cb_used + 255) >> 8;
+    const idx_t units = static_cast<idx_t>(p.rows * chunks);
     const DequantConsts k = dequant_consts(__ldg(p.amax), p.divisor);
-    const idx_t code_ld = static_cast<idx_t>(p.cols_p >> 1), ld_out = static_cast<idx_t>(p.ld_out), rows = static_cast<idx_t>(p.rows);
-    for (uint32_t u = blockIdx.x; u < p.units; u += gridDim.x) {
-        const uint32_t at = u / chunks, cb = ((u - at * chunks) << p.run_log2) + tx, group = at * per_cta + ty;
-        const uint32_t tile_row = group >> 5, in_tile = group & 31u;
-        const idx_t row0 = static_cast<idx_t>(tile_row) * 128 + in_tile;
-        if (cb >= cb_used || row0 >= rows) continue;
-        uint2 c[DEQUANT_ROWS];
-        uint32_t sf[DEQUANT_ROWS];
+    // a unit is (row, chunk of 256 blocks); this CTA's units are blockIdx.x, + gridDim.x, ...: the pair is advanced
+    // by additions (a division per unit cost more than decoding it)
+    const int step_r = static_cast<int>(gridDim.x) / chunks, step_c = static_cast<int>(gridDim.x) % chunks;
+    idx_t row0 = static_cast<idx_t>(blockIdx.x) / static_cast<idx_t>(chunks);
+    int ch0 = static_cast<int>(blockIdx.x - row0 * chunks);
+    const idx_t code_ld = static_cast<idx_t>(p.cols_p >> 1), ld_out = static_cast<idx_t>(p.ld_out);
+    for (idx_t u0 = blockIdx.x; u0 < units; u0 += static_cast<idx_t>(gridDim.x) * DEQUANT_DEPTH) {
+        uint2 c[DEQUANT_DEPTH];
+        uint32_t sfb[DEQUANT_DEPTH];
+        idx_t row[DEQUANT_DEPTH];
+        int col_block[DEQUANT_DEPTH];
 #pragma unroll
-        for (int d = 0; d < DEQUANT_ROWS; ++d) {
-            const idx_t r = row0 + 32 * d;
+        for (int d = 0; d < DEQUANT_DEPTH; ++d) {
+            const idx_t r = row0;
+            const int cb = ch0 * 256 + static_cast<int>(threadIdx.x);
+            row[d] = r;
+            col_block[d] = (u0 + static_cast<idx_t>(d) * gridDim.x < units && cb < cb_used) ? cb : -1;
             c[d] = make_uint2(0u, 0u);
-            if (r < rows) c[d] = *reinterpret_cast<const uint2 *>(p.codes + r * code_ld + cb * 8);
-        }
-        if (p.sf_words) {
-            const uint4 w = *reinterpret_cast<const uint4 *>(
-                p.sf + (static_cast<idx_t>(tile_row) * (n_cb >> 2) + (cb >> 2)) * 512 + in_tile * 16);
-            const uint32_t pick = cb & 3u;                                  // (the other selectors: zeros)
-            sf[0] = __byte_perm(w.x, 0u, pick | 0x4440u);
-            sf[1] = __byte_perm(w.y, 0u, pick | 0x4440u);
-            sf[2] = __byte_perm(w.z, 0u, pick | 0x4440u);
-            sf[3] = __byte_perm(w.w, 0u, pick | 0x4440u);
-        } else {
-#pragma unroll
-            for (int d = 0; d < DEQUANT_ROWS; ++d) {
-                const idx_t r = row0 + 32 * d;
-                sf[d] = 0u;
-                if (r < rows) sf[d] = p.sf[p.sf_tiled ? (static_cast<idx_t>(tile_row) * (n_cb >> 2) + (cb >> 2)) * 512 + in_tile * 16 + d * 4 + (cb & 3u)
-                                                      : r * static_cast<idx_t>(n_cb) + cb];
+            sfb[d] = 0u;
+            if (col_block[d] >= 0) {
+                c[d] = *reinterpret_cast<const uint2 *>(p.codes + r * code_ld + cb * 8);
+                const idx_t sf_off = p.sf_tiled
+                    ? ((r >> 7) * static_cast<idx_t>(n_cb >> 2) + static_cast<idx_t>(cb >> 2)) * 512 +
+                          static_cast<idx_t>((static_cast<int>(r) & 31) * 16 + ((static_cast<int>(r) >> 5) & 3) * 4 + (cb & 3))
+                    : r * static_cast<idx_t>(n_cb) + static_cast<idx_t>(cb);
+                sfb[d] = p.sf[sf_off];
             }
+            row0 += step_r;                      // the next unit of this CTA
+            ch0 += step_c;
+            if (ch0 >= chunks) { ch0 -= chunks; ++row0; }
         }
 #pragma unroll
-        for (int d = 0; d < DEQUANT_ROWS; ++d) {
-            if (row0 + 32 * d >= rows) break;
-            const uint32_t sfb = sf[d];
-            OUT *dst = static_cast<OUT *>(p.out) + ((row0 + 32 * d) * ld_out + static_cast<idx_t>(cb * 16));
+        for (int d = 0; d < DEQUANT_DEPTH; ++d) {
+            const int cb = col_block[d];
+            if (cb < 0) continue;
+            OUT *dst = static_cast<OUT *>(p.out) + (row[d] * ld_out + static_cast<idx_t>(cb * 16));
             const int64_t left = p.cols - static_cast<int64_t>(cb) * 16;
             if constexpr (sizeof(OUT) == 2) {
                 // bf16 / fp16 outputs: the whole block from a table of its eight magnitudes
                 uint32_t o[8];
-                if (dequantize_block_packed<OUT>(c[d], sfb, k, o, p.format == FOS_IF4)) {
+                if (dequantize_block_packed<OUT>(c[d], sfb[d], k, o, p.format == FOS_IF4)) {
                     if (left >= 16 && (reinterpret_cast<uintptr_t>(dst) & 31u) == 0) {
                         stg_32(dst, o);                       // one 32-byte store: whole sectors per instruction
                     } else if (left >= 16 && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
@@ -95,7 +91,7 @@ __global__ void __launch_bounds__(256, DEQUANT_CTAS) dequantize_kernel(const Deq
                 }
             }
             float v[16];
-            dequantize_block(c[d], sfb, p.format == FOS_IF4, k, v);
+            dequantize_block(c[d], sfb[d], p.format == FOS_IF4, k, v);
             if (left >= 16 && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
                 __align__(16) OUT tmp[16];
 #pragma unroll
@@ -220,18 +216,12 @@ extern "C" int fos_dequantize(const uint8_t *codes, const uint8_t *sf, const flo
 
     DequantParams p{codes, sf, amax, out, rows_p, cols_p, rows, cols, ld_out, format,
                     sf_layout == FOS_SF_TILED, dequant_divisor(format, scale_rule)};
-    p.sf_words = p.sf_tiled && reinterpret_cast<uintptr_t>(sf) % 16 == 0;
-    const int64_t cb_used = (cols + 15) / 16;
-    auto chunks_of = [&](int log2) { return (cb_used + (int64_t(1) << log2) - 1) >> log2; };
-    p.run_log2 = 8;
-    for (int log2 = 7; log2 >= 5; --log2)
-        if (chunks_of(log2) << log2 < chunks_of(p.run_log2) << p.run_log2) p.run_log2 = log2;
-    const int64_t units = ((rows + 127) / 128 * 32 >> (8 - p.run_log2)) * chunks_of(p.run_log2);
-    if (units + 148 * DEQUANT_CTAS >= (int64_t(1) << 32)) return FOS_ERR_TOO_LARGE;
-    p.units = static_cast<uint32_t>(units);
-    const unsigned g = static_cast<unsigned>(units < 148 * DEQUANT_CTAS ? units : 148 * DEQUANT_CTAS);
+    const int64_t units = rows * ((((cols + 15) / 16) + 255) / 256);     // runs of 256 blocks of one row
+    int64_t blocks = units;
+    if (blocks > 148 * 8) blocks = 148 * 8;
+    const unsigned g = static_cast<unsigned>(blocks);
     // 32-bit offsets when the padded tensor has fewer than 2^31 elements and the output fits the same bound
-    const bool small = rows_p * cols_p < (int64_t(1) << 31) && rows * ld_out < (int64_t(1) << 31);
+    const bool small = rows_p * cols_p < (int64_t(1) << 31) && rows * ld_out < (int64_t(1) << 31) && units + 4 * blocks < (int64_t(1) << 31);
     if (small) {
         if (out_dtype == FOS_BF16) dequantize_kernel<__nv_bfloat16, true><<<g, 256, 0, stream>>>(p);
         else if (out_dtype == FOS_FP16) dequantize_kernel<__half, true><<<g, 256, 0, stream>>>(p);
