@@ -17,10 +17,12 @@ struct DequantParams {
     int64_t rows_p, cols_p, rows, cols, ld_out;
     int format, sf_tiled;
     float divisor;
+    int run_log2;            // blocks of a row that a run takes, 2^5 .. 2^8
 };
 
 // One thread per 16-value block: 8 bytes of codes and one scale in, 16 values out. A CTA takes
-// runs of 256 blocks of one row (contiguous codes in, contiguous values out), DEPTH runs at a time: the
+// runs of blocks of a row (contiguous codes in, contiguous values out; 256 of one row, or of narrow tensors 2^run_log2 of each
+// of 256 >> run_log2 rows, so that a row of 512 values keeps more than 32 threads busy), DEPTH runs at a time: the
 // loads of all of them are issued before the first block is decoded, so a thread has DEPTH loads in
 // flight instead of one (with one, the kernel waited a memory latency per run: 29 us for 8192 x 4096).
 constexpr int DEQUANT_DEPTH = 4;
@@ -32,10 +34,11 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const DequantParams p) 
     using idx_t = typename std::conditional<SMALL, uint32_t, int64_t>::type;
     const int n_cb = static_cast<int>(p.cols_p >> 4);
     const int cb_used = static_cast<int>((p.cols + 15) >> 4);
-    const int chunks = (cb_used + 255) >> 8;
-    const idx_t units = static_cast<idx_t>(p.rows * chunks);
+    const int chunks = (cb_used + (1 << p.run_log2) - 1) >> p.run_log2, rows_per_unit = 256 >> p.run_log2;
+    const int in_run = static_cast<int>(threadIdx.x) & ((1 << p.run_log2) - 1), in_rows = static_cast<int>(threadIdx.x) >> p.run_log2;
+    const idx_t units = static_cast<idx_t>((p.rows + rows_per_unit - 1) / rows_per_unit * chunks);
     const DequantConsts k = dequant_consts(__ldg(p.amax), p.divisor);
-    // a unit is (row, chunk of 256 blocks); this CTA's units are blockIdx.x, + gridDim.x, ...: the pair is advanced
+    // a unit is (row or rows, run); this CTA's units are blockIdx.x, + gridDim.x, ...: the pair is advanced
     // by additions (a division per unit cost more than decoding it)
     const int step_r = static_cast<int>(gridDim.x) / chunks, step_c = static_cast<int>(gridDim.x) % chunks;
     idx_t row0 = static_cast<idx_t>(blockIdx.x) / static_cast<idx_t>(chunks);
@@ -48,10 +51,10 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const DequantParams p) 
         int col_block[DEQUANT_DEPTH];
 #pragma unroll
         for (int d = 0; d < DEQUANT_DEPTH; ++d) {
-            const idx_t r = row0;
-            const int cb = ch0 * 256 + static_cast<int>(threadIdx.x);
+            const idx_t r = row0 * static_cast<idx_t>(rows_per_unit) + static_cast<idx_t>(in_rows);
+            const int cb = (ch0 << p.run_log2) + in_run;
             row[d] = r;
-            col_block[d] = (u0 + static_cast<idx_t>(d) * gridDim.x < units && cb < cb_used) ? cb : -1;
+            col_block[d] = (u0 + static_cast<idx_t>(d) * gridDim.x < units && cb < cb_used && r < static_cast<idx_t>(p.rows)) ? cb : -1;
             c[d] = make_uint2(0u, 0u);
             sfb[d] = 0u;
             if (col_block[d] >= 0) {
@@ -216,7 +219,13 @@ extern "C" int fos_dequantize(const uint8_t *codes, const uint8_t *sf, const flo
 
     DequantParams p{codes, sf, amax, out, rows_p, cols_p, rows, cols, ld_out, format,
                     sf_layout == FOS_SF_TILED, dequant_divisor(format, scale_rule)};
-    const int64_t units = rows * ((((cols + 15) / 16) + 255) / 256);     // runs of 256 blocks of one row
+    // runs as long as leave the fewest threads idle
+    const int64_t cb_used = (cols + 15) / 16;
+    auto chunks_of = [&](int log2) { return (cb_used + (int64_t(1) << log2) - 1) >> log2; };
+    p.run_log2 = 8;
+    for (int log2 = 7; log2 >= 5; --log2)
+        if (chunks_of(log2) << log2 < chunks_of(p.run_log2) << p.run_log2) p.run_log2 = log2;
+    const int64_t rows_per_unit = 256 >> p.run_log2, units = (rows + rows_per_unit - 1) / rows_per_unit * chunks_of(p.run_log2);
     int64_t blocks = units;
     if (blocks > 148 * 8) blocks = 148 * 8;
     const unsigned g = static_cast<unsigned>(blocks);
