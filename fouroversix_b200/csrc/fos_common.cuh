@@ -84,8 +84,8 @@ int gemm_nvfp4_grouped_scaled(const uint8_t *a_codes, const uint8_t *a_sf, const
 
 // The same for the gate-up projection of an experts layer, gate in the even and up in the odd of its n columns: d is not the
 // product but its clamped SwiGLU with the bias [groups][n] of the output's type (16 bits), n / 2 columns wide, and
-// amax[group] is raised to the largest magnitude written for the group. FOS_ERR_UNSUPPORTED (nothing launched) where the
-// problem is not one for the kernel on CTA pairs.
+// amax[group] is raised to the largest magnitude written for the group. bf16; FOS_ERR_UNSUPPORTED (nothing launched) for other
+// types and where the problem is not one for the kernel on CTA pairs.
 struct GluEpilogue {
     const void *bias;
     float alpha, limit;

@@ -708,7 +708,8 @@ template <bool MX> struct PairCfg {
 // reaches memory (32768 x 5760: 377 MB less written and read, and the kernel that did it, 125 us). A lane holds
 // a row of the tile, so a pair lies in neighbouring registers of one lane, and the bias is the same for all lanes.
 // The accumulators overlap by 96 columns only, so the arithmetic (about 25 instructions per output, 64 outputs per thread
-// and tile) runs while the next tile's MMAs do: at K 2880 a tile's MMAs take some 7000 cycles, the epilogue half of that.
+// and tile) runs while the next tile's MMAs do; on eight warps it takes longer than they do and bounds the kernel (32768 x
+// 5760, K 2880: 382 us, without it 266 and the kernel of its own 125).
 template <typename OUT, int N>
 __device__ __forceinline__ void glu_columns(OUT *dst, const uint32_t *acc, float alpha, const OUT *bias, int64_t cols_left, bool row_ok,
                                             const GluEpilogue &glu, typename Half16<OUT>::Pair limit2,
@@ -1348,8 +1349,9 @@ static int gemm_grouped_entry(const uint8_t *a_codes, const uint8_t *a_sf, const
     if (rows_capacity <= 0 || rows_capacity % 128 || n_p <= 0 || n_p % 128 || k_p < 64 || k_p % 64) return FOS_ERR_INVALID_ARGUMENT;
     if (n <= 0 || n > n_p || ldd < (glu ? n / 2 : n)) return FOS_ERR_INVALID_ARGUMENT;
     if (out_dtype != FOS_BF16 && out_dtype != FOS_FP16 && out_dtype != FOS_FP32) return FOS_ERR_INVALID_ARGUMENT;
-    // (the epilogue's stores are 8 outputs of a row, its loads 8 numbers of the bias)
-    if (glu && (out_dtype == FOS_FP32 || n % 16 || ldd % 8 || reinterpret_cast<uintptr_t>(d) % 16 || reinterpret_cast<uintptr_t>(glu->bias) % 16))
+    // (the epilogue's stores are 8 outputs of a row, its loads 8 numbers of the bias; in fp16 one sigmoid in 60 needs the binary32
+    // sequence, in bf16 one in 500, and the few warps of an epilogue have no room for that many)
+    if (glu && (out_dtype != FOS_BF16 || n % 16 || ldd % 8 || reinterpret_cast<uintptr_t>(d) % 16 || reinterpret_cast<uintptr_t>(glu->bias) % 16))
         return FOS_ERR_UNSUPPORTED;
     if (reinterpret_cast<uintptr_t>(a_codes) % 16 || reinterpret_cast<uintptr_t>(b_codes) % 16 ||
         reinterpret_cast<uintptr_t>(a_sf) % 16 || reinterpret_cast<uintptr_t>(b_sf) % 16)
@@ -1394,9 +1396,7 @@ static int gemm_grouped_entry(const uint8_t *a_codes, const uint8_t *a_sf, const
         if ((st = make_scale_map(&map_sfa, a_sf, rows_capacity / 128, k_p / 64, 1, KB_PER_STAGE)) != FOS_OK) return st;
         if ((st = make_scale_map(&map_sfb, b_sf, b_rows / 128, k_p / 64, 2, KB_PER_STAGE)) != FOS_OK) return st;
         if (glu)
-            return out_dtype == FOS_BF16
-                       ? launch_pair<__nv_bfloat16, false, true, true>(map_a, map_b, map_b_half, map_sfa, map_sfb, p, max_ctas, stream)
-                       : launch_pair<__half, false, true, true>(map_a, map_b, map_b_half, map_sfa, map_sfb, p, max_ctas, stream);
+            return launch_pair<__nv_bfloat16, false, true, true>(map_a, map_b, map_b_half, map_sfa, map_sfb, p, max_ctas, stream);
         return launch_pair_out<false, true>(map_a, map_b, map_b_half, map_sfa, map_sfb, p, max_ctas, stream);
     }
     const bool wide = choice == GEMM_256;
