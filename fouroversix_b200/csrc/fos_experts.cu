@@ -5,6 +5,9 @@
 //   fos_experts_glu           gate-up output + bias -> clamped SwiGLU, the input of the down projection
 //   fos_experts_combine       down output + bias, times the routing weight, summed per token
 //
+// The whole layer as one call (fos_experts_forward) leaves out the second where the quantization gathers the rows itself, and the
+// third where the gate-up GEMM's epilogue does it.
+//
 // The arithmetic follows the reference's GPT-OSS experts module
 // (src/fouroversix/model/modules/gpt_oss.py:297-335), which runs it as a chain of element-wise tensor
 // operations on 16-bit tensors: every operation computes in binary32 and rounds its result to the

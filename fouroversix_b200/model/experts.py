@@ -148,7 +148,7 @@ class FourOverSixExperts(nn.Module):
 
     def _forward_native(self, x: torch.Tensor, routing_indices: torch.Tensor, routing_weights: torch.Tensor) -> torch.Tensor:
         """The same layer on `fos_experts_route`, `fos_experts_gather_rows`, `fos_experts_glu` and
-        `fos_experts_combine` around the grouped launches (as one call nine kernels, one by one eleven): bit-equal to the
+        `fos_experts_combine` around the grouped launches (as one call seven to nine kernels, one by one eleven): bit-equal to the
         tensor-operation form when a token has at most two experts, and to the reference's host loop (which adds
         a token's experts in ascending order) for any number."""
         down, gate_up = self.quantized_weights()
@@ -167,7 +167,7 @@ class FourOverSixExperts(nn.Module):
         if (self.single_call and self.hidden_size % 64 == 0 and self.intermediate_size % 64 == 0
                 and DataType(act_config.dtype) == DataType.nvfp4 and not act_config.block_scale_2d and not act_config.rht
                 and RoundStyle(act_config.round_style) == RoundStyle.nearest):
-            # one host call for the nine launches (fos_experts_forward); the workspace is the call's only scratch
+            # one host call for all launches (fos_experts_forward); the workspace is the call's only scratch
             if routing_indices.dtype not in (torch.int32, torch.int64):
                 routing_indices = routing_indices.to(torch.int64)
             routing_indices = routing_indices.contiguous()
