@@ -363,7 +363,6 @@ __device__ __forceinline__ void tc_mma_f16_pair(uint32_t d_tmem, uint64_t a_desc
 template <typename OUT>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                     const __grid_constant__ CUtensorMap map_b_half,
                      const F16GemmParams p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -411,7 +410,6 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     const int64_t num_tiles = num_m * num_n;
     const int k_tiles = static_cast<int>(p.k_p / 64);
     const int64_t pair_id = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-    const pair::PairUnits units(num_tiles, num_pairs);
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer (both CTAs)
@@ -420,22 +418,18 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         asm volatile("griddepcontrol.wait;" ::: "memory");     // the expanded operands
         uint32_t s = 0, ph = 0;
         bool ok = true;
-        for (int64_t t = pair_id; t < units.count && ok; t += num_pairs) {
+        for (int64_t t = pair_id; t < num_tiles && ok; t += num_pairs) {
             int64_t mb, nb;
-            tile_coords(units.tile(t), num_m, num_n, mb, nb);
-            const bool is_half = units.is_half(t);
-            const int m0 = static_cast<int>(mb * 256 + rank * 128);
-            const int n0 = static_cast<int>(nb * 256) + units.first_col(t) + static_cast<int>(rank) * (is_half ? 64 : 128);
-            const CUtensorMap *const b_map = is_half ? &map_b_half : &map_b;
-            const uint32_t bytes = 2 * (is_half ? PAIR_STAGE_BYTES - 64 * BLOCK_K_BYTES : PAIR_STAGE_BYTES);      // of both CTAs
+            tile_coords(t, num_m, num_n, mb, nb);
+            const int m0 = static_cast<int>(mb * 256 + rank * 128), n0 = static_cast<int>(nb * 256 + rank * 128);
             for (int kt = 0; kt < k_tiles; ++kt) {
                 ok = __all_sync(0xffffffffu, mbar_wait(empty_bar + 8 * s, ph ^ 1u, abort_flag, p.status, 1));
                 if (!ok) break;
                 const uint32_t stage = smem_base + s * PAIR_STAGE_BYTES, bar = leader_full + 8 * s;
                 if (issue) {
-                    if (leader) mbar_expect_tx(full_bar + 8 * s, bytes);
+                    if (leader) mbar_expect_tx(full_bar + 8 * s, 2 * PAIR_STAGE_BYTES);      // the bytes of both CTAs
                     pair::tma_load_2d_pair(stage, &map_a, kt * BLOCK_K_BYTES, m0, bar);
-                    pair::tma_load_2d_pair(stage + A_BYTES, b_map, kt * BLOCK_K_BYTES, n0, bar);
+                    pair::tma_load_2d_pair(stage + A_BYTES, &map_b, kt * BLOCK_K_BYTES, n0, bar);
                 }
                 __syncwarp();
                 if (++s == PAIR_STAGES) { s = 0; ph ^= 1u; }
@@ -453,10 +447,10 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     } else if (warp == 1 && leader) {
         // ------------------------------------------------------------------ MMA issuer, for both CTAs
         const bool issue = elect_one();
+        const uint32_t idesc = f16_idesc(256, 256);
         uint32_t s = 0, ph = 0, tile_i = 0;
         bool ok = true;
-        for (int64_t t = pair_id; t < units.count && ok; t += num_pairs, ++tile_i) {
-            const uint32_t idesc = f16_idesc(units.is_half(t) ? 128 : 256, 256);
+        for (int64_t t = pair_id; t < num_tiles && ok; t += num_pairs, ++tile_i) {
             const uint32_t acc = tile_i % ACC_STAGES, acc_ph = (tile_i / ACC_STAGES) & 1u;
             ok = __all_sync(0xffffffffu, mbar_wait(acc_empty_bar + 8 * acc, acc_ph ^ 1u, abort_flag, p.status, 3));
             if (!ok) break;
@@ -496,26 +490,24 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         const uint32_t leader_acc_empty = map_to_cta(acc_empty_bar, 0);
         uint32_t tile_i = 0;
         bool ok = true;
-        for (int64_t t = pair_id; t < units.count && ok; t += num_pairs, ++tile_i) {
+        for (int64_t t = pair_id; t < num_tiles && ok; t += num_pairs, ++tile_i) {
             int64_t mb, nb;
-            tile_coords(units.tile(t), num_m, num_n, mb, nb);
-            const int cols = units.is_half(t) ? 64 : 128;          // of this warp
-            const int64_t row = mb * 256 + rank * 128 + quad * 32 + lane, n0 = nb * 256 + units.first_col(t) + half * cols;
+            tile_coords(t, num_m, num_n, mb, nb);
+            const int64_t row = mb * 256 + rank * 128 + quad * 32 + lane, n0 = nb * 256 + half * 128;
             const uint32_t acc = tile_i % ACC_STAGES, acc_ph = (tile_i / ACC_STAGES) & 1u;
             // (in the peer this barrier is arrived on from the leader's SM: one lane polls for the warp)
             if (lane == 0) ok = mbar_wait_poll(acc_full_bar + 8 * acc, acc_ph, abort_flag, p.status, 4);
             ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
             if (!ok) break;
             tc_fence_after();
-            const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * 256 + half * cols;
+            const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * 256 + half * 128;
             OUT *dst = out + row * p.ldd + n0;
             const int64_t left = row < p.m ? p.n - n0 : 0;
 #pragma unroll
             for (int c = 0; c < 128; c += 32) {
-                if (c >= cols) break;
                 uint32_t v[32];
                 tc_load_32cols_sync(t_acc + c, v);
-                if (c == cols - 32) {
+                if (c == 96) {
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive_cluster(leader_acc_empty + 8 * acc);
@@ -535,15 +527,14 @@ gemm_f16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 }
 
 template <typename OUT>
-int launch_f16(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mb_pair, const CUtensorMap &mb_half, const F16GemmParams &p,
-               cudaStream_t stream) {
+int launch_f16(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mb_pair, const F16GemmParams &p, cudaStream_t stream) {
     int dev = 0, sms = 0;
     FOS_CUDA_TRY(cudaGetDevice(&dev));
     FOS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int64_t tiles = (p.m_p / BLOCK_M) * ((p.n_p + BLOCK_N - 1) / BLOCK_N);
     const int64_t pair_tiles = ((p.m_p + 255) / 256) * ((p.n_p + 255) / 256);
     if (pairs_pay(tiles, pair_tiles, sms))
-        return pair::launch<gemm_f16_pair_kernel<OUT>>(THREADS, PAIR_SMEM_BYTES, pair_tiles, 0, stream, ma, mb_pair, mb_half, p);
+        return pair::launch<gemm_f16_pair_kernel<OUT>>(THREADS, PAIR_SMEM_BYTES, pair_tiles, 0, stream, ma, mb_pair, p);
     auto kernel = gemm_f16_kernel<OUT>;
     static OncePerDevice configured;   // per instantiation
     FOS_CUDA_TRY(configured.run(dev, [&] {
@@ -594,20 +585,19 @@ int gemm_if4_impl(const uint8_t *a_codes, const uint8_t *a_sf, int a_format, int
     ExpandParams x{{{a_codes, a_sf, a_format, a_sf_layout == FOS_SF_TILED}, {b_codes, b_sf, b_format, b_sf_layout == FOS_SF_TILED}},
                    a16, m_p * (k_p / 16), (m_p + n_p) * (k_p / 16), k_p / 16};
     if ((st = launch_expand(x, stream)) != FOS_OK) return st;
-    CUtensorMap map_a, map_b, map_b_pair, map_b_half;
+    CUtensorMap map_a, map_b, map_b_pair;
     if ((st = make_operand_map(&map_a, a16, m_p, k_p * 2, BLOCK_M)) != FOS_OK) return st;
     if ((st = make_operand_map(&map_b, b16, n_p, k_p * 2, BLOCK_N)) != FOS_OK) return st;
     if ((st = make_operand_map(&map_b_pair, b16, n_p, k_p * 2, 128)) != FOS_OK) return st;
-    if ((st = make_operand_map(&map_b_half, b16, n_p, k_p * 2, 64)) != FOS_OK) return st;
     if (status) {
         FOS_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int32_t), stream));
     } else {
         FOS_CUDA_TRY(wait_failures_ptr(&status));   // the library's sticky word
     }
     F16GemmParams p{alpha.alpha, alpha.amax_a, alpha.amax_b, alpha.denom, d, status, m_p, n_p, k_p, m, n, ldd};
-    if (out_dtype == FOS_BF16) return launch_f16<__nv_bfloat16>(map_a, map_b, map_b_pair, map_b_half, p, stream);
-    if (out_dtype == FOS_FP16) return launch_f16<__half>(map_a, map_b, map_b_pair, map_b_half, p, stream);
-    return launch_f16<float>(map_a, map_b, map_b_pair, map_b_half, p, stream);
+    if (out_dtype == FOS_BF16) return launch_f16<__nv_bfloat16>(map_a, map_b, map_b_pair, p, stream);
+    if (out_dtype == FOS_FP16) return launch_f16<__half>(map_a, map_b, map_b_pair, p, stream);
+    return launch_f16<float>(map_a, map_b, map_b_pair, p, stream);
 }
 
 int check_gemm_if4_args(const uint8_t *a_codes, const uint8_t *a_sf, int a_format, int a_sf_layout,

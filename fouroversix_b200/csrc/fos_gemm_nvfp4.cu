@@ -744,8 +744,8 @@ __device__ __forceinline__ void glu_columns(OUT *dst, const uint32_t *acc, float
 template <typename OUT, bool MX, bool GROUPED = false, bool GLU = false>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                     const __grid_constant__ CUtensorMap map_b_half, const __grid_constant__ CUtensorMap map_sfa,
-                     const __grid_constant__ CUtensorMap map_sfb, const GemmParams p) {
+                     const __grid_constant__ CUtensorMap map_sfa, const __grid_constant__ CUtensorMap map_sfb,
+                     const GemmParams p) {
     using C = PairCfg<MX>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -830,7 +830,6 @@ gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     const int64_t k_blocks = p.k_p / 64;
     const int k_tiles = static_cast<int>((k_blocks + KB_PER_STAGE - 1) / KB_PER_STAGE);
     const int64_t pair_id = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-    const PairUnits units(num_tiles, num_pairs);
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer (both CTAs)
@@ -839,18 +838,13 @@ gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         asm volatile("griddepcontrol.wait;" ::: "memory");   // (a dependent launch) the kernel that packs A is done
         uint32_t s = 0, ph = 0;
         bool ok = true;
-        for (int64_t t = pair_id; t < units.count && ok; t += num_pairs) {
+        for (int64_t t = pair_id; t < num_tiles && ok; t += num_pairs) {
             int64_t mb, nb;
-            tile_coords(units.tile(t), num_m, num_n, mb, nb);
+            tile_coords(t, num_m, num_n, mb, nb);
             int group;
             const int m0 = static_cast<int>(locate(mb, group) + rank * 128);
-            // row of B: of a tile's 256 columns this CTA fetches half, of a half tile's 128 too
-            const bool is_half = units.is_half(t);
-            const int first_col = static_cast<int>(nb * TILE_N) + units.first_col(t);
-            const int n0 = first_col + static_cast<int>(rank) * (is_half ? 64 : 128) + group * static_cast<int>(p.n_p);
-            const int a_group = m0 / 128, b_group = first_col / 128 + group * static_cast<int>(p.n_p / 128);
-            const CUtensorMap *const b_map = is_half ? &map_b_half : &map_b;
-            const uint32_t bytes = 2 * (is_half ? C::STAGE_BYTES - B_HALF_BYTES / 2 : C::STAGE_BYTES);
+            const int n0 = static_cast<int>(nb * TILE_N + rank * 128) + group * static_cast<int>(p.n_p);      // row of B
+            const int a_group = m0 / 128, b_group = static_cast<int>(nb * 2) + group * static_cast<int>(p.n_p / 128);
             for (int kt = 0; kt < k_tiles; ++kt) {
                 ok = __all_sync(0xffffffffu, mbar_wait(empty_bar + 8 * s, ph ^ 1u, abort_flag, p.status, 1));
                 if (!ok) break;
@@ -859,11 +853,11 @@ gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                 // The leader announces the bytes of both CTAs; its barrier may see the peer's bytes
                 // first, which only makes the pending count negative for a moment.
                 if (issue) {
-                    if (leader) mbar_expect_tx(full_bar + 8 * s, bytes);
+                    if (leader) mbar_expect_tx(full_bar + 8 * s, 2 * C::STAGE_BYTES);
                     tma_load_3d_pair(sf, &map_sfa, 0, kt * C::TILES, a_group, bar);
                     tma_load_3d_pair(sf + C::SFA_BYTES, &map_sfb, 0, kt * C::TILES, b_group, bar);
                     tma_load_2d_pair(stage, &map_a, kt * BLOCK_K_BYTES, m0, bar);
-                    tma_load_2d_pair(stage + A_BYTES, b_map, kt * BLOCK_K_BYTES, n0, bar);
+                    tma_load_2d_pair(stage + A_BYTES, &map_b, kt * BLOCK_K_BYTES, n0, bar);
                 }
                 __syncwarp();
                 if (++s == C::STAGES) { s = 0; ph ^= 1u; }
@@ -881,11 +875,10 @@ gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     } else if (warp == 1 && leader) {
         // ------------------------------------------------------------------ scale copies and MMAs, for both CTAs
         const bool issue = elect_one();
+        const uint32_t idesc = mma_idesc(TILE_N, 256);
         uint32_t s = 0, ph = 0, sf_set = 0, tile_i = 0;
         bool ok = true, ready = false;
-        for (int64_t t = pair_id; t < units.count && ok; t += num_pairs, ++tile_i) {
-            const bool is_half = units.is_half(t);
-            const uint32_t idesc = mma_idesc(is_half ? TILE_N / 2 : TILE_N, 256);
+        for (int64_t t = pair_id; t < num_tiles && ok; t += num_pairs, ++tile_i) {
             // the epilogue of the tile before has read the columns that the two accumulators share
             ok = __all_sync(0xffffffffu, mbar_wait(acc_empty_bar, (tile_i & 1u) ^ 1u, abort_flag, p.status, 3));
             if (!ok) break;
@@ -910,7 +903,7 @@ gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                     for (int kb = 0; kb < C::TILES; ++kb) {
                         tc_copy_sf_pair_lo(sfa + 4 * kb, sf_lo + ((kb * SF_TILE_BYTES) >> 4));
                         tc_copy_sf_pair_lo(sfb + 8 * kb, sf_lo + ((C::SFA_BYTES + kb * SF_TILE_BYTES) >> 4));
-                        if (!is_half) tc_copy_sf_pair_lo(sfb + 8 * kb + 4, sf_lo + ((C::SFA_BYTES + (C::TILES + kb) * SF_TILE_BYTES) >> 4));
+                        tc_copy_sf_pair_lo(sfb + 8 * kb + 4, sf_lo + ((C::SFA_BYTES + (C::TILES + kb) * SF_TILE_BYTES) >> 4));
                     }
 #pragma unroll
                     for (int kb = 0; kb < KB_PER_STAGE; ++kb) {
@@ -963,9 +956,9 @@ gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         }
         uint32_t tile_i = 0;
         bool ok = true;
-        for (int64_t t = pair_id; t < units.count && ok; t += num_pairs, ++tile_i) {
+        for (int64_t t = pair_id; t < num_tiles && ok; t += num_pairs, ++tile_i) {
             int64_t mb, nb;
-            tile_coords(units.tile(t), num_m, num_n, mb, nb);
+            tile_coords(t, num_m, num_n, mb, nb);
             int group;
             const int64_t row = locate(mb, group) + rank * 128 + quad * 32 + lane;
             if constexpr (GROUPED) {
@@ -994,29 +987,21 @@ gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                     store_columns<OUT, decltype(n)::value>(dst + col, acc, alpha, bias ? bias + col : nullptr, left - col, vec32, vec16);
                 }
             };
-            uint32_t w[32];
-            if (units.is_half(t)) {
-                // the pair's last unit: columns 0 .. 127 of the accumulator are 128 of the tile's, 64 of them this warp's
-                for (int c = half * 64; c < half * 64 + 64; c += 32) {
-                    tc_load_32cols_sync(t_acc + c, w);
-                    store(w, units.first_col(t) + c, std::integral_constant<int, 32>{});
-                }
-            } else {
-                uint32_t v[FIRST / 48][48];
+            uint32_t v[FIRST / 48][48];
 #pragma unroll
-                for (int i = 0; i < FIRST / 48; ++i) tc_load_48cols_sync(t_acc + first + 48 * i, v[i]);
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(leader_acc_empty);
+            for (int i = 0; i < FIRST / 48; ++i) tc_load_48cols_sync(t_acc + first + 48 * i, v[i]);
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(leader_acc_empty);
 #pragma unroll
-                for (int i = 0; i < FIRST / 48; ++i) store(v[i], first + 48 * i, std::integral_constant<int, 48>{});
-                if constexpr (SECOND == 80) {
-                    tc_load_48cols_sync(t_acc + second, v[0]);
-                    store(v[0], second, std::integral_constant<int, 48>{});
-                }
-                tc_load_32cols_sync(t_acc + second + (SECOND - 32), w);
-                store(w, second + (SECOND - 32), std::integral_constant<int, 32>{});
+            for (int i = 0; i < FIRST / 48; ++i) store(v[i], first + 48 * i, std::integral_constant<int, 48>{});
+            if constexpr (SECOND == 80) {
+                tc_load_48cols_sync(t_acc + second, v[0]);
+                store(v[0], second, std::integral_constant<int, 48>{});
             }
+            uint32_t w[32];
+            tc_load_32cols_sync(t_acc + second + (SECOND - 32), w);
+            store(w, second + (SECOND - 32), std::integral_constant<int, 32>{});
             if constexpr (GLU) {
                 __syncwarp();
                 raise_amax<OUT>(max2, p.glu.amax + group, lane);
@@ -1039,21 +1024,21 @@ gemm_fp4_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 // ---------------------------------------------------------------------------- host side
 
 template <typename OUT, bool MX, bool GROUPED, bool GLU = false>
-int launch_pair(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mb_half, const CUtensorMap &msa, const CUtensorMap &msb,
+int launch_pair(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &msa, const CUtensorMap &msb,
                 const GemmParams &p, int max_ctas, cudaStream_t stream) {
     // (grouped: at most one more row tile per group than the buffer has)
     const int64_t row_tiles = (p.m_p + 255) / 256 + (GROUPED ? p.num_groups : 0);
     return pair::launch<pair::gemm_fp4_pair_kernel<OUT, MX, GROUPED, GLU>>(pair::THREADS, pair::PairCfg<MX>::SMEM_BYTES,
                                                                            row_tiles * ((p.n_p + 255) / 256), max_ctas, stream,
-                                                                           ma, mb, mb_half, msa, msb, p);
+                                                                           ma, mb, msa, msb, p);
 }
 
 template <bool MX, bool GROUPED = false>
-int launch_pair_out(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &mb_half, const CUtensorMap &msa,
-                    const CUtensorMap &msb, const GemmParams &p, int max_ctas, cudaStream_t stream) {
-    if (p.out_dtype == FOS_BF16) return launch_pair<__nv_bfloat16, MX, GROUPED>(ma, mb, mb_half, msa, msb, p, max_ctas, stream);
-    if (p.out_dtype == FOS_FP16) return launch_pair<__half, MX, GROUPED>(ma, mb, mb_half, msa, msb, p, max_ctas, stream);
-    return launch_pair<float, MX, GROUPED>(ma, mb, mb_half, msa, msb, p, max_ctas, stream);
+int launch_pair_out(const CUtensorMap &ma, const CUtensorMap &mb, const CUtensorMap &msa, const CUtensorMap &msb,
+                    const GemmParams &p, int max_ctas, cudaStream_t stream) {
+    if (p.out_dtype == FOS_BF16) return launch_pair<__nv_bfloat16, MX, GROUPED>(ma, mb, msa, msb, p, max_ctas, stream);
+    if (p.out_dtype == FOS_FP16) return launch_pair<__half, MX, GROUPED>(ma, mb, msa, msb, p, max_ctas, stream);
+    return launch_pair<float, MX, GROUPED>(ma, mb, msa, msb, p, max_ctas, stream);
 }
 
 template <int BLOCK_N, typename OUT, bool FUSED_A = false, bool GROUPED = false>
@@ -1228,15 +1213,14 @@ static int gemm_fp4_entry(const uint8_t *a_codes, const uint8_t *a_sf, const uin
     }
 
     if (choice == GEMM_PAIR) {
-        CUtensorMap map_b_half, map_sfa, map_sfb;
+        CUtensorMap map_sfa, map_sfb;
         const int tiles = mx ? KB_PER_STAGE / 2 : KB_PER_STAGE;
-        if ((st = make_operand_map(&map_b_half, b_codes, n_p, k_p / 2, 64)) != FOS_OK) return st;
         if ((st = make_operand_map(&map_a, a_codes, m_p, k_p / 2, 128)) != FOS_OK) return st;
         if ((st = make_operand_map(&map_b, b_codes, n_p, k_p / 2, 128)) != FOS_OK) return st;
         if ((st = make_scale_map(&map_sfa, a_sf, m_p / 128, sf_k_tiles, 1, tiles)) != FOS_OK) return st;
         if ((st = make_scale_map(&map_sfb, b_sf, n_p / 128, sf_k_tiles, 2, tiles)) != FOS_OK) return st;
-        return mx ? launch_pair_out<true>(map_a, map_b, map_b_half, map_sfa, map_sfb, p, max_ctas, stream)
-                  : launch_pair_out<false>(map_a, map_b, map_b_half, map_sfa, map_sfb, p, max_ctas, stream);
+        return mx ? launch_pair_out<true>(map_a, map_b, map_sfa, map_sfb, p, max_ctas, stream)
+                  : launch_pair_out<false>(map_a, map_b, map_sfa, map_sfb, p, max_ctas, stream);
     }
     const bool wide = choice == GEMM_256;
     sms = sms_allowed(sms, max_ctas);                       // leave SMs to concurrent kernels
@@ -1388,16 +1372,15 @@ static int gemm_grouped_entry(const uint8_t *a_codes, const uint8_t *a_sf, const
     } else {
         FOS_CUDA_TRY(wait_failures_ptr(&p.status));
     }
-    CUtensorMap map_a, map_b, map_b_half, map_sfa, map_sfb;
+    CUtensorMap map_a, map_b, map_sfa, map_sfb;
     if (choice == GEMM_PAIR) {
-        if ((st = make_operand_map(&map_b_half, b_codes, b_rows, k_p / 2, 64)) != FOS_OK) return st;
         if ((st = make_operand_map(&map_a, a_codes, rows_capacity, k_p / 2, 128)) != FOS_OK) return st;
         if ((st = make_operand_map(&map_b, b_codes, b_rows, k_p / 2, 128)) != FOS_OK) return st;
         if ((st = make_scale_map(&map_sfa, a_sf, rows_capacity / 128, k_p / 64, 1, KB_PER_STAGE)) != FOS_OK) return st;
         if ((st = make_scale_map(&map_sfb, b_sf, b_rows / 128, k_p / 64, 2, KB_PER_STAGE)) != FOS_OK) return st;
         if (glu)
-            return launch_pair<__nv_bfloat16, false, true, true>(map_a, map_b, map_b_half, map_sfa, map_sfb, p, max_ctas, stream);
-        return launch_pair_out<false, true>(map_a, map_b, map_b_half, map_sfa, map_sfb, p, max_ctas, stream);
+            return launch_pair<__nv_bfloat16, false, true, true>(map_a, map_b, map_sfa, map_sfb, p, max_ctas, stream);
+        return launch_pair_out<false, true>(map_a, map_b, map_sfa, map_sfb, p, max_ctas, stream);
     }
     const bool wide = choice == GEMM_256;
     sms = sms_allowed(sms, max_ctas);

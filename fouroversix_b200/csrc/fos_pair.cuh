@@ -92,23 +92,6 @@ __device__ __forceinline__ void store_columns(OUT *dst, const uint32_t *acc, flo
     }
 }
 
-// The units of work of a persistent launch on CTA pairs: 256 x 256 tiles in their order, except that the tiles of a last round that
-// would keep at most half of the pairs busy are split into two of 256 x 128. Such a half takes about 0.6 of a tile's time
-// (its MMAs half of it, but they need three quarters of a tile's operands), so the round is that much shorter: with 74 pairs
-// 4096 x 4096 outputs (256 tiles, 3.46 rounds) take 3.6 rounds instead of 4. Sums and outputs are those of the whole tile.
-struct PairUnits {
-    int64_t whole, count;        // units that are whole tiles; all units
-    __device__ __forceinline__ PairUnits(int64_t tiles, int64_t pairs) {
-        const int64_t rest = tiles % pairs;
-        whole = 2 * rest <= pairs ? tiles - rest : tiles;
-        count = whole + 2 * (tiles - whole);
-    }
-    __device__ __forceinline__ bool is_half(int64_t unit) const { return unit >= whole; }
-    __device__ __forceinline__ int64_t tile(int64_t unit) const { return unit < whole ? unit : whole + ((unit - whole) >> 1); }
-    // first column of the unit within its tile
-    __device__ __forceinline__ int first_col(int64_t unit) const { return unit < whole ? 0 : static_cast<int>((unit - whole) & 1) * 128; }
-};
-
 // Persistent launch of clusters of two CTAs: one pair per `tiles` at most, as many as can be resident, max_ctas CTAs at
 // most (0: no limit; never 1, which leaves no room for a pair); a programmatic dependent of the kernel before it in the
 // stream (see launch_dependent).
