@@ -219,13 +219,12 @@ extern "C" int fos_dequantize(const uint8_t *codes, const uint8_t *sf, const flo
 
     DequantParams p{codes, sf, amax, out, rows_p, cols_p, rows, cols, ld_out, format,
                     sf_layout == FOS_SF_TILED, dequant_divisor(format, scale_rule)};
-    // runs as long as leave the fewest threads idle
+    // the shortest run that takes a whole row; rows of more than 256 blocks: runs of 256 (shorter runs that leave fewer threads
+    // idle cost more than they save: 2880 values 7.65 -> 7.86 us in runs of 64, 1536 5.66 -> 5.98 in runs of 32, 4096 rows each)
     const int64_t cb_used = (cols + 15) / 16;
-    auto chunks_of = [&](int log2) { return (cb_used + (int64_t(1) << log2) - 1) >> log2; };
-    p.run_log2 = 8;
-    for (int log2 = 7; log2 >= 5; --log2)
-        if (chunks_of(log2) << log2 < chunks_of(p.run_log2) << p.run_log2) p.run_log2 = log2;
-    const int64_t rows_per_unit = 256 >> p.run_log2, units = (rows + rows_per_unit - 1) / rows_per_unit * chunks_of(p.run_log2);
+    p.run_log2 = 5;
+    while (p.run_log2 < 8 && (int64_t(1) << p.run_log2) < cb_used) ++p.run_log2;
+    const int64_t rows_per_unit = 256 >> p.run_log2, units = (rows + rows_per_unit - 1) / rows_per_unit * ((cb_used + (int64_t(1) << p.run_log2) - 1) >> p.run_log2);
     int64_t blocks = units;
     if (blocks > 148 * 8) blocks = 148 * 8;
     const unsigned g = static_cast<unsigned>(blocks);
