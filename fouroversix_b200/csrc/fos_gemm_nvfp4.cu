@@ -74,7 +74,9 @@ constexpr int NUM_THREADS = 384;                   // warps: 0 TMA, 1 MMA, 2-9 e
 // 384 rows leaves half a pair idle), which the host does not know.
 constexpr int PAIR_MIN_GROUP_ROWS = 640;
 // With the SwiGLU in the epilogue, which only pairs have, they also save the kernel that does it otherwise (10 us and more):
-// from the size where they stop being behind by more than that.
+// from the size where they stop being behind by more than that (the whole layer before and after, us, bf16, 32 experts of 2880 x
+// 2880, the rows' gathering of some 10 us left out as well: 256 buffer rows 199 / 183, 384 281 / 260, 1152 772 / 656; 192 rows,
+// without pairs, 161 / 150).
 constexpr int PAIR_MIN_GLU_ROWS = 256;
 // Up to this many rows per group on average a grouped GEMM is bound by the weights (see grouped_kernel_for).
 constexpr int FEW_GROUP_ROWS = 64;
