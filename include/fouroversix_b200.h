@@ -372,8 +372,8 @@ int fos_gemm_nvfp4_grouped(const uint8_t *a_codes, const uint8_t *a_sf, const ui
  */
 /*
  * fos_experts_forward: the whole layer in one host call - what the four calls above compute around two
- * fos_quantize_grouped / fos_gemm_nvfp4_grouped chains (alpha formed in the GEMM), nine kernels enqueued on `stream`
- * without a read-back:
+ * fos_quantize_grouped / fos_gemm_nvfp4_grouped chains (alpha formed in the GEMM), seven to nine kernels enqueued on
+ * `stream` without a read-back:
  *   out[t] = sum over the token's experts e (ascending) of
  *            (glu(x[t] @ gate_up[e]^T + gate_up_bias[e]) @ down[e]^T + down_bias[e]) * routing_weights[t][slot]
  * with both products in NVFP4 (activations quantized per expert with `activation_rule`, the weights packed
@@ -387,6 +387,9 @@ int fos_gemm_nvfp4_grouped(const uint8_t *a_codes, const uint8_t *a_sf, const ui
  * Replaces: GptOssExperts.forward of src/fouroversix/model/modules/gpt_oss.py:270-335 after weight packing.
  */
 int64_t fos_experts_workspace_bytes(int64_t tokens, int top_k, int num_experts, int64_t hidden, int64_t intermediate);
+/* 1 where the gate-up GEMM of a bf16 layer on `sms` SMs applies the SwiGLU itself, 0 where a kernel of its own does (same bits);
+ * rows_capacity = tokens * top_k + 127 * num_experts rounded up to 128. Decides as fos_experts_forward does; needs no GPU. */
+int fos_experts_glu_is_fused(int64_t rows_capacity, int64_t hidden, int64_t intermediate, int num_experts, int sms);
 int fos_experts_forward(const void *x, int dtype, int64_t tokens, int64_t hidden, int64_t ld_x,
                         const void *routing_indices, int index_bytes, const void *routing_weights, int top_k,
                         int num_experts, const uint8_t *gate_up_codes, const uint8_t *gate_up_sf,

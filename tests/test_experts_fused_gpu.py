@@ -21,10 +21,13 @@ def _layer(experts, hidden, inter, dtype, rule="mse"):
                               draw(0.1, experts, hidden), cfg)
 
 
-# tokens, experts per token, experts, hidden, inter; the last three: groups long enough for CTA pairs, with a product that
-# ends within a 256-column tile (640, 896) or on one (1024), and rows that end anywhere
+# tokens, experts per token, experts, hidden, inter; the last three: groups long enough for CTA pairs
 SHAPES = [(1, 1, 2, 64, 64), (37, 3, 5, 128, 192), (256, 4, 32, 192, 128), (2050, 2, 4, 192, 320), (1777, 3, 6, 64, 448),
           (4096, 4, 16, 320, 512)]
+# with the SwiGLU in the gate-up GEMM: 544 to 1152 buffer rows per group, products that end within a 256-column tile (640, 896, 1408)
+# or on one (1024), K of whole and of broken stages
+FUSED = [(2050, 2, 4, 1536, 320), (1777, 3, 6, 1600, 448), (800, 2, 4, 2048, 704), (1030, 3, 5, 2112, 512)]
+SHAPES += FUSED
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
@@ -49,6 +52,13 @@ def test_one_call_equals_the_kernels_one_by_one(tokens, top, experts, hidden, in
     assert torch.equal(got.isnan(), want.isnan())
     assert torch.equal(got.nan_to_num(), want.nan_to_num()), int((got != want).sum())
     assert _native.wait_failure_site() == 0
+
+
+@pytest.mark.parametrize("tokens,top,experts,hidden,inter", FUSED)
+def test_the_fused_shapes_are(tokens, top, experts, hidden, inter):
+    rows = (tokens * top + 127 * experts + 127) // 128 * 128
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert _native.lib().fos_experts_glu_is_fused(rows, hidden, inter, experts, sms) == 1
 
 
 @pytest.mark.parametrize("rule", ["static_6", "mae"])

@@ -46,3 +46,15 @@ def test_where_the_kernel_for_few_rows_is_taken():
     # K is shared by as many CTAs as are resident at once (two per SM), each keeping eight stages, eight at most
     assert [choice(16, n, 16384)[1] for n in (8, 128 * 37, 128 * 38, 128 * 74, 128 * 75, 128 * SMS)] == [8, 8, 4, 4, 2, 2]
     assert [choice(16, 8, k)[1] for k in (4096, 8191, 8192, 16384, 1 << 20)] == [2, 4, 4, 8, 8]
+
+
+def test_where_the_swiglu_is_fused():
+    """From 640 buffer rows per group with K of 1536 and more, from 512 with K of 2048 and more, never with a smaller K: there the
+    epilogue, and below those rows the idle halves of the pairs, cost more than the kernel that they save."""
+    fused = lambda rows, hidden, inter, experts: _native.lib().fos_experts_glu_is_fused(rows, hidden, inter, experts, SMS)
+    for experts, inter in ((8, 1024), (32, 2880)):
+        for rows, hidden, want in ((256, 2880, 0), (384, 4096, 0), (512, 1984, 0), (512, 2048, 1), (640, 1472, 0), (640, 1536, 1), (2048, 1024, 0)):
+            assert fused(rows * experts, hidden, inter, experts) == want, (rows, hidden)
+        assert fused(640 * experts - 128, 1536, inter, experts) == 0 and fused(512 * experts - 128, 2048, inter, experts) == 0
+    assert fused(640, 2048, 64, 1) == 0                      # one narrow tile per row block: not a problem for wide tiles
+    assert fused(100, 2048, 64, 1) < 0 and fused(640, 2000, 64, 1) < 0 and fused(640, 2048, 64, 0) < 0
