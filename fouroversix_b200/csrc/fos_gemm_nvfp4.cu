@@ -89,7 +89,8 @@ constexpr int PAIR_MIN_GROUP_ROWS = 640;
 // (two experts a token with 8, four with 32). Where tokens crowd into few experts it gains more from 640 on and loses more below 385
 // (8 experts of 2048 and 1024, 130 rows: 53 / 42).
 inline int pair_min_glu_rows(int64_t k_p) { return k_p < 1536 ? INT32_MAX : (k_p < 2048 ? 640 : 512); }
-// Up to this many rows per group on average a grouped GEMM is bound by the weights (see grouped_kernel_for).
+// Up to this many rows of a group's own on average, in a buffer with the 127 spare rows per group that unknown routing needs, a
+// grouped GEMM is bound by the weights (see grouped_kernel_for).
 constexpr int FEW_GROUP_ROWS = 64;
 constexpr int MAX_GROUPS = 256;                    // of a grouped launch (their row ranges are kept in shared memory)
 constexpr int SF_COL0 = 256;                       // tensor-memory columns: accumulators first, then per
@@ -1100,9 +1101,10 @@ inline int gemm_kernel_for(int64_t m, int64_t m_p, int64_t n_p, int64_t k_p, int
 
 // 256-row tiles waste half a tile per group on average, 128-row tiles a quarter of that: pairs where groups are long.
 // Groups of a few rows each (a decoding step) are bound by their weights' way out of HBM: a tile then takes the time of its
-// columns, whatever its width, and the width is the one whose last round is fuller. 32 groups of 32 rows, 2880 columns: 12
-// wide tiles a group are 2.6 rounds, which take 3, 23 narrow ones 4.97 half rounds. `pair_min_rows`: buffer rows per group
-// from which pairs are taken.
+// columns, whatever its width, and the width is the one whose last round is fuller, with one row block per group. 32 groups of 32
+// rows, 2880 columns: 12 wide tiles a group are 2.6 rounds, which take 3, 23 narrow ones 4.97 half rounds. (Fewer or more row
+// blocks change the gain and not its sign: n narrow half rounds are never longer than the rounds of half as many wide tiles.)
+// `pair_min_rows`: buffer rows per group from which pairs are taken.
 inline int grouped_kernel_for(int64_t rows_capacity, int num_groups, int64_t n_p, int variant, int max_ctas, int sms,
                               int pair_min_rows = PAIR_MIN_GROUP_ROWS) {
     if (variant == 128) return GEMM_128;

@@ -25,9 +25,9 @@ def _layer(experts, hidden, inter, dtype, rule="mse"):
 SHAPES = [(1, 1, 2, 64, 64), (37, 3, 5, 128, 192), (256, 4, 32, 192, 128), (2050, 2, 4, 192, 320), (1777, 3, 6, 64, 448),
           (4096, 4, 16, 320, 512)]
 # with the SwiGLU in the gate-up GEMM: 544 to 1152 buffer rows per group, products that end within a 256-column tile (640, 896, 1408)
-# or on one (1024), K of whole and of broken stages
+# or on one (1024), K of whole and of broken stages. The last: tiles of 128 columns for few rows per expert
 FUSED = [(2050, 2, 4, 1536, 320), (1777, 3, 6, 1600, 448), (800, 2, 4, 2048, 704), (1030, 3, 5, 2112, 512)]
-SHAPES += FUSED
+SHAPES += FUSED + [(190, 2, 8, 128, 1024)]
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])

@@ -58,3 +58,12 @@ def test_where_the_swiglu_is_fused():
         assert fused(640 * experts - 128, 1536, inter, experts) == 0 and fused(512 * experts - 128, 2048, inter, experts) == 0
     assert fused(640, 2048, 64, 1) == 0                      # one narrow tile per row block: not a problem for wide tiles
     assert fused(100, 2048, 64, 1) < 0 and fused(640, 2000, 64, 1) < 0 and fused(640, 2048, 64, 0) < 0
+
+
+def test_where_few_rows_take_narrow_tiles():
+    """Up to 64 rows of a group's own beside its 127 spare ones, where narrow tiles fill their last round better."""
+    for rows, want in ((47 * 128, NARROW), (48 * 128, WIDE)):                  # 32 groups: 191 rows each are 6112
+        assert choice(rows, 2880, 2880, 32)[0] == want
+    assert choice(40 * 128, 2880, 2880, 32)[0] == NARROW                       # 3 x 256 columns against 5 x 128
+    assert choice(40 * 128, 5760, 2880, 32)[0] == WIDE                         # 5 x 256 either way: the wide tiles stay
+    assert choice(11 * 128, 2048, 1024, 8)[0] == NARROW and choice(12 * 128, 2048, 1024, 8)[0] == WIDE
