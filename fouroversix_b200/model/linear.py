@@ -15,7 +15,7 @@ Like the reference, the backward pass rotates both wgrad operands with the 16-po
 Hadamard transform before quantizing them (the rotation is orthogonal along the contracted
 token axis, so it changes quantization error only) and rounds gradients as
 `gradient_round_style` says (stochastic by default; the noise is seeded from torch's CPU
-generator). Not implemented: `stochastic_unbiased` rounding and the Quartet-II backward.
+generator; `stochastic_unbiased` too). Not implemented: the Quartet-II backward.
 """
 
 from __future__ import annotations
@@ -58,7 +58,7 @@ def _one_call_training_applies(cfg: ModuleQuantizationConfig, *operands: torch.T
     if (cfg.disable_fprop_quantization or cfg.pseudo_quantize or cfg.activation_dtype != DataType.nvfp4
             or cfg.weight_dtype != DataType.nvfp4 or cfg.gradient_dtype != DataType.nvfp4
             or cfg.activation_round_style != RoundStyle.nearest or cfg.weight_round_style != RoundStyle.nearest
-            or cfg.gradient_round_style not in _ROUNDING_CODES
+            or cfg.gradient_round_style not in _ROUNDING_CODES or cfg.output_dtype not in _TORCH_OUT
             or cfg.matmul_backend not in (None, MatmulBackend.cutlass) or cfg.quantize_backend not in (None, QuantizeBackend.cuda)):
         return False
     first = operands[0]
