@@ -77,6 +77,8 @@ SIGNATURES = {
     "fos_linear_forward_bias": (_c_int, [_c_ptr, _c_int, _c_i64, _c_i64, _c_i64, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_i64,
                                         _c_ptr, _c_ptr, _c_int, _c_i64, _c_ptr, _c_i64, _c_ptr, _c_ptr, _c_ptr]),
     "fos_linear_train_workspace_bytes": (_c_i64, [_c_i64, _c_i64, _c_i64]),
+    "fos_linear_train_forward_workspace_bytes": (_c_i64, [_c_i64, _c_i64, _c_i64]),
+    "fos_linear_train_backward_workspace_bytes": (_c_i64, [_c_i64, _c_i64, _c_i64]),
     "fos_linear_train_forward": (_c_int, [_c_ptr, _c_ptr, _c_int, _c_i64, _c_i64, _c_i64, _c_i64, _c_i64, _c_int, _c_int, _c_int, _c_ptr,
                                           _c_int, _c_i64, _c_ptr, _c_i64, _c_ptr]),
     "fos_linear_train_backward": (_c_int, [_c_ptr, _c_ptr, _c_ptr, _c_int, _c_i64, _c_i64, _c_i64, _c_i64, _c_i64, _c_i64, _c_int, _c_int,

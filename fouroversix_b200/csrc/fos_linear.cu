@@ -98,14 +98,23 @@ bool chain_takes(const void *p, int64_t ld, int64_t cols) {
 }  // namespace
 }  // namespace fos
 
-extern "C" int64_t fos_linear_train_workspace_bytes(int64_t rows, int64_t in_features, int64_t out_features) {
+extern "C" int64_t fos_linear_train_forward_workspace_bytes(int64_t rows, int64_t in_features, int64_t out_features) {
     using namespace fos;
     if (rows <= 0 || in_features <= 0 || out_features <= 0) return FOS_ERR_INVALID_ARGUMENT;
-    const int64_t forward = operand_bytes(rows, in_features) + operand_bytes(out_features, in_features);
-    // backward: a slot for dy and then dy^T, one for W^T and then x^T
-    const int64_t backward = larger(operand_bytes(rows, out_features), operand_bytes(out_features, rows)) +
-                             larger(operand_bytes(in_features, out_features), operand_bytes(in_features, rows));
-    return TRAIN_WORDS_BYTES + larger(forward, backward);
+    return TRAIN_WORDS_BYTES + operand_bytes(rows, in_features) + operand_bytes(out_features, in_features);
+}
+
+extern "C" int64_t fos_linear_train_backward_workspace_bytes(int64_t rows, int64_t in_features, int64_t out_features) {
+    using namespace fos;
+    if (rows <= 0 || in_features <= 0 || out_features <= 0) return FOS_ERR_INVALID_ARGUMENT;
+    // a slot for dy and then dy^T, one for W^T and then x^T
+    return TRAIN_WORDS_BYTES + larger(operand_bytes(rows, out_features), operand_bytes(out_features, rows)) +
+           larger(operand_bytes(in_features, out_features), operand_bytes(in_features, rows));
+}
+
+extern "C" int64_t fos_linear_train_workspace_bytes(int64_t rows, int64_t in_features, int64_t out_features) {
+    return fos::larger(fos_linear_train_forward_workspace_bytes(rows, in_features, out_features),
+                       fos_linear_train_backward_workspace_bytes(rows, in_features, out_features));
 }
 
 extern "C" int fos_linear_train_forward(const void *x, const void *w, int dtype, int64_t rows, int64_t in_features, int64_t out_features,
@@ -117,7 +126,7 @@ extern "C" int fos_linear_train_forward(const void *x, const void *w, int dtype,
     if (dtype != FOS_BF16 && dtype != FOS_FP16) return FOS_ERR_INVALID_ARGUMENT;
     if (!chain_takes(x, ld_x, in_features) || !chain_takes(w, ld_w, in_features)) return FOS_ERR_UNSUPPORTED;
     if (reinterpret_cast<uintptr_t>(workspace) % 256 != 0) return FOS_ERR_MISALIGNED;
-    if (workspace_bytes < fos_linear_train_workspace_bytes(rows, in_features, out_features)) return FOS_ERR_INVALID_ARGUMENT;
+    if (workspace_bytes < fos_linear_train_forward_workspace_bytes(rows, in_features, out_features)) return FOS_ERR_INVALID_ARGUMENT;
     int st = check_device();
     if (st != FOS_OK) return st;
     uint8_t *base = static_cast<uint8_t *>(workspace) + TRAIN_WORDS_BYTES;
@@ -149,7 +158,7 @@ extern "C" int fos_linear_train_backward(const void *dy, const void *x, const vo
     if (!chain_takes(dy, ld_dy, out_features) || !chain_takes(x, ld_x, in_features) || !chain_takes(w, ld_w, in_features))
         return FOS_ERR_UNSUPPORTED;
     if (reinterpret_cast<uintptr_t>(workspace) % 256 != 0) return FOS_ERR_MISALIGNED;
-    if (workspace_bytes < fos_linear_train_workspace_bytes(rows, in_features, out_features)) return FOS_ERR_INVALID_ARGUMENT;
+    if (workspace_bytes < fos_linear_train_backward_workspace_bytes(rows, in_features, out_features)) return FOS_ERR_INVALID_ARGUMENT;
     int st = check_device();
     if (st != FOS_OK) return st;
     uint8_t *left = static_cast<uint8_t *>(workspace) + TRAIN_WORDS_BYTES;

@@ -117,7 +117,7 @@ class FourOverSixLinearFunction(torch.autograd.Function):
         dev, (rows, k), n = x.device, x.shape, w.shape[0]
         out = torch.empty(rows, n, dtype=_TORCH_OUT[DataType(config.output_dtype)], device=dev)
         lib = _native.lib()
-        need = lib.fos_linear_train_workspace_bytes(rows, k, n)
+        need = lib.fos_linear_train_forward_workspace_bytes(rows, k, n)
         workspace = torch.empty(need, dtype=torch.uint8, device=dev)
         with _native.on_device(dev):
             _native.check(lib.fos_linear_train_forward(
@@ -138,7 +138,7 @@ class FourOverSixLinearFunction(torch.autograd.Function):
         rounding = _ROUNDING_CODES[cfg.gradient_round_style]
         seeds = [int(torch.randint(0, 2 ** 62, (1,)).item()) for _ in range(2)] if rounding else [0, 0]
         lib = _native.lib()
-        need = lib.fos_linear_train_workspace_bytes(rows, k, n)
+        need = lib.fos_linear_train_backward_workspace_bytes(rows, k, n)
         workspace = torch.empty(need, dtype=torch.uint8, device=dev)
         with _native.on_device(dev):
             _native.check(lib.fos_linear_train_backward(

@@ -271,11 +271,15 @@ int64_t fos_linear_workspace_bytes(int64_t rows, int64_t in_features);
  * stochastically, 2 stochastically with the 16/17 maxima, with the given seeds. Same bits as fos_quantize /
  * fos_quantize_stochastic and fos_gemm_nvfp4_scaled call by call. Base addresses 16-byte aligned, row strides and
  * feature counts multiples of 8, backward also rows a multiple of 16: FOS_ERR_UNSUPPORTED otherwise.
- * `workspace`: fos_linear_train_workspace_bytes(...) bytes of device memory, 256-byte aligned, for either pass.
+ * `workspace`: device memory, 256-byte aligned, of the pass's own fos_linear_train_forward_workspace_bytes(...) or
+ * fos_linear_train_backward_workspace_bytes(...) bytes (the packed operands; one can be far smaller than the other), or of
+ * fos_linear_train_workspace_bytes(...), which do for either.
  *
  * Replaces: FourOverSixLinearFunction.forward / .backward of src/fouroversix/model/modules/linear.py:40-372 in their default
  * configuration, without the bias.
  */
+int64_t fos_linear_train_forward_workspace_bytes(int64_t rows, int64_t in_features, int64_t out_features);
+int64_t fos_linear_train_backward_workspace_bytes(int64_t rows, int64_t in_features, int64_t out_features);
 int64_t fos_linear_train_workspace_bytes(int64_t rows, int64_t in_features, int64_t out_features);
 int fos_linear_train_forward(const void *x, const void *w, int dtype, int64_t rows, int64_t in_features, int64_t out_features,
                              int64_t ld_x, int64_t ld_w, int activation_rule, int weight_rule, int weight_2d, void *out,

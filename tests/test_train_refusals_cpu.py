@@ -8,6 +8,7 @@ import pytest
 import torch
 
 import fouroversix_b200 as fos
+from fouroversix_b200 import _native
 from fouroversix_b200.model.linear import _one_call_training_applies
 
 
@@ -34,3 +35,20 @@ def test_an_output_type_by_its_name_is_one(output):
 def test_operands_it_does_not_take(operand):
     config = fos.ModuleQuantizationConfig(keep_master_weights=True)
     assert not _one_call_training_applies(config, _operand(), operand)
+
+
+def _packed(rows, cols):
+    values = (rows + 127) // 128 * 128 * ((cols + 63) // 64 * 64)
+    return (values // 2 + 255) // 256 * 256 + (values // 16 + 255) // 256 * 256
+
+
+@pytest.mark.parametrize("tokens,k,n", [(16, 16, 16), (4096, 4096, 4096), (32768, 8192, 28672), (272, 520, 1032)])
+def test_a_pass_asks_for_the_room_of_its_own_operands(tokens, k, n):
+    """Forward needs x and W packed and nothing of what backward needs (32768 tokens, 8192 -> 28672: 283 MB of 679)."""
+    lib = _native.lib()
+    forward, backward = (getattr(lib, f"fos_linear_train_{name}_workspace_bytes")(tokens, k, n) for name in ("forward", "backward"))
+    assert forward == 256 + _packed(tokens, k) + _packed(n, k)
+    assert backward == 256 + max(_packed(tokens, n), _packed(n, tokens)) + max(_packed(k, n), _packed(k, tokens))
+    assert lib.fos_linear_train_workspace_bytes(tokens, k, n) == max(forward, backward)
+    for name in ("forward_", "backward_", ""):
+        assert getattr(lib, f"fos_linear_train_{name}workspace_bytes")(tokens, 0, n) == -1

@@ -7,6 +7,7 @@ import torch
 from torch import nn
 
 import fouroversix_b200 as fos
+from fouroversix_b200 import _native
 from fouroversix_b200.model.linear import FourOverSixLinearFunction, _one_call_training_applies
 
 pytestmark = pytest.mark.gpu
@@ -61,3 +62,24 @@ def test_views_and_other_types_keep_their_results(monkeypatch):
     for x, dy in ((base[:20, :64], dense[:20]), (base[:, :64], dense[:1].expand(64, 96))):
         with pytest.raises(ValueError):
             _step(layer, x.detach().requires_grad_(), dy)
+
+
+@pytest.mark.parametrize("tokens,k,n", [(16, 24, 40), (272, 520, 1032), (1024, 512, 64)])
+def test_a_pass_stays_within_its_workspace(tokens, k, n):
+    """Each with exactly the bytes that it asks for, in front of bytes that must stay as they are."""
+    lib, g = _native.lib(), torch.Generator(device="cuda").manual_seed(n)
+    draw = lambda rows, cols: torch.randn(rows, cols, generator=g, device="cuda").bfloat16()
+    x, w, dy = draw(tokens, k), draw(n, k), draw(tokens, n)
+    y, dx, dw = torch.empty_like(dy), torch.empty_like(x), torch.empty_like(w)
+    stream = _native.stream_ptr(x.device)
+    for name in ("forward", "backward"):
+        need = getattr(lib, f"fos_linear_train_{name}_workspace_bytes")(tokens, k, n)
+        work = torch.full((need + 4096,), 0x5A, dtype=torch.uint8, device="cuda")
+        if name == "forward":
+            status = lib.fos_linear_train_forward(x.data_ptr(), w.data_ptr(), _native.FOS_BF16, tokens, k, n, k, k, 3, 3, 1, y.data_ptr(), _native.FOS_BF16, n,
+                                                  work.data_ptr(), need, stream)
+        else:
+            status = lib.fos_linear_train_backward(dy.data_ptr(), x.data_ptr(), w.data_ptr(), _native.FOS_BF16, tokens, k, n, n, k, k, 3, 1, 5, 6, 3, 3, 1,
+                                                   dx.data_ptr(), dw.data_ptr(), _native.FOS_BF16, k, k, work.data_ptr(), need, stream)
+        _native.check(status, name)
+        assert (work[need:] == 0x5A).all(), name
