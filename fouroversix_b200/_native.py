@@ -85,6 +85,7 @@ SIGNATURES = {
                                            ctypes.c_uint64, ctypes.c_uint64, _c_int, _c_int, _c_int, _c_ptr, _c_ptr, _c_int,
                                            _c_i64, _c_i64, _c_ptr, _c_i64, _c_ptr]),
     "fos_experts_glu_is_fused": (_c_int, [_c_i64, _c_i64, _c_i64, _c_int, _c_int]),
+    "fos_experts_forward_workspace_bytes": (_c_i64, [_c_i64, _c_int, _c_int, _c_i64, _c_i64]),
     "fos_experts_workspace_bytes": (_c_i64, [_c_i64, _c_int, _c_int, _c_i64, _c_i64]),
     "fos_experts_forward": (_c_int, [_c_ptr, _c_int, _c_i64, _c_i64, _c_i64, _c_ptr, _c_int, _c_ptr, _c_int, _c_int,
                                      _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_i64, _c_int, _c_int,

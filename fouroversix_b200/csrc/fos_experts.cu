@@ -564,6 +564,7 @@ struct ExpertsWorkspace {
     // byte offsets into the workspace, each a multiple of 256
     int64_t group_start, group_rows, row_token, row_expert, pair_row, pair_expert, route_work, amax, token_max;
     int64_t rows_x, codes_x, sf_x, gate_up, gated, codes_g, sf_g, y, total;
+    int64_t apart;          // the bytes that rows_x, gate_up and y would take beyond these in places of their own
 };
 
 ExpertsWorkspace experts_workspace(int64_t tokens, int top_k, int num_experts, int64_t hidden, int64_t intermediate) {
@@ -581,14 +582,16 @@ ExpertsWorkspace experts_workspace(int64_t tokens, int top_k, int num_experts, i
     w.route_work = take(4 * static_cast<int64_t>(FOS_EXPERTS_ROUTE_WORKSPACE_INTS) * num_experts);
     w.amax = take(4 * 2 * num_experts);
     w.token_max = take(4 * tokens);
-    w.rows_x = take(2 * w.capacity * hidden);
+    // rows_x, gate_up and y share their place: a kernel that writes one of them writes behind its wait for the kernel before it,
+    // which read, or came behind one that read, the last of the one before. (The default path writes y only.)
+    const int64_t rows_bytes = round_up64(2 * w.capacity * hidden, 256), gate_up_bytes = round_up64(4 * w.capacity * intermediate, 256);
+    w.rows_x = w.gate_up = w.y = take(rows_bytes > gate_up_bytes ? rows_bytes : gate_up_bytes);
+    w.apart = rows_bytes + (rows_bytes > gate_up_bytes ? gate_up_bytes : rows_bytes);
     w.codes_x = take(w.capacity * hidden / 2);
     w.sf_x = take(w.capacity * hidden / 16);
-    w.gate_up = take(2 * w.capacity * 2 * intermediate);
     w.gated = take(2 * w.capacity * intermediate);
     w.codes_g = take(w.capacity * intermediate / 2);
     w.sf_g = take(w.capacity * intermediate / 16);
-    w.y = take(2 * w.capacity * hidden);
     w.total = at;
     return w;
 }
@@ -596,9 +599,15 @@ ExpertsWorkspace experts_workspace(int64_t tokens, int top_k, int num_experts, i
 }  // namespace
 }  // namespace fos
 
-extern "C" int64_t fos_experts_workspace_bytes(int64_t tokens, int top_k, int num_experts, int64_t hidden, int64_t intermediate) {
+extern "C" int64_t fos_experts_forward_workspace_bytes(int64_t tokens, int top_k, int num_experts, int64_t hidden, int64_t intermediate) {
     if (tokens <= 0 || top_k <= 0 || num_experts <= 0 || hidden <= 0 || intermediate <= 0) return FOS_ERR_INVALID_ARGUMENT;
     return fos::experts_workspace(tokens, top_k, num_experts, hidden, intermediate).total;
+}
+
+extern "C" int64_t fos_experts_workspace_bytes(int64_t tokens, int top_k, int num_experts, int64_t hidden, int64_t intermediate) {
+    if (tokens <= 0 || top_k <= 0 || num_experts <= 0 || hidden <= 0 || intermediate <= 0) return FOS_ERR_INVALID_ARGUMENT;
+    const fos::ExpertsWorkspace w = fos::experts_workspace(tokens, top_k, num_experts, hidden, intermediate);
+    return w.total + w.apart;
 }
 
 extern "C" int fos_experts_forward(const void *x, int dtype, int64_t tokens, int64_t hidden, int64_t ld_x,

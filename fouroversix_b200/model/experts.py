@@ -173,7 +173,7 @@ class FourOverSixExperts(nn.Module):
             routing_indices = routing_indices.contiguous()
             weights = routing_weights.reshape(-1).contiguous()
             gate_up_bias, down_bias = self.gate_up_proj_bias.contiguous(), self.down_proj_bias.contiguous()
-            need = lib.fos_experts_workspace_bytes(tokens, top_k, self.num_experts, self.hidden_size, self.intermediate_size)
+            need = lib.fos_experts_forward_workspace_bytes(tokens, top_k, self.num_experts, self.hidden_size, self.intermediate_size)
             workspace = torch.empty(need, dtype=torch.uint8, device=dev)
             result = torch.empty(tokens, self.hidden_size, dtype=dtype, device=dev)
             _native.check(lib.fos_experts_forward(

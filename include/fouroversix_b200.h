@@ -385,11 +385,12 @@ int fos_gemm_nvfp4_grouped(const uint8_t *a_codes, const uint8_t *a_sf, const ui
  * expert, as fos_quantize writes them for each expert's matrix) and every element-wise step as described above.
  * x, out, the biases and routing_weights are 16-bit tensors of type `dtype`; hidden and intermediate must be
  * multiples of 64, top_k <= 8, num_experts <= 256 (FOS_ERR_UNSUPPORTED otherwise). workspace: device memory of
- * fos_experts_workspace_bytes(...) bytes, 256-byte aligned, the call's only scratch (the library does not
- * allocate). status as for fos_gemm_nvfp4.
+ * fos_experts_forward_workspace_bytes(...) bytes, 256-byte aligned, the call's only scratch (the library does not
+ * allocate); fos_experts_workspace_bytes(...), which counts every buffer in a place of its own, is more than enough. status as for fos_gemm_nvfp4.
  *
  * Replaces: GptOssExperts.forward of src/fouroversix/model/modules/gpt_oss.py:270-335 after weight packing.
  */
+int64_t fos_experts_forward_workspace_bytes(int64_t tokens, int top_k, int num_experts, int64_t hidden, int64_t intermediate);
 int64_t fos_experts_workspace_bytes(int64_t tokens, int top_k, int num_experts, int64_t hidden, int64_t intermediate);
 /* 1 where the gate-up GEMM of a bf16 layer on `sms` SMs applies the SwiGLU itself, 0 where a kernel of its own does (same bits);
  * rows_capacity = tokens * top_k + 127 * num_experts rounded up to 128. Decides as fos_experts_forward does; needs no GPU. */

@@ -54,6 +54,29 @@ def test_one_call_equals_the_kernels_one_by_one(tokens, top, experts, hidden, in
     assert _native.wait_failure_site() == 0
 
 
+@pytest.mark.parametrize("rule", ["mse", "static_6"])
+@pytest.mark.parametrize("tokens,top,experts,hidden,inter", [SHAPES[1], SHAPES[3], FUSED[2], (300, 2, 4, 512, 64)])
+def test_a_call_stays_within_its_workspace(monkeypatch, tokens, top, experts, hidden, inter, rule):
+    """Two layers one after the other in the same scratch, with bytes behind it that must stay as they are."""
+    layer = _layer(experts, hidden, inter, torch.bfloat16, rule)
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    need = _native.lib().fos_experts_forward_workspace_bytes(tokens, top, experts, hidden, inter)
+    work = torch.full((need + 4096,), 0x5A, dtype=torch.uint8, device="cuda")
+    empty = torch.empty
+    cases = []
+    for _ in range(2):
+        x = torch.randn(tokens, hidden, generator=g, device="cuda").bfloat16()
+        weights, indices = torch.randn(tokens, experts, generator=g, device="cuda").softmax(-1).topk(top)
+        cases.append((x, indices, weights.bfloat16()))
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: work[:need] if a == (need,) else empty(*a, **k))
+    got = [layer(*case) for case in cases]
+    monkeypatch.undo()
+    layer.single_call = False
+    for case, out in zip(cases, got):
+        assert torch.equal(out, layer(*case))
+    assert (work[need:] == 0x5A).all()
+
+
 @pytest.mark.parametrize("tokens,top,experts,hidden,inter", FUSED)
 def test_the_fused_shapes_are(tokens, top, experts, hidden, inter):
     rows = (tokens * top + 127 * experts + 127) // 128 * 128
