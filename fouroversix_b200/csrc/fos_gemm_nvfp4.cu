@@ -76,8 +76,9 @@ constexpr int PAIR_MIN_GROUP_ROWS = 640;
 // With the SwiGLU in the epilogue, which only pairs have, they save the product's way through memory and the kernel that does it
 // otherwise. But the epilogue takes some 9.5 us a tile whatever K is, against 3.5 us for the MMAs of K = 1536 and 6.7 at 2880, and
 // groups of 257 to 384 rows leave half a pair idle: from 640 buffer rows per group where K is at least 1536, from 512 (385 rows
-// of a group's own on average: four row tiles of 128 are two of 256) where it is at least 2048. The whole layer, bf16, random
-// routing, in a graph, us, fused on pairs / not:
+// of a group's own on average: four row tiles of 128 are two of 256) where it is at least 2048, and from 320 where it is at least
+// 2880 and six rounds are sure, which leave the idle halves no more than the kernel saved. The whole layer, bf16, random routing,
+// in a graph, us, fused on pairs / not:
 //   rows of a group's own                          130        200        300        400        500        640       1024
 //   32 experts, 1024 -> 2 x 2880 -> 1024       131/116    157/141    212/184    238/227    280/256    329/295    439/430
 //   32 experts, 1536 -> 2 x 2880 -> 1536       139/125    164/157    259/208    283/256    295/293    345/337    484/502
@@ -86,9 +87,14 @@ constexpr int PAIR_MIN_GROUP_ROWS = 640;
 //   32 experts, 2880 -> 2 x 2880 -> 2880       210/202    230/234    312/307    332/380    383/446    442/497    659/745
 //    8 experts, 2880 -> 2 x 2048 -> 2880         82/79      85/85     104/97     112/114     99/105    118/130    160/170
 //    8 experts, 4096 -> 2 x 2048 -> 4096         79/80      90/85     105/104    112/121    113/123    139/152    183/202
-// (two experts a token with 8, four with 32). Where tokens crowd into few experts it gains more from 640 on and loses more below 385
-// (8 experts of 2048 and 1024, 130 rows: 53 / 42).
-inline int pair_min_glu_rows(int64_t k_p) { return k_p < 1536 ? INT32_MAX : (k_p < 2048 ? 640 : 512); }
+// (two experts a token with 8, four with 32). Where most tokens go to few experts: 32 experts of 2880 and 2880, 256 rows 317 / 350, 300
+// rows 361 / 398; 8 of 2880 and 2048, 200 rows (one to three rounds) 91 / 82; 8 of 2048 and 1024, 130 rows 53 / 42.
+inline int pair_min_glu_rows(int64_t rows_capacity, int num_groups, int64_t n_p, int64_t k_p, int sms) {
+    if (k_p < 1536) return INT32_MAX;
+    if (k_p < 2048) return 640;
+    const int64_t sure_tiles = (rows_capacity - 127 * static_cast<int64_t>(num_groups)) / 256 * ((n_p + 255) / 256);
+    return k_p >= 2880 && sure_tiles >= 6 * (sms / 2) ? 320 : 512;
+}
 // Up to this many rows of a group's own on average, in a buffer with the 127 spare rows per group that unknown routing needs, a
 // grouped GEMM is bound by the weights (see grouped_kernel_for).
 constexpr int FEW_GROUP_ROWS = 64;
@@ -1155,7 +1161,8 @@ extern "C" int fos_experts_glu_is_fused(int64_t rows_capacity, int64_t hidden, i
     if (rows_capacity <= 0 || rows_capacity % 128 || hidden <= 0 || hidden % 64 || intermediate <= 0 || intermediate % 64 ||
         num_experts <= 0 || num_experts > MAX_GROUPS || sms <= 0)
         return FOS_ERR_INVALID_ARGUMENT;
-    return grouped_kernel_for(rows_capacity, num_experts, round_up64(2 * intermediate, 128), 0, 0, sms, pair_min_glu_rows(hidden)) == GEMM_PAIR;
+    const int64_t n_p = round_up64(2 * intermediate, 128);
+    return grouped_kernel_for(rows_capacity, num_experts, n_p, 0, 0, sms, pair_min_glu_rows(rows_capacity, num_experts, n_p, hidden, sms)) == GEMM_PAIR;
 }
 
 static int gemm_fp4_entry(const uint8_t *a_codes, const uint8_t *a_sf, const uint8_t *b_codes,
@@ -1385,7 +1392,7 @@ static int gemm_grouped_entry(const uint8_t *a_codes, const uint8_t *a_sf, const
     p.num_groups = num_groups;
     // how many row blocks are in use is known on the device only: the grid is sized for the buffers, and
     // CTAs that find no tile leave at once
-    const int choice = grouped_kernel_for(rows_capacity, num_groups, n_p, variant, max_ctas, sms, glu ? pair_min_glu_rows(k_p) : PAIR_MIN_GROUP_ROWS);
+    const int choice = grouped_kernel_for(rows_capacity, num_groups, n_p, variant, max_ctas, sms, glu ? pair_min_glu_rows(rows_capacity, num_groups, n_p, k_p, sms) : PAIR_MIN_GROUP_ROWS);
     if (glu) {
         if (choice != GEMM_PAIR) return FOS_ERR_UNSUPPORTED;
         p.glu = *glu;

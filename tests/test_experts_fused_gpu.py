@@ -24,9 +24,9 @@ def _layer(experts, hidden, inter, dtype, rule="mse"):
 # tokens, experts per token, experts, hidden, inter; the last three: groups long enough for CTA pairs
 SHAPES = [(1, 1, 2, 64, 64), (37, 3, 5, 128, 192), (256, 4, 32, 192, 128), (2050, 2, 4, 192, 320), (1777, 3, 6, 64, 448),
           (4096, 4, 16, 320, 512)]
-# with the SwiGLU in the gate-up GEMM: 544 to 1152 buffer rows per group, products that end within a 256-column tile (640, 896, 1408)
-# or on one (1024), K of whole and of broken stages. The last: tiles of 128 columns for few rows per expert
-FUSED = [(2050, 2, 4, 1536, 320), (1777, 3, 6, 1600, 448), (800, 2, 4, 2048, 704), (1030, 3, 5, 2112, 512)]
+# with the SwiGLU in the gate-up GEMM: 327 to 1152 buffer rows per group, products that end within a 256-column tile (640, 896, 1408,
+# 5760) or on one (1024), K of whole and of broken stages. The last: tiles of 128 columns for few rows per expert
+FUSED = [(2050, 2, 4, 1536, 320), (1777, 3, 6, 1600, 448), (800, 2, 4, 2048, 704), (1030, 3, 5, 2112, 512), (1600, 4, 32, 2880, 2880)]
 SHAPES += FUSED + [(190, 2, 8, 128, 1024)]
 
 

@@ -49,13 +49,17 @@ def test_where_the_kernel_for_few_rows_is_taken():
 
 
 def test_where_the_swiglu_is_fused():
-    """From 640 buffer rows per group with K of 1536 and more, from 512 with K of 2048 and more, never with a smaller K: there the
-    epilogue, and below those rows the idle halves of the pairs, cost more than the kernel that they save."""
+    """From 640 buffer rows per group with K of 1536 and more, from 512 with K of 2048 and more, from 320 with K of 2880 and six sure
+    rounds, never with a smaller K: there the epilogue, and below those rows the idle halves of the pairs, cost more than the
+    kernel that they save."""
     fused = lambda rows, hidden, inter, experts: _native.lib().fos_experts_glu_is_fused(rows, hidden, inter, experts, SMS)
     for experts, inter in ((8, 1024), (32, 2880)):
-        for rows, hidden, want in ((256, 2880, 0), (384, 4096, 0), (512, 1984, 0), (512, 2048, 1), (640, 1472, 0), (640, 1536, 1), (2048, 1024, 0)):
+        for rows, hidden, want in ((256, 2880, 0), (384, 2816, 0), (512, 1984, 0), (512, 2048, 1), (640, 1472, 0), (640, 1536, 1), (2048, 1024, 0)):
             assert fused(rows * experts, hidden, inter, experts) == want, (rows, hidden)
         assert fused(640 * experts - 128, 1536, inter, experts) == 0 and fused(512 * experts - 128, 2048, inter, experts) == 0
+    # 32 groups of 320 buffer rows, 23 column tiles: 24 row tiles of their own at least, 552 tiles on 74 pairs
+    assert fused(320 * 32, 2880, 2880, 32) == 1 and fused(320 * 32 - 128, 2880, 2880, 32) == 0
+    assert fused(320 * 32, 2880, 1024, 32) == 0 and fused(384 * 8, 4096, 2048, 8) == 0                # 192 tiles; 128
     assert fused(640, 2048, 64, 1) == 0                      # one narrow tile per row block: not a problem for wide tiles
     assert fused(100, 2048, 64, 1) < 0 and fused(640, 2000, 64, 1) < 0 and fused(640, 2048, 64, 0) < 0
 
