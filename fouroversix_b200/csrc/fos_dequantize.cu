@@ -17,25 +17,28 @@ struct DequantParams {
     int64_t rows_p, cols_p, rows, cols, ld_out;
     int format, sf_tiled;
     float divisor;
-    int run_log2;            // blocks of a row that a run takes, 2^5 .. 2^8
 };
 
 // One thread per 16-value block: 8 bytes of codes and one scale in, 16 values out. A CTA takes
-// runs of blocks of a row (contiguous codes in, contiguous values out; 256 of one row, or of narrow tensors 2^run_log2 of each
-// of 256 >> run_log2 rows, so that a row of 512 values keeps more than 32 threads busy), DEPTH runs at a time: the
+// runs of 2^RUN_LOG2 blocks of a row (contiguous codes in, contiguous values out; 256 of one row, or 32, 64 or 128 of each of 8, 4
+// or 2 rows, so that a row of 512 values keeps more than 32 threads busy), DEPTH runs at a time: the
 // loads of all of them are issued before the first block is decoded, so a thread has DEPTH loads in
 // flight instead of one (with one, the kernel waited a memory latency per run: 29 us for 8192 x 4096).
 constexpr int DEQUANT_DEPTH = 4;
 
 // SMALL: every offset (bytes of codes and scales, elements of the output) fits 32 bits, so the address arithmetic
 // of a block is 32-bit (a third of the kernel's instructions were 64-bit multiplies and compares).
-template <typename OUT, bool SMALL>
-__global__ void __launch_bounds__(256) dequantize_kernel(const DequantParams p) {
+// (RUN_LOG2 is known to the compiler: with a number that is not, the kernel takes 64 registers for whole rows of 256 blocks too, not
+// 48, and a CTA per SM less: 8192 x 4096 16.3 us instead of 15.2. Five CTAs: what 16-bit outputs have without being told.)
+template <typename OUT, bool SMALL, int RUN_LOG2>
+__global__ void __launch_bounds__(256, SMALL && sizeof(OUT) == 4 && RUN_LOG2 == 8 ? 5 : 0) dequantize_kernel(const DequantParams p) {
     using idx_t = typename std::conditional<SMALL, uint32_t, int64_t>::type;
     const int n_cb = static_cast<int>(p.cols_p >> 4);
     const int cb_used = static_cast<int>((p.cols + 15) >> 4);
-    const int chunks = (cb_used + (1 << p.run_log2) - 1) >> p.run_log2, rows_per_unit = 256 >> p.run_log2;
-    const int in_run = static_cast<int>(threadIdx.x) & ((1 << p.run_log2) - 1), in_rows = static_cast<int>(threadIdx.x) >> p.run_log2;
+    constexpr int RUN = 1 << RUN_LOG2, rows_per_unit = 256 >> RUN_LOG2;
+    const int chunks = (cb_used + RUN - 1) >> RUN_LOG2;
+    const int in_run = rows_per_unit == 1 ? static_cast<int>(threadIdx.x) : static_cast<int>(threadIdx.x) & (RUN - 1);
+    const int in_rows = rows_per_unit == 1 ? 0 : static_cast<int>(threadIdx.x) >> RUN_LOG2;
     const idx_t units = static_cast<idx_t>((p.rows + rows_per_unit - 1) / rows_per_unit * chunks);
     const DequantConsts k = dequant_consts(__ldg(p.amax), p.divisor);
     // a unit is (row or rows, run); this CTA's units are blockIdx.x, + gridDim.x, ...: the pair is advanced
@@ -52,9 +55,9 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const DequantParams p) 
 #pragma unroll
         for (int d = 0; d < DEQUANT_DEPTH; ++d) {
             const idx_t r = row0 * static_cast<idx_t>(rows_per_unit) + static_cast<idx_t>(in_rows);
-            const int cb = (ch0 << p.run_log2) + in_run;
+            const int cb = ch0 * RUN + in_run;
             row[d] = r;
-            col_block[d] = (u0 + static_cast<idx_t>(d) * gridDim.x < units && cb < cb_used && r < static_cast<idx_t>(p.rows)) ? cb : -1;
+            col_block[d] = (u0 + static_cast<idx_t>(d) * gridDim.x < units && cb < cb_used && (rows_per_unit == 1 || r < static_cast<idx_t>(p.rows))) ? cb : -1;
             c[d] = make_uint2(0u, 0u);
             sfb[d] = 0u;
             if (col_block[d] >= 0) {
@@ -219,26 +222,35 @@ extern "C" int fos_dequantize(const uint8_t *codes, const uint8_t *sf, const flo
 
     DequantParams p{codes, sf, amax, out, rows_p, cols_p, rows, cols, ld_out, format,
                     sf_layout == FOS_SF_TILED, dequant_divisor(format, scale_rule)};
-    // the shortest run that takes a whole row; rows of more than 256 blocks: runs of 256 (shorter runs that leave fewer threads
-    // idle cost more than they save: 2880 values 7.65 -> 7.86 us in runs of 64, 1536 5.66 -> 5.98 in runs of 32, 4096 rows each)
+    // the shortest run that takes a whole row and leaves every SM a unit; rows of more than 256 blocks: runs of 256 (shorter runs that
+    // leave fewer threads idle cost more than they save: 2880 values 7.65 -> 7.86 us in runs of 64, 1536 5.66 -> 5.98 in runs of 32,
+    // 4096 rows each; fewer units than SMs: 128 x 512 to fp32 2.41 -> 2.91). To fp32 a half-filled run of 256 stores 8 KB, which is
+    // enough up to some thousand rows (2400 x 2048 8.5 us, in runs of 128 8.9; 4096 x 2048 12.8 / 12.5).
     const int64_t cb_used = (cols + 15) / 16;
-    p.run_log2 = 5;
-    while (p.run_log2 < 8 && (int64_t(1) << p.run_log2) < cb_used) ++p.run_log2;
-    const int64_t rows_per_unit = 256 >> p.run_log2, units = (rows + rows_per_unit - 1) / rows_per_unit * ((cb_used + (int64_t(1) << p.run_log2) - 1) >> p.run_log2);
+    int run_log2 = 5;
+    while (run_log2 < 8 && ((int64_t(1) << run_log2) < cb_used || rows < (256 >> run_log2) * int64_t(148))) ++run_log2;
+    if (run_log2 == 7 && out_dtype == FOS_FP32 && rows < 4096) run_log2 = 8;
+    const int64_t rows_per_unit = 256 >> run_log2, units = (rows + rows_per_unit - 1) / rows_per_unit * ((cb_used + (int64_t(1) << run_log2) - 1) >> run_log2);
     int64_t blocks = units;
     if (blocks > 148 * 8) blocks = 148 * 8;
     const unsigned g = static_cast<unsigned>(blocks);
     // 32-bit offsets when the padded tensor has fewer than 2^31 elements and the output fits the same bound
     const bool small = rows_p * cols_p < (int64_t(1) << 31) && rows * ld_out < (int64_t(1) << 31) && units + 4 * blocks < (int64_t(1) << 31);
-    if (small) {
-        if (out_dtype == FOS_BF16) dequantize_kernel<__nv_bfloat16, true><<<g, 256, 0, stream>>>(p);
-        else if (out_dtype == FOS_FP16) dequantize_kernel<__half, true><<<g, 256, 0, stream>>>(p);
-        else dequantize_kernel<float, true><<<g, 256, 0, stream>>>(p);
-    } else {
-        if (out_dtype == FOS_BF16) dequantize_kernel<__nv_bfloat16, false><<<g, 256, 0, stream>>>(p);
-        else if (out_dtype == FOS_FP16) dequantize_kernel<__half, false><<<g, 256, 0, stream>>>(p);
-        else dequantize_kernel<float, false><<<g, 256, 0, stream>>>(p);
-    }
+    auto launch_run = [&](auto out_element, auto run) {
+        using OUT = decltype(out_element);
+        constexpr int RUN_LOG2 = decltype(run)::value;
+        if (small) dequantize_kernel<OUT, true, RUN_LOG2><<<g, 256, 0, stream>>>(p);
+        else dequantize_kernel<OUT, false, RUN_LOG2><<<g, 256, 0, stream>>>(p);
+    };
+    auto launch = [&](auto out_element) {
+        if (run_log2 == 5) launch_run(out_element, std::integral_constant<int, 5>{});
+        else if (run_log2 == 6) launch_run(out_element, std::integral_constant<int, 6>{});
+        else if (run_log2 == 7) launch_run(out_element, std::integral_constant<int, 7>{});
+        else launch_run(out_element, std::integral_constant<int, 8>{});
+    };
+    if (out_dtype == FOS_BF16) launch(__nv_bfloat16{});
+    else if (out_dtype == FOS_FP16) launch(__half{});
+    else launch(0.0f);
     FOS_CUDA_TRY(cudaGetLastError());
     return FOS_OK;
 }
