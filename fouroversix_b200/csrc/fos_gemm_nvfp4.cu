@@ -33,9 +33,9 @@
 //               219 us). (The CTA-pair kernel below does issue them from its MMA warp: two SMs share
 //               that warp's waits, and its barriers are probed a stage ahead.)
 //
-// What bounds the kernel: 218 us at 8192^3 (K 8192, 128 x 256 tiles). Parts switched off in a
-// -DFOS_GEMM_DEBUG build, before the MMA warp probed its barriers a stage ahead: MMAs alone 150 us,
-// loads alone 148, loads + MMAs 176, everything 219. The scale copies are the largest single cost: twelve per stage, each
+// What bounds the kernel: 218 us at 8192^3 (K 8192, 128 x 256 tiles). Parts of it by themselves,
+// before the MMA warp probed its barriers a stage ahead: MMAs alone 150 us, loads alone 148, loads
+// + MMAs 176, everything 219. The scale copies are the largest single cost: twelve per stage, each
 // about 30 ns of the copying warp and about 14 cycles of the tensor pipe that no MMA gets.
 // Loads and MMAs together lose 26 us to the round trip of a stage (four 48 KB stages cannot cover
 // it) and to the shared-memory port both use. The probes gain where few stages are in flight per tile:
@@ -138,7 +138,6 @@ struct GemmParams {
     int64_t m_p, n_p, k_p;   // padded problem (k_p in values)
     int64_t m, n, ldd;       // region of D that is written
     int out_dtype;
-    int debug;               // timing-experiment bits; only read in builds with -DFOS_GEMM_DEBUG (results are wrong with any set)
     int mx;                  // operands are MXFP4: E8M0 scales per 32 values, a 512-byte scale tile spans 128 values of K
     // Row-parallel layers: this rank's partial product is not stored to d but scattered, tile by tile as
     // the tiles complete, into the staging buffers of the ranks that will reduce them. Row block mb (128
@@ -278,13 +277,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     const int64_t k_blocks = p.k_p / 64;                       // MMA K-blocks in the problem
     const int64_t k_tiles = (k_blocks + KB_PER_STAGE - 1) / KB_PER_STAGE;
 
-#ifdef FOS_GEMM_DEBUG
-    const bool dbg_no_sf = p.debug & 1, dbg_no_load = p.debug & 2, dbg_no_store = p.debug & 4;
-    const bool dbg_no_mma = p.debug & 16;
-#else
-    constexpr bool dbg_no_sf = false, dbg_no_load = false, dbg_no_store = false, dbg_no_mma = false;
-#endif
-    if (warp == 0 && !dbg_no_load) {
+    if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer: operands and scales
         // One warp, one elected lane: per stage the two operand tiles and, SF_LEAD stages ahead of them (their
         // way into the MMA is longer: shared memory -> tcgen05.cp -> tensor memory), the two scale copies into
@@ -301,7 +294,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             b_group = static_cast<int>(nb * C::N_GROUPS) + group_of(mb) * static_cast<int>(p.n_p / 128);
         };
         auto issue_next_scales = [&]() {
-            if (f_t >= num_tiles || dbg_no_sf) return;
+            if (f_t >= num_tiles) return;
             // two tensor copies per stage: [K-blocks kb0 .. kb0+3] x [one / N_GROUPS row groups] of 512-byte tiles;
             // what lies beyond K or N is zero-filled and still counted (MXFP4: a tile spans two K-blocks, so the
             // box of its maps is two tiles per group)
@@ -381,9 +374,9 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + acc * BLOCK_N;
             for (int64_t kt = 0; kt < k_tiles; ++kt) {
-                if (!dbg_no_load && !ready) {
+                if (!ready) {
                     ok = mbar_wait(full_bar + 8 * s, ph, abort_flag, p.status, 2);
-                    if (ok && !dbg_no_sf) ok = mbar_wait(sf_ready_bar + 8 * j, jph, abort_flag, p.status, 5);
+                    if (ok) ok = mbar_wait(sf_ready_bar + 8 * j, jph, abort_flag, p.status, 5);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                 }
@@ -400,14 +393,14 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 const uint32_t a_lo = desc_lo(stage, 16), b_lo = desc_lo(stage + A_BYTES, 16);
                 const uint32_t sfa_tmem = tmem_base + SF_COL0 + j * C::SF_STAGE_COLS, sfb_tmem = sfa_tmem + 16;
                 if (p.mx) {
-                    for (int kb = 0; kb < nkb && !dbg_no_mma && issue; ++kb)
+                    for (int kb = 0; kb < nkb && issue; ++kb)
                         tc_mma_mxf4_lo(d_tmem, a_lo + 2 * kb, b_lo + 2 * kb, mma_idesc_mx(idesc, (kb & 1) * 2),
                                        sfa_tmem + 4 * (kb >> 1), sfb_tmem + (BLOCK_N / 32) * (kb >> 1),
                                        (kt > 0 || kb > 0) ? 1u : 0u);
                 } else {
 #pragma unroll
                     for (int kb = 0; kb < KB_PER_STAGE; ++kb) {
-                        if (kb < nkb && !dbg_no_mma && issue)
+                        if (kb < nkb && issue)
                             tc_mma_nvf4_lo(d_tmem, a_lo + 2 * kb, b_lo + 2 * kb, idesc, sfa_tmem + 4 * kb,
                                            sfb_tmem + (BLOCK_N / 32) * kb, (kt > 0 || kb > 0) ? 1u : 0u);
                     }
@@ -538,7 +531,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             if (!ok) break;
             tc_fence_after();
             const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * BLOCK_N + half * COLS;
-            const bool row_ok = row < row_end && !dbg_no_store;
+            const bool row_ok = row < row_end;
             if constexpr (sizeof(OUT) == 2) {
                 // 16-bit outputs: scale, convert and pack while reading, so that the warp's whole
                 // row segment fits in registers and the accumulator goes back to the MMA warp
@@ -566,17 +559,6 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                         for (int i = 0; i < COLS / 2; ++i) pk[i] = add_bias<OUT>(pk[i], bias + 2 * i, left - 2 * i);
                     }
                     if (left >= COLS && vec32_ok) {
-#ifdef FOS_GEMM_DEBUG
-                        if (p.debug & 8) {
-                            // timing experiment (values land in the wrong places): the same bytes stored so that
-                            // every instruction of the warp fills four whole 256-byte row segments
-                            uint8_t *wbase = reinterpret_cast<uint8_t *>(out + (row - lane) * p.ldd + n0);
-#pragma unroll
-                            for (int i = 0; i < COLS / 16; ++i)
-                                if (row - lane + 4 * i + (lane >> 3) < row_end)
-                                    stg_32_stream(wbase + (4 * i + (lane >> 3)) * p.ldd * sizeof(OUT) + (lane & 7) * 32, &pk[8 * i]);
-                        } else
-#endif
                         // 32 bytes per store: every instruction of the warp fills whole 32-byte sectors
 #pragma unroll
                         for (int i = 0; i < COLS / 16; ++i) stg_32_stream(reinterpret_cast<uint8_t *>(dst) + 32 * i, &pk[8 * i]);
@@ -610,7 +592,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 }
             }
         }
-    } else if (warp >= 10 && warp < 10 + SF_CP_WARPS && !dbg_no_load && !dbg_no_sf) {
+    } else if (warp >= 10 && warp < 10 + SF_CP_WARPS) {
         // ------------------------------------------------------------------ scale copies by tcgen05.cp
         const bool issue = elect_one();
         // The warps take the stages in turn, and every (warp, slot) pair has a landing barrier of its own, which
@@ -1126,21 +1108,8 @@ inline int grouped_kernel_for(int64_t rows_capacity, int num_groups, int64_t n_p
     return wide ? GEMM_256 : GEMM_128;
 }
 
-#ifdef FOS_GEMM_DEBUG
-int g_gemm_debug = 0;     // timing experiments of a debug build (fos_gemm_debug_set)
-#endif
-
 }  // namespace
 }  // namespace fos
-
-#ifdef FOS_GEMM_DEBUG
-// Debug builds only (not declared in the public header): bit 0 skips the scale copies, bit 1 the operand
-// loads, bit 2 the output stores, bit 4 the MMAs. The GEMM's result is wrong with any of them set.
-extern "C" int fos_gemm_debug_set(int bits) {
-    fos::g_gemm_debug = bits;
-    return FOS_OK;
-}
-#endif
 
 extern "C" int fos_gemm_fp4_kernel(int64_t m, int64_t n, int64_t k, int num_groups, const fos_gemm_opts *opts, int sms, int *k_split) {
     using namespace fos;
@@ -1198,12 +1167,6 @@ static int gemm_fp4_entry(const uint8_t *a_codes, const uint8_t *a_sf, const uin
     FOS_CUDA_TRY(cudaGetDevice(&dev));
     FOS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const int choice = gemm_kernel_for(m, m_p, n_p, k_p, variant, max_ctas, d_peers != nullptr, sms);
-
-#ifdef FOS_GEMM_DEBUG
-    const int debug_bits = g_gemm_debug;
-#else
-    const int debug_bits = 0;
-#endif
     GemmParams p{};
     p.a_sf = a_sf; p.b_sf = b_sf;
     p.alpha = alpha;
@@ -1215,7 +1178,7 @@ static int gemm_fp4_entry(const uint8_t *a_codes, const uint8_t *a_sf, const uin
     }
     p.d = d; p.status = status;
     p.m_p = m_p; p.n_p = n_p; p.k_p = k_p; p.m = m; p.n = n; p.ldd = ldd;
-    p.out_dtype = out_dtype; p.debug = debug_bits; p.mx = mx;
+    p.out_dtype = out_dtype; p.mx = mx;
     if (d_peers) {
         p.scatter_world = world;
         p.scatter_rank = rank;
