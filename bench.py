@@ -730,8 +730,8 @@ def run_case(args) -> None:
 
 def experts_pipeline(dev, steps: int) -> dict:
     """The grouped experts layer (32 experts of GPT-OSS-20B shape, 4 per token, uniformly random routing) as CUDA-graph
-    replays: routing tables (2 kernels), gather, 2 x (quantize, grouped GEMM), SwiGLU, combine - nine kernels of the
-    library and no read-back."""
+    replays: routing tables (2 kernels), 2 x (quantize, grouped GEMM), combine, and where they are kernels of their own
+    the gather and the SwiGLU - seven to nine kernels of the library and no read-back."""
     from fouroversix_b200.model import FourOverSixExperts
 
     e, h, i, top_k = 32, 2880, 2880, 4

@@ -95,7 +95,8 @@ __device__ __forceinline__ bool expand_block_packed(uint2 c, uint32_t sfb, bool 
 // round, their loads issued before the first is decoded. Both operands are one range of blocks, in which codes and outputs
 // (and row-major scales, IF4's) lie one after the other: no row and column to be found. Tiled scales (an NVFP4 operand beside an
 // IF4 one) need them: by a 32-bit division where the operand's blocks allow, because a 64-bit one costs about as much as
-// decoding the block (IF4 x NVFP4, us, 64-bit / 32-bit: 128 x 8192 x 8192 82.3 / 77.5, 512 x 14336 x 2048 90.3 / 87.4). Launched as the dependent of the kernel that packs an operand, so what it reads is loaded coherently.
+// decoding the block (IF4 x NVFP4, us, 64-bit / 32-bit: 128 x 8192 x 8192 82.3 / 77.5, 512 x 14336 x 2048 90.3 / 87.4). Launched as
+// the dependent of the kernel that packs an operand, so what it reads is loaded coherently.
 constexpr int EXPAND_DEPTH = 4;
 __global__ void __launch_bounds__(256) expand_kernel(const ExpandParams p) {
     asm volatile("griddepcontrol.wait;" ::: "memory");

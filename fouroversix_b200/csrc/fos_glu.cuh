@@ -58,7 +58,7 @@ __device__ __forceinline__ void raise_amax(typename Half16<T>::Pair m2, float *a
 // within (12 + 1.5 |t|) units of 2^-23 for |t| <= 64 (__expf: 2 + 1.173 |t| units in the last place by CUDA's own bound, the
 // addition and __fdividef 3, and the binary32 sequence itself is within 4 of the true value); where both ends of that
 // interval round to the same number, the binary32 sequence does too. The rest - a value within the interval of a
-// rounding boundary (one in 500 in bf16, one in 60 in fp16), a large |t|, NaN - runs the sequence itself.
+// rounding boundary (one in 500 in bf16, one in 60 in fp16), a large |t| - runs the sequence itself; NaN gives NaN either way.
 template <typename T> __device__ __noinline__ uint32_t sigmoid16x2_sequence(float t0, float t1) {
     return Half16<T>::pack(1.0f / (1.0f + expf(-t0)), 1.0f / (1.0f + expf(-t1)));
 }

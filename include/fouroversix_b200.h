@@ -260,6 +260,18 @@ int fos_gemm_mxfp4_unscaled(const uint8_t *a_codes, const uint8_t *a_sf, const u
  * (quantize the input, quantized_matmul), without its bias addition.
  */
 int64_t fos_linear_workspace_bytes(int64_t rows, int64_t in_features);
+int fos_linear_forward(const void *x, int x_dtype, int64_t rows, int64_t in_features, int64_t ld_x, int activation_rule,
+                       const uint8_t *w_codes, const uint8_t *w_sf, const float *w_amax, int weight_rule,
+                       int64_t out_features, void *out, int out_dtype, int64_t ld_out, void *workspace,
+                       int64_t workspace_bytes, const fos_gemm_opts *opts, int32_t *status, void *stream);
+
+/* The same with the layer's bias [out_features] (of the output's type, bf16 / fp16; NULL: none) added to the rounded
+ * product, as a separate 16-bit addition would. FOS_ERR_UNSUPPORTED for a bias with fp32 output. */
+int fos_linear_forward_bias(const void *x, int x_dtype, int64_t rows, int64_t in_features, int64_t ld_x,
+                            int activation_rule, const uint8_t *w_codes, const uint8_t *w_sf, const float *w_amax,
+                            int weight_rule, int64_t out_features, const void *bias, void *out, int out_dtype,
+                            int64_t ld_out, void *workspace, int64_t workspace_bytes, const fos_gemm_opts *opts,
+                            int32_t *status, void *stream);
 
 /*
  * A training step's forward and backward pass with a high-precision weight W [out_features, in_features], each as ONE host
@@ -289,18 +301,6 @@ int fos_linear_train_backward(const void *dy, const void *x, const void *w, int 
                               int gradient_rounding, uint64_t seed_dgrad, uint64_t seed_wgrad, int activation_rule, int weight_rule,
                               int weight_2d, void *dx, void *dw, int out_dtype, int64_t ld_dx, int64_t ld_dw, void *workspace,
                               int64_t workspace_bytes, void *stream);
-int fos_linear_forward(const void *x, int x_dtype, int64_t rows, int64_t in_features, int64_t ld_x, int activation_rule,
-                       const uint8_t *w_codes, const uint8_t *w_sf, const float *w_amax, int weight_rule,
-                       int64_t out_features, void *out, int out_dtype, int64_t ld_out, void *workspace,
-                       int64_t workspace_bytes, const fos_gemm_opts *opts, int32_t *status, void *stream);
-
-/* The same with the layer's bias [out_features] (of the output's type, bf16 / fp16; NULL: none) added to the rounded
- * product, as a separate 16-bit addition would. FOS_ERR_UNSUPPORTED for a bias with fp32 output. */
-int fos_linear_forward_bias(const void *x, int x_dtype, int64_t rows, int64_t in_features, int64_t ld_x,
-                            int activation_rule, const uint8_t *w_codes, const uint8_t *w_sf, const float *w_amax,
-                            int weight_rule, int64_t out_features, const void *bias, void *out, int out_dtype,
-                            int64_t ld_out, void *workspace, int64_t workspace_bytes, const fos_gemm_opts *opts,
-                            int32_t *status, void *stream);
 
 /*
  * Grouped problems in one launch: num_groups GEMMs that share n, k and the output type, each with its own A rows,
